@@ -526,7 +526,7 @@ mtx_status mtx_profiler_region(mtx_profiler_t prof, uint32_t i, char name[64], d
  * workgroup sizes and specialization constants (extractionPipeline.cpp:238-256). */
 typedef struct mtx_tuning {
     uint32_t minmaxZChunk;  /* block slabs per warp in the min/max pass */
-    uint32_t minmaxSlices;  /* 0 (default): a TMA ring of z slices for 2- and 4-byte voxels (else 2);
+    uint32_t minmaxSlices;  /* 0 (default): a TMA ring of z slices for 2- and 4-byte voxels, row words for uint8;
                                1, 2 or 4: the load-based pass with that many z slices in flight */
     uint32_t extractWarps;  /* warps per CTA of the extraction passes: 1, 2, 4 (default) or 8 */
     uint32_t staging;       /* mtx_staging used when the extract options say AUTO */

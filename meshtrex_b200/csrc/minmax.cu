@@ -337,12 +337,24 @@ __global__ void __launch_bounds__(256) minmax_xface_patch_kernel(uint2 *__restri
     }
 }
 
-// Fallback for any block edge and any row alignment: one thread per block.
+// Leaf pass for any block edge and any row alignment (minmax_leaf_rows_warp).
+constexpr int kRowsWarps = 4;
+template <typename T, int W, int NR, bool ALIGNED>
+__global__ void __launch_bounds__(kRowsWarps * 32)
+    minmax_leaf_rows_kernel(const T *__restrict__ vol, uint32_t X, uint32_t Y, uint32_t Z, uint32_t B, uint32_t GX,
+                            uint32_t GY, uint32_t GZ, uint32_t nXS, uint32_t nbs, uint32_t zchunk, uint64_t nwarps,
+                            uint2 *__restrict__ leaf) {
+    __shared__ uint32_t s_col[kRowsWarps][64 * W];
+    const uint64_t w = (uint64_t)blockIdx.x * kRowsWarps + (threadIdx.x >> 5);
+    if (w >= nwarps) return;  // uniform per warp
+    minmax_leaf_rows_warp<T, W, NR, ALIGNED>(vol, X, Y, Z, B, GX, GY, GZ, nXS, nbs, zchunk, w, leaf,
+                                             s_col[threadIdx.x >> 5]);
+}
+
 template <typename T>
-__global__ void __launch_bounds__(128) minmax_leaf_generic_kernel(const T *__restrict__ vol, uint32_t X,
-                                                                  uint32_t Y, uint32_t Z, uint32_t B,
-                                                                  uint32_t GX, uint32_t GY,
-                                                                  uint64_t nblocks, uint2 *__restrict__ leaf) {
+__global__ void __launch_bounds__(128) minmax_leaf_one_kernel(const T *__restrict__ vol, uint32_t X, uint32_t Y,
+                                                              uint32_t Z, uint32_t B, uint32_t GX, uint32_t GY,
+                                                              uint64_t nblocks, uint2 *__restrict__ leaf) {
     const uint64_t b = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (b < nblocks) minmax_leaf_one<T>(vol, X, Y, Z, B, GX, GY, b, leaf);
 }
@@ -454,12 +466,55 @@ static cudaError_t launch_vec(const Problem &p, uint2 *leaf, cudaStream_t s, int
     return cudaGetLastError();
 }
 
-template <typename T>
-static cudaError_t launch_generic(const Problem &p, uint2 *leaf, cudaStream_t s) {
-    uint64_t blocks = (p.nblocks + 127) / 128;
-    minmax_leaf_generic_kernel<T><<<(unsigned)blocks, 128, 0, s>>>((const T *)p.vol, p.X, p.Y, p.Z, p.B, p.GX,
-                                                                   p.GY, p.nblocks, leaf);
+// Slabs a warp of the rows pass takes: enough warps for four waves of them
+// where the runs stay 8 slices long, else for one wave.
+static uint32_t rows_zchunk(const Problem &p, uint64_t cols, int sm_count, uint32_t zover) {
+    if (zover) return zover;
+    auto chunk = [&](uint64_t warps) {
+        const uint64_t nzc = std::min<uint64_t>(p.GZ, std::max<uint64_t>(1, (warps + cols - 1) / cols));
+        return ceil_div(p.GZ, (uint32_t)nzc);
+    };
+    const uint64_t wave = (uint64_t)sm_count * 48;
+    return std::max(chunk(4 * wave), std::min(ceil_div(8, p.B), chunk(wave)));
+}
+
+template <typename T, int W, int NR>
+static cudaError_t launch_rows_nr(const Problem &p, const RowCut &c, uint2 *leaf, cudaStream_t s, int sm_count,
+                                  uint32_t zover) {
+    const uint64_t cols = (uint64_t)c.nXS * p.GY;
+    const uint32_t zchunk = rows_zchunk(p, cols, sm_count, zover);
+    const uint64_t nwarps = cols * ceil_div(p.GZ, zchunk);
+    const unsigned blocks = (unsigned)((nwarps + kRowsWarps - 1) / kRowsWarps);
+    auto k = c.aligned || sizeof(T) == 4 ? minmax_leaf_rows_kernel<T, W, NR, true>
+                                         : minmax_leaf_rows_kernel<T, W, NR, sizeof(T) == 4>;
+    k<<<blocks, kRowsWarps * 32, 0, s>>>((const T *)p.vol, p.X, p.Y, p.Z, p.B, p.GX, p.GY, p.GZ, c.nXS, c.nbs, zchunk,
+                                         nwarps, leaf);
     return cudaGetLastError();
+}
+
+template <typename T, int W>
+static cudaError_t launch_rows_w(const Problem &p, const RowCut &c, uint2 *leaf, cudaStream_t s, int sm_count,
+                                 uint32_t zover) {
+    switch (p.B) {
+    case 3: return launch_rows_nr<T, W, 4>(p, c, leaf, s, sm_count, zover);
+    case 4: return launch_rows_nr<T, W, 5>(p, c, leaf, s, sm_count, zover);
+    case 8: return launch_rows_nr<T, W, 9>(p, c, leaf, s, sm_count, zover);
+    case 16: return launch_rows_nr<T, W, 17>(p, c, leaf, s, sm_count, zover);
+    default: return launch_rows_nr<T, W, 0>(p, c, leaf, s, sm_count, zover);
+    }
+}
+
+template <typename T>
+static cudaError_t launch_rows(const Problem &p, uint2 *leaf, cudaStream_t s, int sm_count, uint32_t zover) {
+    if (!rows_ok(p, sizeof(T))) {
+        const uint64_t blocks = (p.nblocks + 127) / 128;
+        minmax_leaf_one_kernel<T><<<(unsigned)blocks, 128, 0, s>>>((const T *)p.vol, p.X, p.Y, p.Z, p.B, p.GX, p.GY,
+                                                                   p.nblocks, leaf);
+        return cudaGetLastError();
+    }
+    const RowCut c = row_cut(p, sizeof(T));
+    if (sizeof(T) == 1 && !c.wide) return launch_rows_w<T, sizeof(T) == 1 ? 1 : 2>(p, c, leaf, s, sm_count, zover);
+    return launch_rows_w<T, 2>(p, c, leaf, s, sm_count, zover);
 }
 
 template <typename T, int B>
@@ -529,7 +584,10 @@ static cudaError_t dispatch_leaf(const Problem &p, uint2 *leaf, cudaStream_t s, 
                                  uint32_t slices) {
     const bool vec_ok = ((uintptr_t)p.vol % 16 == 0) && (((uint64_t)p.X * sizeof(T)) % 16 == 0) &&
                         (p.B == 4 || p.B == 8 || p.B == 16);
-    if (!vec_ok) return launch_generic<T>(p, leaf, s);
+    // uint8 takes the rows pass for 16-byte rows too: a 512-byte strip of 16
+    // voxels a lane leaves a 256^3 volume half of its lanes and few warps (19.8
+    // against 7.7 us at B = 8)
+    if (!vec_ok || (sizeof(T) == 1 && !slices)) return launch_rows<T>(p, leaf, s, sm, zover);
     switch (slices) {
     case 1: return dispatch_b<T, 1>(p, leaf, s, sm, zover);
     case 4: return dispatch_b<T, 4>(p, leaf, s, sm, zover);

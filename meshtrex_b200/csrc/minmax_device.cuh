@@ -11,6 +11,8 @@
 // so it is loaded once.
 #pragma once
 
+#include <algorithm>
+
 #include "mtx_internal.h"
 
 namespace mtx {
@@ -231,7 +233,287 @@ __device__ __forceinline__ void minmax_leaf_vec_warp(const T *__restrict__ vol, 
     }
 }
 
-// Fallback for any block edge and any row alignment: one thread per block.
+// ------------------------------------------- any block edge, any alignment
+// One aligned 32-bit word of a voxel row as operands of packed three-input
+// min/max.  uint8 takes two: the even bytes alone, and the word as it is, in
+// whose 16-bit halves the odd byte decides every comparison (the even byte
+// below it only breaks ties), so that the winners' high bytes are the odd
+// bytes' min and max.
+template <typename T> struct RowWord;
+template <> struct RowWord<uint8_t> {
+    static constexpr int N = 2, VPW = 4;
+    __device__ __forceinline__ static void split(uint32_t w, uint32_t v[2]) {
+        v[0] = w & 0x00ff00ffu;
+        v[1] = w;
+    }
+    __device__ __forceinline__ static uint32_t join(const uint32_t v[2]) {
+        return (v[0] & 0x00ff00ffu) | (v[1] & 0xff00ff00u);
+    }
+    __device__ __forceinline__ static uint32_t lo(uint32_t a, uint32_t b) { return __vminu2(a, b); }
+    __device__ __forceinline__ static uint32_t hi(uint32_t a, uint32_t b) { return __vmaxu2(a, b); }
+    __device__ __forceinline__ static uint32_t lo3(uint32_t a, uint32_t b, uint32_t c) { return __vimin3_u16x2(a, b, c); }
+    __device__ __forceinline__ static uint32_t hi3(uint32_t a, uint32_t b, uint32_t c) { return __vimax3_u16x2(a, b, c); }
+    __device__ __forceinline__ static uint32_t column(const uint32_t *s, uint32_t c) {
+        return reinterpret_cast<const uint8_t *>(s)[c];
+    }
+};
+template <> struct RowWord<uint16_t> {
+    static constexpr int N = 1, VPW = 2;
+    __device__ __forceinline__ static void split(uint32_t w, uint32_t v[1]) { v[0] = w; }
+    __device__ __forceinline__ static uint32_t join(const uint32_t v[1]) { return v[0]; }
+    __device__ __forceinline__ static uint32_t lo(uint32_t a, uint32_t b) { return __vminu2(a, b); }
+    __device__ __forceinline__ static uint32_t hi(uint32_t a, uint32_t b) { return __vmaxu2(a, b); }
+    __device__ __forceinline__ static uint32_t lo3(uint32_t a, uint32_t b, uint32_t c) { return __vimin3_u16x2(a, b, c); }
+    __device__ __forceinline__ static uint32_t hi3(uint32_t a, uint32_t b, uint32_t c) { return __vimax3_u16x2(a, b, c); }
+    __device__ __forceinline__ static uint32_t column(const uint32_t *s, uint32_t c) {
+        return reinterpret_cast<const uint16_t *>(s)[c];
+    }
+};
+template <> struct RowWord<float> {
+    static constexpr int N = 1, VPW = 1;
+    __device__ __forceinline__ static void split(uint32_t w, uint32_t v[1]) {
+        v[0] = Vox<float>::key(__uint_as_float(w));
+    }
+    __device__ __forceinline__ static uint32_t join(const uint32_t v[1]) { return v[0]; }
+    __device__ __forceinline__ static uint32_t lo(uint32_t a, uint32_t b) { return min(a, b); }
+    __device__ __forceinline__ static uint32_t hi(uint32_t a, uint32_t b) { return max(a, b); }
+    __device__ __forceinline__ static uint32_t lo3(uint32_t a, uint32_t b, uint32_t c) { return __vimin3_u32(a, b, c); }
+    __device__ __forceinline__ static uint32_t hi3(uint32_t a, uint32_t b, uint32_t c) { return __vimax3_u32(a, b, c); }
+    __device__ __forceinline__ static uint32_t column(const uint32_t *s, uint32_t c) { return s[c]; }
+};
+
+// How a volume is cut into strips of whole blocks: nbs blocks a strip, nXS
+// strips of almost equal width.  aligned: every row of every strip starts on a
+// word, so no row has to be shifted.  wide: two words of a row a lane (strips
+// of up to 64 float32, 128 uint16 or 256 uint8 columns), else one.
+struct RowCut {
+    uint32_t nbs, nXS, aligned, wide;
+};
+inline RowCut row_cut(const Problem &p, uint32_t esz) {
+    RowCut c{};
+    // uint8 rows of up to 160 voxels leave most of a 256-column strip's lanes idle
+    c.wide = esz > 1 || p.X > 160;
+    const uint32_t W = c.wide ? 2u : 1u, vpw = 4u / esz;
+    // blocks are word-aligned columns apart when `step` of them are
+    uint32_t step = 1;
+    while ((step * p.B * esz) % 4) ++step;
+    c.aligned = (uintptr_t)p.vol % 4 == 0 && ((uint64_t)p.X * esz) % 4 == 0 && (32 * W * vpw - 1) / p.B >= step;
+    // a strip's columns: its blocks and the next block's first column
+    uint32_t most = std::max(1u, ((c.aligned ? 32 * W : 32 * W - 1) * vpw - 1) / p.B);
+    if (c.aligned) most = most / step * step;
+    c.nXS = ceil_div(p.GX, most);
+    c.nbs = ceil_div(p.GX, c.nXS);
+    if (c.aligned) c.nbs = std::min(most, ceil_div(c.nbs, step) * step);
+    c.nXS = ceil_div(p.GX, c.nbs);
+    return c;
+}
+
+// Whether the byte offsets of a block's rows fit 32 bits; wider rows take
+// minmax_leaf_one.
+inline bool rows_ok(const Problem &p, uint32_t esz) { return (uint64_t)p.X * esz * p.B < (1ull << 32); }
+
+// One warp's share of the leaf pass for any block edge and any row alignment:
+// a strip of nbs whole blocks of one block row over a run of zchunk slabs.
+// Lanes own columns (W words of consecutive voxels each): per z slice the
+// B + 1 rows of the strip are loaded as aligned words, a slice ahead of their
+// use; rows that do not start on a word (ALIGNED false) are shifted into
+// place with the next lane's word.  Rows fold column by column, slices fold
+// into the running slab, and only when a slab is complete -- once every B
+// slices -- do the columns go to shared memory, where each lane takes the
+// B + 1 columns of its blocks.  NR = B + 1 at compile time, 0: at run time,
+// four rows in flight.  s: 64 * W words of the warp's own shared memory.  The
+// B + 1 rows of a strip span less than 4 GiB (rows_ok).
+// Bound by instruction issue (about 2.5 a cycle and SM): every word costs an
+// address, a load, for unaligned rows a shuffle and a shift, and half a
+// min/max pair.  Against one thread a block, whose byte loads read every voxel
+// of a block alone: 1024 x 1024 x 314 uint8 at B = 3, 477 -> 112 us (one word
+// a lane instead of two: 152); 509 x 387 x 301 uint16 at B = 8, 74 -> 39;
+// 250 x 198 x 171 float32 at B = 8, 75 -> 10.
+template <typename T, int W, int NR, bool ALIGNED>
+__device__ __forceinline__ void minmax_leaf_rows_warp(const T *__restrict__ vol, uint32_t X, uint32_t Y, uint32_t Z,
+                                                      uint32_t B_, uint32_t GX, uint32_t GY, uint32_t GZ, uint32_t nXS,
+                                                      uint32_t nbs, uint32_t zchunk, uint64_t w,
+                                                      uint2 *__restrict__ leaf, uint32_t *s) {
+    using RW = RowWord<T>;
+    constexpr int N = RW::N;
+    const uint32_t B = NR ? NR - 1 : B_, lane = threadIdx.x & 31;
+    const uint32_t xs = (uint32_t)(w % nXS);
+    const uint64_t rest = w / nXS;
+    const uint32_t by = (uint32_t)(rest % GY);
+    const uint64_t zc = rest / GY;
+    if (zc * zchunk >= GZ) return;
+    const uint32_t bz0 = (uint32_t)zc * zchunk, bz1 = min(GZ, bz0 + zchunk);
+    const uint32_t xb0 = xs * nbs, x0 = xb0 * B, nb = min(nbs, GX - xb0);
+    const uint32_t ncol = min(X - x0, nb * B + 1);  // columns the strip's blocks cover
+    const uint32_t y0 = by * B, ny = min(B + 1, Y - y0);
+    const uint64_t rowb = (uint64_t)X * sizeof(T), planeb = rowb * Y;
+    const uintptr_t vbeg = reinterpret_cast<uintptr_t>(vol), vend = vbeg + planeb * Z;
+    const uint32_t zend = min(bz1 * B, Z - 1);
+    uint32_t *smn = s, *smx = s + 32 * W;
+
+    uint32_t amn[W][N], amx[W][N];
+#pragma unroll
+    for (int j = 0; j < W; ++j)
+#pragma unroll
+        for (int n = 0; n < N; ++n) {
+            amn[j][n] = ~0u;
+            amx[j][n] = 0u;
+        }
+    uint32_t bz = bz0;
+    // this lane's first word of the strip's first row, and its word's place in the strip
+    uintptr_t slice = vbeg + (uint64_t)bz0 * B * planeb + (uint64_t)y0 * rowb + (uint64_t)x0 * sizeof(T) + 4u * lane;
+    bool on[W];  // words that hold a column of the strip (or the bytes after one)
+#pragma unroll
+    for (int j = 0; j < W; ++j) on[j] = 4u * (32 * j + lane) < ncol * (uint32_t)sizeof(T) + (ALIGNED ? 0u : 3u);
+    // byte offset of row r; a row past the block repeats its last one, which changes no min or max
+    auto row_off = [&](uint32_t r) { return (uint32_t)rowb * min(r, ny - 1); };
+    auto close = [&](uint32_t b) {  // the slab's columns -> its blocks
+#pragma unroll
+        for (int j = 0; j < W; ++j) {
+            smn[32 * j + lane] = RW::join(amn[j]);
+            smx[32 * j + lane] = RW::join(amx[j]);
+        }
+        __syncwarp();
+        for (uint32_t i = lane; i < nb; i += 32) {
+            const uint32_t c1 = min(i * B + B, ncol - 1);
+            uint32_t lo = ~0u, hi = 0u;
+            for (uint32_t c = i * B; c <= c1; ++c) {
+                lo = min(lo, RW::column(smn, c));
+                hi = max(hi, RW::column(smx, c));
+            }
+            if (MTX_BC(((uint64_t)b * GY + by) * GX + xb0 + i, (uint64_t)GX * GY * GZ, kBcLeaf))
+                leaf[((uint64_t)b * GY + by) * GX + xb0 + i] = make_uint2(lo, hi);
+        }
+        __syncwarp();
+    };
+    auto load = [&](uintptr_t at, uint32_t r, uint32_t raw[W]) {
+        const uintptr_t a = at + row_off(r);
+        const uint32_t *src = reinterpret_cast<const uint32_t *>(ALIGNED ? a : a & ~(uintptr_t)3);
+#pragma unroll
+        for (int j = 0; j < W; ++j) raw[j] = on[j] ? __ldg(src + 32 * j) : 0u;
+    };
+    // the same for a row with a word that may reach past the volume: its bytes one by one
+    auto load_edge = [&](uintptr_t at, uint32_t r, uint32_t raw[W]) {
+        const uintptr_t a = (at + row_off(r)) & ~(uintptr_t)3;
+#pragma unroll
+        for (int j = 0; j < W; ++j) {
+            raw[j] = 0;
+            for (uint32_t k = 0; k < 4; ++k) {
+                const uintptr_t q = a + 128 * j + k;
+                if (q >= vbeg && q < vend) raw[j] |= (uint32_t)__ldg(reinterpret_cast<const uint8_t *>(q)) << (8 * k);
+            }
+        }
+    };
+    // a row's columns, this lane's starting sh bits into its word
+    auto place = [&](uintptr_t at, uint32_t r, const uint32_t raw[W], uint32_t v[W][N]) {
+        const uint32_t sh = ALIGNED ? 0u : 8u * (((uint32_t)at + row_off(r)) & 3u);
+#pragma unroll
+        for (int j = 0; j < W; ++j) {
+            uint32_t x = raw[j];
+            if constexpr (!ALIGNED) {
+                const uint32_t give = j + 1 < W && lane == 0 ? raw[j + 1 < W ? j + 1 : j] : raw[j];
+                x = __funnelshift_r(x, __shfl_sync(0xffffffffu, give, (lane + 1) & 31), sh);
+            }
+            RW::split(x, v[j]);
+        }
+    };
+    uint32_t tmn[W][N], tmx[W][N];  // the slice
+    auto fold_pair = [&](bool start, const uint32_t v[W][N], const uint32_t u[W][N]) {
+#pragma unroll
+        for (int j = 0; j < W; ++j)
+#pragma unroll
+            for (int n = 0; n < N; ++n) {
+                tmn[j][n] = start ? RW::lo(v[j][n], u[j][n]) : RW::lo3(tmn[j][n], v[j][n], u[j][n]);
+                tmx[j][n] = start ? RW::hi(v[j][n], u[j][n]) : RW::hi3(tmx[j][n], v[j][n], u[j][n]);
+            }
+    };
+    // only the volume's first and last row have a word that reaches past the volume
+    auto is_edge = [&](uint32_t z) {
+        return !ALIGNED && ((z == 0 && y0 == 0) || (z == Z - 1 && y0 + ny == Y));
+    };
+    constexpr int NA = NR ? NR : 1;
+    uint32_t raw[NA][W];  // NR > 0: the slice's rows, loaded one slice ahead
+    if constexpr (NR > 0) {
+        if (!is_edge(bz0 * B)) {
+#pragma unroll
+            for (int r = 0; r < NR; ++r) load(slice, r, raw[r]);
+        }
+    }
+    for (uint32_t z = bz0 * B; z <= zend; ++z, slice += planeb) {
+        uint32_t v[W][N], u[W][N];
+        const bool edge = is_edge(z);
+        if (edge) {
+            for (uint32_t r = 0; r < ny; ++r) {
+                uint32_t w1[W];
+                load_edge(slice, r, w1);
+                place(slice, r, w1, v);
+                if (r == 0) fold_pair(true, v, v);
+                else fold_pair(false, v, v);
+            }
+        }
+        if constexpr (NR > 0) {
+            uint32_t cur[NA][W];
+#pragma unroll
+            for (int r = 0; r < NR; ++r)
+#pragma unroll
+                for (int j = 0; j < W; ++j) cur[r][j] = raw[r][j];
+            if (z < zend && !is_edge(z + 1)) {
+#pragma unroll
+                for (int r = 0; r < NR; ++r) load(slice + planeb, r, raw[r]);
+            }
+            if (!edge) {
+                constexpr int R0 = (NR & 1) ? 1 : 2;
+                place(slice, 0, cur[0], v);
+                if (R0 == 2) {
+                    place(slice, 1, cur[R0 - 1], u);
+                    fold_pair(true, v, u);
+                } else {
+                    fold_pair(true, v, v);
+                }
+#pragma unroll
+                for (int r = R0; r < NR; r += 2) {
+                    place(slice, r, cur[r], v);
+                    place(slice, r + 1, cur[r + 1], u);
+                    fold_pair(false, v, u);
+                }
+            }
+        } else if (!edge) {
+            for (uint32_t r = 0; r < ny; r += 4) {
+                uint32_t four[4][W];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) load(slice, r + k, four[k]);
+                place(slice, r, four[0], v);
+                place(slice, r + 1, four[1], u);
+                if (r == 0) fold_pair(true, v, u);
+                else fold_pair(false, v, u);
+                place(slice, r + 2, four[2], v);
+                place(slice, r + 3, four[3], u);
+                fold_pair(false, v, u);
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < W; ++j)
+#pragma unroll
+            for (int n = 0; n < N; ++n) {
+                amn[j][n] = RW::lo(amn[j][n], tmn[j][n]);
+                amx[j][n] = RW::hi(amx[j][n], tmx[j][n]);
+            }
+        if (z == bz * B + B) {  // the halo slice of slab bz is the first slice of slab bz + 1
+            close(bz);
+            ++bz;
+#pragma unroll
+            for (int j = 0; j < W; ++j)
+#pragma unroll
+                for (int n = 0; n < N; ++n) {
+                    amn[j][n] = tmn[j][n];
+                    amx[j][n] = tmx[j][n];
+                }
+        }
+    }
+    if (bz < bz1) close(bz);
+}
+
+// One block by one thread: rows too long for the 32-bit offsets above.
 template <typename T>
 __device__ __forceinline__ void minmax_leaf_one(const T *__restrict__ vol, uint32_t X, uint32_t Y, uint32_t Z,
                                                 uint32_t B, uint32_t GX, uint32_t GY, uint64_t b,
