@@ -336,7 +336,7 @@ __device__ __forceinline__ void minmax_leaf_rows_warp(const T *__restrict__ vol,
                                                       uint2 *__restrict__ leaf, uint32_t *s) {
     using RW = RowWord<T>;
     constexpr int N = RW::N;
-    const uint32_t B = NR ? NR - 1 : B_, lane = threadIdx.x & 31;
+    const uint32_t B = NR ? (uint32_t)(NR - 1) : B_, lane = threadIdx.x & 31;
     const uint32_t xs = (uint32_t)(w % nXS);
     const uint64_t rest = w / nXS;
     const uint32_t by = (uint32_t)(rest % GY);
@@ -532,6 +532,102 @@ __device__ __forceinline__ void minmax_leaf_one(const T *__restrict__ vol, uint3
             }
         }
     leaf[b] = make_uint2(mn, mx);
+}
+
+// ------------------------------------------------------------ octree
+// Every octree level in one launch (minMaxOctreeReduce.comp.glsl:23-59 runs
+// one dispatch per level).  A CTA takes 32 x 8 x 8 texels of the launch's first
+// level (the leaf level, or level 1 when the leaf pass wrote it): each thread
+// reads the 2 x 2 x 2 texels of one texel of the next level, all eight loads in
+// flight, and the two levels after that follow by shuffles and one exchange
+// through shared memory.  The CTA that finishes last builds the rest from the
+// third level and zeroes the counter (zero since the context's creation) for
+// the next launch.  Each texel is the min/max of its up-to-8 children; children
+// past their level's extent are skipped (minMaxOctreeReduce.comp.glsl:37-47),
+// which the identity {~0, 0} in their place does.
+// Latency-bound: a tile costs one round of loads, one barrier and one counter.
+// An 8^3 tile a CTA of 512 threads, a barrier pair a level, took 203 us for the
+// 342 x 342 x 105 grid of a 1024 x 1024 x 314 volume at B = 3; this takes 56.
+constexpr int kPyrMaxLevels = 32;
+constexpr uint32_t kPyrThreads = 256, kPyrTileX = 32, kPyrTileYZ = 8;
+struct PyrAll {
+    uint2 *base[kPyrMaxLevels];
+    uint32_t ext[kPyrMaxLevels][3];
+    int levels;
+    uint32_t tiles_x, tiles_y, ntiles;
+    uint32_t *done;
+};
+
+__device__ __forceinline__ uint2 texel_join(uint2 a, uint2 b) { return make_uint2(min(a.x, b.x), max(a.y, b.y)); }
+__device__ __forceinline__ uint2 texel_xor(uint2 a, int o) {
+    return texel_join(a, make_uint2(__shfl_xor_sync(0xffffffffu, a.x, o), __shfl_xor_sync(0xffffffffu, a.y, o)));
+}
+__device__ __forceinline__ void texel_store(const PyrAll &L, int k, uint32_t x, uint32_t y, uint32_t z, uint2 v) {
+    if (k < L.levels && x < L.ext[k][0] && y < L.ext[k][1] && z < L.ext[k][2])
+        L.base[k][((uint64_t)z * L.ext[k][1] + y) * L.ext[k][0] + x] = v;
+}
+
+// One tile of the launch by a CTA of kPyrThreads threads (all of them).
+__device__ __forceinline__ void pyramid_tile(const PyrAll &L, uint32_t tile, uint2 (*s_part)[8], uint32_t *s_last) {
+    const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const uint32_t tx = tile % L.tiles_x, ty = (tile / L.tiles_x) % L.tiles_y, tz = tile / (L.tiles_x * L.tiles_y);
+    {
+        // next level: 16 x 4 x 4 texels a tile, a warp 16 x 2 of them
+        const uint32_t x = tx * 16 + (t & 15), y = ty * 4 + ((t >> 4) & 3), z = tz * 4 + (t >> 6);
+        uint2 v[8];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+            const uint32_t ux = 2 * x + (c & 1), uy = 2 * y + ((c >> 1) & 1), uz = 2 * z + (c >> 2);
+            v[c] = make_uint2(~0u, 0u);
+            if (ux < L.ext[0][0] && uy < L.ext[0][1] && uz < L.ext[0][2])
+                v[c] = L.base[0][((uint64_t)uz * L.ext[0][1] + uy) * L.ext[0][0] + ux];
+        }
+        uint2 r = v[0];
+#pragma unroll
+        for (int c = 1; c < 8; ++c) r = texel_join(r, v[c]);
+        texel_store(L, 1, x, y, z, r);
+        if (L.levels <= 2) return;
+        r = texel_xor(texel_xor(r, 1), 16);  // pairs in x and y
+        if (lane < 16 && !(lane & 1)) s_part[warp][lane >> 1] = r;
+    }
+    __syncthreads();
+    if (warp == 0) {
+        // level 2: 8 x 2 x 2 texels, lane = x | y << 3 | z << 4; warp 2 z + (y of level 1) / 2 holds a pair in y
+        const uint32_t x = lane & 7, y = (lane >> 3) & 1, z = lane >> 4;
+        uint2 r = texel_join(s_part[4 * z + y][x], s_part[4 * z + 2 + y][x]);
+        texel_store(L, 2, tx * 8 + x, ty * 2 + y, tz * 2 + z, r);
+        r = texel_xor(texel_xor(texel_xor(r, 1), 8), 16);
+        if (!(lane & 25)) texel_store(L, 3, tx * 4 + (x >> 1), ty, tz, r);
+        if (L.levels > 4) {  // level 3 of every tile is written: the last CTA to get here builds the rest
+            __threadfence();
+            __syncwarp();
+            if (lane == 0) *s_last = atomicAdd(L.done, 1u) == L.ntiles - 1;
+        }
+    }
+    if (L.levels <= 4) return;
+    __syncthreads();
+    if (!*s_last) return;
+    __threadfence();
+    for (int k = 4; k < L.levels; ++k) {
+        const uint32_t ex = L.ext[k][0], ey = L.ext[k][1], ez = L.ext[k][2];
+        const uint32_t px = L.ext[k - 1][0], py = L.ext[k - 1][1], pz = L.ext[k - 1][2];
+        const uint64_t cnt = (uint64_t)ex * ey * ez;
+#pragma unroll 2
+        for (uint64_t i = t; i < cnt; i += kPyrThreads) {
+            const uint32_t x = (uint32_t)(i % ex), y = (uint32_t)((i / ex) % ey), z = (uint32_t)(i / ((uint64_t)ex * ey));
+            uint2 r = make_uint2(~0u, 0u);
+#pragma unroll
+            for (int c = 0; c < 8; ++c) {
+                const uint32_t ux = 2 * x + (c & 1), uy = 2 * y + ((c >> 1) & 1), uz = 2 * z + (c >> 2);
+                if (ux < px && uy < py && uz < pz)
+                    r = texel_join(r, __ldcg(&L.base[k - 1][((uint64_t)uz * py + uy) * px + ux]));
+            }
+            L.base[k][i] = r;
+        }
+        __threadfence();
+        __syncthreads();
+    }
+    if (t == 0) *L.done = 0;
 }
 
 }  // namespace mtx

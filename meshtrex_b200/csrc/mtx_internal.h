@@ -128,7 +128,11 @@ struct Problem {
 mtx_status launch_minmax_leaf(mtx_context *c, const Problem &p, uint2 *leaf, cudaStream_t s,
                               uint32_t zchunk_override = 0, uint2 *l1 = nullptr, const uint32_t *l1ext = nullptr,
                               bool *l1_done = nullptr);
-// Octree levels start+1.. from level start (already in all_levels at offset[start]).
+// Octree levels start+1.. from level start (already in all_levels at offset[start]):
+// the launch's view of them (PyrAll, ntiles 0 when there is no level above), or the launch itself.
+struct PyrAll;
+mtx_status pyramid_levels(mtx_context *c, uint2 *all_levels, int levels, const uint32_t ext[][3],
+                          const uint64_t *offset, int start, PyrAll *out);
 mtx_status launch_pyramid(mtx_context *c, uint2 *all_levels, int levels, const uint32_t ext[][3],
                           const uint64_t *offset, cudaStream_t s, int start = 0);
 
