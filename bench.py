@@ -286,19 +286,14 @@ def run_reference(args):
 # --------------------------------------------------------------- GPU side
 def launches_per_extraction(grid, shape_zyx=None, esz=2, block=BLOCK):
     """Kernel launches of one plain extraction: leaf min/max (with the strip-column
-    patch when the TMA leaf pass covers more than one 512-byte x-strip), octree,
-    filter, count + scan, emit."""
-    m = max(grid)
-    levels = 1
-    while m > 1:
-        m >>= 1
-        levels += 1
+    patch when the TMA leaf pass covers more than one 512-byte x-strip), filter
+    with octree, count + scan, emit."""
     patch = 0
     if shape_zyx is not None:
         X = shape_zyx[2]
         tma_leaf = esz >= 2 and (X * esz) % 16 == 0 and block in (4, 8, 16)
         patch = 1 if tma_leaf and X * esz > 512 else 0
-    return 1 + patch + (1 if levels > 1 else 0) + 1 + 2 + 1
+    return 1 + patch + 1 + 2 + 1
 
 
 def read_traffic():

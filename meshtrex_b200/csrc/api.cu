@@ -12,7 +12,7 @@
 #include <unordered_map>
 #include <vector>
 
-#include "mtx_internal.h"
+#include "minmax_device.cuh"
 
 using namespace mtx;
 
@@ -750,7 +750,7 @@ mtx_status mtx_filter_active_blocks(mtx_context_t c, const mtx_minmax_output *mm
     }
     prof_begin(prof, "Active_Block_Filtering", c->stream);
     r = launch_filter(c, p, (const uint2 *)mm->minMaxImage.ptr, (uint32_t *)ids, (uint32_t *)rank, (uint32_t *)cnt,
-                      nullptr, c->stream);
+                      c->stream);
     prof_end(prof, c->stream);
     if (r != MTX_OK) {
         dev_free(c, ids);
@@ -860,7 +860,6 @@ mtx_status mtx_extract_meshlet_descriptors(mtx_context_t c, const mtx_minmax_out
     a.block_capacity = n;
     a.faces = (uint32_t *)c->faces.ptr;
     a.state = sb ? (uint8_t *)c->state.ptr : nullptr;
-    a.count_status = (uint64_t *)c->count_status.ptr;
     a.totals = (uint32_t *)counters;
     a.cell_cases = o.cellCases;
     a.vertex_format = o.vertexFormat;
@@ -960,17 +959,21 @@ mtx_status mtx_extract_plain_async(mtx_context_t c, const mtx_volume *vol, const
                            &l1_done);
     prof_end(P, s);
     if (r != MTX_OK) return r;
-    if (L > 1) {
+    // the octree goes with the filter, unless a profiler wants its own time
+    PyrAll octree{};
+    if (P && L > 1) {
         prof_begin(P, "MinMax_Octree_Reduction", s);
         r = launch_pyramid(c, (uint2 *)c->leaf.ptr, L, ext, off, s, l1_done ? 1 : 0);
         prof_end(P, s);
-        if (r != MTX_OK) return r;
+    } else if (L > 1) {
+        r = pyramid_levels(c, (uint2 *)c->leaf.ptr, L, ext, off, l1_done ? 1 : 0, &octree);
     }
+    if (r != MTX_OK) return r;
     // the filter overwrites the ids, ranks and count a previous call's extraction may still read
     if ((r = join_extract(c)) != MTX_OK) return r;
     prof_begin(P, "Active_Block_Filtering", s);
     r = launch_filter(c, p, (const uint2 *)c->leaf.ptr, (uint32_t *)c->ids.ptr, (uint32_t *)c->rank.ptr,
-                      &c->ctrl->active_count, nullptr, s);
+                      &c->ctrl->active_count, s, &octree);
     prof_end(P, s);
     if (r != MTX_OK) return r;
     cudaStream_t es = s;  // the extraction passes' stream
@@ -990,8 +993,8 @@ mtx_status mtx_extract_plain_async(mtx_context_t c, const mtx_volume *vol, const
     a.block_capacity = maxa;
     a.faces = (uint32_t *)c->faces.ptr;
     a.state = sb ? (uint8_t *)c->state.ptr : nullptr;
-    a.count_status = (uint64_t *)c->count_status.ptr;
     a.totals = out->counters;
+    a.status_out = out->counters + 4;
     a.cell_cases = o.cellCases;
     a.vertices = out->vertices;
     a.vertex_capacity = out->vertexCapacity;
@@ -1015,7 +1018,6 @@ mtx_status mtx_extract_plain_async(mtx_context_t c, const mtx_volume *vol, const
         MTX_CUDA(c, cudaMemcpyAsync(out->meshlets, desc, out->meshletCapacity * sizeof(mtx_meshlet_descriptor),
                                     cudaMemcpyDeviceToDevice, es));
     }
-    MTX_CUDA(c, cudaMemcpyAsync(out->counters + 4, &c->ctrl->status.code, 4, cudaMemcpyDeviceToDevice, es));
     if (c->has_xstream) {
         MTX_CUDA(c, cudaEventRecord(c->ev_extracted, es));
         c->extract_pending = true;

@@ -35,8 +35,10 @@ __global__ void __launch_bounds__(kMaxWarps * 32, BC ? 0 : 4)
     pmb_count_kernel(Problem p_, const __grid_constant__ CUtensorMap map, const uint32_t *__restrict__ ids,
                      const uint32_t *__restrict__ count_ptr, mtx_meshlet_descriptor *__restrict__ desc,
                      uint64_t desc_cap, uint32_t *__restrict__ faces, uint8_t *__restrict__ state,
-                     uint32_t *totals, uint8_t *__restrict__ cell_cases, uint64_t block_cap, DevStatus *st) {
+                     uint32_t *totals, uint8_t *__restrict__ cell_cases, uint64_t block_cap, DevStatus *st,
+                     uint64_t *scan_status, uint32_t scan_tiles, uint32_t *scan_ticket) {
     extern __shared__ __align__(128) unsigned char smem[];
+    scan_reset(scan_status, scan_tiles, scan_ticket, totals);
     Problem p = p_;
     if (BC) p.B = BC;
     const WPlan pl = make_wplan(p.B, sizeof(T), TMA, false, kSingleBuffer, p.B <= 8);
@@ -98,11 +100,12 @@ __global__ void __launch_bounds__(kMaxWarps * 32, BC ? 0 : 4)
 // -------------------------------------------------------------- scan pass
 __global__ void __launch_bounds__(kScanThreads)
     pmb_scan_kernel(mtx_meshlet_descriptor *__restrict__ desc, const uint32_t *__restrict__ count_ptr,
-                    uint64_t *tile_status, uint32_t *ticket, uint32_t *totals, DevStatus *st, uint32_t spin_limit) {
+                    uint64_t *tile_status, uint32_t *ticket, uint32_t *totals, DevStatus *st, uint32_t spin_limit,
+                    uint32_t skip) {
     __shared__ uint32_t s_tile, s_ok;
     __shared__ uint64_t s_tmp[kScanThreads / 32 + 1];
     __shared__ uint64_t s_pre[2];
-    if (threadIdx.x == 0) s_tile = atomicAdd(ticket, 1u);
+    if (threadIdx.x == 0) s_tile = atomicAdd(ticket, 1u) + skip;
     __syncthreads();
     const uint32_t t = s_tile;
     const uint32_t count = *count_ptr;
@@ -124,7 +127,7 @@ __global__ void __launch_bounds__(kMaxWarps * 32, (!GENERIC && CPL == 8) ? 3 : 1
                     const mtx_meshlet_descriptor *__restrict__ desc, const uint32_t *__restrict__ faces,
                     const uint8_t *__restrict__ state, uint32_t *__restrict__ indices, uint64_t tcap,
                     uint64_t block_cap, void *__restrict__ vertices, uint64_t vcap, uint32_t vfmt, uint32_t frame,
-                    uint32_t normals, DevStatus *st) {
+                    uint32_t normals, DevStatus *st, uint32_t *done, uint32_t *status_out) {
     // B <= 8 with TMA: the count pass's block state comes with each tile
     constexpr bool STATE = TMA && CPL == 8;
     extern __shared__ __align__(128) unsigned char smem[];
@@ -152,8 +155,8 @@ __global__ void __launch_bounds__(kMaxWarps * 32, (!GENERIC && CPL == 8) ? 3 : 1
         fence_mbar_init();
     }
     __syncthreads();
-    const uint32_t count = *count_ptr;
-    if (count > block_cap) return;  // reported by the count pass
+    uint32_t count = *count_ptr;
+    if (count > block_cap) count = 0;  // reported by the count pass
     const uint32_t gw = blockIdx.x * W + warp, nw = gridDim.x * W;
     uint32_t parity = 0, buf = 0;
 
@@ -204,6 +207,19 @@ __global__ void __launch_bounds__(kMaxWarps * 32, (!GENERIC && CPL == 8) ? 3 : 1
         g = gn;
         nb_rk = nb_rk_n;
     }
+    // the CTA that ends last hands out the error code the call's kernels left
+    // (a copy after the kernel cost 1.5 us and its gap)
+    if (status_out) {
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            __threadfence();
+            if (atomicAdd(done, 1u) == gridDim.x - 1) {
+                __threadfence();
+                *done = 0;
+                *status_out = ld_volatile(&st->code);
+            }
+        }
+    }
 }
 
 // ------------------------------------------------------------------ host
@@ -243,7 +259,8 @@ static mtx_status run_count(mtx_context *c, const Problem &p, const ExtractArgs 
     mtx_status r = grid_for(c, k, W * 32, smem, a.host_count, W, grid);
     if (r != MTX_OK) return r;
     k<<<grid, W * 32, smem, s>>>(p, map, a.ids, a.count, a.desc, a.desc_capacity, a.faces, a.state, a.totals,
-                                 a.cell_cases, a.block_capacity, &c->ctrl->status);
+                                 a.cell_cases, a.block_capacity, &c->ctrl->status, (uint64_t *)c->count_status.ptr,
+                                 scan_tiles(std::min(a.block_capacity, a.desc_capacity)), &c->ctrl->count_ticket);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(c, e, "count launch");
     return MTX_OK;
@@ -252,7 +269,8 @@ static mtx_status run_count(mtx_context *c, const Problem &p, const ExtractArgs 
 template <typename T, int CPL, bool TMA, int BC = 0>
 static void (*emit_fn(bool generic))(Problem, CUtensorMap, const uint32_t *, const uint32_t *, const uint32_t *,
                                      const mtx_meshlet_descriptor *, const uint32_t *, const uint8_t *, uint32_t *,
-                                     uint64_t, uint64_t, void *, uint64_t, uint32_t, uint32_t, uint32_t, DevStatus *) {
+                                     uint64_t, uint64_t, void *, uint64_t, uint32_t, uint32_t, uint32_t, DevStatus *,
+                                     uint32_t *, uint32_t *) {
     return generic ? pmb_emit_kernel<T, CPL, TMA, true, BC> : pmb_emit_kernel<T, CPL, TMA, false, BC>;
 }
 
@@ -270,7 +288,7 @@ static mtx_status run_emit(mtx_context *c, const Problem &p, const ExtractArgs &
     if (r != MTX_OK) return r;
     k<<<grid, W * 32, smem, s>>>(p, map, a.ids, a.rank_map, a.count, a.desc, a.faces, a.state, a.indices,
                                  a.tri_capacity, a.block_capacity, a.vertices, a.vertex_capacity, a.vertex_format,
-                                 a.frame, a.normals, &c->ctrl->status);
+                                 a.frame, a.normals, &c->ctrl->status, &c->ctrl->emit_done, a.status_out);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(c, e, "emit launch");
     return MTX_OK;
@@ -308,44 +326,41 @@ static mtx_status launch_stage(mtx_context *c, const Problem &p, const ExtractAr
 
 uint32_t block_state_bytes(uint32_t B) { return make_wplan(B, 2, true, false, kSingleBuffer, B <= 8).state_bytes; }
 
-// Counts, faces and the scan: after this the descriptors and totals are final.
-mtx_status launch_count(mtx_context *c, const Problem &p, const ExtractArgs &a, cudaStream_t s) {
-    const uint64_t cap = std::min<uint64_t>(a.block_capacity, a.desc_capacity);
-    const uint32_t ntiles = (uint32_t)std::max<uint64_t>(1, (cap + kScanTile - 1) / kScanTile);
-    mtx_status r = scratch_reserve(c, c->count_status, sizeof(uint64_t) * (size_t)ntiles);
-    if (r != MTX_OK) return r;
-    MTX_CUDA(c, cudaMemsetAsync(&c->ctrl->count_ticket, 0, sizeof(uint32_t), s));
-    MTX_CUDA(c, cudaMemsetAsync(a.totals, 0, 4 * sizeof(uint32_t), s));
-    MTX_CUDA(c, cudaMemsetAsync(c->count_status.ptr, 0, sizeof(uint64_t) * ntiles, s));
-    if ((r = launch_stage<false>(c, p, a, s)) != MTX_OK) return r;
-    if (c->withhold & 2u) {  // failure injection: scan tile 0 is never handed out
-        static const uint32_t kOne = 1;
-        MTX_CUDA(c, cudaMemcpyAsync(&c->ctrl->count_ticket, &kOne, sizeof(uint32_t), cudaMemcpyHostToDevice, s));
-    }
-    pmb_scan_kernel<<<ntiles, kScanThreads, 0, s>>>(a.desc, a.count, (uint64_t *)c->count_status.ptr,
-                                                    &c->ctrl->count_ticket, a.totals, &c->ctrl->status,
-                                                    c->wait_polls ? c->wait_polls : kSpinLimit);
+// The scan over up to `capacity` descriptors, behind a kernel that ran scan_reset for it.
+static mtx_status run_scan(mtx_context *c, mtx_meshlet_descriptor *desc, const uint32_t *count, uint64_t capacity,
+                           uint32_t *totals, uint32_t skip, cudaStream_t s) {
+    pmb_scan_kernel<<<scan_tiles(capacity), kScanThreads, 0, s>>>(desc, count, (uint64_t *)c->count_status.ptr,
+                                                                  &c->ctrl->count_ticket, totals, &c->ctrl->status,
+                                                                  c->wait_polls ? c->wait_polls : kSpinLimit, skip);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(c, e, "scan launch");
     return MTX_OK;
 }
 
+// Counts, faces and the scan: after this the descriptors and totals are final.
+mtx_status launch_count(mtx_context *c, const Problem &p, const ExtractArgs &a, cudaStream_t s) {
+    const uint64_t cap = std::min<uint64_t>(a.block_capacity, a.desc_capacity);
+    mtx_status r = scratch_reserve(c, c->count_status, sizeof(uint64_t) * (size_t)scan_tiles(cap));
+    if (r != MTX_OK) return r;
+    if ((r = launch_stage<false>(c, p, a, s)) != MTX_OK) return r;
+    return run_scan(c, a.desc, a.count, cap, a.totals, (c->withhold >> 1) & 1u, s);
+}
+
 // The descriptor scan on its own: vertexOffset / indexOffset of count
 // descriptors from their vertexCount / primitiveCount (totals as launch_count).
+// The kernel that fills the counts runs scan_reset with the words of desc_scan_words.
+mtx_status desc_scan_words(mtx_context *c, uint64_t capacity, uint64_t **words, uint32_t *tiles, uint32_t **ticket) {
+    mtx_status r = scratch_reserve(c, c->count_status, sizeof(uint64_t) * (size_t)scan_tiles(capacity));
+    if (r != MTX_OK) return r;
+    *words = (uint64_t *)c->count_status.ptr;
+    *tiles = scan_tiles(capacity);
+    *ticket = &c->ctrl->count_ticket;
+    return MTX_OK;
+}
+
 mtx_status launch_desc_scan(mtx_context *c, mtx_meshlet_descriptor *desc, const uint32_t *count, uint64_t capacity,
                             uint32_t *totals, cudaStream_t s) {
-    const uint32_t ntiles = (uint32_t)std::max<uint64_t>(1, (capacity + kScanTile - 1) / kScanTile);
-    mtx_status r = scratch_reserve(c, c->count_status, sizeof(uint64_t) * (size_t)ntiles);
-    if (r != MTX_OK) return r;
-    MTX_CUDA(c, cudaMemsetAsync(&c->ctrl->count_ticket, 0, sizeof(uint32_t), s));
-    MTX_CUDA(c, cudaMemsetAsync(totals, 0, 4 * sizeof(uint32_t), s));
-    MTX_CUDA(c, cudaMemsetAsync(c->count_status.ptr, 0, sizeof(uint64_t) * ntiles, s));
-    pmb_scan_kernel<<<ntiles, kScanThreads, 0, s>>>(desc, count, (uint64_t *)c->count_status.ptr,
-                                                    &c->ctrl->count_ticket, totals, &c->ctrl->status,
-                                                    c->wait_polls ? c->wait_polls : kSpinLimit);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return cuda_fail(c, e, "scan launch");
-    return MTX_OK;
+    return run_scan(c, desc, count, capacity, totals, 0, s);
 }
 
 // Vertices (when a.vertices is set) and triangles.

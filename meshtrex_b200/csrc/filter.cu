@@ -7,15 +7,14 @@
 // each CTA takes a tile of consecutive block ids by ticket (4096 a tile, 16
 // per thread, so that a 1024^3 volume at block 8 is one wave of CTAs; 1024 in
 // the no-allocation entry point, whose scratch is sized for them), counts its
-// active blocks (warp scan + CTA scan), and resolves its global offset with a
+// active blocks (two ballots a round of 64 blocks), and resolves its global offset with a
 // single-pass decoupled look-back over the tiles before it: the list comes out
 // in ascending block order, which is the order the CPU rule produces.  It
 // also writes the rank of every block (0xffffffff for inactive ones), which
 // the extraction uses to find a neighbouring block's vertices.
-#include <cstddef>
 #include <mutex>
 
-#include "mtx_internal.h"
+#include "minmax_device.cuh"
 
 namespace mtx {
 
@@ -25,67 +24,112 @@ constexpr int kNoallocItems = 4;       // tiles of 1024 in mtx_filter_active_blo
 constexpr int kFilterTile = kFilterThreads * kFilterItems;
 constexpr int kNoallocTile = kFilterThreads * kNoallocItems;
 
-// tile status word: [31:30] flag (0 empty, 1 aggregate, 2 inclusive, 3 aborted), [29:0] count
+// Look-back words and tickets of one launch.  EPOCH (the context's own
+// scratch): a status word is flag << 62 | epoch << 32 | count and the ticket
+// word epoch << 32 | ticket; the CTA that draws a launch's last ticket starts
+// the next epoch, so that the words of earlier launches read as empty and
+// nothing has to be zeroed between launches (three memsets of about 4 us
+// each on the timeline before; the words are zeroed once, when the scratch
+// grows).  Otherwise (the no-allocation entry point, whose array holds 32-bit
+// words): flag << 30 | count, zeroed before the launch.
+// flag: 0 empty, 1 aggregate, 2 inclusive, 3 aborted.
 constexpr uint32_t kFlagAgg = 1u, kFlagInc = 2u, kFlagAbort = 3u;
+template <bool EPOCH> struct TileWord;
+template <> struct TileWord<false> {
+    using U = uint32_t;
+    __device__ __forceinline__ static U make(uint32_t flag, uint32_t, uint32_t count) { return (flag << 30) | count; }
+    __device__ __forceinline__ static uint32_t flag(U w, uint32_t) { return w >> 30; }
+    __device__ __forceinline__ static uint32_t count(U w) { return w & 0x3fffffffu; }
+    __device__ __forceinline__ static uint32_t draw(U *ticket, uint32_t, uint32_t &epoch) {
+        epoch = 0;
+        return atomicAdd(ticket, 1u);
+    }
+};
+template <> struct TileWord<true> {
+    using U = uint64_t;
+    __device__ __forceinline__ static U make(uint32_t flag, uint32_t epoch, uint32_t count) {
+        return ((U)flag << 62) | ((U)epoch << 32) | count;
+    }
+    __device__ __forceinline__ static uint32_t flag(U w, uint32_t epoch) {
+        return ((uint32_t)(w >> 32) & 0x3fffffffu) == epoch ? (uint32_t)(w >> 62) : 0u;
+    }
+    __device__ __forceinline__ static uint32_t count(U w) { return (uint32_t)w; }
+    __device__ __forceinline__ static uint32_t draw(U *ticket, uint32_t ntiles, uint32_t &epoch) {
+        const U t = atomicAdd(reinterpret_cast<unsigned long long *>(ticket), 1ull);
+        epoch = (uint32_t)(t >> 32);
+        if ((uint32_t)t == ntiles - 1) st_volatile(ticket, (U)((epoch + 1) & 0x3fffffffu) << 32);
+        return (uint32_t)t;
+    }
+};
 
-template <int ITEMS>
-__global__ void __launch_bounds__(kFilterThreads)
-    filter_compact_kernel(const uint2 *__restrict__ leaf, uint64_t nblocks, uint32_t ntiles, uint32_t dtype,
-                          float iso, uint32_t *__restrict__ ids, uint32_t *__restrict__ rank_map,
-                          uint32_t *__restrict__ count_out, uint64_t *__restrict__ count_status,
-                          uint32_t *tile_status, uint32_t *ticket, DevStatus *st, uint32_t spin_limit) {
-    __shared__ uint32_t s_tile, s_prefix, s_abort;
-    __shared__ uint32_t s_tmp[kFilterThreads / 32 + 1];
+// A CTA's tile is ITEMS / 2 rounds of 64 consecutive blocks a warp, lane l
+// taking blocks 2 l and 2 l + 1 of each round: the loads and the rank stores
+// are coalesced and the ranks follow from two ballots a round.  skip: failure
+// injection, the tickets start at tile `skip`.
+template <int ITEMS, bool EPOCH>
+__device__ __forceinline__ void filter_tile(const uint2 *__restrict__ leaf, uint64_t nblocks, uint32_t ntiles,
+                                            uint32_t dtype, float iso, uint32_t *__restrict__ ids,
+                                            uint32_t *__restrict__ rank_map, uint32_t *__restrict__ count_out,
+                                            typename TileWord<EPOCH>::U *tile_status,
+                                            typename TileWord<EPOCH>::U *ticket, DevStatus *st, uint32_t spin_limit,
+                                            uint32_t skip) {
+    using TW = TileWord<EPOCH>;
+    constexpr int R = ITEMS / 2;
+    __shared__ uint32_t s_tile, s_epoch, s_prefix, s_abort;
+    __shared__ uint32_t s_tmp[kFilterThreads / 32];
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (threadIdx.x == 0) {
-        s_tile = atomicAdd(ticket, 1u);
-        s_abort = 0;
+        uint32_t epoch;
+        s_tile = TW::draw(ticket, ntiles, epoch) + skip;
+        s_epoch = epoch;
     }
     __syncthreads();
-    const uint32_t t = s_tile;
+    const uint32_t t = s_tile, epoch = s_epoch;
     if (t >= ntiles) return;
 
-    const uint64_t base = (uint64_t)t * (kFilterThreads * ITEMS) + (uint64_t)threadIdx.x * ITEMS;
-    uint32_t f[ITEMS];
-    if (base + ITEMS <= nblocks) {
-        const uint4 *p = reinterpret_cast<const uint4 *>(leaf + base);
-        uint4 v[ITEMS / 2];
+    const uint64_t base = (uint64_t)t * (kFilterThreads * ITEMS) + (uint64_t)warp * (32 * ITEMS) + 2 * lane;
+    uint4 v[R];
 #pragma unroll
-        for (int i = 0; i < ITEMS / 2; ++i) v[i] = __ldg(p + i);  // all loads before any use
-#pragma unroll
-        for (int i = 0; i < ITEMS / 2; ++i) {
-            f[2 * i] = block_active(dtype, v[i].x, v[i].y, iso);
-            f[2 * i + 1] = block_active(dtype, v[i].z, v[i].w, iso);
-        }
-    } else {
-#pragma unroll
-        for (int i = 0; i < ITEMS; ++i) {
-            f[i] = 0;
-            if (base + i < nblocks) {
-                uint2 v = leaf[base + i];
-                f[i] = block_active(dtype, v.x, v.y, iso);
-            }
+    for (int k = 0; k < R; ++k) {  // all loads before any use; {0, 0} is an inactive block
+        const uint64_t i = base + 64 * k;
+        v[k] = make_uint4(0, 0, 0, 0);
+        if (i + 1 < nblocks) {
+            v[k] = __ldg(reinterpret_cast<const uint4 *>(leaf + i));
+        } else if (i < nblocks) {
+            const uint2 one = __ldg(leaf + i);
+            v[k].x = one.x;
+            v[k].y = one.y;
         }
     }
-    uint32_t c = 0;
+    uint32_t b0[R], b1[R], total_w = 0;  // active first and second blocks of each round's lanes
 #pragma unroll
-    for (int i = 0; i < ITEMS; ++i) c += f[i];
-    uint32_t total;
-    const uint32_t excl = cta_exclusive_scan<kFilterThreads>(c, s_tmp, &total);
+    for (int k = 0; k < R; ++k) {
+        b0[k] = __ballot_sync(0xffffffffu, block_active(dtype, v[k].x, v[k].y, iso));
+        b1[k] = __ballot_sync(0xffffffffu, block_active(dtype, v[k].z, v[k].w, iso));
+        total_w += __popc(b0[k]) + __popc(b1[k]);
+    }
+    if (lane == 0) s_tmp[warp] = total_w;
+    __syncthreads();
+    uint32_t total = 0, excl = 0;
+#pragma unroll
+    for (uint32_t w = 0; w < kFilterThreads / 32; ++w) {
+        if (w == warp) excl = total;
+        total += s_tmp[w];
+    }
 
-    if (threadIdx.x < 32) {
-        const uint32_t lane = threadIdx.x;
+    if (warp == 0) {
         uint32_t prefix = 0;
         bool abort = false;
         if (t == 0) {
-            if (lane == 0) st_volatile(&tile_status[0], (kFlagInc << 30) | total);
+            if (lane == 0) st_volatile(&tile_status[0], TW::make(kFlagInc, epoch, total));
         } else {
-            if (lane == 0) st_volatile(&tile_status[t], (kFlagAgg << 30) | total);
+            if (lane == 0) st_volatile(&tile_status[t], TW::make(kFlagAgg, epoch, total));
             int64_t j = (int64_t)t - 1;
             uint32_t spins = 0;
             while (true) {
                 const int64_t k = j - (int64_t)lane;
-                const uint32_t w = k >= 0 ? ld_volatile(&tile_status[k]) : (kFlagInc << 30);
-                const uint32_t flag = w >> 30;
+                const typename TW::U w = k >= 0 ? ld_volatile(&tile_status[k]) : TW::make(kFlagInc, epoch, 0);
+                const uint32_t flag = TW::flag(w, epoch);
                 if (__any_sync(0xffffffffu, flag == kFlagAbort)) { abort = true; break; }
                 const uint32_t inc = __ballot_sync(0xffffffffu, flag == kFlagInc);
                 const uint32_t emp = __ballot_sync(0xffffffffu, flag == 0u);
@@ -100,74 +144,92 @@ __global__ void __launch_bounds__(kFilterThreads)
                     backoff(spins);
                     continue;
                 }
-                uint32_t v = lane <= first ? (w & 0x3fffffffu) : 0u;
+                uint32_t c = lane <= first ? TW::count(w) : 0u;
 #pragma unroll
-                for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-                prefix += v;
+                for (int o = 16; o; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
+                prefix += c;
                 if (first < 32) break;
                 j -= 32;
             }
             if (lane == 0)
-                st_volatile(&tile_status[t], abort ? (kFlagAbort << 30) : ((kFlagInc << 30) | (prefix + total)));
+                st_volatile(&tile_status[t],
+                            abort ? TW::make(kFlagAbort, epoch, 0) : TW::make(kFlagInc, epoch, prefix + total));
         }
         if (lane == 0) {
             s_prefix = prefix;
             s_abort = abort ? 1u : 0u;
+            if (t == ntiles - 1) *count_out = abort ? 0u : prefix + total;
         }
     }
     __syncthreads();
     if (s_abort) return;
     uint32_t r = s_prefix + excl;
-    // rank of every block of the tile: its rank if active, else kNoRank
-    uint32_t rk[ITEMS];
+    const uint32_t lt = (1u << lane) - 1u;
 #pragma unroll
-    for (int i = 0; i < ITEMS; ++i) {
-        rk[i] = 0xffffffffu;
-        if (f[i] && MTX_BC(r, nblocks, kBcRank)) {
-            const uint32_t id = (uint32_t)(base + i);
-            ids[r] = id;
-            rk[i] = r;
-            if (count_status) count_status[r] = 0ull;
-            ++r;
-        }
+    for (int k = 0; k < R; ++k) {
+        const uint64_t i = base + 64 * k;
+        const bool f0 = (b0[k] >> lane) & 1u, f1 = (b1[k] >> lane) & 1u;
+        const uint32_t r0 = r + __popc(b0[k] & lt) + __popc(b1[k] & lt), r1 = r0 + f0;
+        if (f0 && MTX_BC(r0, nblocks, kBcRank)) ids[r0] = (uint32_t)i;
+        if (f1 && MTX_BC(r1, nblocks, kBcRank)) ids[r1] = (uint32_t)i + 1;
+        // rank of every block of the tile: its rank if active, else kNoRank
+        const uint2 rk = make_uint2(f0 ? r0 : 0xffffffffu, f1 ? r1 : 0xffffffffu);
+        if (i + 1 < nblocks) *reinterpret_cast<uint2 *>(rank_map + i) = rk;
+        else if (i < nblocks) rank_map[i] = rk.x;
+        r += __popc(b0[k]) + __popc(b1[k]);
     }
-    if (base + ITEMS <= nblocks) {
-#pragma unroll
-        for (int i = 0; i < ITEMS / 4; ++i)
-            reinterpret_cast<uint4 *>(rank_map + base)[i] = make_uint4(rk[4 * i], rk[4 * i + 1], rk[4 * i + 2],
-                                                                       rk[4 * i + 3]);
-    } else {
-#pragma unroll
-        for (int i = 0; i < ITEMS; ++i)
-            if (base + i < nblocks) rank_map[base + i] = rk[i];
-    }
-    if (t == ntiles - 1 && threadIdx.x == 0) *count_out = s_prefix + total;
+}
+
+template <int ITEMS, bool EPOCH>
+__global__ void __launch_bounds__(kFilterThreads, 4)
+    filter_compact_kernel(const uint2 *__restrict__ leaf, uint64_t nblocks, uint32_t ntiles, uint32_t dtype,
+                          float iso, uint32_t *__restrict__ ids, uint32_t *__restrict__ rank_map,
+                          uint32_t *__restrict__ count_out, typename TileWord<EPOCH>::U *tile_status,
+                          typename TileWord<EPOCH>::U *ticket, DevStatus *st, uint32_t spin_limit, uint32_t skip) {
+    filter_tile<ITEMS, EPOCH>(leaf, nblocks, ntiles, dtype, iso, ids, rank_map, count_out, tile_status, ticket, st,
+                              spin_limit, skip);
+}
+
+// The compaction and the octree in one launch (the asynchronous whole-path
+// call): both read the leaf level, neither waits for the other, and the
+// octree's few CTAs run under the compaction's look-back chain.  As two
+// launches they took 6.4 + 6.4 us for a 256^3 volume at B = 8, and a gap.
+__global__ void __launch_bounds__(kFilterThreads, 4)
+    filter_octree_kernel(const uint2 *__restrict__ leaf, uint64_t nblocks, uint32_t ntiles, uint32_t dtype, float iso,
+                         uint32_t *__restrict__ ids, uint32_t *__restrict__ rank_map, uint32_t *__restrict__ count_out,
+                         uint64_t *tile_status, uint64_t *ticket, DevStatus *st, uint32_t spin_limit, uint32_t skip,
+                         const __grid_constant__ PyrAll L) {
+    static_assert(kPyrThreads == kFilterThreads, "one CTA size for both");
+    __shared__ uint2 s_part[8][8];
+    __shared__ uint32_t s_last;
+    if (blockIdx.x < ntiles)
+        filter_tile<kFilterItems, true>(leaf, nblocks, ntiles, dtype, iso, ids, rank_map, count_out, tile_status,
+                                        ticket, st, spin_limit, skip);
+    else
+        pyramid_tile(L, blockIdx.x - ntiles, s_part, &s_last);
 }
 
 MTX_BC_READER(bc_take_filter)
 
 mtx_status launch_filter(mtx_context *c, const Problem &p, const uint2 *leaf, uint32_t *ids, uint32_t *rank_map,
-                         uint32_t *count, uint64_t *count_status, cudaStream_t s) {
+                         uint32_t *count, cudaStream_t s, const PyrAll *octree) {
     if (p.nblocks >= (1ull << 30)) return fail(c, MTX_ERR_UNSUPPORTED, "more than 2^30 blocks");
     const uint32_t ntiles = (uint32_t)((p.nblocks + kFilterTile - 1) / kFilterTile);
-    mtx_status rs = scratch_reserve(c, c->filter_status, sizeof(uint32_t) * (size_t)ntiles);
+    const size_t before = c->filter_status.size;
+    mtx_status rs = scratch_reserve(c, c->filter_status, sizeof(uint64_t) * (size_t)ntiles);
     if (rs != MTX_OK) return rs;
-    MTX_CUDA(c, cudaMemsetAsync(c->filter_status.ptr, 0, sizeof(uint32_t) * (size_t)ntiles, s));
-    if (count == &c->ctrl->active_count) {  // ticket, count ticket (reset by the count pass too) and count: one memset
-        static_assert(offsetof(Ctrl, active_count) == offsetof(Ctrl, filter_ticket) + 8, "Ctrl layout");
-        MTX_CUDA(c, cudaMemsetAsync(&c->ctrl->filter_ticket, 0, 3 * sizeof(uint32_t), s));
-    } else {
-        MTX_CUDA(c, cudaMemsetAsync(&c->ctrl->filter_ticket, 0, sizeof(uint32_t), s));
-        MTX_CUDA(c, cudaMemsetAsync(count, 0, sizeof(uint32_t), s));
-    }
-    if (c->withhold & 1u) {  // failure injection: tile 0 is never handed out, so its successors wait and give up
-        static const uint32_t kOne = 1;
-        MTX_CUDA(c, cudaMemcpyAsync(&c->ctrl->filter_ticket, &kOne, sizeof(uint32_t), cudaMemcpyHostToDevice, s));
-    }
-    filter_compact_kernel<kFilterItems><<<ntiles, kFilterThreads, 0, s>>>(
-        leaf, p.nblocks, ntiles, p.dtype, p.iso, ids, rank_map, count, count_status,
-        (uint32_t *)c->filter_status.ptr, &c->ctrl->filter_ticket, &c->ctrl->status,
-        c->wait_polls ? c->wait_polls : kSpinLimit);
+    if (c->filter_status.size != before)  // new words: no epoch's
+        MTX_CUDA(c, cudaMemsetAsync(c->filter_status.ptr, 0, c->filter_status.size, s));
+    uint64_t *words = (uint64_t *)c->filter_status.ptr;
+    const uint32_t polls = c->wait_polls ? c->wait_polls : kSpinLimit, skip = c->withhold & 1u;
+    if (octree && octree->ntiles)
+        filter_octree_kernel<<<ntiles + octree->ntiles, kFilterThreads, 0, s>>>(
+            leaf, p.nblocks, ntiles, p.dtype, p.iso, ids, rank_map, count, words, &c->ctrl->filter_ticket,
+            &c->ctrl->status, polls, skip, *octree);
+    else
+        filter_compact_kernel<kFilterItems, true><<<ntiles, kFilterThreads, 0, s>>>(
+            leaf, p.nblocks, ntiles, p.dtype, p.iso, ids, rank_map, count, words, &c->ctrl->filter_ticket,
+            &c->ctrl->status, polls, skip);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(c, e, "filter launch");
     return MTX_OK;
@@ -289,9 +351,9 @@ extern "C" mtx_status mtx_filter_active_blocks_noalloc(const uint32_t *leaf_minm
         cudaGetLastError();
         return MTX_ERR_CUDA;
     }
-    filter_compact_kernel<kNoallocItems><<<ntiles, kFilterThreads, 0, s>>>(
+    filter_compact_kernel<kNoallocItems, false><<<ntiles, kFilterThreads, 0, s>>>(
         reinterpret_cast<const uint2 *>(leaf_minmax), total_blocks, ntiles, dtype, isovalue, compacted_ids, block_rank,
-        active_count, nullptr, sc, sc + kNoallocTicket, st, kSpinLimit);
+        active_count, sc, sc + kNoallocTicket, st, kSpinLimit, 0u);
     if (cudaGetLastError() != cudaSuccess) return MTX_ERR_CUDA;
     return MTX_OK;
 }

@@ -30,7 +30,9 @@ __global__ void __launch_bounds__(kMeshletWarps * 32)
     meshlet_kernel(const mtx_meshlet_descriptor *__restrict__ blocks, const uint32_t *__restrict__ count_ptr,
                    const uint32_t *__restrict__ indices, uint32_t maxV, uint32_t maxP,
                    mtx_meshlet_descriptor *__restrict__ per_block, mtx_meshlet_descriptor *__restrict__ meshlets,
-                   uint32_t *__restrict__ mverts, uint32_t *__restrict__ midx) {
+                   uint32_t *__restrict__ mverts, uint32_t *__restrict__ midx, uint64_t *scan_words,
+                   uint32_t scan_ntiles, uint32_t *scan_ticket, uint32_t *totals) {
+    if (!EMIT) scan_reset(scan_words, scan_ntiles, scan_ticket, totals);
     __shared__ uint32_t s_list[kMeshletWarps][kMaxMeshletVertices];
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint32_t *list = s_list[warp];
@@ -139,10 +141,13 @@ extern "C" mtx_status mtx_build_meshlets(mtx_context_t c, const mtx_extraction_o
     const auto *blocks = (const mtx_meshlet_descriptor *)ext->meshletDescriptorBuffer.ptr;
     const auto *count = (const uint32_t *)ext->meshletDescriptorCountBuffer.ptr;
     const auto *indices = (const uint32_t *)ext->indexBuffer.ptr;
+    uint64_t *words;
+    uint32_t ntiles, *ticket;
+    if ((r = desc_scan_words(c, nb, &words, &ntiles, &ticket)) != MTX_OK) return bail(r);
     const uint32_t grid = std::min<uint32_t>((nb + kMeshletWarps - 1) / kMeshletWarps, 16u * c->sm_count);
     meshlet_kernel<false><<<grid, kMeshletWarps * 32, 0, s>>>(blocks, count, indices, maxVertices, maxPrimitives,
                                                               (mtx_meshlet_descriptor *)per_block, nullptr, nullptr,
-                                                              nullptr);
+                                                              nullptr, words, ntiles, ticket, (uint32_t *)counters);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return bail(cuda_fail(c, e, "meshlet count launch"));
     if ((r = launch_desc_scan(c, (mtx_meshlet_descriptor *)per_block, count, nb, (uint32_t *)counters, s)) != MTX_OK)
@@ -164,7 +169,7 @@ extern "C" mtx_status mtx_build_meshlets(mtx_context_t c, const mtx_extraction_o
     meshlet_kernel<true><<<grid, kMeshletWarps * 32, 0, s>>>(blocks, count, indices, maxVertices, maxPrimitives,
                                                              (mtx_meshlet_descriptor *)per_block,
                                                              (mtx_meshlet_descriptor *)p_desc, (uint32_t *)p_mv,
-                                                             (uint32_t *)p_idx);
+                                                             (uint32_t *)p_idx, nullptr, 0, nullptr, nullptr);
     if ((e = cudaGetLastError()) != cudaSuccess) return bail(cuda_fail(c, e, "meshlet emit launch"));
     const uint64_t work = (uint64_t)MV * stride;
     const uint32_t ggrid = (uint32_t)std::min<uint64_t>((work + 255) / 256, 8ull * c->sm_count);

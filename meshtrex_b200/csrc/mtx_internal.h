@@ -15,14 +15,14 @@ namespace mtx {
 // Per-pipeline control words in device memory.
 struct Ctrl {
     DevStatus status;        // first error recorded by any kernel
-    uint32_t filter_ticket;  // tile tickets of the compaction scan
-    uint32_t count_ticket;   // block tickets of the count scan
+    uint64_t filter_ticket;  // compaction: epoch << 32 | tile ticket
+    uint32_t count_ticket;   // tile tickets of the count scan
     uint32_t active_count;   // compaction result
-    uint32_t pad0;
     uint32_t totals[4];      // vertexCount, indexCount, meshletCount, activeBlockCount
     uint32_t batch_ticket[4];
     uint32_t pyr_done;       // octree tiles finished (the last one builds the top levels)
-    uint32_t pad1[3];
+    uint32_t emit_done;      // CTAs of the emit pass finished (the last one writes status_out)
+    uint32_t pad1[2];
 };
 
 // A grow-only device allocation owned by the context.
@@ -138,10 +138,10 @@ mtx_status launch_pyramid(mtx_context *c, uint2 *all_levels, int levels, const u
 
 // Stage 2: ordered compaction of active blocks.
 //   ids[rank] = block id, rank_map[id] = rank (0xffffffff if inactive),
-//   *count = number of active blocks.  count_status: optional per-rank words
-//   to zero (pass null).
+//   *count = number of active blocks.
+// octree: build these levels in the same launch.
 mtx_status launch_filter(mtx_context *c, const Problem &p, const uint2 *leaf, uint32_t *ids,
-                         uint32_t *rank_map, uint32_t *count, uint64_t *count_status, cudaStream_t s);
+                         uint32_t *rank_map, uint32_t *count, cudaStream_t s, const PyrAll *octree = nullptr);
 
 // Stage 3: per-active-block counts and face records, the scan that fills the
 // meshlet descriptors and totals (launch_count); then vertices and triangles
@@ -155,9 +155,9 @@ struct ExtractArgs {
     uint64_t desc_capacity;
     uint32_t *faces;            // 3*B*B words per active block
     uint8_t *state;             // block_state_bytes(B) per active block (count -> emit), B <= 8
-    uint64_t block_capacity;    // active blocks that desc/faces/count_status can hold
-    uint64_t *count_status;     // unused (the scan keeps its own look-back words)
+    uint64_t block_capacity;    // active blocks that desc/faces/state can hold
     uint32_t *totals;           // device uint32[4] {vertexCount, indexCount, meshletCount, activeCount}
+    uint32_t *status_out;       // optional device word: the context's error code when the emit pass is done
     uint8_t *cell_cases;        // optional
     void *vertices;             // vertex buffer written by the emit pass, or null
     uint64_t vertex_capacity;
@@ -168,7 +168,24 @@ struct ExtractArgs {
 mtx_status launch_count(mtx_context *c, const Problem &p, const ExtractArgs &a, cudaStream_t s);
 // Bytes of the block state the count pass hands to the emit pass (0: none, B > 8).
 uint32_t block_state_bytes(uint32_t B);
-// The descriptor scan alone over *count descriptors (capacity bounds them).
+// The descriptor scan alone over *count descriptors (capacity bounds them); the
+// kernel before it in the stream zeroes the scan's words (scan_reset).
+mtx_status desc_scan_words(mtx_context *c, uint64_t capacity, uint64_t **words, uint32_t *tiles, uint32_t **ticket);
+inline uint32_t scan_tiles(uint64_t capacity) {  // look-back words of the descriptor scan, at least one
+    return capacity ? (uint32_t)((capacity + 1023) / 1024) : 1u;
+}
+#ifdef __CUDACC__
+// Zeroes the descriptor scan's look-back words, ticket and totals from the
+// kernel that runs before it (three memsets of about 4 us each on the
+// timeline before); called at the start of that kernel by every thread.
+__device__ __forceinline__ void scan_reset(uint64_t *words, uint32_t tiles, uint32_t *ticket, uint32_t *totals) {
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < tiles; i += gridDim.x * blockDim.x) words[i] = 0;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        *ticket = 0;
+        totals[0] = totals[1] = totals[2] = totals[3] = 0;
+    }
+}
+#endif
 mtx_status launch_desc_scan(mtx_context *c, mtx_meshlet_descriptor *desc, const uint32_t *count, uint64_t capacity,
                             uint32_t *totals, cudaStream_t s);
 mtx_status launch_emit(mtx_context *c, const Problem &p, const ExtractArgs &a, cudaStream_t s);

@@ -1167,6 +1167,7 @@ __device__ __forceinline__ void emit_block(const Problem &p, const WPlan &pl, un
 constexpr int kScanThreads = 256;
 constexpr int kScanItems = 4;
 constexpr int kScanTile = kScanThreads * kScanItems;
+static_assert(kScanTile == 1024, "scan_tiles");
 
 __device__ __forceinline__ void scan_tile(mtx_meshlet_descriptor *desc, uint32_t count, uint32_t t, uint64_t *status,
                                           uint32_t *totals, DevStatus *st, uint64_t *s_tmp, uint32_t *s_ok,
