@@ -43,6 +43,7 @@ struct BVol {
     WPlan pl;       // region sizes of this volume, offsets of the batch's shared warp layout
     GridDiv dv;     // reciprocals of the grid's row and slice sizes (block_geo)
     uint32_t nXS, nbs, zchunk, wide;  // min/max: strips, blocks a strip, words a lane (RowCut); slabs a warp
+    bool nan_zero;      // minmax_leaf_rows_warp
     uint64_t leaf_off;  // first leaf entry of the volume in the pooled leaf array
     uint64_t mm_begin;  // first min/max warp of the volume
 };
@@ -121,7 +122,7 @@ __global__ void __launch_bounds__(128) batch_minmax_kernel(const BVol *__restric
     }
 #define MTX_MM(T, W, NR)                                                                                               \
     minmax_leaf_rows_warp<T, W, NR, sizeof(T) == 4>((const T *)p.vol, p.X, p.Y, p.Z, p.B, p.GX, p.GY, p.GZ, v.nXS, v.nbs, \
-                                                    v.zchunk, lw, out, s_col[threadIdx.x >> 5])
+                                                    v.zchunk, lw, out, s_col[threadIdx.x >> 5], v.nan_zero)
     switch (p.dtype * 4 + (p.B == 8) * 2 + v.wide) {
     case MTX_DTYPE_U8 * 4: MTX_MM(uint8_t, 1, 0); break;
     case MTX_DTYPE_U8 * 4 + 1: MTX_MM(uint8_t, 2, 0); break;
@@ -637,7 +638,7 @@ KernelFn batch_kernel(int variant) {
 
 WPlan plan_in_layout(uint32_t B, const WPlan &L) {
     WPlan p = make_wplan_balanced(B);
-    p.off_tile[0] = p.off_tile[1] = L.off_tile[0];
+    p.off_tile = L.off_tile;
     p.off_vtab = L.off_vtab;
     p.off_bar = L.off_bar;
     p.off_rows = L.off_rows;
@@ -743,6 +744,7 @@ mtx_status mtx_batch_create(mtx_context_t c, const mtx_batch_desc *d, mtx_batch_
         }
         const RowCut cut = row_cut(p, esz);
         bv.wide = cut.wide;
+        bv.nan_zero = (uintptr_t)p.vol % 16 != 0 || ((uint64_t)p.X * esz) % 16 != 0 || (B != 4 && B != 8 && B != 16);
         bv.nXS = cut.nXS;
         bv.nbs = cut.nbs;
         const uint64_t cols = (uint64_t)bv.nXS * p.GY;

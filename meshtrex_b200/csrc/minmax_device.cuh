@@ -321,7 +321,10 @@ inline bool rows_ok(const Problem &p, uint32_t esz) { return (uint64_t)p.X * esz
 // into the running slab, and only when a slab is complete -- once every B
 // slices -- do the columns go to shared memory, where each lane takes the
 // B + 1 columns of its blocks.  NR = B + 1 at compile time, 0: at run time,
-// four rows in flight.  s: 64 * W words of the warp's own shared memory.  The
+// four rows in flight.  s: 64 * W words of the warp's own shared memory.
+// nan_zero (float32): a NaN of positive sign takes the key of -0.0 instead of one
+// above +inf, which would leave its block without an isovalue -- what volumes
+// off the 16-byte passes have always had, while those passes keep the NaN's key.  The
 // B + 1 rows of a strip span less than 4 GiB (rows_ok).
 // Bound by instruction issue (about 2.5 a cycle and SM): every word costs an
 // address, a load, for unaligned rows a shuffle and a shift, and half a
@@ -333,7 +336,7 @@ template <typename T, int W, int NR, bool ALIGNED>
 __device__ __forceinline__ void minmax_leaf_rows_warp(const T *__restrict__ vol, uint32_t X, uint32_t Y, uint32_t Z,
                                                       uint32_t B_, uint32_t GX, uint32_t GY, uint32_t GZ, uint32_t nXS,
                                                       uint32_t nbs, uint32_t zchunk, uint64_t w,
-                                                      uint2 *__restrict__ leaf, uint32_t *s) {
+                                                      uint2 *__restrict__ leaf, uint32_t *s, bool nan_zero = true) {
     using RW = RowWord<T>;
     constexpr int N = RW::N;
     const uint32_t B = NR ? (uint32_t)(NR - 1) : B_, lane = threadIdx.x & 31;
@@ -415,6 +418,7 @@ __device__ __forceinline__ void minmax_leaf_rows_warp(const T *__restrict__ vol,
                 x = __funnelshift_r(x, __shfl_sync(0xffffffffu, give, (lane + 1) & 31), sh);
             }
             RW::split(x, v[j]);
+            if constexpr (sizeof(T) == 4) v[j][0] = nan_zero && v[j][0] > 0xff800000u ? 0x7fffffffu : v[j][0];
         }
     };
     uint32_t tmn[W][N], tmx[W][N];  // the slice

@@ -57,3 +57,28 @@ def test_rows_leaf_matches_oracle(ctx, oracle, shape, dtype, block, offset, zchu
         mm.free()
     finally:
         ctx.set_tuning()
+
+
+@pytest.mark.parametrize("block,offset", [(7, 0), (8, 1), (3, 0)])
+def test_rows_leaf_keys_of_nan_and_infinities(ctx, block, offset):
+    """A NaN of positive sign counts as -0.0, so that it does not take its block
+    out of every isovalue's range; one of negative sign and the infinities keep
+    their place in the order of the keys."""
+    from meshtrex_b200 import api
+    rng = np.random.default_rng(5)
+    a = rng.standard_normal((2 * block + 1, block + 3, 3 * block + 2)).astype(np.float32)
+    r = rng.random(a.shape)
+    for lo, v in ((.0, np.float32(np.nan)), (.01, -np.float32(np.nan)), (.02, np.inf), (.03, -np.inf), (.04, -0.0)):
+        a[(r >= lo) & (r < lo + .01)] = v
+    buf = torch.zeros(a.size + offset, dtype=torch.float32, device="cuda")
+    buf[offset:] = torch.from_numpy(a.reshape(-1)).cuda()
+    mm = api.compute_min_max_mip(ctx, api.wrap_volume(buf[offset:].view(a.shape)),
+                                 api.push_constants(a.shape[::-1], block, 0.0))
+    got = u32(mm.level(0))
+    mm.free()
+    bits = a.view(np.uint32)
+    keys = np.where(bits >> 31, ~bits, bits | 0x80000000)
+    keys = np.where(keys > 0xff800000, np.uint32(0x7fffffff), keys)
+    for z, y, x in np.ndindex(got.shape[:3]):
+        s = keys[z * block:(z + 1) * block + 1, y * block:(y + 1) * block + 1, x * block:(x + 1) * block + 1]
+        assert (got[z, y, x, 0], got[z, y, x, 1]) == (s.min(), s.max())
