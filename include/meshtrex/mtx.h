@@ -178,10 +178,10 @@ typedef struct mtx_mesh_buffers {
     uint32_t *counters;
     /* Upper bound on active blocks, sizing the scratch of the extraction
      * (0 = every block of the grid); more active blocks -> MTX_ERR_CAPACITY.
-     * The scratch per active block is 12 B^2 bytes of face records, 16 B of
-     * descriptor and, for B <= 8, the block state the count pass hands to the
-     * emit pass (1920 B at B = 8): about 2.7 KB at B = 8, so a bound well
-     * under the grid's block count saves gigabytes on large volumes. */
+     * The scratch per active block is 6 B^2 bytes of face records, 16 B of
+     * descriptor and what the count pass hands to the emit pass: 4 B^3 bytes
+     * for B <= 8, else 4 (B+1)^2 (each rounded up): about 2.4 KB at B = 8, so a
+     * bound well under the grid's block count saves gigabytes on large volumes. */
     uint64_t maxActiveBlocks;
 } mtx_mesh_buffers;
 

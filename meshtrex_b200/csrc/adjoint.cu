@@ -47,10 +47,10 @@ template <bool DET>
 __global__ void __launch_bounds__(kAdjWarps * 32) adjoint_block_kernel(const __grid_constant__ AdjArgs a) {
     extern __shared__ __align__(128) unsigned char smem[];
     const Problem &p = a.p;
-    const WPlan pl = make_wplan(p.B, 4, false, false, true);
+    const WPlan pl = make_wplan(p.B);
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, W = blockDim.x >> 5;
     unsigned char *ws = smem + warp * a.ws_bytes;
-    float *tile = reinterpret_cast<float *>(ws + pl.off_tile[0]);
+    float *tile = reinterpret_cast<float *>(ws + pl.off_tile);
     float *acc = reinterpret_cast<float *>(ws + a.off_acc);
     const uint32_t *cross = reinterpret_cast<const uint32_t *>(ws + pl.off_cross);
     const uint32_t *vp = reinterpret_cast<const uint32_t *>(ws + pl.off_vp);
@@ -62,9 +62,9 @@ __global__ void __launch_bounds__(kAdjWarps * 32) adjoint_block_kernel(const __g
         const uint4 dq = __ldg(reinterpret_cast<const uint4 *>(a.desc + r));
         const uint32_t vbase = dq.x, nv = dq.z;
         tile_load_float(p, pl, tile, g);
-        build_rows<float>(p, pl, ws, 0, g);
+        build_rows<float>(p, pl, ws, g);
         uint32_t bnv, bnt;
-        block_counts(p, pl, ws, g, nullptr, false, nullptr, bnv, bnt);
+        block_counts(p, pl, ws, g, nullptr, false, bnv, bnt);
         const bool ok = bnv == nv && (uint64_t)vbase + nv <= a.vcount;
         if (!ok && lane == 0) report(a.st, MTX_ERR_INTERNAL, kSiteAdjoint, r, bnv);
         if (DET) {
@@ -238,7 +238,7 @@ extern "C" mtx_status mtx_extract_backward(mtx_context_t c, const mtx_volume *vo
     a.iso_part = (float *)c->adj_iso.ptr;
     a.T3 = T3;
     a.st = &c->ctrl->status;
-    const WPlan pl = make_wplan(B, 4, false, false, true);
+    const WPlan pl = make_wplan(B);
     a.off_acc = pl.bytes;
     a.ws_bytes = pl.bytes + (det ? align_up(4 * T3, 128) : 0u);
     const uint32_t smem = kAdjWarps * a.ws_bytes;

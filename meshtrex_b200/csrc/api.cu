@@ -845,9 +845,8 @@ mtx_status mtx_extract_meshlet_descriptors(mtx_context_t c, const mtx_minmax_out
         memset(out, 0, sizeof(*out));
         return s;
     };
-    if ((r = scratch_reserve(c, c->faces, (size_t)n * 3 * B * B * 4)) != MTX_OK) return bail(r);
-    const uint32_t sb = block_state_bytes(B);
-    if (sb && (r = scratch_reserve(c, c->state, (size_t)n * sb)) != MTX_OK) return bail(r);
+    if ((r = scratch_reserve(c, c->faces, n * face_record_bytes(B))) != MTX_OK) return bail(r);
+    if ((r = scratch_reserve(c, c->state, n * block_state_bytes(B))) != MTX_OK) return bail(r);
 
     ExtractArgs a;
     memset(&a, 0, sizeof(a));
@@ -858,8 +857,8 @@ mtx_status mtx_extract_meshlet_descriptors(mtx_context_t c, const mtx_minmax_out
     a.desc = (mtx_meshlet_descriptor *)desc;
     a.desc_capacity = n;
     a.block_capacity = n;
-    a.faces = (uint32_t *)c->faces.ptr;
-    a.state = sb ? (uint8_t *)c->state.ptr : nullptr;
+    a.faces = (uint16_t *)c->faces.ptr;
+    a.state = (uint32_t *)c->state.ptr;
     a.totals = (uint32_t *)counters;
     a.cell_cases = o.cellCases;
     a.vertex_format = o.vertexFormat;
@@ -941,9 +940,8 @@ mtx_status mtx_extract_plain_async(mtx_context_t c, const mtx_volume *vol, const
     if ((r = scratch_reserve(c, c->leaf, texels * 8)) != MTX_OK) return r;
     if ((r = scratch_reserve(c, c->ids, p.nblocks * 4)) != MTX_OK) return r;
     if ((r = scratch_reserve(c, c->rank, p.nblocks * 4)) != MTX_OK) return r;
-    if ((r = scratch_reserve(c, c->faces, maxa * 3 * B * B * 4)) != MTX_OK) return r;
-    const uint32_t sb = block_state_bytes(B);
-    if (sb && (r = scratch_reserve(c, c->state, maxa * sb)) != MTX_OK) return r;
+    if ((r = scratch_reserve(c, c->faces, maxa * face_record_bytes(B))) != MTX_OK) return r;
+    if ((r = scratch_reserve(c, c->state, maxa * block_state_bytes(B))) != MTX_OK) return r;
     mtx_meshlet_descriptor *desc = out->meshlets;
     uint64_t dcap = out->meshletCapacity;
     if (!desc || dcap < maxa) {
@@ -991,8 +989,8 @@ mtx_status mtx_extract_plain_async(mtx_context_t c, const mtx_volume *vol, const
     a.desc = desc;
     a.desc_capacity = dcap;
     a.block_capacity = maxa;
-    a.faces = (uint32_t *)c->faces.ptr;
-    a.state = sb ? (uint8_t *)c->state.ptr : nullptr;
+    a.faces = (uint16_t *)c->faces.ptr;
+    a.state = (uint32_t *)c->state.ptr;
     a.totals = out->counters;
     a.status_out = out->counters + 4;
     a.cell_cases = o.cellCases;

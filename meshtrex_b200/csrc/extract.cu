@@ -2,55 +2,51 @@
 // (meshtrex: marching_cubes_pmb.task.glsl:101-216 and
 // marching_cubes_pmb.mesh.glsl:185-393, drawn by extractionManager.cpp:638-640).
 //
-// One warp owns one active block at a time; a CTA runs several such warps
-// that share only the case tables (and, in the emit pass, the context-layer
-// map).  Each warp stages the (B+1)^3 voxel tile of its block in shared
-// memory (a TMA 3D tile, or plain loads when the volume's rows are not
-// 16-byte aligned); the next block's tile is issued as soon as the current
-// block is done.
+// One warp owns one active block at a time (block bodies: pmb_lists.cuh); a CTA
+// runs several such warps that share only the tables.  The count pass stages
+// the (B+1)^3 voxel tile of its block in shared memory by TMA, or, when the
+// volume's rows are not 16-byte aligned, takes the inside bits straight from
+// plain loads; the next block's tile is issued as soon as the current block's
+// inside bits are built.
 //
-//  count pass  per-block vertex/triangle counts, low-face records and, for
-//              B <= 8, the block state the emit pass takes over
+//  count pass  per-block vertex/triangle counts, low-face records and the list
+//              of the block's cells (B > 8: its inside bits) for the emit pass
 //  scan pass   decoupled look-back scan of the counts -> meshlet descriptors, totals
 //  emit pass   vertices (each exactly once) and triangles, indices resolved
-//              through the block's voxel table and the neighbours' face records
-#include "pmb_device.cuh"
+//              through the block's vertex table and the neighbours' face records
+#include "pmb_lists.cuh"
 
 namespace mtx {
 
-// One tile buffer a warp in the count and emit passes: without the second
-// (prefetch) buffer a warp's region shrinks by a tile (2.7 KB for uint16 at
-// B = 8), more CTAs fit an SM (emit: seven instead of five), and the other
-// warps hide a tile's latency better than the prefetch did (per 1024^3
-// extraction: emit 0.41 -> 0.33 ms, count 0.101 -> 0.095 ms).
-constexpr bool kSingleBuffer = true;
-
 // ------------------------------------------------------------- count pass
-// BC: the block edge at compile time (0: p.B at run time).  The bench's edge 8
-// has its own instantiation, in which the warp's shared-memory plan and every
-// division by the edge fold to constants (48 registers).  The run-time form is
-// held to 64 registers (no spills), where it would otherwise take up to 128.
+// BC: the block edge at compile time (0: p.B at run time): the warp's
+// shared-memory plan and every division by the edge fold to constants.
+// Bound by instruction issue (2.6 a cycle and SM, 880 a block at B = 8).  Row
+// walks over the crossing rows with case bytes and prefixes kept for every cell
+// took 108 us for the 80,600 active blocks of the 1024^3 uint16 ball at B = 8;
+// the list takes 94; 1024 x 1024 x 314 uint8 at B = 3 179 -> 127; 384 x 320 x
+// 256 float32 at B = 4 58 -> 42; 640 x 512 x 448 uint16 at B = 16 53 -> 36.
 template <typename T, bool TMA, int BC>
-__global__ void __launch_bounds__(kMaxWarps * 32, BC ? 0 : 4)
+__global__ void __launch_bounds__(kMaxWarps * 32, 4)
     pmb_count_kernel(Problem p_, const __grid_constant__ CUtensorMap map, const uint32_t *__restrict__ ids,
                      const uint32_t *__restrict__ count_ptr, mtx_meshlet_descriptor *__restrict__ desc,
-                     uint64_t desc_cap, uint32_t *__restrict__ faces, uint8_t *__restrict__ state,
+                     uint64_t desc_cap, uint16_t *__restrict__ faces, uint32_t *__restrict__ state,
                      uint32_t *totals, uint8_t *__restrict__ cell_cases, uint64_t block_cap, DevStatus *st,
-                     uint64_t *scan_status, uint32_t scan_tiles, uint32_t *scan_ticket) {
+                     uint64_t *scan_status, uint32_t scan_tiles, uint32_t *scan_ticket, bool use_off) {
     extern __shared__ __align__(128) unsigned char smem[];
     scan_reset(scan_status, scan_tiles, scan_ticket, totals);
     Problem p = p_;
     if (BC) p.B = BC;
-    const WPlan pl = make_wplan(p.B, sizeof(T), TMA, false, kSingleBuffer, p.B <= 8);
+    const WPlan pl = make_count_plan(p.B, sizeof(T), TMA);
     const GridDiv dv = grid_div(p);
-    uint8_t *ntab = smem + 2048;
+    uint8_t *ntab = smem;
+    uint32_t *off = reinterpret_cast<uint32_t *>(smem + 256);
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, W = blockDim.x >> 5;
-    unsigned char *ws = smem + kTableBytes + warp * pl.bytes;
+    unsigned char *ws = smem + count_fixed_bytes(p.B, !TMA && use_off) + warp * pl.bytes;
     for (uint32_t i = threadIdx.x; i < 256; i += blockDim.x) ntab[i] = (uint8_t)(c_mc_cases[i] & 0xFu);
+    if (!TMA && use_off) row_offsets(p, pl, off);
     if (lane == 0 && TMA) {
-        uint64_t *bar = reinterpret_cast<uint64_t *>(ws + pl.off_bar);
-        mbar_init(bar, 1);
-        mbar_init(bar + 1, 1);
+        mbar_init(reinterpret_cast<uint64_t *>(ws + pl.off_bar), 1);
         fence_mbar_init();
     }
     __syncthreads();
@@ -62,36 +58,32 @@ __global__ void __launch_bounds__(kMaxWarps * 32, BC ? 0 : 4)
         }
         return;
     }
-    const uint32_t B3 = pl.BB * pl.B;
-    const uint32_t gw = blockIdx.x * W + warp, nw = gridDim.x * W;
-    uint32_t parity = 0, buf = 0;
+    const uint32_t B3 = pl.BB * pl.B, slot = list_state_words(p.B), fslot = face_stride16(p.B);
+    uint32_t parity = 0;
 
-    uint32_t r = gw;
+    uint32_t r = blockIdx.x * W + warp;
+    const uint32_t nw = gridDim.x * W;
     Geo g{};
     if (r < count) {
         g = block_geo(__ldg(ids + r), p, TMA, sizeof(T), dv);
-        tile_issue<T, TMA>(pl, ws, buf, g, &map);
+        if constexpr (TMA) tile_issue<T>(pl, ws, g, &map);
     }
     while (r < count) {
         const uint32_t rn = r + nw;
         Geo gn{};
         const bool have_next = rn < count;
-        if (have_next) {
-            gn = block_geo(__ldg(ids + rn), p, TMA, sizeof(T), dv);
-            if (pl.nbuf == 2) tile_issue<T, TMA>(pl, ws, buf ^ 1u, gn, &map);
+        if (have_next) gn = block_geo(__ldg(ids + rn), p, TMA, sizeof(T), dv);
+        if constexpr (TMA) {
+            if (!tile_wait(pl, ws, g, parity, st)) break;
+            if constexpr (BC != 0) tile_rows<T, BC>(p, pl, ws, g);
+            else build_rows<T>(p, pl, ws, g);
+            if (have_next) tile_issue<T>(pl, ws, gn, &map);  // the tile is dead once the rows are built
+        } else {
+            load_rows<T, BC>(p, pl, ws, g, use_off ? off : nullptr);
         }
-        if (!tile_wait<T, TMA>(p, pl, ws, buf, g, parity, st)) {
-            if (have_next && pl.nbuf == 2) tile_drain<TMA>(pl, ws, buf ^ 1u, parity);
-            break;
-        }
-        // one tile buffer: the next tile is issued as soon as this block's rows are built
-        const bool early = have_next && pl.nbuf == 1;
-        count_block<T, TMA>(p, pl, ws, buf, g, ntab, cell_cases ? cell_cases + (uint64_t)r * B3 : nullptr, desc + r,
-                            faces + (uint64_t)r * 3 * pl.BB,
-                            (state && pl.state_bytes) ? state + (uint64_t)r * pl.state_bytes : nullptr,
-                            early ? &gn : nullptr, &map);
+        count_block_list<BC>(p, pl, ws, g, ntab, cell_cases ? cell_cases + (uint64_t)r * B3 : nullptr, desc + r,
+                             faces + (uint64_t)r * fslot, state + (uint64_t)r * slot);
         if (!have_next) break;
-        if (pl.nbuf != 1) buf ^= 1u;
         r = rn;
         g = gn;
     }
@@ -101,7 +93,8 @@ __global__ void __launch_bounds__(kMaxWarps * 32, BC ? 0 : 4)
 __global__ void __launch_bounds__(kScanThreads)
     pmb_scan_kernel(mtx_meshlet_descriptor *__restrict__ desc, const uint32_t *__restrict__ count_ptr,
                     uint64_t *tile_status, uint32_t *ticket, uint32_t *totals, DevStatus *st, uint32_t spin_limit,
-                    uint32_t skip) {
+                    uint32_t skip, uint32_t *emit_ticket) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) *emit_ticket = 0;  // for the emit pass that follows
     __shared__ uint32_t s_tile, s_ok;
     __shared__ uint64_t s_tmp[kScanThreads / 32 + 1];
     __shared__ uint64_t s_pre[2];
@@ -113,98 +106,210 @@ __global__ void __launch_bounds__(kScanThreads)
     scan_tile(desc, count, t, tile_status, totals, st, s_tmp, &s_ok, s_pre, spin_limit);
 }
 
+// A warp's blocks in the emit pass: three quarters of the list by a fixed stride,
+// the rest by ticket, drawn one block ahead.  Warps' blocks differ in work, and
+// with about ten blocks a warp (80,000 active blocks of a 1024^3 volume) fixed
+// shares alone leave most warps waiting for the unluckiest; tickets alone are
+// bound by the counter, which serves fewer than one draw a nanosecond
+// (emit of the 1024^3 uint16
+// ball at block 8: 183 us by stride, 161 by tickets, 158 so; the count pass, at
+// half the work a block, gets slower, 94 -> 134 us, and keeps the stride).
+struct BlockShare {
+    uint32_t fixed, stride;  // blocks given out by stride, warps of the grid
+    uint32_t *ticket;
+    __device__ __forceinline__ BlockShare(uint32_t count, uint32_t warps, uint32_t *t) : stride(warps), ticket(t) {
+        const uint32_t rounds = count / warps;
+        fixed = rounds ? rounds * 3 / 4 * warps : ~0u;
+    }
+    // The block after block r of this warp (lane 0's value is the block for tickets: take it by shuffle).
+    __device__ __forceinline__ uint32_t after(uint32_t r) const {
+        if (fixed == ~0u || (uint64_t)r + stride < fixed) return min((uint64_t)r + stride, (uint64_t)~0u);
+        uint32_t t = 0;
+        if ((threadIdx.x & 31) == 0) t = fixed + atomicAdd(ticket, 1u);
+        return t;
+    }
+};
+
 // -------------------------------------------------------------- emit pass
-// CPL: context voxels per lane, ceil((3B^2 + 3B + 1) / 32): 8 covers B <= 8, 32 covers B <= 16.
-// The xyz form of B <= 8 is bounded to 85 registers (three CTAs of 256
-// threads); it uses 60 at the compile-time edge 8 and about 68 otherwise, with
-// no spills; with 27.9 KB of shared memory a CTA of four warps (8- and 16-bit
-// voxels) eight CTAs share an SM at edge 8.  The other forms would spill
-// under that bound.
-template <typename T, int CPL, bool TMA, bool GENERIC, int BC>
-__global__ void __launch_bounds__(kMaxWarps * 32, (!GENERIC && CPL == 8) ? 3 : 1)
-    pmb_emit_kernel(Problem p_, const __grid_constant__ CUtensorMap map, const uint32_t *__restrict__ ids,
-                    const uint32_t *__restrict__ rank_map, const uint32_t *__restrict__ count_ptr,
-                    const mtx_meshlet_descriptor *__restrict__ desc, const uint32_t *__restrict__ faces,
-                    const uint8_t *__restrict__ state, uint32_t *__restrict__ indices, uint64_t tcap,
-                    uint64_t block_cap, void *__restrict__ vertices, uint64_t vcap, uint32_t vfmt, uint32_t frame,
-                    uint32_t normals, DevStatus *st, uint32_t *done, uint32_t *status_out) {
-    // B <= 8 with TMA: the count pass's block state comes with each tile
-    constexpr bool STATE = TMA && CPL == 8;
+// Bound by instruction issue (2.5 a cycle and SM, 1380 a block at B = 8) and the
+// latency of each block's dependent loads (rank -> descriptor and face records;
+// list -> voxels), under which four CTAs of eight warps an SM run; five, at 48
+// registers, take the L1 that serves the second reading of the list and are
+// slower.  Against the tile, the rows and the row walks of the former pass:
+// 1024^3 uint16 ball at B = 8, 231 -> 157 us; 512^3 float32 gyroid at B = 8,
+// 225 -> 135; 640 x 512 x 448 uint16 at B = 16, one CTA of four warps an SM
+// before, 411 -> 110; 1024 x 1024 x 314 uint8 at B = 3, 251 -> 152.
+template <typename T, bool GENERIC, int BC, bool BIG>
+__global__ void __launch_bounds__(kMaxWarps * 32, GENERIC ? 1 : 4)
+    pmb_emit_kernel(Problem p_, const uint32_t *__restrict__ ids, const uint32_t *__restrict__ rank_map,
+                    const uint32_t *__restrict__ count_ptr, const mtx_meshlet_descriptor *__restrict__ desc,
+                    const uint16_t *__restrict__ faces, const uint32_t *__restrict__ state,
+                    uint32_t *__restrict__ indices, uint64_t tcap, uint64_t block_cap, void *__restrict__ vertices,
+                    uint64_t vcap, uint32_t vfmt, uint32_t frame, uint32_t normals, DevStatus *st, uint32_t *done,
+                    uint32_t *status_out, uint32_t *ticket) {
+    // context voxels a lane loads at once: all of them for B <= 8
+    constexpr int N = BIG ? 8 : BC == 3 || BC == 4 ? 2 : 7;
     extern __shared__ __align__(128) unsigned char smem[];
     Problem p = p_;
     if (BC) p.B = BC;
-    const WPlan pl = make_wplan(p.B, sizeof(T), TMA, true, kSingleBuffer);
+    const WPlan pl = make_emit_plan(p.B);
     const GridDiv dv = grid_div(p);
-    uint64_t *tab = reinterpret_cast<uint64_t *>(smem);
-    uint8_t *ntab = smem + 2048;
-    uint8_t *owner = smem + 2048 + 256;
-    uint32_t *cmap = reinterpret_cast<uint32_t *>(smem + kTableBytes);
+    uint64_t *tri = reinterpret_cast<uint64_t *>(smem);
+    uint16_t *first = reinterpret_cast<uint16_t *>(smem + 8 * kTris);
+    uint32_t *cmap = reinterpret_cast<uint32_t *>(smem + 8 * kTris + 512);
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, W = blockDim.x >> 5;
-    unsigned char *ws = smem + cta_fixed_bytes(p.B, true) + warp * pl.bytes;
-    for (uint32_t i = threadIdx.x; i < 256; i += blockDim.x) {
-        tab[i] = c_mc_cases[i];
-        ntab[i] = (uint8_t)(c_mc_cases[i] & 0xFu);
-    }
-    for (uint32_t j = threadIdx.x; j < pl.nb3; j += blockDim.x) cmap[j] = ctx_map_entry(pl, j);
-    if (threadIdx.x < 12) owner[threadIdx.x] = c_mc_owner[threadIdx.x];
-    if (CPL == 8) edge_offsets(reinterpret_cast<uint16_t *>(owner + 16), pl.B1);
-    if (lane == 0 && TMA) {
-        uint64_t *bar = reinterpret_cast<uint64_t *>(ws + pl.off_bar);
-        mbar_init(bar, 1);
-        mbar_init(bar + 1, 1);
-        fence_mbar_init();
-    }
+    unsigned char *ws = smem + emit_fixed_bytes(p.B) + warp * pl.bytes;
+    build_tris(pl, tri, first);
+    for (uint32_t j = threadIdx.x; j < pl.nb3; j += blockDim.x) cmap[j] = ctx_entry(pl, j);
     __syncthreads();
     uint32_t count = *count_ptr;
     if (count > block_cap) count = 0;  // reported by the count pass
-    const uint32_t gw = blockIdx.x * W + warp, nw = gridDim.x * W;
-    uint32_t parity = 0, buf = 0;
+    const uint32_t slot = list_state_words(p.B), B3 = pl.BB * pl.B;
+    const uint64_t face_words = block_cap * face_stride16(p.B);
+    uint32_t *jobs = reinterpret_cast<uint32_t *>(ws + pl.off_jobs);
+    uint32_t *nbase = reinterpret_cast<uint32_t *>(ws + pl.off_nvid);
+    unsigned char *vtab_b = ws + pl.off_vtab;
+    uint16_t *vtab = reinterpret_cast<uint16_t *>(vtab_b);
+    const uint32_t edge8 = BC == 8 ? ctx8_edge(lane) : 0u;
 
-    uint32_t r = gw;
+    const BlockShare share(count, gridDim.x * W, ticket);
+    uint32_t r = blockIdx.x * W + warp, drawn = share.after(r), nb_rk = kNoVertex;
     Geo g{};
     mtx_meshlet_descriptor d{};
-    uint32_t nb_rk = kNoVertex;
-    auto state_of = [&](uint32_t rr) -> const unsigned char * {
-        return STATE ? state + (uint64_t)rr * pl.state_bytes : nullptr;
-    };
     if (r < count) {
         const uint32_t id = __ldg(ids + r);
-        g = block_geo(id, p, TMA, sizeof(T), dv);
-        tile_issue<T, TMA>(pl, ws, buf, g, &map, state_of(r));
         d = desc[r];
+        g = block_geo(id, p, false, sizeof(T), dv);
         nb_rk = neighbour_rank(p, g, id, rank_map);
     }
     while (r < count) {
-        // prefetch the next block: its tile, descriptor and neighbour ranks
-        const uint32_t rn = r + nw;
-        const bool have_next = rn < count;
-        Geo gn{};
-        mtx_meshlet_descriptor dn{};
-        uint32_t nb_rk_n = kNoVertex;
-        if (have_next) {
-            const uint32_t idn = __ldg(ids + rn);
-            gn = block_geo(idn, p, TMA, sizeof(T), dv);
-            if (pl.nbuf == 2) tile_issue<T, TMA>(pl, ws, buf ^ 1u, gn, &map, state_of(rn));
-            dn = desc[rn];
-            nb_rk_n = neighbour_rank(p, gn, idn, rank_map);
-        }
         const uint32_t nb_vb =
             (nb_rk != kNoVertex && MTX_BC(nb_rk, count, kBcDesc)) ? __ldg(&desc[nb_rk].vertexOffset) : kNoVertex;
-        uint32_t rec[CPL];
-        gather_issue_map<CPL>(p, pl, g, nb_rk, faces, 3 * pl.BB, cmap, rec, block_cap * 3 * pl.BB);
-        if (!tile_wait<T, TMA>(p, pl, ws, buf, g, parity, st)) {
-            if (have_next && pl.nbuf == 2) tile_drain<TMA>(pl, ws, buf ^ 1u, parity);
-            break;
+        const uint32_t miss = __ballot_sync(0xffffffffu, nb_rk == kNoVertex) & 0xfeu;
+        uint32_t rec[N];
+        Ctx8 c8;
+        if (BC == 8) c8 = ctx8_load(faces, nb_rk, edge8, face_words);
+        else if (!BIG) ctx_load<N>(pl, faces, nb_rk, cmap, 0, rec, face_words);
+        // the next block's place, descriptor and neighbour ranks
+        const uint32_t rn = __shfl_sync(0xffffffffu, drawn, 0);
+        drawn = share.after(rn);
+        uint32_t nb_rk_n = kNoVertex;
+        Geo gn{};
+        mtx_meshlet_descriptor dn{};
+        if (rn < count) {
+            const uint32_t idn = __ldg(ids + rn);
+            dn = desc[rn];
+            gn = block_geo(idn, p, false, sizeof(T), dv);
+            nb_rk_n = neighbour_rank(p, gn, idn, rank_map);
         }
-        gather_finish<CPL, CPL == 8>(pl, nb_vb, rec, ws, d.vertexOffset);
-        emit_block<T, GENERIC, false, CPL == 8, STATE>(p, pl, ws, buf, g, d, tab, ntab, owner, indices, tcap,
-                                                       vertices, vcap, vfmt, frame, normals, st, r, cmap);
-        if (!have_next) break;
-        if (pl.nbuf == 1) tile_issue<T, TMA>(pl, ws, buf, gn, &map, state_of(rn));
-        else buf ^= 1u;
+        const uint32_t tbase = d.indexOffset / 3u, nv = d.vertexCount, nt = d.primitiveCount;
+        const bool fits = (uint64_t)tbase + nt <= tcap && !(vertices && (uint64_t)d.vertexOffset + nv > vcap);
+        if (!fits && lane == 0) report(st, MTX_ERR_CAPACITY, kSiteEmitCapacity, r, 2);
+        if (fits && (nt || (vertices && nv))) {
+            const uint32_t *own = state + (uint64_t)r * slot;
+            const bool inner = g.ox + pl.B < p.X && g.oy + pl.B < p.Y && g.oz + pl.B < p.Z;
+            if (BIG) {
+                uint32_t *rows = reinterpret_cast<uint32_t *>(ws + pl.off_rows);
+                for (uint32_t i = lane; i < pl.B1 * pl.B1; i += 32) rows[i] = __ldg(own + i);
+                __syncwarp();
+                list_bits<BC>(p, pl, ws, g);
+            }
+            if (lane < 8) nbase[lane] = lane ? nb_vb : d.vertexOffset;
+
+            // vertices, and this block's entries of the vertex table
+            const uint32_t *rows = reinterpret_cast<const uint32_t *>(ws + pl.off_rows);
+            const uint16_t *list = reinterpret_cast<const uint16_t *>(ws + pl.off_list);
+            ListWalk l;
+            uint32_t vrun = 0, out = 0, ahead = BIG ? 0u : __ldg(own + lane);
+            for (uint32_t s0 = 0; vrun < nv && (BIG || s0 < slot); s0 += 32) {
+                uint32_t e = ahead;
+                if (BIG) {
+                    const uint32_t n = list_next<true>(l, pl, ws);
+                    if (!n) break;
+                    e = lane < n ? listed_cell(p, pl, g, rows, list[l.done + lane], inner) : 0u;
+                    l.done += n;
+                } else if (s0 + 32 < slot) {
+                    ahead = __ldg(own + s0 + 32 + lane);  // past the list's end: not used
+                }
+                if (!BIG && (e & 0xfffu) >= B3) e = 0;  // a list the count pass did not finish (reported there)
+                uint32_t vt;
+                const uint32_t rel = vrun + step_vertices(e >> 28, vt);
+                queue_vertices(pl, e, rel, vtab, jobs);
+                vrun += vt;
+                __syncwarp();
+                if (vertices) {
+                    const uint32_t avail = min(vrun, nv);  // never past the block's vertices
+                    while (avail - out >= (vrun >= nv ? 1u : 32u)) {
+                        const uint32_t k = min(32u, avail - out);
+                        put_vertices<T, GENERIC>(p, pl, g, jobs, out, k, inner, vertices, d.vertexOffset, vfmt,
+                                                 frame, normals);
+                        out += k;
+                    }
+                }
+            }
+            // the context layer's entries
+            if (BC == 8) {
+                ctx8_store(c8, edge8, vtab);
+            } else if (!BIG) {
+                ctx_store<N>(pl, vtab, cmap, 0, rec);
+            } else {
+                for (uint32_t j0 = 0; j0 < pl.nb3; j0 += 32 * N) {
+                    ctx_load<N>(pl, faces, nb_rk, cmap, j0, rec, face_words);
+                    ctx_store<N>(pl, vtab, cmap, j0, rec);
+                }
+            }
+            __syncwarp();
+
+            // triangles: each cell queues its jobs, resolved 32 at a time
+            bool bad = false;
+            uint32_t top = 0;
+            out = 0;
+            l = ListWalk{};
+            ahead = BIG ? 0u : __ldg(own + lane);
+            for (uint32_t s0 = 0; top < nt && (BIG || s0 < slot); s0 += 32) {
+                uint32_t e = ahead;
+                if (BIG) {
+                    const uint32_t n = list_next<true>(l, pl, ws);
+                    if (!n) break;
+                    e = lane < n ? listed_cell(p, pl, g, rows, list[l.done + lane], inner) : 0u;
+                    l.done += n;
+                } else if (s0 + 32 < slot) {
+                    ahead = __ldg(own + s0 + 32 + lane);
+                }
+                if (!BIG && (e & 0xfffu) >= B3) e = 0;
+                const uint32_t f = first[(e >> 12) & 0xffu], n = f >> 12;
+                uint32_t before, total;
+                if (BIG) {
+                    before = warp_excl_scan(n, total);
+                } else {
+                    before = (e >> 20) & 0xffu;
+                    total = __shfl_sync(0xffffffffu, before + n, 31);
+                }
+                const uint32_t cell = e & 0xfffu, q = fdiv(cell, pl.rB), x = cell - q * pl.B;
+                const uint32_t z = fdiv(q, pl.rB), y = q - z * pl.B;
+                const uint32_t end = (x + 1 == pl.B ? 1u << 26 : 0u) | (y + 1 == pl.B ? 1u << 27 : 0u) |
+                                     (z + 1 == pl.B ? 1u << 28 : 0u);
+                const uint32_t job = (((q + z) * pl.B1 + x) << 1) | ((f & 0xfffu) << 16) | end;
+#pragma unroll
+                for (uint32_t t = 0; t < 5; ++t)  // at most five triangles a case
+                    if (t < n) jobs[(top + before + t) & (kJobWin - 1)] = job + (t << 16);
+                top += total;
+                __syncwarp();
+                const uint32_t avail = min(top, nt);  // never past the block's triangles
+                const bool last = top >= nt;
+                while (avail - out >= (last ? 1u : 32u)) {
+                    const uint32_t k = min(32u, avail - out);
+                    put_triangles(vtab_b, tri, jobs, nbase, out, k, indices + 3ull * tbase, miss, bad);
+                    out += k;
+                }
+            }
+            if (vrun != nv || top != nt) bad = true;
+            if (bad) report(st, MTX_ERR_INTERNAL, kSiteEmitNeighbour, r, 3);
+            __syncwarp();
+        }
         r = rn;
-        d = dn;
         g = gn;
+        d = dn;
         nb_rk = nb_rk_n;
     }
     // the CTA that ends last hands out the error code the call's kernels left
@@ -248,47 +353,79 @@ static mtx_status grid_for(mtx_context *c, K kernel, int threads, uint32_t smem,
     return MTX_OK;
 }
 
+// Warps a CTA: threads/32 of the options, else the context's tuning, else the
+// pass's own choice, and no more than the shared memory holds.
+static uint32_t cta_warps(const mtx_context *c, const ExtractArgs &a, uint32_t fixed, uint32_t per_warp,
+                          uint32_t own) {
+    uint32_t W = a.threads ? a.threads / 32 : (c->tuning.extractWarps ? c->tuning.extractWarps : own);
+    W = std::min<uint32_t>(std::max<uint32_t>(W, 1), kMaxWarps);
+    const uint32_t room = c->max_smem_optin > (int)fixed ? (uint32_t)c->max_smem_optin - fixed : 0u;
+    return std::min<uint32_t>(W, std::max<uint32_t>(1, room / per_warp));
+}
+
+template <typename T, bool TMA>
+static auto count_fn(uint32_t B) {
+    switch (B) {
+    case 3: return pmb_count_kernel<T, TMA, 3>;
+    case 4: return pmb_count_kernel<T, TMA, 4>;
+    case 8: return pmb_count_kernel<T, TMA, 8>;
+    case 16: return pmb_count_kernel<T, TMA, 16>;
+    default: return pmb_count_kernel<T, TMA, 0>;
+    }
+}
+
 template <typename T>
-static mtx_status run_count(mtx_context *c, const Problem &p, const ExtractArgs &a, const CUtensorMap &map, bool tma,
-                            uint32_t W, cudaStream_t s) {
-    const WPlan pl = make_wplan(p.B, sizeof(T), tma, false, kSingleBuffer, p.B <= 8);
-    const uint32_t smem = kTableBytes + W * pl.bytes;
-    auto k = tma ? (p.B == 8 ? pmb_count_kernel<T, true, 8> : pmb_count_kernel<T, true, 0>)
-                 : pmb_count_kernel<T, false, 0>;
+static mtx_status run_count(mtx_context *c, const Problem &p, const ExtractArgs &a, cudaStream_t s) {
+    const uint32_t staging = a.staging ? a.staging : c->tuning.staging;
+    const bool tma = use_tma(p, staging);
+    CUtensorMap map;
+    memset(&map, 0, sizeof(map));
+    if (tma) {
+        const mtx_status rs = make_volume_tensor_map(c, p, tile_pitch(p.B, sizeof(T), true), &map);
+        if (rs != MTX_OK) return rs;
+    }
+    // the tile's element offsets in shared memory, where they fit 32 bits and B <= 8 keeps them small
+    const bool use_off = !tma && p.B <= 8 && (uint64_t)(p.B + 1) * p.X * p.Y < (1ull << 32);
+    const WPlan pl = make_count_plan(p.B, sizeof(T), tma);
+    const uint32_t fixed = count_fixed_bytes(p.B, use_off), W = cta_warps(c, a, fixed, pl.bytes, 4);
+    const uint32_t smem = fixed + W * pl.bytes;
+    auto k = tma ? count_fn<T, true>(p.B) : count_fn<T, false>(p.B);
     unsigned grid;
     mtx_status r = grid_for(c, k, W * 32, smem, a.host_count, W, grid);
     if (r != MTX_OK) return r;
     k<<<grid, W * 32, smem, s>>>(p, map, a.ids, a.count, a.desc, a.desc_capacity, a.faces, a.state, a.totals,
                                  a.cell_cases, a.block_capacity, &c->ctrl->status, (uint64_t *)c->count_status.ptr,
-                                 scan_tiles(std::min(a.block_capacity, a.desc_capacity)), &c->ctrl->count_ticket);
+                                 scan_tiles(std::min(a.block_capacity, a.desc_capacity)), &c->ctrl->count_ticket,
+                                 use_off);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(c, e, "count launch");
     return MTX_OK;
 }
 
-template <typename T, int CPL, bool TMA, int BC = 0>
-static void (*emit_fn(bool generic))(Problem, CUtensorMap, const uint32_t *, const uint32_t *, const uint32_t *,
-                                     const mtx_meshlet_descriptor *, const uint32_t *, const uint8_t *, uint32_t *,
-                                     uint64_t, uint64_t, void *, uint64_t, uint32_t, uint32_t, uint32_t, DevStatus *,
-                                     uint32_t *, uint32_t *) {
-    return generic ? pmb_emit_kernel<T, CPL, TMA, true, BC> : pmb_emit_kernel<T, CPL, TMA, false, BC>;
+template <typename T, bool GENERIC>
+static auto emit_fn(uint32_t B) {
+    switch (B) {
+    case 3: return pmb_emit_kernel<T, GENERIC, 3, false>;
+    case 4: return pmb_emit_kernel<T, GENERIC, 4, false>;
+    case 8: return pmb_emit_kernel<T, GENERIC, 8, false>;
+    case 16: return pmb_emit_kernel<T, GENERIC, 16, true>;
+    default: return B <= 8 ? pmb_emit_kernel<T, GENERIC, 0, false> : pmb_emit_kernel<T, GENERIC, 0, true>;
+    }
 }
 
 template <typename T>
-static mtx_status run_emit(mtx_context *c, const Problem &p, const ExtractArgs &a, const CUtensorMap &map, bool tma,
-                           uint32_t W, cudaStream_t s) {
-    const WPlan pl = make_wplan(p.B, sizeof(T), tma, true, kSingleBuffer);
-    const uint32_t smem = cta_fixed_bytes(p.B, true) + W * pl.bytes;
+static mtx_status run_emit(mtx_context *c, const Problem &p, const ExtractArgs &a, cudaStream_t s) {
+    const WPlan pl = make_emit_plan(p.B);
+    const uint32_t fixed = emit_fixed_bytes(p.B), W = cta_warps(c, a, fixed, pl.bytes, 8);
+    const uint32_t smem = fixed + W * pl.bytes;
     const bool generic = a.vertices && (a.vertex_format != MTX_VERTEX_XYZ || a.frame != MTX_FRAME_VOXEL);
-    auto k = p.B == 8 && tma ? emit_fn<T, 8, true, 8>(generic)
-             : p.B <= 8    ? (tma ? emit_fn<T, 8, true>(generic) : emit_fn<T, 8, false>(generic))
-                           : (tma ? emit_fn<T, 32, true>(generic) : emit_fn<T, 32, false>(generic));
+    auto k = generic ? emit_fn<T, true>(p.B) : emit_fn<T, false>(p.B);
     unsigned grid;
     mtx_status r = grid_for(c, k, W * 32, smem, a.host_count, W, grid);
     if (r != MTX_OK) return r;
-    k<<<grid, W * 32, smem, s>>>(p, map, a.ids, a.rank_map, a.count, a.desc, a.faces, a.state, a.indices,
-                                 a.tri_capacity, a.block_capacity, a.vertices, a.vertex_capacity, a.vertex_format,
-                                 a.frame, a.normals, &c->ctrl->status, &c->ctrl->emit_done, a.status_out);
+    k<<<grid, W * 32, smem, s>>>(p, a.ids, a.rank_map, a.count, a.desc, a.faces, a.state, a.indices, a.tri_capacity,
+                                 a.block_capacity, a.vertices, a.vertex_capacity, a.vertex_format, a.frame, a.normals,
+                                 &c->ctrl->status, &c->ctrl->emit_done, a.status_out, &c->ctrl->emit_ticket);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(c, e, "emit launch");
     return MTX_OK;
@@ -297,41 +434,25 @@ static mtx_status run_emit(mtx_context *c, const Problem &p, const ExtractArgs &
 template <bool EMIT>
 static mtx_status launch_stage(mtx_context *c, const Problem &p, const ExtractArgs &a, cudaStream_t s) {
     if (p.B < 2 || p.B > MTX_MAX_BLOCK_EDGE) return fail(c, MTX_ERR_UNSUPPORTED, "block edge must be in [2, 16]");
-    mtx_status rs = load_case_tables(c);
+    mtx_status rs = load_list_tables(c);
     if (rs != MTX_OK) return rs;
-    const uint32_t staging = a.staging ? a.staging : c->tuning.staging;
-    const bool tma = use_tma(p, staging);
-    CUtensorMap map;
-    memset(&map, 0, sizeof(map));
-    if (tma) {
-        rs = make_volume_tensor_map(c, p, tile_pitch(p.B, dtype_size(p.dtype), true), &map);
-        if (rs != MTX_OK) return rs;
-    }
-    // warps per CTA: threads/32 of the options, else the context's tuning, else 4
-    uint32_t W = a.threads ? a.threads / 32 : (c->tuning.extractWarps ? c->tuning.extractWarps : 4);
-    W = std::min<uint32_t>(std::max<uint32_t>(W, 1), kMaxWarps);
-    // no more warps than the shared memory holds (16^3 float tiles fit 7, not 8)
-    const WPlan pl = make_wplan(p.B, dtype_size(p.dtype), tma, EMIT, kSingleBuffer, p.B <= 8);
-    // the emit pass with TMA and B <= 8 reads the block state the count pass wrote
-    if (EMIT && tma && pl.state_bytes && !a.state) return fail(c, MTX_ERR_INTERNAL, "emit without block state");
-    const uint32_t fixed = cta_fixed_bytes(p.B, EMIT);
-    const uint32_t room = c->max_smem_optin > (int)fixed ? (uint32_t)c->max_smem_optin - fixed : 0u;
-    W = std::min<uint32_t>(W, std::max<uint32_t>(1, room / pl.bytes));
     switch (p.dtype) {
-    case MTX_DTYPE_U8: return EMIT ? run_emit<uint8_t>(c, p, a, map, tma, W, s) : run_count<uint8_t>(c, p, a, map, tma, W, s);
-    case MTX_DTYPE_U16: return EMIT ? run_emit<uint16_t>(c, p, a, map, tma, W, s) : run_count<uint16_t>(c, p, a, map, tma, W, s);
-    default: return EMIT ? run_emit<float>(c, p, a, map, tma, W, s) : run_count<float>(c, p, a, map, tma, W, s);
+    case MTX_DTYPE_U8: return EMIT ? run_emit<uint8_t>(c, p, a, s) : run_count<uint8_t>(c, p, a, s);
+    case MTX_DTYPE_U16: return EMIT ? run_emit<uint16_t>(c, p, a, s) : run_count<uint16_t>(c, p, a, s);
+    default: return EMIT ? run_emit<float>(c, p, a, s) : run_count<float>(c, p, a, s);
     }
 }
 
-uint32_t block_state_bytes(uint32_t B) { return make_wplan(B, 2, true, false, kSingleBuffer, B <= 8).state_bytes; }
+size_t block_state_bytes(uint32_t B) { return 4 * (size_t)list_state_words(B); }
+size_t face_record_bytes(uint32_t B) { return 2 * (size_t)face_stride16(B); }
 
 // The scan over up to `capacity` descriptors, behind a kernel that ran scan_reset for it.
 static mtx_status run_scan(mtx_context *c, mtx_meshlet_descriptor *desc, const uint32_t *count, uint64_t capacity,
                            uint32_t *totals, uint32_t skip, cudaStream_t s) {
     pmb_scan_kernel<<<scan_tiles(capacity), kScanThreads, 0, s>>>(desc, count, (uint64_t *)c->count_status.ptr,
                                                                   &c->ctrl->count_ticket, totals, &c->ctrl->status,
-                                                                  c->wait_polls ? c->wait_polls : kSpinLimit, skip);
+                                                                  c->wait_polls ? c->wait_polls : kSpinLimit, skip,
+                                                                  &c->ctrl->emit_ticket);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(c, e, "scan launch");
     return MTX_OK;

@@ -239,17 +239,6 @@ __device__ __forceinline__ void tma_load_3d(void *smem_dst, const CUtensorMap *m
         : "memory");
 }
 
-// Untiled bulk copy (no multicast) of `bytes` from global to shared memory,
-// completing on the mbarrier; both addresses 16-byte aligned, bytes a
-// multiple of 16.
-__device__ __forceinline__ void bulk_load(void *smem_dst, const void *src, uint32_t bytes, uint64_t *bar) {
-    asm volatile(
-        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-            smem_u32(smem_dst)),
-        "l"((uint64_t)src), "r"(bytes), "r"(smem_u32(bar))
-        : "memory");
-}
-
 __device__ __forceinline__ void prefetch_tensormap(const CUtensorMap *map) {
     asm volatile("prefetch.tensormap [%0];" ::"l"((uint64_t)map) : "memory");
 }

@@ -22,7 +22,8 @@ struct Ctrl {
     uint32_t batch_ticket[4];
     uint32_t pyr_done;       // octree tiles finished (the last one builds the top levels)
     uint32_t emit_done;      // CTAs of the emit pass finished (the last one writes status_out)
-    uint32_t pad1[2];
+    uint32_t emit_ticket;    // emit pass: blocks handed out by ticket (zeroed by the scan pass)
+    uint32_t pad1;
 };
 
 // A grow-only device allocation owned by the context.
@@ -153,8 +154,8 @@ struct ExtractArgs {
     uint32_t host_count;        // > 0 when the host knows it (sizes the grid), else 0
     mtx_meshlet_descriptor *desc;  // per active block {vbase, 3*tbase, nv, nt}
     uint64_t desc_capacity;
-    uint32_t *faces;            // 3*B*B words per active block
-    uint8_t *state;             // block_state_bytes(B) per active block (count -> emit), B <= 8
+    uint16_t *faces;            // face_record_bytes(B) per active block
+    uint32_t *state;            // block_state_bytes(B) per active block (count -> emit)
     uint64_t block_capacity;    // active blocks that desc/faces/state can hold
     uint32_t *totals;           // device uint32[4] {vertexCount, indexCount, meshletCount, activeCount}
     uint32_t *status_out;       // optional device word: the context's error code when the emit pass is done
@@ -166,8 +167,10 @@ struct ExtractArgs {
     uint32_t vertex_format, frame, normals, staging, threads;
 };
 mtx_status launch_count(mtx_context *c, const Problem &p, const ExtractArgs &a, cudaStream_t s);
-// Bytes of the block state the count pass hands to the emit pass (0: none, B > 8).
-uint32_t block_state_bytes(uint32_t B);
+// Bytes an active block takes of the state the count pass hands to the emit
+// pass, and of its face records.
+size_t block_state_bytes(uint32_t B);
+size_t face_record_bytes(uint32_t B);
 // The descriptor scan alone over *count descriptors (capacity bounds them); the
 // kernel before it in the stream zeroes the scan's words (scan_reset).
 mtx_status desc_scan_words(mtx_context *c, uint64_t capacity, uint64_t **words, uint32_t *tiles, uint32_t **ticket);

@@ -32,14 +32,11 @@ __host__ __device__ inline WPlan make_wplan_balanced(uint32_t B) {
     p.nb3 = 3 * B * B + 3 * B + 1;
     p.rB = (uint32_t)((0x100000000ull + B - 1) / B);
     p.rB1 = (uint32_t)((0x100000000ull + B) / (B + 1));
-    p.rBB = (uint32_t)((0x100000000ull + B * B - 1) / (B * B));
-    p.R = 32 / B;
     p.PX = B + 1;
     const uint32_t T3 = p.B1 * p.B1 * p.B1;
     p.tile_bytes = 4 * T3;
-    p.nbuf = 1;
     uint32_t o = 0;
-    p.off_tile[0] = p.off_tile[1] = o;
+    p.off_tile = o;
     p.off_vtab = o;  // the vertex table replaces the tile (same size)
     o = align_up(o + p.tile_bytes, 16);
     p.off_bar = 0;   // unused: tiles are staged by plain loads
@@ -54,8 +51,8 @@ __host__ __device__ inline WPlan make_wplan_balanced(uint32_t B) {
     p.off_jobs = o;
     o = align_up(o + 4 * kRing, 16);
     p.off_vp = p.off_jobs;  // 4 * BB <= 4 * kRing for B <= 16
-    p.off_tp = p.off_tile[0];  // the count phase's triangle prefixes: the tile is dead there
-    p.off_nvid = p.off_nm = 0;  // unused
+    p.off_tp = p.off_tile;  // the count phase's triangle prefixes: the tile is dead there
+    p.off_nvid = 0;  // unused
     p.bytes = o;
     return p;
 }
@@ -77,7 +74,7 @@ __device__ __forceinline__ void tile_load_rows_from(const Problem &p, const WPla
     // per-load branch, 34.6 ms)
     constexpr uint32_t kLdgBatch = 4;
     const S *vol = reinterpret_cast<const S *>(p.vol);
-    float *tile = reinterpret_cast<float *>(ws + pl.off_tile[0]);
+    float *tile = reinterpret_cast<float *>(ws + pl.off_tile);
     uint32_t *words = reinterpret_cast<uint32_t *>(ws + pl.off_list);
     uint32_t *rows = reinterpret_cast<uint32_t *>(ws + pl.off_rows);
     const uint32_t lane = threadIdx.x & 31, B1 = pl.B1, n = B1 * B1 * B1, nw = (n + 31) / 32;
@@ -191,7 +188,7 @@ __device__ __forceinline__ uint32_t listed_case(const WPlan &pl, const uint32_t 
 __device__ __forceinline__ void block_counts_balanced(const Problem &p, const WPlan &pl, unsigned char *ws,
                                                       const Geo &g, const uint8_t *ntab, bool want_tris,
                                                       uint32_t &nv, uint32_t &nt) {
-    block_counts(p, pl, ws, g, ntab, want_tris, nullptr, nv, nt);
+    block_counts(p, pl, ws, g, ntab, want_tris, nv, nt);
     if (!want_tris) nt = 0;
 }
 
@@ -204,7 +201,7 @@ __device__ __forceinline__ void count_block_balanced(const Problem &p, const WPl
     uint32_t bnv, bnt;
     block_counts_balanced(p, pl, ws, g, ntab, true, bnv, bnt);
     if (lane == 0) *reinterpret_cast<uint2 *>(&dr->vertexCount) = make_uint2(bnv, bnt);
-    write_face_records<false>(pl, ws, fr);
+    write_face_records(pl, ws, fr);
 }
 
 // ---------------------------------------------------------- vertex table
@@ -296,7 +293,7 @@ __device__ __forceinline__ void resolve_vertices(const Problem &p, const WPlan &
                                                  uint32_t done, uint32_t n, uint32_t vbase, void *vertices,
                                                  uint32_t vfmt, uint32_t frame, uint32_t normals) {
     const uint32_t lane = threadIdx.x & 31, B1 = pl.B1;
-    const float *tile = reinterpret_cast<const float *>(ws + pl.off_tile[0]);
+    const float *tile = reinterpret_cast<const float *>(ws + pl.off_tile);
     const uint32_t *jobs = reinterpret_cast<const uint32_t *>(ws + pl.off_jobs);
     const bool xyz = !GENERIC || vfmt == MTX_VERTEX_XYZ;
     if (lane < n) {

@@ -1,8 +1,8 @@
 // Device building blocks of the PMB marching-cubes passes, shared by the
-// single-volume kernels (extract.cu) and the batched kernel (batched.cu):
-// per-warp shared-memory plans, tile staging, inside bitmasks, PMB edge
-// ownership by bit operations, the per-block count and emit bodies, and the
-// decoupled look-back used by the scans.
+// single-volume kernels (extract.cu), the batched kernel (batched.cu) and the
+// adjoint: per-warp shared-memory plans, tile staging, inside bitmasks, PMB
+// edge ownership by bit operations, and the decoupled look-back used by the
+// scans.
 //
 // Output order is canonical and equals the CPU oracle's: vertices by (block
 // rank, owner voxel x-fastest in the block, axis x<y<z); triangles by (block
@@ -41,22 +41,13 @@ constexpr int kMaxWarps = 8;                        // warps per CTA of the extr
 
 __host__ __device__ inline uint32_t align_up(uint32_t v, uint32_t a) { return (v + a - 1) / a * a; }
 
-// Bytes of a CTA's shared memory before its warps' regions: the case tables,
-// and for the emit pass the context-layer map (ctx_map_entry, one word per
-// voxel of the (B+1)^3 context outside the block).
-__host__ __device__ inline uint32_t cta_fixed_bytes(uint32_t B, bool emit) {
-    return kTableBytes + (emit ? align_up(4 * (3 * B * B + 3 * B + 1), 128) : 0u);
-}
-
 // ------------------------------------------------------- per-warp smem plan
 struct WPlan {
-    uint32_t B, B1, BB, PX, nbuf, nb3;
-    uint32_t rB, rB1, rBB;  // ceil(2^32 / d) reciprocals: n / d == __umulhi(n, r) for the sizes used here
-    uint32_t R;             // block rows walked per round of 32 lanes (32 / B)
-    uint32_t off_tile[2], off_bar, off_rows, off_cross, off_vp, off_tp, off_nvid, off_nm, off_jobs;
-    uint32_t off_case, off_mm;  // case byte of each mixed cell, mixed-cell mask of each cell row (kept)
-    uint32_t state_bytes;       // block state handed from count to emit (B <= 8): [off_cross, off_mm + 2BB)
-    uint32_t off_vtab, off_vmsk, off_list;  // balanced bodies only (pmb_balanced.cuh)
+    uint32_t B, B1, BB, PX, nb3;
+    uint32_t rB, rB1;  // ceil(2^32 / d) reciprocals: n / d == __umulhi(n, r) for the sizes used here
+    uint32_t off_tile, off_bar, off_rows, off_cross, off_vp, off_tp, off_nvid, off_jobs;
+    uint32_t off_case, off_mm;             // pmb_lists.cuh: face records and bitstream, list bits
+    uint32_t off_vtab, off_vmsk, off_list;
     uint32_t bytes;       // per warp
     uint32_t tile_bytes;  // one tile (the TMA transaction size)
 };
@@ -71,12 +62,9 @@ __host__ __device__ inline uint32_t tile_pitch(uint32_t B, uint32_t esz, bool tm
     return align_up(xoff_max + B + 1, A);
 }
 
-// tri_pass: the emit pass's plan.  keep: room for the case bytes and mixed
-// masks (always in the emit pass); for B <= 8 the count pass keeps them too
-// and hands the block state -- crossing rows, row prefixes, case bytes and
-// mixed masks, one contiguous range -- to the emit pass through global memory.
-__host__ __device__ inline WPlan make_wplan(uint32_t B, uint32_t esz, bool tma, bool tri_pass,
-                                            bool single_buffer = false, bool keep = false) {
+// A warp's shared memory for a float tile staged by plain loads, its inside
+// rows, crossing rows and row prefixes (the adjoint).
+__host__ __device__ inline WPlan make_wplan(uint32_t B) {
     WPlan p{};
     p.B = B;
     p.B1 = B + 1;
@@ -84,46 +72,15 @@ __host__ __device__ inline WPlan make_wplan(uint32_t B, uint32_t esz, bool tma, 
     p.nb3 = 3 * B * B + 3 * B + 1;  // voxels of the (B+1)^3 context outside the block
     p.rB = (uint32_t)((0x100000000ull + B - 1) / B);
     p.rB1 = (uint32_t)((0x100000000ull + B) / (B + 1));
-    p.rBB = (uint32_t)((0x100000000ull + B * B - 1) / (B * B));
-    p.R = 32 / B;
-    p.PX = tile_pitch(B, esz, tma);
-    p.tile_bytes = p.PX * p.B1 * p.B1 * esz;
-    p.nbuf = (p.tile_bytes <= 4096 && !single_buffer) ? 2 : 1;
-    // the emit pass puts its vertex table (build_utab, B <= 8) in the tile's slot
-    const uint32_t slot = (tri_pass && B <= 8) ? std::max(p.tile_bytes, 3 * p.B1 * p.B1 * p.B1) : p.tile_bytes;
-    uint32_t o = 0;
-    for (uint32_t b = 0; b < 2; ++b) {  // a TMA destination is 128-byte aligned; what follows the last, 16
-        p.off_tile[b] = o;
-        if (b < p.nbuf) o = align_up(o + slot, b + 1 < p.nbuf ? 128 : 16);
-    }
-    if (p.nbuf == 1) p.off_tile[1] = p.off_tile[0];
-    p.off_bar = o;
-    o += 16;
-    if (tri_pass && B <= 8) o += 32;  // first vertex of the block and of its seven +x/+y/+z neighbours (emit)
+    p.PX = B + 1;
+    p.tile_bytes = 4 * p.PX * p.B1 * p.B1;
+    uint32_t o = align_up(p.tile_bytes, 16);
     p.off_rows = o;
-    // the emit pass with TMA and B <= 8 takes the count pass's block state and builds no rows
-    if (!(tri_pass && tma && B <= 8)) o = align_up(o + 4 * p.B1 * p.B1, 16);
+    o = align_up(o + 4 * p.B1 * p.B1, 16);
     p.off_cross = o;
     o = align_up(o + 12 * p.BB, 16);
     p.off_vp = o;
     o = align_up(o + 4 * p.BB, 16);
-    p.off_tp = o;
-    o = align_up(o + 4 * p.BB, 16);
-    if (tri_pass || keep) {
-        p.off_case = o;
-        o = align_up(o + B * B * B, 16);
-        p.off_mm = o;
-        o = align_up(o + 2 * B * B, 16);
-        p.state_bytes = B <= 8 ? o - p.off_cross : 0u;
-    }
-    if (tri_pass) {  // context first vertices: 16-bit packed entries for B <= 8 (gather_finish<CPL, true>)
-        p.off_nvid = o;
-        o = align_up(o + (B <= 8 ? 2 : 4) * p.nb3, 16);
-        p.off_nm = o;  // owned-edge masks (B > 8; packed into the entries for B <= 8)
-        if (B > 8) o = align_up(o + p.nb3, 16);
-    }
-    p.off_jobs = o;  // a window of packed jobs (triangles or vertices) in output order: the emit pass only
-    if (tri_pass) o = align_up(o + 4 * kJobWin, 16);
     p.bytes = align_up(o, 128);
     return p;
 }
@@ -188,64 +145,30 @@ __device__ __forceinline__ Geo block_geo(uint32_t id, const Problem &p, bool tma
 }
 
 // ----------------------------------------------------------- warp tiles
-// Starts the load of a block's (B+1)^3 tile into buffer `buf`.  TMA: lane 0
-// issues one cp.async.bulk.tensor (zero fill outside the volume).  Plain
-// loads are done in tile_wait instead.
-// state: also bring the block's state (pl.state_bytes from global memory)
-// into [off_cross, ...) on the same barrier (TMA only).
-template <typename T, bool TMA>
-__device__ __forceinline__ void tile_issue(const WPlan &pl, unsigned char *ws, uint32_t buf, const Geo &g,
-                                           const CUtensorMap *map, const unsigned char *state = nullptr) {
-    if (!TMA) return;
+// Starts the TMA load of a block's (B+1)^3 tile (zero fill outside the volume):
+// lane 0 issues one cp.async.bulk.tensor.
+template <typename T>
+__device__ __forceinline__ void tile_issue(const WPlan &pl, unsigned char *ws, const Geo &g, const CUtensorMap *map) {
     __syncwarp();
     if ((threadIdx.x & 31) == 0) {
-        uint64_t *bar = reinterpret_cast<uint64_t *>(ws + pl.off_bar) + buf;
-        fence_proxy_async();  // earlier generic reads of this buffer come first
-        mbar_arrive_expect_tx(bar, pl.tile_bytes + (state ? pl.state_bytes : 0u));
-        tma_load_3d(ws + pl.off_tile[buf], map, bar, (int)(g.ox - g.xoff), (int)g.oy, (int)g.oz);
-        if (state) bulk_load(ws + pl.off_cross, state, pl.state_bytes, bar);
+        uint64_t *bar = reinterpret_cast<uint64_t *>(ws + pl.off_bar);
+        fence_proxy_async();  // earlier generic reads of the tile come first
+        mbar_arrive_expect_tx(bar, pl.tile_bytes);
+        tma_load_3d(ws + pl.off_tile, map, bar, (int)(g.ox - g.xoff), (int)g.oy, (int)g.oz);
     }
 }
 
-template <typename T, bool TMA>
-__device__ __forceinline__ bool tile_wait(const Problem &p, const WPlan &pl, unsigned char *ws, uint32_t buf,
-                                          const Geo &g, uint32_t &parity, DevStatus *st) {
-    if (TMA) {
-        uint64_t *bar = reinterpret_cast<uint64_t *>(ws + pl.off_bar) + buf;
-        const bool ok = mbar_wait_bounded(bar, (parity >> buf) & 1u);
-        if (!__all_sync(0xffffffffu, ok)) {
-            if ((threadIdx.x & 31) == 0) report(st, MTX_ERR_TIMEOUT, kSiteTmaWait, g.ox, g.oy);
-            // give the copy in flight one more bounded wait before the warp leaves
-            mbar_wait_bounded(bar, (parity >> buf) & 1u);
-            parity ^= 1u << buf;
-            return false;
-        }
-        parity ^= 1u << buf;
-        return true;
+__device__ __forceinline__ bool tile_wait(const WPlan &pl, unsigned char *ws, const Geo &g, uint32_t &parity,
+                                          DevStatus *st) {
+    uint64_t *bar = reinterpret_cast<uint64_t *>(ws + pl.off_bar);
+    const bool ok = mbar_wait_bounded(bar, parity);
+    if (!__all_sync(0xffffffffu, ok)) {
+        if ((threadIdx.x & 31) == 0) report(st, MTX_ERR_TIMEOUT, kSiteTmaWait, g.ox, g.oy);
+        // give the copy in flight one more bounded wait before the warp leaves
+        mbar_wait_bounded(bar, parity);
+        return false;
     }
-    // plain loads, kLdgBatch per lane in flight before any is stored
-    constexpr uint32_t kLdgBatch = 8;
-    T *tile = reinterpret_cast<T *>(ws + pl.off_tile[buf]);
-    const T *vol = reinterpret_cast<const T *>(p.vol);
-    const uint32_t n = pl.B1 * pl.B1 * pl.B1;
-    for (uint32_t i0 = 0; i0 < n; i0 += 32 * kLdgBatch) {
-        T v[kLdgBatch];
-        uint32_t dst[kLdgBatch];
-#pragma unroll
-        for (uint32_t k = 0; k < kLdgBatch; ++k) {
-            const uint32_t i = i0 + k * 32 + (threadIdx.x & 31);
-            const uint32_t iq = fdiv(i, pl.rB1);
-            const uint32_t x = i - iq * pl.B1, z = fdiv(iq, pl.rB1), y = iq - z * pl.B1;
-            const uint32_t gx = g.ox + x, gy = g.oy + y, gz = g.oz + z;
-            v[k] = T(0);
-            dst[k] = i < n ? (z * pl.B1 + y) * pl.PX + x : 0xffffffffu;
-            if (i < n && gx < p.X && gy < p.Y && gz < p.Z) v[k] = __ldg(vol + ((uint64_t)gz * p.Y + gy) * p.X + gx);
-        }
-#pragma unroll
-        for (uint32_t k = 0; k < kLdgBatch; ++k)
-            if (dst[k] != 0xffffffffu && MTX_BC(dst[k], pl.PX * pl.B1 * pl.B1, kBcTile)) tile[dst[k]] = v[k];
-    }
-    __syncwarp();
+    parity ^= 1u;
     return true;
 }
 
@@ -284,23 +207,12 @@ __device__ __forceinline__ void tile_load_float(const Problem &p, const WPlan &p
     else tile_load_float_from<float>(p, pl, tile, g);
 }
 
-// Waits (bounded) for a prefetched tile that will not be used, so that no
-// copy into this warp's shared memory is in flight when it leaves.
-template <bool TMA>
-__device__ __forceinline__ void tile_drain(const WPlan &pl, unsigned char *ws, uint32_t buf, uint32_t &parity) {
-    if (!TMA) return;
-    uint64_t *bar = reinterpret_cast<uint64_t *>(ws + pl.off_bar) + buf;
-    mbar_wait_bounded(bar, (parity >> buf) & 1u);
-    parity ^= 1u << buf;
-}
-
 // Inside bitmask of every tile row: bit x <=> voxel at or below iso and inside
 // the volume.  Integer voxels compare against floor(iso); rows that start on a
 // 4-byte boundary are tested 2 (uint16) or 4 (uint8) voxels per instruction.
 template <typename T>
-__device__ __forceinline__ void build_rows(const Problem &p, const WPlan &pl, unsigned char *ws, uint32_t buf,
-                                           const Geo &g) {
-    const T *tile = reinterpret_cast<const T *>(ws + pl.off_tile[buf]);
+__device__ __forceinline__ void build_rows(const Problem &p, const WPlan &pl, unsigned char *ws, const Geo &g) {
+    const T *tile = reinterpret_cast<const T *>(ws + pl.off_tile);
     uint32_t *rows = reinterpret_cast<uint32_t *>(ws + pl.off_rows);
     const uint32_t xin = min(pl.B1, p.X - g.ox);
     const uint32_t xmask = (1u << xin) - 1u;  // xin <= 17
@@ -402,13 +314,10 @@ __device__ __forceinline__ uint32_t mixed_cells(const Problem &p, const WPlan &p
 
 // Per-row crossing masks, vertex prefixes and (want_tris) triangle prefixes,
 // and the block's vertex/triangle counts.  Lane l owns rows [l*R, l*R + R) so
-// that the row prefixes follow from one warp scan.  Optionally writes the
-// per-cell case bytes (cases_out: every cell, 0 / 255 for cells that are not
-// mixed) and keeps, in the warp's shared memory, the mixed-cell mask of each
-// cell row and the case byte of each mixed cell (keep: the emit pass).
+// that the row prefixes follow from one warp scan. 
 __device__ __forceinline__ void block_counts(const Problem &p, const WPlan &pl, unsigned char *ws, const Geo &g,
-                                             const uint8_t *ntab, bool want_tris, uint8_t *cases_out,
-                                             uint32_t &nv, uint32_t &nt, bool keep = false) {
+                                             const uint8_t *ntab, bool want_tris, uint32_t &nv,
+                                             uint32_t &nt) {
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t *rows = reinterpret_cast<const uint32_t *>(ws + pl.off_rows);
     uint32_t *cross = reinterpret_cast<uint32_t *>(ws + pl.off_cross);
@@ -432,9 +341,6 @@ __device__ __forceinline__ void block_counts(const Problem &p, const WPlan &pl, 
             tp[q] = stri;
             uint32_t inside;
             uint32_t mm = mixed_cells(p, pl, g, rows, y, z, inside);
-            if (cases_out)
-                for (uint32_t x = 0; x < B; ++x) cases_out[q * B + x] = ((inside >> x) & 1u) ? 255 : 0;
-            if (keep) reinterpret_cast<uint16_t *>(ws + pl.off_mm)[q] = (uint16_t)mm;
             // the four rows of the cell row, read once for all its mixed cells
             const uint32_t r00 = mm ? rows[z * pl.B1 + y] : 0u, r01 = mm ? rows[z * pl.B1 + y + 1] : 0u;
             const uint32_t r10 = mm ? rows[(z + 1) * pl.B1 + y] : 0u, r11 = mm ? rows[(z + 1) * pl.B1 + y + 1] : 0u;
@@ -445,9 +351,6 @@ __device__ __forceinline__ void block_counts(const Problem &p, const WPlan &pl, 
                 const uint32_t cfg = (a & 3u) | ((b & 2u) << 1) | ((b & 1u) << 3) | ((c & 3u) << 4) | ((e & 2u) << 5) |
                                      ((e & 1u) << 7);
                 stri += ntab[cfg];
-                if (!MTX_BC(q * B + x, B * BB, kBcRows)) continue;
-                if (cases_out) cases_out[q * B + x] = (uint8_t)cfg;
-                if (keep) ws[pl.off_case + q * B + x] = (uint8_t)cfg;
             }
         }
     }
@@ -463,11 +366,6 @@ __device__ __forceinline__ void block_counts(const Problem &p, const WPlan &pl, 
     __syncwarp();
     nv = tv;
     nt = tt;
-}
-
-// Owned-edge mask of voxel (x, y, z) of the block, from the crossing rows.
-__device__ __forceinline__ uint32_t voxel_mask(const uint32_t *cross, uint32_t BB, uint32_t q, uint32_t x) {
-    return ((cross[q] >> x) & 1u) | (((cross[BB + q] >> x) & 1u) << 1) | (((cross[2 * BB + q] >> x) & 1u) << 2);
 }
 
 // Block-relative index of the first vertex owned by voxel (x, y, z).
@@ -568,103 +466,9 @@ __device__ __forceinline__ float3 vertex_pos(const Problem &p, const WPlan &pl, 
 }
 
 
-// Writes the block's own vertices (vbase .. vbase + nv) in canonical order.
-// Each lane walks the cut edges of its rows and writes one job per vertex
-// (voxel index | axis << 12) at the vertex's own position in a window of
-// kJobWin jobs; the warp then resolves the window 32 vertices at a time, one
-// per lane, each lane storing its own vertex record.
-// GENERIC selects the VertexData / NDC / normals options; the plain form
-// writes xyz in the voxel frame.  ANY: the tile holds the voxels converted to
-// T = float and the volume's own dtype is p.dtype (used for the normals).
-template <typename T, bool GENERIC, bool ANY = false>
-__device__ __forceinline__ void emit_vertices(const Problem &p, const WPlan &pl, unsigned char *ws, uint32_t buf,
-                                              const Geo &g, uint32_t vbase, uint32_t nv, void *vertices, uint32_t vfmt,
-                                              uint32_t frame, uint32_t normals) {
-    const uint32_t lane = threadIdx.x & 31;
-    const uint32_t B = pl.B, BB = pl.BB, R = (BB + 31) / 32;
-    const uint32_t *cross = reinterpret_cast<const uint32_t *>(ws + pl.off_cross);
-    const uint32_t *vp = reinterpret_cast<const uint32_t *>(ws + pl.off_vp);
-    const T *tile = reinterpret_cast<const T *>(ws + pl.off_tile[buf]);
-    uint32_t *jobs = reinterpret_cast<uint32_t *>(ws + pl.off_jobs);
-    const bool xyz = !GENERIC || vfmt == MTX_VERTEX_XYZ;
-    for (uint32_t w0 = 0; w0 < nv; w0 += kJobWin) {
-        const uint32_t w1 = w0 + kJobWin;
-        if (nv <= kJobWin) {  // one window (the common case): no window checks
-            for (uint32_t k = 0; k < R; ++k) {
-                const uint32_t q = lane * R + k;
-                if (q >= BB) break;
-                const uint32_t xc = cross[q], yc = cross[BB + q], zc = cross[2 * BB + q];
-                uint32_t j = vp[q], any = xc | yc | zc;
-                while (any) {
-                    const uint32_t x = __ffs(any) - 1;
-                    any &= any - 1u;
-                    const uint32_t base = (q * B + x);
-                    if ((xc >> x) & 1u) jobs[j++] = base;
-                    if ((yc >> x) & 1u) jobs[j++] = base | (1u << 12);
-                    if ((zc >> x) & 1u) jobs[j++] = base | (2u << 12);
-                }
-            }
-        } else {
-            for (uint32_t k = 0; k < R; ++k) {
-                const uint32_t q = lane * R + k;
-                if (q >= BB) break;
-                const uint32_t xc = cross[q], yc = cross[BB + q], zc = cross[2 * BB + q];
-                uint32_t j = vp[q];
-                if (j >= w1 || j + __popc(xc) + __popc(yc) + __popc(zc) <= w0) continue;
-                uint32_t any = xc | yc | zc;
-                while (any) {
-                    const uint32_t x = __ffs(any) - 1;
-                    any &= any - 1u;
-                    const uint32_t base = (q * B + x);
-                    if ((xc >> x) & 1u) { if (j >= w0 && j < w1) jobs[j - w0] = base; ++j; }
-                    if ((yc >> x) & 1u) { if (j >= w0 && j < w1) jobs[j - w0] = base | (1u << 12); ++j; }
-                    if ((zc >> x) & 1u) { if (j >= w0 && j < w1) jobs[j - w0] = base | (2u << 12); ++j; }
-                }
-            }
-        }
-        __syncwarp();
-        const uint32_t cnt = min(kJobWin, nv - w0);
-        for (uint32_t b = 0; b < cnt; b += 32) {
-            const uint32_t n = min(32u, cnt - b);
-            if (lane < n && MTX_BC(w0 + b + lane, nv, kBcVertex)) {
-                const uint32_t job = jobs[b + lane];
-                const uint32_t i = job & 0xfffu, a = job >> 12;
-                const uint32_t q = fdiv(i, pl.rB), x = i - q * B;
-                const uint32_t z = fdiv(q, pl.rB), y = q - z * B;
-                float t;
-                const float3 pos =
-                    vertex_pos<T>(p, pl, tile, g, x, y, z, a, GENERIC && frame == MTX_FRAME_NDC, &t);
-                if (xyz) {  // each lane its own 12 bytes: L2 merges the warp's 384-byte span
-                    float *o = reinterpret_cast<float *>(vertices) + 3ull * (vbase + w0 + b + lane);
-                    o[0] = pos.x;
-                    o[1] = pos.y;
-                    o[2] = pos.z;
-                } else {
-                    float3 nn = make_float3(0.0f, 0.0f, 0.0f);
-                    if (normals) {
-                        if constexpr (ANY) nn = vertex_normal_any(p, g.ox + x, g.oy + y, g.oz + z, a, t);
-                        else nn = vertex_normal<T>(p, g.ox + x, g.oy + y, g.oz + z, a, t);
-                    }
-                    float4 *v = reinterpret_cast<float4 *>(vertices) + 2ull * (vbase + w0 + b + lane);
-                    v[0] = make_float4(pos.x, pos.y, pos.z, 1.0f);
-                    v[1] = make_float4(nn.x, nn.y, nn.z, 0.0f);
-                }
-            }
-            __syncwarp();
-        }
-    }
-}
-
 // -------------------------------------------------------------- emit pass
-// Index of a voxel of the (B+1)^3 context outside the block (some coordinate == B).
-__device__ __forceinline__ uint32_t ctx_index(uint32_t B, uint32_t x, uint32_t y, uint32_t z) {
-    const uint32_t B1 = B + 1;
-    if (x == B) return z * B1 + y;
-    if (y == B) return B1 * B1 + z * B + x;
-    return B1 * B1 + B * B1 + y * B + x;
-}
-
-// Context voxel of compact index j (inverse of ctx_index).
+// Context voxel of compact index j: the (B+1)^2 voxels with x == B first, then
+// those with y == B, then those with z == B.
 __device__ __forceinline__ void ctx_voxel(const WPlan &pl, uint32_t j, uint32_t &x, uint32_t &y, uint32_t &z) {
     const uint32_t B = pl.B, B1 = pl.B1;
     if (j < B1 * B1) {
@@ -684,79 +488,7 @@ __device__ __forceinline__ void ctx_voxel(const WPlan &pl, uint32_t j, uint32_t 
     }
 }
 
-// Resolves the vertex id of edge e of the cell at block cell (x, y, z).
-__device__ __forceinline__ uint32_t edge_vertex(uint32_t x, uint32_t y, uint32_t z, uint32_t e, const uint8_t *owner,
-                                                const uint32_t *cross, const uint32_t *vp, const uint32_t *nvid,
-                                                const uint8_t *nm, uint32_t B, uint32_t BB, uint32_t vbase,
-                                                bool &bad) {
-    const uint32_t own = owner[e];
-    const uint32_t ux = x + (own & 1u), uy = y + ((own >> 1) & 1u), uz = z + ((own >> 2) & 1u);
-    const uint32_t ax = own >> 3;
-    uint32_t base, m;
-    if (ux < B && uy < B && uz < B) {
-        const uint32_t q = uz * B + uy;
-        base = vbase + voxel_prefix(cross, vp, BB, q, ux);
-        m = voxel_mask(cross, BB, q, ux);
-    } else {
-        const uint32_t jx = ctx_index(B, ux, uy, uz);
-        if (!MTX_BC(jx, 3 * B * B + 3 * B + 1, kBcContext)) {
-            bad = true;
-            return 0;
-        }
-        base = nvid[jx];
-        m = nm[jx];
-    }
-    if (base == kNoVertex || !((m >> ax) & 1u)) {
-        bad = true;
-        return 0;
-    }
-    return base + __popc(m & ((1u << ax) - 1u));
-}
-
-// Unified vertex table over the block's (B+1)^3 voxels for B <= 8, built in
-// the tile's slot once the vertices are written: a 16-bit entry per voxel,
-// the first vertex of the voxel relative to its block's first vertex (11
-// bits) | the block's number c << 11 (0 = this block, 1-7 = the +x/+y/+z
-// neighbour dx | dy << 1 | dz << 2), then a mask byte per voxel with its
-// owned cut edges.  Own voxels come from the crossing rows; the context layer
-// from the packed gather (gather_finish<CPL, true>).  A triangle corner is
-// then one entry, one mask and one base word.  Only voxels that own a cut
-// edge are written; triangle corners refer to no other.
-__device__ __forceinline__ void build_utab(const WPlan &pl, unsigned char *ws, uint16_t *ut, uint8_t *um,
-                                           const uint32_t *cmap) {
-    const uint32_t lane = threadIdx.x & 31, B = pl.B, B1 = pl.B1, BB = pl.BB, R = (BB + 31) / 32;
-    const uint32_t *cross = reinterpret_cast<const uint32_t *>(ws + pl.off_cross);
-    const uint32_t *vp = reinterpret_cast<const uint32_t *>(ws + pl.off_vp);
-    for (uint32_t k = 0; k < R; ++k) {
-        const uint32_t q = lane * R + k;
-        if (q >= BB) break;
-        const uint32_t xc = cross[q], yc = cross[BB + q], zc = cross[2 * BB + q];
-        const uint32_t z = fdiv(q, pl.rB), y = q - z * B, row = (z * B1 + y) * B1;
-        uint32_t any = xc | yc | zc, run = vp[q];
-        while (any) {
-            const uint32_t x = __ffs(any) - 1;
-            any &= any - 1u;
-            const uint32_t m = ((xc >> x) & 1u) | (((yc >> x) & 1u) << 1) | (((zc >> x) & 1u) << 2);
-            if (MTX_BC(row + x, B1 * B1 * B1, kBcVoxTab)) {
-                ut[row + x] = (uint16_t)run;
-                um[row + x] = (uint8_t)m;
-            }
-            run += __popc(m);
-        }
-    }
-    const uint16_t *nvid = reinterpret_cast<const uint16_t *>(ws + pl.off_nvid);
-    for (uint32_t j = lane; j < pl.nb3; j += 32) {
-        const uint32_t e = cmap[j], v = nvid[j];
-        const uint32_t ti = (((e >> 23) & 31u) * B1 + ((e >> 18) & 31u)) * B1 + ((e >> 13) & 31u);
-        if (MTX_BC(ti, B1 * B1 * B1, kBcVoxTab)) {
-            ut[ti] = (uint16_t)((v & 0x7ffu) | ((e & 7u) << 11));
-            um[ti] = (uint8_t)(v >> 11);
-        }
-    }
-    __syncwarp();
-}
-
-// Edge offsets of the unified table for one CTA (B <= 8): entry e holds the
+// Edge offsets of the vertex table for one CTA (B <= 8): entry e holds the
 // table offset of cube edge e's owner voxel from the cell's low corner,
 // dx + dy (B+1) + dz (B+1)^2, and its axis << 8 (from the owner table).
 __device__ __forceinline__ void edge_offsets(uint16_t *eoff, uint32_t B1) {
@@ -764,21 +496,6 @@ __device__ __forceinline__ void edge_offsets(uint16_t *eoff, uint32_t B1) {
         const uint32_t o = c_mc_owner[threadIdx.x];
         eoff[threadIdx.x] = (uint16_t)((o & 1u) + ((o >> 1) & 1u) * B1 + ((o >> 2) & 1u) * B1 * B1 + ((o >> 3) << 8));
     }
-}
-
-// The vertex id of cube edge e of the cell whose low corner is tile voxel ti,
-// from the unified table (build_utab); nbase: the eight block first vertices.
-__device__ __forceinline__ uint32_t edge_vertex_ut(uint32_t ti, uint32_t e, const uint16_t *eoff, const uint16_t *ut,
-                                                   const uint8_t *um, const uint32_t *nbase, uint32_t B1, bool &bad) {
-    const uint32_t eo = eoff[e];
-    const uint32_t i = ti + (eo & 0xffu), ax = eo >> 8;
-    if (!MTX_BC(i, B1 * B1 * B1, kBcVoxTab)) {
-        bad = true;
-        return 0;
-    }
-    const uint32_t m = um[i], v = ut[i];
-    bad |= !((m >> ax) & 1u);
-    return nbase[v >> 11] + (v & 0x7ffu) + __popc(m & ((1u << ax) - 1u));
 }
 
 // -------------------------------------------------------------- scan pass
@@ -901,104 +618,15 @@ __device__ __forceinline__ void gather_issue(const Problem &p, const WPlan &pl, 
     }
 }
 
-// Map entry of context voxel j: neighbour number c (bits 0-2), the index of its
-// face record in that neighbour (bits 3-12), and the voxel's block coordinates
-// x, y, z (5 bits each from bit 13).  It depends on B alone, so the emit kernel
-// builds the map once per CTA.
-__device__ __forceinline__ uint32_t ctx_map_entry(const WPlan &pl, uint32_t j) {
-    const uint32_t B = pl.B, BB = pl.BB;
-    uint32_t x, y, z;
-    ctx_voxel(pl, j, x, y, z);
-    const uint32_t dx = x == B, dy = y == B, dz = z == B;
-    const uint32_t lx = dx ? 0 : x, ly = dy ? 0 : y, lz = dz ? 0 : z;
-    const uint32_t e = dx ? lz * B + ly : (dy ? BB + lz * B + lx : 2 * BB + ly * B + lx);
-    return (dx | (dy << 1) | (dz << 2)) | (e << 3) | (x << 13) | (y << 18) | (z << 23);
-}
-
-// gather_issue with the context-layer map in shared memory.
-template <int CPL>
-__device__ __forceinline__ void gather_issue_map(const Problem &p, const WPlan &pl, const Geo &g, uint32_t nb_rk,
-                                                 const uint32_t *faces, uint32_t face_stride, const uint32_t *cmap,
-                                                 uint32_t rec[CPL], uint64_t face_words = ~0ull) {
-    const uint32_t lane = threadIdx.x & 31, nb3 = pl.nb3;
-    // the whole context layer lies in the volume unless the block reaches a high face
-    const bool inner = g.ox + pl.B < p.X && g.oy + pl.B < p.Y && g.oz + pl.B < p.Z;
-#pragma unroll
-    for (uint32_t k = 0; k < CPL; ++k) {
-        rec[k] = 0;
-        if (k * 32 >= nb3) continue;  // warp-uniform
-        const uint32_t j = k * 32 + lane;
-        const uint32_t m = cmap[j < nb3 ? j : 0];
-        const uint32_t c = j < nb3 ? (m & 7u) : 1u;
-        const uint32_t rk = __shfl_sync(0xffffffffu, nb_rk, c);
-        bool take = j < nb3 && rk != kNoVertex;
-        if (!inner)
-            take = take && g.ox + ((m >> 13) & 31u) < p.X && g.oy + ((m >> 18) & 31u) < p.Y &&
-                   g.oz + ((m >> 23) & 31u) < p.Z;
-        if (take && MTX_BC((uint64_t)rk * face_stride + ((m >> 3) & 1023u), face_words, kBcFaces))
-            rec[k] = __ldg(faces + (uint64_t)rk * face_stride + ((m >> 3) & 1023u)) | 0x80000000u | (c << 27);
-    }
-}
-
-// Turns the gathered records into first-vertex ids and owned-edge masks of the
-// context layer (nb_vb: lane c holds neighbour c's first vertex id).
-// PACKED (B <= 8, the unified table of build_utab): each entry keeps the
-// neighbour-relative first vertex and the voxel's owned-edge mask, rel | m <<
-// 11 (the neighbour's number comes from the context map), and lanes 0-7 store
-// the first vertex of the block (vbase, entry 0) and of its neighbours into
-// the plan's eight base words.
-template <int CPL, bool PACKED = false>
-__device__ __forceinline__ void gather_finish(const WPlan &pl, uint32_t nb_vb, const uint32_t rec[CPL],
-                                              unsigned char *ws, uint32_t vbase = 0) {
-    const uint32_t lane = threadIdx.x & 31, nb3 = pl.nb3;
-    uint32_t *nvid = reinterpret_cast<uint32_t *>(ws + pl.off_nvid);
-    uint16_t *nvid16 = reinterpret_cast<uint16_t *>(ws + pl.off_nvid);
-    uint8_t *nm = ws + pl.off_nm;
-    if constexpr (PACKED) {
-        if (lane < 8) reinterpret_cast<uint32_t *>(ws + pl.off_bar + 16)[lane] = lane ? nb_vb : vbase;
-    }
-#pragma unroll
-    for (uint32_t k = 0; k < CPL; ++k) {
-        if (k * 32 >= nb3) continue;
-        const uint32_t j = k * 32 + lane;
-        const uint32_t vb = PACKED ? 0u : __shfl_sync(0xffffffffu, nb_vb, (rec[k] >> 27) & 7u);
-        if (j < nb3) {
-            const bool present = rec[k] >> 31;
-            if constexpr (PACKED) {
-                nvid16[j] = (uint16_t)((rec[k] & 0x7ffu) | (present ? ((rec[k] >> 24) & 7u) << 11 : 0u));
-            } else {
-                nvid[j] = present ? vb + (rec[k] & 0xffffffu) : kNoVertex;
-                nm[j] = present ? (uint8_t)((rec[k] >> 24) & 7u) : (uint8_t)0;
-            }
-        }
-    }
-}
-
 // The block's low-face records from its crossing rows and row prefixes:
 // block-relative first vertex | owned-edge mask << 24 of the voxels with
 // x == 0 (index z*B + y), y == 0 (BB + z*B + x) and z == 0 (2BB + y*B + x).
-// SPREAD: each y == 0 / z == 0 record computed by its own lane from its row's
-// prefix (coalesced stores; the single-volume count pass); otherwise 2B lanes
-// walk those rows along x with a running first vertex (the batched count phase).
-template <bool SPREAD = true>
+// 2B lanes walk the y == 0 and z == 0 rows along x with a running first vertex.
 __device__ __forceinline__ void write_face_records(const WPlan &pl, const unsigned char *ws, uint32_t *fr) {
     const uint32_t lane = threadIdx.x & 31, B = pl.B, BB = pl.BB;
     const uint32_t *cross = reinterpret_cast<const uint32_t *>(ws + pl.off_cross);
     const uint32_t *vp = reinterpret_cast<const uint32_t *>(ws + pl.off_vp);
-    if constexpr (SPREAD) {
-        // records BB + i for i < 2BB: record i is voxel x of row q (y == 0:
-        // q = z*B; z == 0: q = y); consecutive lanes take consecutive records
-        for (uint32_t i = lane; i < 2 * BB; i += 32) {
-            const uint32_t face = i >= BB, rem = face ? i - BB : i;
-            const uint32_t r = fdiv(rem, pl.rB), x = rem - r * B;
-            const uint32_t q = face ? r : r * B;
-            const uint32_t xc = cross[q], yc = cross[BB + q], zc = cross[2 * BB + q];
-            const uint32_t below = (1u << x) - 1u;
-            const uint32_t run = vp[q] + __popc(xc & below) + __popc(yc & below) + __popc(zc & below);
-            const uint32_t m = ((xc >> x) & 1u) | (((yc >> x) & 1u) << 1) | (((zc >> x) & 1u) << 2);
-            if (MTX_BC(BB + i, 3 * BB, kBcFaces)) fr[BB + i] = run | (m << 24);
-        }
-    } else if (lane < 2 * B) {
+    if (lane < 2 * B) {
         // lane l < 2B walks row (y = 0, z = l) or (y = l - B, z = 0) along x
         const bool yface = lane < B;
         const uint32_t q = yface ? lane * B : lane - B;
@@ -1014,150 +642,6 @@ __device__ __forceinline__ void write_face_records(const WPlan &pl, const unsign
     // x == 0 face: record z*B + y is voxel (0, y, z), the first of row q = z*B + y
     for (uint32_t q = lane; q < BB; q += 32)
         fr[q] = vp[q] | (((cross[q] & 1u) | ((cross[BB + q] & 1u) << 1) | ((cross[2 * BB + q] & 1u) << 2)) << 24);
-}
-
-// Count body of one block whose tile is staged: the (vertices, triangles)
-// counts into *dr and the low-face records -- block-relative prefix | mask
-// << 24 of the voxels with x == 0 (index z*B+y), y == 0 (BB + z*B+x) and
-// z == 0 (2BB + y*B+x) -- into fr.  The tile is dead once the inside rows
-// are built: next (TMA, one tile buffer) is then issued into the same buffer,
-// so that its load runs under the rest of this block.
-template <typename T, bool TMA = false>
-__device__ __forceinline__ void count_block(const Problem &p, const WPlan &pl, unsigned char *ws, uint32_t buf,
-                                            const Geo &g, const uint8_t *ntab, uint8_t *cases_out,
-                                            mtx_meshlet_descriptor *dr, uint32_t *fr, uint8_t *state,
-                                            const Geo *next = nullptr, const CUtensorMap *map = nullptr) {
-    const uint32_t lane = threadIdx.x & 31;
-    build_rows<T>(p, pl, ws, buf, g);
-    if (next) tile_issue<T, TMA>(pl, ws, buf, *next, map);
-    uint32_t bnv, bnt;
-    block_counts(p, pl, ws, g, ntab, true, cases_out, bnv, bnt, state != nullptr);
-    if (lane == 0) *reinterpret_cast<uint2 *>(&dr->vertexCount) = make_uint2(bnv, bnt);
-    if (state) {  // the block state for the emit pass: 16-byte words, coalesced
-        const uint4 *src = reinterpret_cast<const uint4 *>(ws + pl.off_cross);
-        uint4 *dst = reinterpret_cast<uint4 *>(state);
-        for (uint32_t i = lane; i < pl.state_bytes / 16; i += 32) dst[i] = src[i];
-    }
-    write_face_records(pl, ws, fr);
-}
-
-// Emit body of one block whose tile is staged and whose context layer has
-// been gathered: its own vertices (when `vertices` is set) and its triangles.
-// ANY as in emit_vertices.  VT: resolve triangle corners through the voxel
-// table (build_utab; B <= 8 only).  STATE: the count pass's block state came
-// with the tile (tile_issue), so the rows and counts are not rebuilt.
-template <typename T, bool GENERIC, bool ANY = false, bool VT = false, bool STATE = false>
-__device__ __forceinline__ void emit_block(const Problem &p, const WPlan &pl, unsigned char *ws, uint32_t buf,
-                                           const Geo &g, const mtx_meshlet_descriptor &d, const uint64_t *tab,
-                                           const uint8_t *ntab, const uint8_t *owner, uint32_t *indices,
-                                           uint64_t tcap, void *vertices, uint64_t vcap, uint32_t vfmt,
-                                           uint32_t frame, uint32_t normals, DevStatus *st, uint32_t r,
-                                           const uint32_t *cmap = nullptr) {
-    const uint32_t lane = threadIdx.x & 31, B = pl.B, BB = pl.BB;
-    const uint32_t *cross = reinterpret_cast<const uint32_t *>(ws + pl.off_cross);
-    const uint32_t *vp = reinterpret_cast<const uint32_t *>(ws + pl.off_vp);
-    const uint32_t *tp = reinterpret_cast<const uint32_t *>(ws + pl.off_tp);
-    const uint32_t *nvid = reinterpret_cast<const uint32_t *>(ws + pl.off_nvid);
-    const uint8_t *nm = ws + pl.off_nm;
-    uint32_t *jobs = reinterpret_cast<uint32_t *>(ws + pl.off_jobs);
-    const uint32_t tbase = d.indexOffset / 3u;
-    if ((uint64_t)tbase + d.primitiveCount > tcap || (vertices && (uint64_t)d.vertexOffset + d.vertexCount > vcap)) {
-        if (lane == 0) report(st, MTX_ERR_CAPACITY, kSiteEmitCapacity, r, 2);
-        return;
-    }
-    if (!(d.primitiveCount || (vertices && d.vertexCount))) return;
-    uint32_t bnv = d.vertexCount;
-    if constexpr (!STATE) {
-        uint32_t bnt;
-        build_rows<T>(p, pl, ws, buf, g);
-        block_counts(p, pl, ws, g, ntab, true, nullptr, bnv, bnt, true);
-        if (lane == 0 && (bnv != d.vertexCount || bnt != d.primitiveCount))
-            report(st, MTX_ERR_INTERNAL, kSiteEmitNeighbour, r, 2);
-    }
-    if (vertices && bnv)
-        emit_vertices<T, GENERIC, ANY>(p, pl, ws, buf, g, d.vertexOffset, bnv, vertices, vfmt, frame, normals);
-    // triangles in canonical order: each lane walks the mixed cells of its rows
-    // (masks and case bytes kept by block_counts) and writes one job per
-    // triangle (cell | t << 12 | case << 16) at the triangle's own position in
-    // a window of kJobWin jobs; the warp resolves 32 triangles at a time.  With
-    // the vertex table (VT) the cell is given by its low corner's table index
-    // (z (B+1) + y) (B+1) + x, which the resolve uses as is.
-    const uint16_t *mmk = reinterpret_cast<const uint16_t *>(ws + pl.off_mm);
-    const uint8_t *ck = ws + pl.off_case;
-    uint16_t *vt = reinterpret_cast<uint16_t *>(ws + pl.off_tile[buf]);  // the tile is dead past the vertices
-    uint8_t *um = ws + pl.off_tile[buf] + 2 * pl.B1 * pl.B1 * pl.B1;
-    const uint32_t *nbase = reinterpret_cast<const uint32_t *>(ws + pl.off_bar + 16);
-    if constexpr (VT) build_utab(pl, ws, vt, um, cmap);
-    const uint32_t R = (BB + 31) / 32, nt = d.primitiveCount;
-    bool bad = false;
-    for (uint32_t w0 = 0; w0 < nt; w0 += kJobWin) {
-        const uint32_t w1 = w0 + kJobWin;
-        if (nt <= kJobWin) {  // one window (the common case): no window checks
-            for (uint32_t k = 0; k < R; ++k) {
-                const uint32_t q = lane * R + k;
-                if (q >= BB) break;
-                uint32_t j = tp[q], mm = mmk[q];
-                const uint32_t cell0 = VT ? (q + fdiv(q, pl.rB)) * pl.B1 : q * B;  // row q = z B + y
-                while (mm) {
-                    const uint32_t x = __ffs(mm) - 1;
-                    mm &= mm - 1u;
-                    const uint32_t cfg = ck[q * B + x];
-                    const uint32_t n = ntab[cfg], job = (cell0 + x) | (cfg << 16);
-#pragma unroll
-                    for (uint32_t t = 0; t < 5; ++t)  // at most five triangles a case
-                        if (t < n) jobs[j + t] = job | (t << 12);
-                    j += n;
-                }
-            }
-        } else {
-            for (uint32_t k = 0; k < R; ++k) {
-                const uint32_t q = lane * R + k;
-                if (q >= BB) break;
-                uint32_t j = tp[q];
-                const uint32_t jend = (q + 1 < BB) ? tp[q + 1] : nt;
-                if (j >= w1 || jend <= w0) continue;
-                uint32_t mm = mmk[q];
-                const uint32_t cell0 = VT ? (q + fdiv(q, pl.rB)) * pl.B1 : q * B;
-                while (mm) {
-                    const uint32_t x = __ffs(mm) - 1;
-                    mm &= mm - 1u;
-                    const uint32_t cfg = ck[q * B + x];
-                    const uint32_t n = ntab[cfg];
-                    for (uint32_t t = 0; t < n; ++t, ++j)
-                        if (j >= w0 && j < w1) jobs[j - w0] = (cell0 + x) | (t << 12) | (cfg << 16);
-                }
-            }
-        }
-        __syncwarp();
-        const uint32_t cnt = min(kJobWin, nt - w0);
-        for (uint32_t b = 0; b < cnt; b += 32) {
-            const uint32_t n = min(32u, cnt - b);
-            if (lane < n && MTX_BC(w0 + b + lane, nt, kBcIndex)) {
-                const uint32_t job = jobs[b + lane];
-                const uint32_t i = job & 0xfffu, t = (job >> 12) & 7u;
-                const uint64_t w = tab[job >> 16] >> (4 + 12 * t);
-                uint32_t *o = indices + 3ull * (tbase + w0 + b + lane);  // each lane its own 12 bytes
-                if constexpr (VT) {
-                    const uint32_t ti = i;  // the cell's low corner in the vertex table
-                    const uint16_t *eoff = reinterpret_cast<const uint16_t *>(owner + 16);  // edge_offsets
-                    o[0] = edge_vertex_ut(ti, (uint32_t)(w & 0xFu), eoff, vt, um, nbase, pl.B1, bad);
-                    o[1] = edge_vertex_ut(ti, (uint32_t)((w >> 4) & 0xFu), eoff, vt, um, nbase, pl.B1, bad);
-                    o[2] = edge_vertex_ut(ti, (uint32_t)((w >> 8) & 0xFu), eoff, vt, um, nbase, pl.B1, bad);
-                } else {
-                    const uint32_t q = fdiv(i, pl.rB), x = i - q * B;
-                    const uint32_t z = fdiv(q, pl.rB), y = q - z * B;
-                    o[0] = edge_vertex(x, y, z, (uint32_t)(w & 0xFu), owner, cross, vp, nvid, nm, B, BB,
-                                       d.vertexOffset, bad);
-                    o[1] = edge_vertex(x, y, z, (uint32_t)((w >> 4) & 0xFu), owner, cross, vp, nvid, nm, B, BB,
-                                       d.vertexOffset, bad);
-                    o[2] = edge_vertex(x, y, z, (uint32_t)((w >> 8) & 0xFu), owner, cross, vp, nvid, nm, B, BB,
-                                       d.vertexOffset, bad);
-                }
-            }
-            __syncwarp();
-        }
-    }
-    if (bad) report(st, MTX_ERR_INTERNAL, kSiteEmitNeighbour, r, 3);
 }
 
 // Exclusive scan of the per-block vertex and triangle counts in rank order,

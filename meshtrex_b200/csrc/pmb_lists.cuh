@@ -46,7 +46,13 @@ static mtx_status load_list_tables(mtx_context *c) {
 }
 
 // ------------------------------------------------------------------ plans
-constexpr uint32_t kListRing = 64;  // listed cells not yet taken: fewer than 32, and a word's 32
+// List bits come in units, one a lane: 16 cells for B <= 8 (all of a block's in
+// one round of 32 lanes), else 32.  A warp's list holds a round's cells and up
+// to 31 not yet taken.
+__host__ __device__ inline uint32_t list_unit(uint32_t B) { return B <= 8 ? 16u : 32u; }
+__host__ __device__ inline uint32_t list_cap(uint32_t B) {
+    return B <= 8 ? (B * B * B + 15) / 16 * 16 : 32u * 32u + 32u;
+}
 
 // State handed from count to emit, words a block: the list, padded to whole
 // steps of 32 (B <= 8), or the inside bits of the (B+1)^2 rows.
@@ -63,19 +69,16 @@ __host__ __device__ inline void plan_block(WPlan &p, uint32_t B) {
     p.nb3 = 3 * B * B + 3 * B + 1;
     p.rB = (uint32_t)((0x100000000ull + B - 1) / B);
     p.rB1 = (uint32_t)((0x100000000ull + B) / (B + 1));
-    p.rBB = (uint32_t)((0x100000000ull + B * B - 1) / (B * B));
-    p.R = 32 / B;
-    p.nbuf = 1;
 }
 
 // A warp's shared memory in the count pass: TMA tile and barrier, inside rows,
-// list bits, ring, face records (which share the region of the plain loads'
+// list bits, list, face records (which share the region of the plain loads'
 // bitstream: that is dead once the rows are built).
 __host__ __device__ inline WPlan make_count_plan(uint32_t B, uint32_t esz, bool tma) {
     WPlan p{};
     plan_block(p, B);
     uint32_t o = 0;
-    p.off_tile[0] = p.off_tile[1] = 0;
+    p.off_tile = 0;
     if (tma) {
         p.PX = tile_pitch(B, esz, true);
         p.tile_bytes = p.PX * p.B1 * p.B1 * esz;
@@ -87,8 +90,8 @@ __host__ __device__ inline WPlan make_count_plan(uint32_t B, uint32_t esz, bool 
     o = align_up(o + 4 * p.B1 * p.B1, 16);
     p.off_mm = o;  // list bits
     o = align_up(o + 4 * list_words(B), 16);
-    p.off_list = o;  // ring
-    o = align_up(o + 2 * kListRing, 16);
+    p.off_list = o;
+    o = align_up(o + 2 * list_cap(B), 16);
     p.off_case = o;  // face records / bitstream
     const uint32_t bits = 4 * ((p.B1 * p.B1 * p.B1 + 31) / 32 + 1);
     o = align_up(o + std::max(2 * face_stride16(B), tma ? 0u : bits), 16);
@@ -103,7 +106,7 @@ __host__ __device__ inline uint32_t count_fixed_bytes(uint32_t B, bool off) {
 }
 
 // In the emit pass: vertex table, job ring, first vertices of the block and
-// its seven neighbours, and for B > 8 the inside rows, list bits and ring.
+// its seven neighbours, and for B > 8 the inside rows, list bits and list.
 __host__ __device__ inline WPlan make_emit_plan(uint32_t B) {
     WPlan p{};
     plan_block(p, B);
@@ -113,14 +116,14 @@ __host__ __device__ inline WPlan make_emit_plan(uint32_t B) {
     p.off_nvid = o;
     o += 32;
     p.off_vtab = o;
-    o = align_up(o + (B <= 8 ? 2 : 4) * p.B1 * p.B1 * p.B1, 16);
+    o = align_up(o + 2 * p.B1 * p.B1 * p.B1, 16);
     if (B > 8) {
         p.off_rows = o;
         o = align_up(o + 4 * p.B1 * p.B1, 16);
         p.off_mm = o;
         o = align_up(o + 4 * list_words(B), 16);
         p.off_list = o;
-        o = align_up(o + 2 * kListRing, 16);
+        o = align_up(o + 2 * list_cap(B), 16);
     }
     p.bytes = align_up(o, 16);
     return p;
@@ -182,6 +185,66 @@ __device__ __forceinline__ void load_rows(const Problem &p, const WPlan &pl, uns
     __syncwarp();
 }
 
+// Inside bits of the rows of a staged tile for a block edge known at compile
+// time (build_rows otherwise).  Integer voxels: the sign of floor(iso) - value,
+// shifted in voxel by voxel from the row's end; float voxels: the compare.
+template <typename T, int BC>
+__device__ __forceinline__ void tile_rows(const Problem &p, const WPlan &pl, unsigned char *ws, const Geo &g) {
+    constexpr uint32_t B1 = BC + 1;
+    const T *tile = reinterpret_cast<const T *>(ws + pl.off_tile);
+    uint32_t *rows = reinterpret_cast<uint32_t *>(ws + pl.off_rows);
+    const uint32_t xin = min(B1, p.X - g.ox);
+    // integer voxels: value <= iso  <=>  value <= floor(iso) (never when iso < 0 or NaN)
+    const bool never = Vox<T>::code != 2 && !(p.iso >= 0.0f);
+    const int thr = never || Vox<T>::code == 2 ? 0 : (int)fminf(floorf(p.iso), sizeof(T) == 1 ? 255.0f : 65535.0f);
+    const uint32_t xmask = never ? 0u : (1u << xin) - 1u;
+    // rows of 8 and 16 voxels start on 8 (uint8) or 16 bytes
+    constexpr bool kWide = BC == 8 || BC == 16;
+    constexpr uint32_t NW = BC * sizeof(T) / 4;  // words of a row but its last voxel
+    for (uint32_t q = threadIdx.x & 31; q < B1 * B1; q += 32) {
+        const uint32_t z = q / B1, y = q - z * B1;
+        const T *r = tile + q * pl.PX + g.xoff;
+        uint32_t m = 0;
+        if constexpr (kWide) {
+            uint32_t w[NW];
+#pragma unroll
+            for (uint32_t i = 0; i < NW; i += (NW % 4 ? 2 : 4)) {
+                if constexpr (NW % 4 == 0) {
+                    const uint4 v = reinterpret_cast<const uint4 *>(r)[i / 4];
+                    w[i] = v.x, w[i + 1] = v.y, w[i + 2] = v.z, w[i + 3] = v.w;
+                } else {
+                    const uint2 v = reinterpret_cast<const uint2 *>(r)[i / 2];
+                    w[i] = v.x, w[i + 1] = v.y;
+                }
+            }
+            const T last = r[BC];
+#pragma unroll
+            for (int x = BC; x >= 0; --x) {
+                if constexpr (Vox<T>::code == 2) {
+                    const float v = x == BC ? (float)last : __uint_as_float(w[x < BC ? x : 0]);
+                    m = 2 * m + (v <= p.iso ? 1u : 0u);
+                } else {
+                    constexpr int PER = 4 / sizeof(T);
+                    const int xi = x < BC ? x : 0;
+                    const int v = x == BC ? (int)last
+                                          : (int)((w[xi / PER] >> (8 * sizeof(T) * (xi % PER))) &
+                                                  (sizeof(T) == 1 ? 0xffu : 0xffffu));
+                    m = __funnelshift_l((uint32_t)(thr - v), m, 1);
+                }
+            }
+        } else {
+#pragma unroll
+            for (int x = BC; x >= 0; --x) {
+                if constexpr (Vox<T>::code == 2) m = 2 * m + (Vox<T>::val(r[x]) <= p.iso ? 1u : 0u);
+                else m = __funnelshift_l((uint32_t)(thr - (int)r[x]), m, 1);
+            }
+        }
+        if (Vox<T>::code != 2) m = ~m;
+        rows[q] = g.oy + y < p.Y && g.oz + z < p.Z ? m & xmask : 0u;
+    }
+    __syncwarp();
+}
+
 // Element offsets of the (B+1)^3 tile's voxels from the block's first one,
 // for one CTA.
 __device__ __forceinline__ void row_offsets(const Problem &p, const WPlan &pl, uint32_t *off) {
@@ -194,7 +257,7 @@ __device__ __forceinline__ void row_offsets(const Problem &p, const WPlan &pl, u
 }
 
 // ---------------------------------------------------------------- the list
-// Bits of the listed cells, cell q B + x at bit (q B + x) of the word array.
+// Bits of the listed cells, cell q B + x at bit (q B + x) of the units.
 template <int BC>
 __device__ __forceinline__ void list_bits(const Problem &p, const WPlan &pl, unsigned char *ws, const Geo &g) {
     const uint32_t lane = threadIdx.x & 31, B = pl.B, B1 = pl.B1;
@@ -233,34 +296,41 @@ __device__ __forceinline__ void list_bits(const Problem &p, const WPlan &pl, uns
     __syncwarp();
 }
 
-// Takes the listed cells in order, up to 32 at a time.
+// Takes the listed cells in order, up to 32 at a time, from the warp's list.  A
+// round turns 32 units of list bits into cells: a warp scan of the units' counts
+// gives every lane its place, and each lane writes its own unit's cells.
 struct ListWalk {
-    uint32_t top = 0, done = 0;          // cells put into the ring, cells taken out of it
-    uint32_t next = 0, group = 0, nz = 0;  // words not looked at, the 32 words held, those with cells left
-    uint32_t word = 0;                   // this lane's word of the 32 held
+    uint32_t top = 0, done = 0;  // cells in the list, cells taken from it
+    uint32_t next = 0;           // units not looked at
 };
-// The next n <= 32 cells are ring[(done + i) & 63]; advance done by n after use.  0 at the end.
+// The next n <= 32 cells are list[done + i]; advance done by n after use.  0 at the end.
+template <bool BIG>
 __device__ __forceinline__ uint32_t list_next(ListWalk &l, const WPlan &pl, unsigned char *ws) {
-    const uint32_t lane = threadIdx.x & 31, lt = (1u << lane) - 1u, nw = list_words(pl.B);
-    const uint32_t *bits = reinterpret_cast<const uint32_t *>(ws + pl.off_mm);
-    uint16_t *ring = reinterpret_cast<uint16_t *>(ws + pl.off_list);
-    __syncwarp();
-    while (l.top - l.done < 32) {
-        if (!l.nz) {
-            if (l.next >= nw) break;
-            l.group = l.next;
-            l.word = l.group + lane < nw ? bits[l.group + lane] : 0u;
-            l.nz = __ballot_sync(0xffffffffu, l.word != 0);
-            l.next += 32;
-            continue;
+    const uint32_t lane = threadIdx.x & 31, unit = BIG ? 32u : 16u, nu = (pl.BB * pl.B + unit - 1) / unit;
+    uint16_t *list = reinterpret_cast<uint16_t *>(ws + pl.off_list);
+    while (l.top - l.done < 32 && l.next < nu) {
+        if (BIG) {  // what is left moves to the front
+            const uint32_t left = l.top - l.done;
+            __syncwarp();
+            const uint16_t v = lane < left ? list[l.done + lane] : (uint16_t)0;
+            __syncwarp();
+            if (lane < left) list[lane] = v;
+            l.top = left;
+            l.done = 0;
         }
-        const uint32_t k = __ffs(l.nz) - 1;
-        l.nz &= l.nz - 1u;
-        const uint32_t w = __shfl_sync(0xffffffffu, l.word, k);
-        if ((w >> lane) & 1u) ring[(l.top + __popc(w & lt)) & (kListRing - 1)] = (uint16_t)((l.group + k) * 32 + lane);
-        l.top += __popc(w);
+        const uint32_t u = l.next + lane;
+        uint32_t b = 0;
+        if (u < nu) {
+            if (BIG) b = reinterpret_cast<const uint32_t *>(ws + pl.off_mm)[u];
+            else b = reinterpret_cast<const uint16_t *>(ws + pl.off_mm)[u];
+        }
+        uint32_t total;
+        uint32_t at = l.top + warp_excl_scan(__popc(b), total);
+        for (uint32_t c = u * unit; b; b &= b - 1u) list[at++] = (uint16_t)(c + __ffs(b) - 1);
+        l.top += total;
+        l.next += 32;
+        __syncwarp();
     }
-    __syncwarp();
     return min(32u, l.top - l.done);
 }
 
@@ -301,7 +371,7 @@ __device__ __forceinline__ void count_block_list(const Problem &p, const WPlan &
                                                  uint16_t *faces, uint32_t *state) {
     const uint32_t lane = threadIdx.x & 31, B = pl.B, BB = pl.BB;
     const uint32_t *rows = reinterpret_cast<const uint32_t *>(ws + pl.off_rows);
-    const uint16_t *ring = reinterpret_cast<const uint16_t *>(ws + pl.off_list);
+    const uint16_t *list = reinterpret_cast<const uint16_t *>(ws + pl.off_list);
     uint16_t *fr = reinterpret_cast<uint16_t *>(ws + pl.off_case);
     const bool inner = g.ox + B < p.X && g.oy + B < p.Y && g.oz + B < p.Z;
     for (uint32_t i = lane; i < face_stride16(B) / 8; i += 32) reinterpret_cast<uint4 *>(fr)[i] = make_uint4(0, 0, 0, 0);
@@ -313,16 +383,18 @@ __device__ __forceinline__ void count_block_list(const Problem &p, const WPlan &
         }
     if (B > 8)
         for (uint32_t i = lane; i < pl.B1 * pl.B1; i += 32) state[i] = rows[i];
+    constexpr bool kBig = BC > 8;  // the run-time form takes the rounds of B > 8
     ListWalk l;
-    uint32_t nv = 0, nt = 0;
-    while (const uint32_t n = list_next(l, pl, ws)) {
+    uint32_t nv = 0, nt = 0, steps = 0;
+    while (const uint32_t n = BC ? list_next<kBig>(l, pl, ws) : B > 8 ? list_next<true>(l, pl, ws) : list_next<false>(l, pl, ws)) {
         uint32_t e = 0;
-        if (lane < n) e = listed_cell(p, pl, g, rows, ring[(l.done + lane) & (kListRing - 1)], inner);
+        if (lane < n) e = listed_cell(p, pl, g, rows, list[l.done + lane], inner);
         const uint32_t m = e >> 28, tris = lane < n ? ntab[(e >> 12) & 0xffu] : 0u;
         uint32_t vt, tt;
         const uint32_t rel = nv + step_vertices(m, vt);
         const uint32_t before = warp_excl_scan(tris, tt);
-        if (B <= 8 && MTX_BC(l.done + lane, list_state_words(B), kBcState)) state[l.done + lane] = e | (before << 20);
+        if (B <= 8 && MTX_BC(steps + lane, list_state_words(B), kBcState)) state[steps + lane] = e | (before << 20);
+        steps += 32;
         if (m) {
             const uint32_t cell = e & 0xfffu, q = fdiv(cell, pl.rB), x = cell - q * B, z = fdiv(q, pl.rB), y = q - z * B;
             const uint16_t rec = (uint16_t)(rel | ((m & 3u) << 14));
@@ -342,33 +414,26 @@ __device__ __forceinline__ void count_block_list(const Problem &p, const WPlan &
 }
 
 // -------------------------------------------------------------- emit body
-// Entry of the vertex table, one a voxel of the (B+1)^3 tile: the voxel's
-// first vertex relative to its block's, whether its x and y edges are cut, and
-// the block (0 = this one, 1-7 the +x/+y/+z neighbour dx | dy << 1 | dz << 2).
-// 16 bits for B <= 8 (11 + 2 + 3), else 32 (14 + 2 + 3).
-template <bool BIG> struct VEntry;
-template <> struct VEntry<false> {
-    using E = uint16_t;
-    static constexpr uint32_t kRel = 11, kShift = 1;  // log2 of the entry's bytes
-};
-template <> struct VEntry<true> {
-    using E = uint32_t;
-    static constexpr uint32_t kRel = 14, kShift = 2;
-};
+// Vertex table: for each voxel of the (B+1)^3 tile the first vertex it owns,
+// relative to its block's (14 bits), and whether its x and y edges are cut
+// (bits 14, 15) -- the face records' form, so that the context layer's entries
+// are copies of them.  Which block a corner's voxel belongs to follows from the
+// cell: the neighbour in +x / +y / +z exactly where the cell is the block's
+// last along that axis and the edge's owner is the cell's far voxel.
+constexpr uint32_t kRelMask = 0x3fffu, kCutMask = 0xc000u;
 
 // The CTA's triangle table: three 16-bit corners a triangle, each the owner
-// voxel's byte offset in the vertex table from the cell's low corner, and the
-// two edge bits of the entry that count before the corner's axis.
-template <bool BIG>
+// voxel's byte offset in the vertex table from the cell's low corner (bits
+// 0-9), its steps along x, y and z (10-12) and the cut bits of the entry that
+// count before the corner's axis (14, 15).
 __device__ __forceinline__ void build_tris(const WPlan &pl, uint64_t *tri, uint16_t *first) {
-    constexpr uint32_t kRel = VEntry<BIG>::kRel, kShift = VEntry<BIG>::kShift;
     for (uint32_t i = threadIdx.x; i < kTris; i += blockDim.x) {
         const uint32_t e3 = __ldg(&g_mc_tri[i]);
         uint64_t w = 0;
         for (uint32_t k = 0; k < 3; ++k) {
             const uint32_t o = c_mc_owner[(e3 >> (4 * k)) & 0xfu], ax = o >> 3;
             const uint32_t off = (o & 1u) + ((o >> 1) & 1u) * pl.B1 + ((o >> 2) & 1u) * pl.B1 * pl.B1;
-            w |= (uint64_t)((off << kShift) | (((1u << ax) - 1u) << kRel)) << (16 * k);
+            w |= (uint64_t)((off << 1) | ((o & 7u) << 10) | (((1u << ax) - 1u) << 14)) << (16 * k);
         }
         tri[i] = w;
     }
@@ -387,8 +452,50 @@ __device__ __forceinline__ uint32_t ctx_entry(const WPlan &pl, uint32_t j) {
     return (dx | (dy << 1) | (dz << 2)) | (e << 3) | (((z * pl.B1 + y) * pl.B1 + x) << 13);
 }
 
-// Face records of up to 32 N context voxels from j0 on, all loads issued; nb_rk: lane c
-// holds neighbour c's rank or kNoVertex.
+// The context layer: face records of the neighbours (nb_rk: lane c holds
+// neighbour c's rank or kNoVertex) into the vertex table, loads first.
+// B = 8: two records a lane from each of the three faces and the 25 of the
+// edges and the corner, four loads a lane in all.
+struct Ctx8 {
+    uint32_t face[3], edge;
+};
+__device__ __forceinline__ uint32_t ctx8_edge(uint32_t lane) {  // map entry (ctx_entry) of the lane's edge voxel
+    const uint32_t k = lane & 7u;
+    if (lane < 8) return 3u | ((8 * k) << 3) | (((k * 9 + 8) * 9 + 8) << 13);
+    if (lane < 16) return 5u | (k << 3) | (((8 * 9 + k) * 9 + 8) << 13);
+    if (lane < 24) return 6u | ((64 + k) << 3) | (((8 * 9 + 8) * 9 + k) << 13);
+    return lane == 24 ? 7u | (728u << 13) : 0u;
+}
+__device__ __forceinline__ Ctx8 ctx8_load(const uint16_t *faces, uint32_t nb_rk, uint32_t edge, uint64_t face_words) {
+    const uint32_t lane = threadIdx.x & 31;
+    Ctx8 c;
+#pragma unroll
+    for (int f = 0; f < 3; ++f) {
+        const uint32_t rk = __shfl_sync(0xffffffffu, nb_rk, 1 << f);
+        const uint64_t at = (uint64_t)rk * 192 + 64 * f + 2 * lane;
+        c.face[f] = 0;
+        if (rk != kNoVertex && MTX_BC(at + 1, face_words, kBcFaces))
+            c.face[f] = __ldg(reinterpret_cast<const uint32_t *>(faces + at));
+    }
+    const uint32_t rk = __shfl_sync(0xffffffffu, nb_rk, edge & 7u);
+    const uint64_t at = (uint64_t)rk * 192 + ((edge >> 3) & 1023u);
+    c.edge = 0;
+    if (edge && rk != kNoVertex && MTX_BC(at, face_words, kBcFaces)) c.edge = __ldg(faces + at);
+    return c;
+}
+__device__ __forceinline__ void ctx8_store(const Ctx8 &c, uint32_t edge, uint16_t *vtab) {
+    const uint32_t lane = threadIdx.x & 31, u = lane >> 2, v = 2 * (lane & 3u);
+    uint16_t *x = vtab + (u * 9 + v) * 9 + 8, *y = vtab + (u * 9 + 8) * 9 + v, *z = vtab + (8 * 9 + u) * 9 + v;
+    x[0] = (uint16_t)c.face[0];
+    x[9] = (uint16_t)(c.face[0] >> 16);
+    y[0] = (uint16_t)c.face[1];
+    y[1] = (uint16_t)(c.face[1] >> 16);
+    z[0] = (uint16_t)c.face[2];
+    z[1] = (uint16_t)(c.face[2] >> 16);
+    if (edge) vtab[edge >> 13] = (uint16_t)c.edge;
+}
+
+// Any B, through the map: up to 32 N context voxels from j0 on.
 template <int N>
 __device__ __forceinline__ void ctx_load(const WPlan &pl, const uint16_t *faces, uint32_t nb_rk, const uint32_t *cmap,
                                          uint32_t j0, uint32_t rec[N], uint64_t face_words) {
@@ -404,99 +511,92 @@ __device__ __forceinline__ void ctx_load(const WPlan &pl, const uint16_t *faces,
         if (j < pl.nb3 && rk != kNoVertex && MTX_BC(at, face_words, kBcFaces)) rec[k] = __ldg(faces + at);
     }
 }
-
-template <bool BIG, int N>
-__device__ __forceinline__ void ctx_store(const WPlan &pl, typename VEntry<BIG>::E *vtab, const uint32_t *cmap,
-                                          uint32_t j0, const uint32_t rec[N]) {
-    constexpr uint32_t kRel = VEntry<BIG>::kRel;
+template <int N>
+__device__ __forceinline__ void ctx_store(const WPlan &pl, uint16_t *vtab, const uint32_t *cmap, uint32_t j0,
+                                          const uint32_t rec[N]) {
     const uint32_t lane = threadIdx.x & 31;
 #pragma unroll
     for (int k = 0; k < N; ++k) {
         const uint32_t j = j0 + 32 * k + lane;
-        if (j < pl.nb3) {
-            const uint32_t c = cmap[j];
-            if (MTX_BC(c >> 13, pl.B1 * pl.B1 * pl.B1, kBcVoxTab))
-                vtab[c >> 13] = (typename VEntry<BIG>::E)((rec[k] & ((1u << kRel) - 1u)) | ((rec[k] >> 14) << kRel) |
-                                                          ((c & 7u) << (kRel + 2)));
+        if (j < pl.nb3 && MTX_BC(cmap[j] >> 13, pl.B1 * pl.B1 * pl.B1, kBcVoxTab)) vtab[cmap[j] >> 13] = (uint16_t)rec[k];
+    }
+}
+
+// One step of the vertex phase: this lane's list word e (0: none) and its first
+// vertex rel -> the voxel's table entry, and a job (cell | axis << 12) for each
+// of its vertices, queued at the vertex's own number.
+__device__ __forceinline__ void queue_vertices(const WPlan &pl, uint32_t e, uint32_t rel, uint16_t *vtab,
+                                               uint32_t *jobs) {
+    const uint32_t m = e >> 28, cell = e & 0xfffu;
+    if (!m) return;
+    const uint32_t q = fdiv(cell, pl.rB), x = cell - q * pl.B;
+    const uint32_t ti = (q + fdiv(q, pl.rB)) * pl.B1 + x;  // row q = z B + y
+    if (MTX_BC(ti, pl.B1 * pl.B1 * pl.B1, kBcVoxTab)) vtab[ti] = (uint16_t)(rel | (m << 14));
+    if (m & 1u) jobs[rel++ & (kJobWin - 1)] = cell;
+    if (m & 2u) jobs[rel++ & (kJobWin - 1)] = cell | (1u << 12);
+    if (m & 4u) jobs[rel & (kJobWin - 1)] = cell | (2u << 12);
+}
+
+// Writes vertices [done, done + n) of the block, n <= 32, one a lane; the first
+// is vertex vbase of the mesh.
+template <typename T, bool GENERIC>
+__device__ __forceinline__ void put_vertices(const Problem &p, const WPlan &pl, const Geo &g, const uint32_t *jobs,
+                                             uint32_t done, uint32_t n, bool inner, void *vertices, uint64_t vbase,
+                                             uint32_t vfmt, uint32_t frame, uint32_t normals) {
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t job = jobs[(done + lane) & (kJobWin - 1)];
+    const uint32_t cell = job & 0xfffu, a = job >> 12;
+    const uint32_t q = fdiv(cell, pl.rB), x = cell - q * pl.B, z = fdiv(q, pl.rB), y = q - z * pl.B;
+    const uint32_t gx = g.ox + x, gy = g.oy + y, gz = g.oz + z;
+    // (a list the count pass did not finish must not lead past the volume)
+    if (lane < n && (inner || (gx + (a == 0) < p.X && gy + (a == 1) < p.Y && gz + (a == 2) < p.Z))) {
+        const T *v = reinterpret_cast<const T *>(p.vol) + ((uint64_t)gz * p.Y + gy) * p.X + gx;
+        const uint64_t step = a == 0 ? 1ull : a == 1 ? (uint64_t)p.X : (uint64_t)p.X * p.Y;
+        const float t = edge_t(Vox<T>::val(__ldg(v)), Vox<T>::val(__ldg(v + step)), p.iso);
+        float3 pos = make_float3((float)gx, (float)gy, (float)gz);
+        if (a == 0) pos.x = __fadd_rn(pos.x, t);
+        if (a == 1) pos.y = __fadd_rn(pos.y, t);
+        if (a == 2) pos.z = __fadd_rn(pos.z, t);
+        if (GENERIC && frame == MTX_FRAME_NDC) {
+            pos.x = __fsub_rn(__fmul_rn(__fdiv_rn(pos.x, (float)p.X), 2.0f), 1.0f);
+            pos.y = __fsub_rn(__fmul_rn(__fdiv_rn(pos.y, (float)p.Y), 2.0f), 1.0f);
+            pos.z = __fsub_rn(__fmul_rn(__fdiv_rn(pos.z, (float)p.Z), 2.0f), 1.0f);
+        }
+        const uint64_t at = vbase + done + lane;
+        if (!GENERIC || vfmt == MTX_VERTEX_XYZ) {  // each lane its own 12 bytes: L2 merges the warp's span
+            float *o = reinterpret_cast<float *>(vertices) + 3 * at;
+            o[0] = pos.x;
+            o[1] = pos.y;
+            o[2] = pos.z;
+        } else {
+            float3 nn = make_float3(0.0f, 0.0f, 0.0f);
+            if (normals) nn = vertex_normal<T>(p, gx, gy, gz, a, t);
+            float4 *o = reinterpret_cast<float4 *>(vertices) + 2 * at;
+            o[0] = make_float4(pos.x, pos.y, pos.z, 1.0f);
+            o[1] = make_float4(nn.x, nn.y, nn.z, 0.0f);
         }
     }
+    __syncwarp();
 }
 
-// Writes vertex `at` on the +A edge of voxel (gx, gy, gz) whose value is fa and
-// whose neighbour's is fb.
-template <typename T, bool GENERIC, int A>
-__device__ __forceinline__ void put_vertex(const Problem &p, uint32_t gx, uint32_t gy, uint32_t gz, float fa, float fb,
-                                           void *vertices, uint64_t at, uint32_t vfmt, uint32_t frame,
-                                           uint32_t normals) {
-    const float t = edge_t(fa, fb, p.iso);
-    float3 pos = make_float3((float)gx, (float)gy, (float)gz);
-    if (A == 0) pos.x = __fadd_rn(pos.x, t);
-    if (A == 1) pos.y = __fadd_rn(pos.y, t);
-    if (A == 2) pos.z = __fadd_rn(pos.z, t);
-    if (GENERIC && frame == MTX_FRAME_NDC) {
-        pos.x = __fsub_rn(__fmul_rn(__fdiv_rn(pos.x, (float)p.X), 2.0f), 1.0f);
-        pos.y = __fsub_rn(__fmul_rn(__fdiv_rn(pos.y, (float)p.Y), 2.0f), 1.0f);
-        pos.z = __fsub_rn(__fmul_rn(__fdiv_rn(pos.z, (float)p.Z), 2.0f), 1.0f);
-    }
-    if (!GENERIC || vfmt == MTX_VERTEX_XYZ) {  // each lane its own 12 bytes: L2 merges the warp's span
-        float *o = reinterpret_cast<float *>(vertices) + 3 * at;
-        o[0] = pos.x;
-        o[1] = pos.y;
-        o[2] = pos.z;
-    } else {
-        float3 nn = make_float3(0.0f, 0.0f, 0.0f);
-        if (normals) nn = vertex_normal<T>(p, gx, gy, gz, A, t);
-        float4 *v = reinterpret_cast<float4 *>(vertices) + 2 * at;
-        v[0] = make_float4(pos.x, pos.y, pos.z, 1.0f);
-        v[1] = make_float4(nn.x, nn.y, nn.z, 0.0f);
-    }
-}
-
-// One step of the vertex phase: this lane's list word e (0: none) and its
-// first vertex rel -> the voxel's table entry and its vertices.
-template <typename T, bool GENERIC, bool BIG>
-__device__ __forceinline__ void emit_step_vertices(const Problem &p, const WPlan &pl, const Geo &g, uint32_t e,
-                                                   uint32_t rel, typename VEntry<BIG>::E *vtab, void *vertices,
-                                                   uint64_t vbase, uint32_t nv, uint32_t vfmt, uint32_t frame,
-                                                   uint32_t normals) {
-    const uint32_t m = e >> 28;
-    if (!m) return;
-    const uint32_t cell = e & 0xfffu, q = fdiv(cell, pl.rB), x = cell - q * pl.B, z = fdiv(q, pl.rB), y = q - z * pl.B;
-    const uint32_t ti = (z * pl.B1 + y) * pl.B1 + x;
-    if (MTX_BC(ti, pl.B1 * pl.B1 * pl.B1, kBcVoxTab))
-        vtab[ti] = (typename VEntry<BIG>::E)(rel | ((m & 3u) << VEntry<BIG>::kRel));
-    if (!vertices || rel + __popc(m) > nv) return;
-    const uint32_t gx = g.ox + x, gy = g.oy + y, gz = g.oz + z;
-    const T *v = reinterpret_cast<const T *>(p.vol) + ((uint64_t)gz * p.Y + gy) * p.X + gx;
-    // the voxel and its cut neighbours, all loads in flight
-    const T a = __ldg(v), bx = m & 1u ? __ldg(v + 1) : T(0), by = m & 2u ? __ldg(v + p.X) : T(0),
-            bz = m & 4u ? __ldg(v + (uint64_t)p.X * p.Y) : T(0);
-    const float fa = Vox<T>::val(a);
-    uint64_t at = vbase + rel;
-    if (m & 1u) put_vertex<T, GENERIC, 0>(p, gx, gy, gz, fa, Vox<T>::val(bx), vertices, at++, vfmt, frame, normals);
-    if (m & 2u) put_vertex<T, GENERIC, 1>(p, gx, gy, gz, fa, Vox<T>::val(by), vertices, at++, vfmt, frame, normals);
-    if (m & 4u) put_vertex<T, GENERIC, 2>(p, gx, gy, gz, fa, Vox<T>::val(bz), vertices, at, vfmt, frame, normals);
-}
-
-// Resolves triangle jobs [done, done + n), n <= 32, one a lane, each lane storing its own 12 bytes.
-template <bool BIG>
+// Writes triangles [done, done + n) of the block, n <= 32, one a lane, each lane
+// its own 12 bytes from dst on.  Job: the cell's byte offset in the vertex table
+// (bits 0-15), the triangle (16-25), whether the cell is the block's last along
+// x, y and z (26-28).  miss: bit c, neighbour c is not active.
 __device__ __forceinline__ void put_triangles(const unsigned char *vtab, const uint64_t *tri, const uint32_t *jobs,
                                               const uint32_t *nbase, uint32_t done, uint32_t n, uint32_t *dst,
                                               uint32_t miss, bool &bad) {
-    using V = VEntry<BIG>;
-    using E = typename V::E;
-    constexpr uint32_t kOff = (1u << V::kRel) - 1u, kCut = 3u << V::kRel;
     const uint32_t lane = threadIdx.x & 31;
     if (lane < n) {
         const uint32_t job = jobs[(done + lane) & (kJobWin - 1)];
-        const uint64_t w = tri[job >> 16];
+        const uint64_t w = tri[(job >> 16) & 0x3ffu];
         const uint32_t ti = job & 0xffffu, c[3] = {(uint32_t)w, (uint32_t)w >> 16, (uint32_t)(w >> 32)};
         uint32_t id[3], from = 0;
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
-            const uint32_t e = *reinterpret_cast<const E *>(vtab + ti + (c[k] & kOff));
-            const uint32_t b = (e >> (V::kRel + 2)) & 7u;
-            id[k] = nbase[b] + (e & kOff) + __popc(e & c[k] & kCut);
+            const uint32_t e = *reinterpret_cast<const uint16_t *>(vtab + ti + (c[k] & 0x3ffu));
+            const uint32_t b = (c[k] >> 10) & (job >> 26) & 7u;
+            id[k] = nbase[b] + (e & kRelMask) + __popc(e & c[k] & kCutMask);
             from |= miss >> b;
         }
         bad |= from & 1u;
