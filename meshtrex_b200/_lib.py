@@ -224,6 +224,8 @@ def lib():
             f = getattr(L, name)
             f.restype = res
             f.argtypes = args
+        L.mtxpy_copy.restype = C.c_int
+        L.mtxpy_copy.argtypes = [_P, _P, C.c_uint64, _P]
         _lib = L
     return _lib
 

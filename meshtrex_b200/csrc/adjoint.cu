@@ -243,9 +243,8 @@ extern "C" mtx_status mtx_extract_backward(mtx_context_t c, const mtx_volume *vo
     a.ws_bytes = pl.bytes + (det ? align_up(4 * T3, 128) : 0u);
     const uint32_t smem = kAdjWarps * a.ws_bytes;
     auto kern = det ? adjoint_block_kernel<true> : adjoint_block_kernel<false>;
-    MTX_CUDA(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int occ = 0;
-    MTX_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kAdjWarps * 32, smem));
+    if ((rs = ctas_per_sm(c, reinterpret_cast<const void *>(kern), kAdjWarps * 32, smem, &occ)) != MTX_OK) return rs;
     if (occ < 1) return fail(c, MTX_ERR_UNSUPPORTED, "adjoint warp layout does not fit shared memory");
     const uint32_t grid = std::min<uint32_t>((n + kAdjWarps - 1) / kAdjWarps, (uint32_t)(occ * c->sm_count));
     kern<<<grid, kAdjWarps * 32, smem, s>>>(a);

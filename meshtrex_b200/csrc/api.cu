@@ -6,6 +6,7 @@
 #include <cstdio>
 #include <cstring>
 #include <map>
+#include <memory>
 #include <mutex>
 #include <new>
 #include <string>
@@ -72,21 +73,60 @@ struct LiveAlloc {
     int device;
     size_t bytes;
 };
+// One free call's event, shared by the buffers it freed; null when the free
+// waited already.  Events go back to a pool (their creation and destruction cost
+// more than the record).
+struct FreeMark {
+    int device;
+    cudaEvent_t ev;
+    ~FreeMark();
+};
 struct IdleBuf {
-    void *ptr;
-    cudaEvent_t freed;  // recorded on the freeing stream; null when the free waited already
+    void *ptr = nullptr;
+    std::shared_ptr<FreeMark> freed;
 };
 std::mutex g_alloc_mu;
 std::unordered_map<void *, LiveAlloc> g_live;                  // every buffer dev_alloc handed out
-std::map<std::pair<int, size_t>, std::vector<IdleBuf>> g_idle;  // (device, bytes) -> freed buffers
+// (device, bytes) -> freed buffers; never destroyed, as its marks return events to the pool below
+std::map<std::pair<int, size_t>, std::vector<IdleBuf>> &g_idle = *new std::map<std::pair<int, size_t>, std::vector<IdleBuf>>;
 size_t g_idle_bytes[kCacheDevices];
 uint32_t g_idle_count[kCacheDevices];
+std::vector<cudaEvent_t> *g_events = new std::vector<cudaEvent_t>[kCacheDevices];  // idle events, at most kCacheBuffers a device
+
+// An event of the current device (which is `device`), null if there is none to be had.
+cudaEvent_t take_event(int device) {
+    {
+        std::lock_guard<std::mutex> lk(g_alloc_mu);
+        if (!g_events[device].empty()) {
+            cudaEvent_t e = g_events[device].back();
+            g_events[device].pop_back();
+            return e;
+        }
+    }
+    cudaEvent_t e = nullptr;
+    if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    return e;
+}
+
+FreeMark::~FreeMark() {  // never under g_alloc_mu
+    {
+        std::lock_guard<std::mutex> lk(g_alloc_mu);
+        if (g_events[device].size() < kCacheBuffers) {
+            g_events[device].push_back(ev);
+            return;
+        }
+    }
+    cudaEventDestroy(ev);
+}
 
 bool take_idle(int device, size_t bytes, IdleBuf *out) {
     std::lock_guard<std::mutex> lk(g_alloc_mu);
     auto it = g_idle.find({device, bytes});
     if (it == g_idle.end() || it->second.empty()) return false;
-    *out = it->second.back();
+    *out = std::move(it->second.back());
     it->second.pop_back();
     g_idle_bytes[device] -= bytes;
     --g_idle_count[device];
@@ -97,8 +137,10 @@ bool take_idle(int device, size_t bytes, IdleBuf *out) {
 // Hands the freed buffers of `device` back to the driver (that device current).
 void dev_cache_release(int device) {
     std::vector<IdleBuf> drop;
+    std::vector<cudaEvent_t> events;
     {
         std::lock_guard<std::mutex> lk(g_alloc_mu);
+        if (device >= 0 && device < kCacheDevices) events.swap(g_events[device]);
         for (auto it = g_idle.begin(); it != g_idle.end();) {
             if (it->first.first == device) {
                 for (const IdleBuf &b : it->second) {
@@ -116,12 +158,10 @@ void dev_cache_release(int device) {
         }
     }
     for (const IdleBuf &b : drop) {
-        if (b.freed) {
-            cudaEventSynchronize(b.freed);
-            cudaEventDestroy(b.freed);
-        }
+        if (b.freed) cudaEventSynchronize(b.freed->ev);
         cudaFree(b.ptr);
     }
+    for (cudaEvent_t e : events) cudaEventDestroy(e);
 }
 
 mtx_status dev_alloc(mtx_context *c, void **p, size_t bytes) {
@@ -131,16 +171,15 @@ mtx_status dev_alloc(mtx_context *c, void **p, size_t bytes) {
     }
     if (bytes == 0) bytes = 16;
     const bool cached = c->device >= 0 && c->device < kCacheDevices;
-    IdleBuf idle{nullptr, nullptr};
+    IdleBuf idle;
     if (cached && take_idle(c->device, bytes, &idle)) {
         if (idle.freed) {
             // the freeing stream's work must be done before this stream uses the buffer
-            cudaError_t e = cudaEventQuery(idle.freed);
-            if (e == cudaErrorNotReady) e = cudaStreamWaitEvent(c->stream, idle.freed, 0);
-            cudaEventDestroy(idle.freed);
+            cudaError_t e = cudaEventQuery(idle.freed->ev);
+            if (e == cudaErrorNotReady) e = cudaStreamWaitEvent(c->stream, idle.freed->ev, 0);
             if (e != cudaSuccess) {
                 cudaGetLastError();
-                cudaEventSynchronize(idle.freed);
+                cudaEventSynchronize(idle.freed->ev);
             }
         }
         *p = idle.ptr;
@@ -164,55 +203,65 @@ mtx_status dev_alloc(mtx_context *c, void **p, size_t bytes) {
     return MTX_OK;
 }
 
-void dev_free(mtx_context *c, void *p) {
-    if (!p) return;
-    LiveAlloc a{-1, 0};
-    {
-        std::lock_guard<std::mutex> lk(g_alloc_mu);
-        auto it = g_live.find(p);
-        if (it != g_live.end()) a = it->second;
-    }
-    if (a.device < 0) {
-        cudaFree(p);
-        return;
-    }
+void dev_free(mtx_context *c, std::initializer_list<void *> ptrs) {
+    std::shared_ptr<FreeMark> mark;
+    bool marked = false;
     int cur = -1;
-    cudaGetDevice(&cur);
-    if (cur != a.device) cudaSetDevice(a.device);
-    // ordered on the freeing context's stream; without one, as cudaFree (the whole device)
-    cudaEvent_t ev = nullptr;
-    if (c && c->device == a.device) {
-        if (cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) != cudaSuccess ||
-            cudaEventRecord(ev, c->stream) != cudaSuccess) {
-            cudaGetLastError();
-            if (ev) cudaEventDestroy(ev);
-            ev = nullptr;
-            cudaDeviceSynchronize();
+    for (void *p : ptrs) {
+        if (!p) continue;
+        LiveAlloc a{-1, 0};
+        {
+            std::lock_guard<std::mutex> lk(g_alloc_mu);
+            auto it = g_live.find(p);
+            if (it != g_live.end()) a = it->second;
         }
-    } else {
-        cudaDeviceSynchronize();
-    }
-    bool keep = false;
-    {
-        std::lock_guard<std::mutex> lk(g_alloc_mu);
-        if (g_idle_bytes[a.device] + a.bytes <= kCacheBytes && g_idle_count[a.device] < kCacheBuffers) {
-            g_idle[{a.device, a.bytes}].push_back(IdleBuf{p, ev});
-            g_idle_bytes[a.device] += a.bytes;
-            ++g_idle_count[a.device];
-            keep = true;
-        } else {
-            g_live.erase(p);
+        if (a.device < 0) {
+            cudaFree(p);
+            continue;
+        }
+        int now = -1;
+        cudaGetDevice(&now);
+        if (now != a.device) {
+            if (cur < 0) cur = now;
+            cudaSetDevice(a.device);
+            marked = false;
+        }
+        if (!marked) {
+            // ordered on the freeing context's stream; without one, as cudaFree (the whole device)
+            marked = true;
+            mark.reset();
+            cudaEvent_t ev = c && c->device == a.device ? take_event(a.device) : nullptr;
+            if (ev) mark.reset(new FreeMark{a.device, ev});
+            if (!ev || cudaEventRecord(ev, c->stream) != cudaSuccess) {
+                cudaGetLastError();
+                mark.reset();
+                cudaDeviceSynchronize();
+            }
+        }
+        bool keep = false;
+        {
+            std::lock_guard<std::mutex> lk(g_alloc_mu);
+            if (g_idle_bytes[a.device] + a.bytes <= kCacheBytes && g_idle_count[a.device] < kCacheBuffers) {
+                IdleBuf b;
+                b.ptr = p;
+                b.freed = mark;
+                g_idle[{a.device, a.bytes}].push_back(std::move(b));
+                g_idle_bytes[a.device] += a.bytes;
+                ++g_idle_count[a.device];
+                keep = true;
+            } else {
+                g_live.erase(p);
+            }
+        }
+        if (!keep) {
+            if (mark) cudaEventSynchronize(mark->ev);
+            cudaFree(p);
         }
     }
-    if (!keep) {
-        if (ev) {
-            cudaEventSynchronize(ev);
-            cudaEventDestroy(ev);
-        }
-        cudaFree(p);
-    }
-    if (cur >= 0 && cur != a.device) cudaSetDevice(cur);
+    if (cur >= 0) cudaSetDevice(cur);
 }
+
+void dev_free(mtx_context *c, void *p) { dev_free(c, {p}); }
 
 mtx_status scratch_reserve(mtx_context *c, Scratch &s, size_t bytes) {
     if (s.size >= bytes && s.ptr) return MTX_OK;
@@ -281,6 +330,22 @@ void mip_layout(const uint32_t g[3], int levels, uint32_t ext[][3], uint64_t *of
         off += (uint64_t)ext[l][0] * ext[l][1] * ext[l][2];
     }
     *total = off;
+}
+
+// CTAs of a kernel that fit an SM, asked for once a context: the two runtime
+// calls cost 3 us a launch.  The kernel's dynamic shared memory limit is raised to
+// the device's own, so that no later launch of it with more meets a lower one.
+mtx_status ctas_per_sm(mtx_context *c, const void *kernel, int threads, uint32_t smem, int *out) {
+    for (const auto &o : c->occupancy)
+        if (o.kernel == kernel && o.threads == threads && o.smem == smem) {
+            *out = o.ctas;
+            return MTX_OK;
+        }
+    MTX_CUDA(c, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, c->max_smem_optin));
+    MTX_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(out, kernel, threads, smem));
+    if (c->occupancy.size() >= 64) c->occupancy.clear();
+    c->occupancy.push_back({kernel, threads, smem, *out});
+    return MTX_OK;
 }
 
 // ------------------------------------------------------------ tensor maps
@@ -376,7 +441,15 @@ DevStatus bc_take_batched();
 DevStatus bc_take_adjoint();
 #endif
 
-static mtx_status check_device_status(mtx_context *c) {
+// Waits for the context's stream and reports (and clears) any error its kernels
+// recorded.  words: also copies that many words from src to c->pinned, in the
+// same wait -- a blocking copy of the error word after each count cost 10 us of
+// a small extraction's time, three times a pass.
+static mtx_status sync_and_check(mtx_context *c, const void *src = nullptr, uint32_t words = 0) {
+    DevStatus *h = reinterpret_cast<DevStatus *>(c->pinned + 8);
+    if (words) MTX_CUDA(c, cudaMemcpyAsync(c->pinned, src, 4 * words, cudaMemcpyDeviceToHost, c->stream));
+    MTX_CUDA(c, cudaMemcpyAsync(h, &c->ctrl->status, sizeof(*h), cudaMemcpyDeviceToHost, c->stream));
+    MTX_CUDA(c, cudaStreamSynchronize(c->stream));
 #ifdef MTX_BOUNDS_CHECK
     // a bounds-check build: the translation units' check records first
     for (DevStatus b : {bc_take_extract(), bc_take_filter(), bc_take_minmax(), bc_take_batched(), bc_take_adjoint()})
@@ -387,13 +460,12 @@ static mtx_status check_device_status(mtx_context *c) {
             return fail(c, MTX_ERR_INTERNAL, buf);
         }
 #endif
-    DevStatus h;
-    MTX_CUDA(c, cudaMemcpy(&h, &c->ctrl->status, sizeof(h), cudaMemcpyDeviceToHost));
-    if (h.code == 0) return MTX_OK;
-    MTX_CUDA(c, cudaMemset(&c->ctrl->status, 0, sizeof(h)));
+    if (h->code == 0) return MTX_OK;
+    const DevStatus e = *h;
+    MTX_CUDA(c, cudaMemset(&c->ctrl->status, 0, sizeof(e)));
     char buf[160];
-    snprintf(buf, sizeof(buf), "device error %u at site %u (info %u, %u)", h.code, h.where, h.info0, h.info1);
-    return fail(c, (mtx_status)h.code, buf);
+    snprintf(buf, sizeof(buf), "device error %u at site %u (info %u, %u)", e.code, e.where, e.info0, e.info1);
+    return fail(c, (mtx_status)e.code, buf);
 }
 
 }  // namespace mtx
@@ -489,8 +561,7 @@ mtx_status mtx_synchronize(mtx_context_t c) {
     if (!c) return MTX_ERR_INVALID_ARG;
     DeviceGuard g(c->device);
     join_extract(c);
-    MTX_CUDA(c, cudaStreamSynchronize(c->stream));
-    return check_device_status(c);
+    return sync_and_check(c);
 }
 
 mtx_status mtx_debug_fail_allocation(mtx_context_t c, uint32_t k) {
@@ -771,9 +842,7 @@ mtx_status mtx_read_active_block_count(mtx_context_t c, mtx_filtering_output *f)
     if (!c || !f || !f->activeBlockCountBuffer.ptr) return MTX_ERR_INVALID_ARG;
     DeviceGuard g(c->device);
     join_extract(c);
-    MTX_CUDA(c, cudaMemcpyAsync(c->pinned, f->activeBlockCountBuffer.ptr, 4, cudaMemcpyDeviceToHost, c->stream));
-    MTX_CUDA(c, cudaStreamSynchronize(c->stream));
-    mtx_status r = check_device_status(c);
+    mtx_status r = sync_and_check(c, f->activeBlockCountBuffer.ptr, 1);
     if (r != MTX_OK) return r;
     f->activeBlockCount = c->pinned[0];
     return MTX_OK;
@@ -794,9 +863,7 @@ mtx_status mtx_filtering_free(mtx_context_t c, mtx_filtering_output *f) {
     if (!c || !f) return MTX_ERR_INVALID_ARG;
     DeviceGuard g(c->device);
     join_extract(c);
-    dev_free(c, f->compactedBlockIdBuffer.ptr);
-    dev_free(c, f->activeBlockCountBuffer.ptr);
-    dev_free(c, f->blockRankBuffer.ptr);
+    dev_free(c, {f->compactedBlockIdBuffer.ptr, f->activeBlockCountBuffer.ptr, f->blockRankBuffer.ptr});
     memset(f, 0, sizeof(*f));
     return MTX_OK;
 }
@@ -872,10 +939,7 @@ mtx_status mtx_extract_meshlet_descriptors(mtx_context_t c, const mtx_minmax_out
     prof_end(prof, c->stream);
     if (r != MTX_OK) return bail(r);
     // exact output sizes: one 8-byte readback instead of worst-case buffers
-    cudaError_t e = cudaMemcpyAsync(c->pinned, counters, 8, cudaMemcpyDeviceToHost, c->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-    if (e != cudaSuccess) return bail(cuda_fail(c, e, "count readback"));
-    if ((r = check_device_status(c)) != MTX_OK) return bail(r);
+    if ((r = sync_and_check(c, counters, 2)) != MTX_OK) return bail(r);
     const uint32_t V = c->pinned[0], I = c->pinned[1];
     void *vb = nullptr, *ib = nullptr;
     if ((r = dev_alloc(c, &vb, (size_t)V * out->vertexStride)) != MTX_OK) return bail(r);
@@ -905,10 +969,8 @@ mtx_status mtx_extraction_free(mtx_context_t c, mtx_extraction_output *x) {
     if (!c || !x) return MTX_ERR_INVALID_ARG;
     DeviceGuard g(c->device);
     join_extract(c);
-    dev_free(c, x->vertexBuffer.ptr);
-    dev_free(c, x->indexBuffer.ptr);
-    dev_free(c, x->meshletDescriptorBuffer.ptr);
-    dev_free(c, x->vertexCountBuffer.ptr);  // the three counters share one allocation
+    dev_free(c, {x->vertexBuffer.ptr, x->indexBuffer.ptr, x->meshletDescriptorBuffer.ptr,
+                 x->vertexCountBuffer.ptr});  // the three counters share one allocation
     const uint32_t stride = x->vertexStride;
     memset(x, 0, sizeof(*x));
     x->vertexStride = stride;
@@ -1124,6 +1186,14 @@ mtx_status mtx_profiler_export_csv(mtx_profiler_t p, const char *path) {
         fprintf(f, "%s,%.6f,%.6f,%u\n", r.name.c_str(), r.last_ms, r.frames ? r.sum_ms / r.frames : 0.0, r.frames);
     fclose(f);
     return MTX_OK;
+}
+
+// A copy between device buffers on the given stream, for the Python front end's
+// accessors (not part of the C ABI).
+int mtxpy_copy(void *dst, const void *src, uint64_t bytes, void *stream) {
+    const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToDevice, (cudaStream_t)stream);
+    if (e != cudaSuccess) cudaGetLastError();
+    return (int)e;
 }
 
 }  // extern "C"

@@ -342,9 +342,9 @@ static bool use_tma(const Problem &p, uint32_t staging) {
 template <typename K>
 static mtx_status grid_for(mtx_context *c, K kernel, int threads, uint32_t smem, uint32_t host_count, int warps,
                            unsigned &grid) {
-    MTX_CUDA(c, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int per_sm = 0;
-    MTX_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem));
+    const mtx_status r = ctas_per_sm(c, reinterpret_cast<const void *>(kernel), threads, smem, &per_sm);
+    if (r != MTX_OK) return r;
     if (per_sm < 1) return fail(c, MTX_ERR_UNSUPPORTED, "extraction kernel does not fit on an SM");
     if (c->tuning.extractCtasPerSm) per_sm = std::min(per_sm, (int)c->tuning.extractCtasPerSm);
     uint64_t g = (uint64_t)per_sm * c->sm_count;

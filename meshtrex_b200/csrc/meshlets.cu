@@ -202,8 +202,8 @@ extern "C" mtx_status mtx_build_meshlets(mtx_context_t c, const mtx_extraction_o
     if (e != cudaSuccess) return bail(cuda_fail(c, e, "meshlet count launch"));
     if ((r = launch_desc_scan(c, (mtx_meshlet_descriptor *)per_block, count, nb, (uint32_t *)counters, s)) != MTX_OK)
         return bail(r);
-    uint32_t tot[4];
-    if ((e = cudaMemcpyAsync(tot, counters, sizeof(tot), cudaMemcpyDeviceToHost, s)) == cudaSuccess)
+    uint32_t *tot = c->pinned;
+    if ((e = cudaMemcpyAsync(tot, counters, 16, cudaMemcpyDeviceToHost, s)) == cudaSuccess)
         e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return bail(cuda_fail(c, e, "meshlet totals"));
     const uint32_t MV = tot[0], M = tot[1] / 3u;
@@ -235,8 +235,7 @@ extern "C" mtx_status mtx_build_meshlets(mtx_context_t c, const mtx_extraction_o
                                                                (const uint32_t *)p_mv, MV, stride, (float *)p_vd);
     if ((e = cudaGetLastError()) != cudaSuccess) return bail(cuda_fail(c, e, "meshlet gather launch"));
     if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return bail(cuda_fail(c, e, "meshlet build"));
-    dev_free(c, per_block);
-    dev_free(c, counters);
+    dev_free(c, {per_block, counters});
     out->meshletCount = M;
     out->vertexCount = MV;
     out->indexCount = 3u * T;
@@ -247,10 +246,8 @@ extern "C" mtx_status mtx_meshlet_output_free(mtx_context_t c, mtx_meshlet_outpu
     if (!c || !out) return MTX_ERR_INVALID_ARG;
     DeviceGuard dg(c->device);
     join_extract(c);
-    dev_free(c, out->meshletDescriptorBuffer.ptr);
-    dev_free(c, out->meshletVertexBuffer.ptr);
-    dev_free(c, out->vertexBuffer.ptr);
-    dev_free(c, out->indexBuffer.ptr);
+    dev_free(c, {out->meshletDescriptorBuffer.ptr, out->meshletVertexBuffer.ptr, out->vertexBuffer.ptr,
+                 out->indexBuffer.ptr});
     const uint32_t stride = out->vertexStride;
     memset(out, 0, sizeof(*out));
     out->vertexStride = stride;

@@ -5,7 +5,9 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <initializer_list>
 #include <string>
+#include <vector>
 
 #include "meshtrex/mtx.h"
 #include "mtx_device.cuh"
@@ -59,6 +61,13 @@ struct mtx_context {
     cudaEvent_t ev_filtered = nullptr;   // filter done on `stream` (the extraction may start)
     cudaEvent_t ev_extracted = nullptr;  // extraction done on `xstream` (the scratch is free again)
     bool extract_pending = false;        // ev_extracted recorded and not yet joined into `stream`
+    struct Occupancy {
+        const void *kernel;
+        int threads;
+        uint32_t smem;
+        int ctas;
+    };
+    std::vector<Occupancy> occupancy;  // ctas_per_sm
 };
 
 namespace mtx {
@@ -85,7 +94,9 @@ mtx_status cuda_fail(mtx_context *c, cudaError_t e, const char *what);
     } while (0)
 
 mtx_status dev_alloc(mtx_context *c, void **p, size_t bytes);
+void dev_free(mtx_context *c, std::initializer_list<void *> ptrs);
 void dev_free(mtx_context *c, void *p);  // ordered on c's stream (c may be null: a device-wide wait)
+mtx_status ctas_per_sm(mtx_context *c, const void *kernel, int threads, uint32_t smem, int *out);
 mtx_status scratch_reserve(mtx_context *c, Scratch &s, size_t bytes);
 // Makes the context's stream wait for an extraction still running on its
 // extraction stream (mtx_context_set_extract_stream); every entry point that
