@@ -3,21 +3,28 @@
 // this differentiates is the vertex placement of marching_cubes_pmb.mesh.glsl:
 // 122-141, p = u + t * e_axis with t = (iso - f(u)) / (f(u + e_axis) - f(u)).
 //
-// One warp per active block restages the block's (B+1)^3 tile as float,
-// rebuilds the crossing masks and vertex prefixes exactly as the forward
-// passes do (so vertex ids follow the forward's canonical order), and for
-// each of the block's vertices recomputes t's inputs from the volume:
+// One warp per active block builds the inside bits of the block's rows from the
+// volume, lists the voxels that own a cut edge in canonical order (so vertex
+// ids follow the forward's) and, axis by axis, one voxel a lane, recomputes t's
+// inputs:
 //   dL/df(u)  = g (iso - f(v)) / d^2,  dL/df(v) = g (f(u) - iso) / d^2,
 //   dL/diso   = g / d,                 d = f(v) - f(u), v = u + e_axis.
 // ATOMIC mode adds the field terms into dL/dfield with FP32 atomics.
 // DETERMINISTIC mode accumulates them into a private (B+1)^3 tile in shared
 // memory in six sweeps (axis x, y, z; the edge's first, then second voxel),
-// in each of which every tile voxel has at most one writer, writes the tile
-// out as the block's partial, and a gather pass then gives every voxel one
-// designated block that sums the partials of the up to 8 blocks whose tiles
-// hold it, in a fixed order.  dL/diso is summed per block and then over
-// blocks in rank order in both modes.
-#include "pmb_device.cuh"
+// in each of which every tile voxel has at most one writer.  The tile's inner
+// voxels belong to this block alone and go straight to dL/dfield; the others
+// are kept as the block's partial, and a gather pass gives each of them one
+// designated block that sums the partials of the blocks that own an edge at it
+// -- its own block and those before it in x, y and z -- in that order.  dL/diso
+// is summed per block -- each lane over its rows, axis by axis, so that the sum does
+// not depend on how the list fell into steps -- and then over blocks in rank order
+// in both modes.
+// Staging each tile as float and walking its rows took 49 us (ATOMIC) for the
+// 7,700 active blocks of a 512^3 volume, after 88 us of zeroing, and 34 us, with
+// 36 us for a gather over whole tiles, for the 1,250 of 250 x 198 x 171
+// (DETERMINISTIC); this takes 31, and 14 with 9.
+#include "pmb_lists.cuh"
 
 namespace mtx {
 
@@ -38,77 +45,198 @@ struct AdjArgs {
     float *partial;       // DETERMINISTIC: T3 floats per active block
     float *iso_part;      // dL/diso of each active block
     uint32_t T3;          // (B+1)^3
-    uint32_t ws_bytes;    // shared memory per warp
-    uint32_t off_acc;     // accumulation tile inside the warp's shared memory
     DevStatus *st;
 };
 
-template <bool DET>
+// Listed voxels of a block whose dL/diso terms are kept in shared memory.
+__host__ __device__ inline uint32_t iso_terms(uint32_t B) { return B <= 8 ? 256u : 768u; }
+
+// A warp's shared memory: inside rows, list bits, list, the plain loads'
+// bitstream, dL/diso terms, and for DETERMINISTIC the accumulation tile
+// (off_tile).
+__host__ __device__ inline WPlan make_adjoint_plan(uint32_t B, bool det) {
+    WPlan p{};
+    plan_block(p, B);
+    const uint32_t T3 = p.B1 * p.B1 * p.B1;
+    uint32_t o = 0;
+    p.off_rows = o;
+    o = align_up(o + 4 * p.B1 * p.B1, 16);
+    p.off_mm = o;
+    o = align_up(o + 4 * list_words(B), 16);
+    p.off_list = o;
+    o = align_up(o + 2 * list_cap(B), 16);
+    p.off_case = o;
+    o = align_up(o + 4 * ((T3 + 31) / 32 + 1), 16);
+    p.off_vp = o;  // dL/diso terms, axis by axis
+    o += 12 * iso_terms(B);
+    p.off_tile = o;
+    if (det) o = align_up(o + 4 * T3, 16);
+    p.bytes = o;
+    return p;
+}
+
+// List bits of the voxels that own a cut edge.  Lane l takes rows [l R, l R + R),
+// R = ceil(B^2 / 32): its listed voxels are list[at, at + n), its vertices the
+// block's from vat on; nl and nv are the block's.
+struct CutRows {
+    uint32_t at, n, vat, nl, nv;
+};
+template <int BC>
+__device__ __forceinline__ CutRows cut_bits(const Problem &p, const WPlan &pl, unsigned char *ws, const Geo &g) {
+    const uint32_t lane = threadIdx.x & 31, B = pl.B, R = (pl.BB + 31) / 32;
+    const uint32_t *rows = reinterpret_cast<const uint32_t *>(ws + pl.off_rows);
+    uint32_t *bits = reinterpret_cast<uint32_t *>(ws + pl.off_mm);
+    for (uint32_t i = lane; i < list_words(B); i += 32) bits[i] = 0;
+    __syncwarp();
+    CutRows c{};
+    uint32_t nv = 0;
+    for (uint32_t q = lane * R; q < min(pl.BB, lane * R + R); ++q) {
+        const uint32_t z = fdiv(q, pl.rB), y = q - z * B;
+        uint32_t xc, yc, zc;
+        row_cross(p, pl, g, rows, y, z, xc, yc, zc);
+        nv += __popc(xc) + __popc(yc) + __popc(zc);
+        const uint32_t m = xc | yc | zc;
+        c.n += __popc(m);
+        if constexpr (BC == 8) {
+            reinterpret_cast<uint8_t *>(bits)[q] = (uint8_t)m;
+        } else if (m) {
+            const uint32_t b = q * B, w = b >> 5, s = b & 31u;
+            atomicOr(&bits[w], m << s);
+            if (s + B > 32) atomicOr(&bits[w + 1], m >> (32 - s));
+        }
+    }
+    __syncwarp();
+    c.at = warp_excl_scan(c.n, c.nl);
+    c.vat = warp_excl_scan(nv, c.nv);
+    return c;
+}
+
+// One vertex's dL/diso term (the gradient along its edge over the edge's value
+// difference); 0 where t = 0.5.
+__device__ __forceinline__ float iso_term(float gv, float scale, float den) {
+    return fabsf(den) > 1e-5f ? __fdiv_rn(__fmul_rn(gv, scale), den) : 0.0f;
+}
+
+template <typename T, bool DET, int BC>
 __global__ void __launch_bounds__(kAdjWarps * 32) adjoint_block_kernel(const __grid_constant__ AdjArgs a) {
+    constexpr bool kBig = BC == 0;  // the run-time form's list rounds; BC = 8 has one
     extern __shared__ __align__(128) unsigned char smem[];
-    const Problem &p = a.p;
-    const WPlan pl = make_wplan(p.B);
+    Problem p = a.p;
+    if (BC) p.B = BC;
+    const WPlan pl = make_adjoint_plan(p.B, DET);
+    const GridDiv dv = grid_div(p);
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, W = blockDim.x >> 5;
-    unsigned char *ws = smem + warp * a.ws_bytes;
-    float *tile = reinterpret_cast<float *>(ws + pl.off_tile);
-    float *acc = reinterpret_cast<float *>(ws + a.off_acc);
-    const uint32_t *cross = reinterpret_cast<const uint32_t *>(ws + pl.off_cross);
-    const uint32_t *vp = reinterpret_cast<const uint32_t *>(ws + pl.off_vp);
-    const uint32_t B = pl.B, BB = pl.BB, B1 = pl.B1, R = (BB + 31) / 32;
+    unsigned char *ws = smem + warp * pl.bytes;
+    float *acc = reinterpret_cast<float *>(ws + pl.off_tile);
+    const uint32_t *rows = reinterpret_cast<const uint32_t *>(ws + pl.off_rows);
+    const uint16_t *list = reinterpret_cast<const uint16_t *>(ws + pl.off_list);
+    float *term = reinterpret_cast<float *>(ws + pl.off_vp);
+    const uint32_t B = pl.B, B1 = pl.B1, T3 = B1 * B1 * B1;
     const float iso = p.iso;
     for (uint32_t r = blockIdx.x * W + warp; r < a.n; r += gridDim.x * W) {
-        const uint32_t id = __ldg(a.ids + r);
-        const Geo g = block_geo(id, p, false, 4);
+        const Geo g = block_geo(__ldg(a.ids + r), p, false, 4, dv);
         const uint4 dq = __ldg(reinterpret_cast<const uint4 *>(a.desc + r));
         const uint32_t vbase = dq.x, nv = dq.z;
-        tile_load_float(p, pl, tile, g);
-        build_rows<float>(p, pl, ws, g);
-        uint32_t bnv, bnt;
-        block_counts(p, pl, ws, g, nullptr, false, bnv, bnt);
-        const bool ok = bnv == nv && (uint64_t)vbase + nv <= a.vcount;
-        if (!ok && lane == 0) report(a.st, MTX_ERR_INTERNAL, kSiteAdjoint, r, bnv);
+        const bool inner = g.ox + B < p.X && g.oy + B < p.Y && g.oz + B < p.Z;
+        load_rows<T, BC>(p, pl, ws, g, nullptr);
+        const CutRows cr = cut_bits<BC>(p, pl, ws, g);
+        const bool ok = cr.nv == nv && (uint64_t)vbase + nv <= a.vcount;
+        if (!ok && lane == 0) report(a.st, MTX_ERR_INTERNAL, kSiteAdjoint, r, cr.nv);
         if (DET) {
-            for (uint32_t i = lane; i < a.T3; i += 32) acc[i] = 0.0f;
+            for (uint32_t i = lane; i < T3; i += 32) acc[i] = 0.0f;
             __syncwarp();
         }
-        float diso = 0.0f;
-        if (ok) {
-            for (uint32_t ax = 0; ax < 3; ++ax) {
-                const uint32_t step = ax == 0 ? 1u : ax == 1 ? B1 : B1 * B1;
-                const uint64_t gstep = ax == 0 ? 1ull : ax == 1 ? (uint64_t)p.X : (uint64_t)p.X * p.Y;
-                for (uint32_t role = 0; role < (DET ? 2u : 1u); ++role) {
-                    for (uint32_t k = 0; k < R; ++k) {
-                        const uint32_t q = lane * R + k;
-                        if (q >= BB) break;
-                        const uint32_t z = fdiv(q, pl.rB), y = q - z * B;
-                        uint32_t m = cross[ax * BB + q];
-                        while (m) {
-                            const uint32_t x = __ffs(m) - 1;
-                            m &= m - 1u;
-                            uint32_t vid = vbase + voxel_prefix(cross, vp, BB, q, x);
-                            for (uint32_t b = 0; b < ax; ++b) vid += (cross[b * BB + q] >> x) & 1u;
-                            const uint32_t i0 = (z * B1 + y) * B1 + x, i1 = i0 + step;
-                            const float fa = tile[i0], fb = tile[i1];
-                            const float den = __fsub_rn(fb, fa);
-                            if (!(fabsf(den) > 1e-5f)) continue;  // t = 0.5: no gradient
-                            const float gv = __fmul_rn(__ldg(a.g + (uint64_t)vid * a.gstride + ax), a.gscale[ax]);
-                            const float s = __fdiv_rn(gv, den);
-                            if (DET) {
-                                if (role == 0) {
-                                    acc[i0] = __fadd_rn(acc[i0], __fdiv_rn(__fmul_rn(s, __fsub_rn(iso, fb)), den));
-                                    diso = __fadd_rn(diso, s);
-                                } else {
-                                    acc[i1] = __fadd_rn(acc[i1], __fdiv_rn(__fmul_rn(s, __fsub_rn(fa, iso)), den));
-                                }
-                            } else {
-                                const uint64_t v0 = ((uint64_t)(g.oz + z) * p.Y + (g.oy + y)) * p.X + (g.ox + x);
-                                atomicAdd(a.dfield + v0, __fdiv_rn(__fmul_rn(s, __fsub_rn(iso, fb)), den));
-                                atomicAdd(a.dfield + v0 + gstep, __fdiv_rn(__fmul_rn(s, __fsub_rn(fa, iso)), den));
-                                diso = __fadd_rn(diso, s);
-                            }
-                        }
+        const uint32_t nterm = iso_terms(B);
+        const bool keep = cr.nl <= nterm;  // else the terms are computed again below
+        ListWalk l;
+        uint32_t run = vbase, seen = 0;
+        while (const uint32_t n = !ok ? 0u : !kBig ? list_next<false>(l, pl, ws)
+                                           : B > 8 ? list_next<true>(l, pl, ws) : list_next<false>(l, pl, ws)) {
+            uint32_t m = 0, cell = 0;
+            if (lane < n) {
+                cell = list[l.done + lane];
+                m = listed_cell(p, pl, g, rows, cell, inner) >> 28;
+            }
+            uint32_t vt;
+            const uint32_t first = run + step_vertices(m, vt);
+            const uint32_t q = fdiv(cell, pl.rB), x = cell - q * B, z = fdiv(q, pl.rB), y = q - z * B;
+            const uint64_t v0 = ((uint64_t)(g.oz + z) * p.Y + (g.oy + y)) * p.X + (g.ox + x);
+            const uint64_t gstep[3] = {1ull, (uint64_t)p.X, (uint64_t)p.X * p.Y};
+            const T *v = reinterpret_cast<const T *>(p.vol) + v0;
+            // the voxel, its cut neighbours and their vertices' gradients, all loads in flight
+            T raw[4] = {T(0), T(0), T(0), T(0)};
+            float gv[3] = {0.0f, 0.0f, 0.0f};
+            if (m) raw[3] = __ldg(v);
+#pragma unroll
+            for (uint32_t k = 0; k < 3; ++k)
+                if ((m >> k) & 1u) {
+                    raw[k] = __ldg(v + gstep[k]);
+                    gv[k] = __ldg(a.g + (uint64_t)(first + __popc(m & ((1u << k) - 1u))) * a.gstride + k);
+                }
+            const float fa = Vox<T>::val(raw[3]);
+            float own = 0.0f, far[3];
+            bool on[3];
+#pragma unroll
+            for (uint32_t k = 0; k < 3; ++k) {
+                const float fb = Vox<T>::val(raw[k]), den = __fsub_rn(fb, fa);
+                on[k] = ((m >> k) & 1u) && fabsf(den) > 1e-5f;  // else t = 0.5: no gradient
+                far[k] = 0.0f;
+                const float s = (m >> k) & 1u ? iso_term(gv[k], a.gscale[k], den) : 0.0f;
+                if (keep && lane < n) term[k * nterm + seen + lane] = s;
+                if (on[k]) {
+                    const float ta = __fdiv_rn(__fmul_rn(s, __fsub_rn(iso, fb)), den);
+                    far[k] = __fdiv_rn(__fmul_rn(s, __fsub_rn(fa, iso)), den);
+                    if (DET) {
+                        own = __fadd_rn(own, ta);
+                    } else {
+                        atomicAdd(a.dfield + v0, ta);
+                        atomicAdd(a.dfield + v0 + gstep[k], far[k]);
                     }
-                    if (DET) __syncwarp();
+                }
+            }
+            if (DET) {
+                // one writer a tile voxel in each of the four additions
+                const uint32_t i = (z * B1 + y) * B1 + x;
+                if (m) acc[i] = __fadd_rn(acc[i], own);
+                __syncwarp();
+#pragma unroll
+                for (uint32_t k = 0; k < 3; ++k) {
+                    const uint32_t j = i + (k == 0 ? 1u : k == 1 ? B1 : B1 * B1);
+                    if (on[k]) acc[j] = __fadd_rn(acc[j], far[k]);
+                    __syncwarp();
+                }
+            }
+            run += vt;
+            seen += n;
+            l.done += n;
+        }
+        // dL/diso: each lane its rows' terms, axis by axis in canonical order, then the lanes' sums
+        float diso = 0.0f;
+        __syncwarp();
+        if (ok && keep) {
+            for (uint32_t k = 0; k < 3; ++k)
+                for (uint32_t i = cr.at; i < cr.at + cr.n; ++i) diso = __fadd_rn(diso, term[k * nterm + i]);
+        } else if (ok) {
+            const uint32_t R = (pl.BB + 31) / 32;
+            for (uint32_t k = 0; k < 3; ++k) {
+                uint64_t vid = vbase + cr.vat;
+                for (uint32_t q = lane * R; q < min(pl.BB, lane * R + R); ++q) {
+                    const uint32_t z = fdiv(q, pl.rB), y = q - z * B;
+                    uint32_t xc, yc, zc;
+                    row_cross(p, pl, g, rows, y, z, xc, yc, zc);
+                    for (uint32_t any = xc | yc | zc; any; any &= any - 1u) {
+                        const uint32_t x = __ffs(any) - 1;
+                        const uint32_t m = ((xc >> x) & 1u) | (((yc >> x) & 1u) << 1) | (((zc >> x) & 1u) << 2);
+                        if ((m >> k) & 1u) {
+                            const T *v = reinterpret_cast<const T *>(p.vol) +
+                                         ((uint64_t)(g.oz + z) * p.Y + (g.oy + y)) * p.X + (g.ox + x);
+                            const uint64_t step = k == 0 ? 1ull : k == 1 ? (uint64_t)p.X : (uint64_t)p.X * p.Y;
+                            const float den = __fsub_rn(Vox<T>::val(__ldg(v + step)), Vox<T>::val(__ldg(v)));
+                            const float gk = __ldg(a.g + (vid + __popc(m & ((1u << k) - 1u))) * a.gstride + k);
+                            diso = __fadd_rn(diso, iso_term(gk, a.gscale[k], den));
+                        }
+                        vid += __popc(m);
+                    }
                 }
             }
         }
@@ -116,51 +244,105 @@ __global__ void __launch_bounds__(kAdjWarps * 32) adjoint_block_kernel(const __g
         for (int o = 16; o; o >>= 1) diso = __fadd_rn(diso, __shfl_xor_sync(0xffffffffu, diso, o));
         if (lane == 0) a.iso_part[r] = diso;
         if (DET) {
-            float *dst = a.partial + (uint64_t)r * a.T3;
-            for (uint32_t i = lane; i < a.T3; i += 32) dst[i] = acc[i];
+            __syncwarp();
+            float *dst = a.partial + (uint64_t)r * T3;
+            for (uint32_t i = lane; i < T3; i += 32) {
+                const uint32_t iq = fdiv(i, pl.rB1), lx = i - iq * B1, lz = fdiv(iq, pl.rB1), ly = iq - lz * B1;
+                const float t = acc[i];
+                if (lx % B == 0 || ly % B == 0 || lz % B == 0)  // shared with a neighbour: the gather pass's
+                    dst[i] = t;
+                else if (t != 0.0f)  // (voxels outside the volume have none)
+                    a.dfield[((uint64_t)(g.oz + lz) * p.Y + (g.oy + ly)) * p.X + (g.ox + lx)] = t;
+            }
         }
         __syncwarp();
     }
 }
 
-// DETERMINISTIC: each voxel of an active block's (B+1)^3 tile is written by
-// one designated block, the first active block in the order
-// c(w) - (0,0,0), -(1,0,0), -(0,1,0), -(1,1,0), -(0,0,1), ... among those
-// whose tiles hold w (c(w) the block containing w), as the sum of their
-// partials in that order.
+// DETERMINISTIC: the voxels on the faces of the active blocks' tiles.  A voxel w
+// of block c gets terms from edges that c owns and, where it lies on c's low x,
+// y or z face, from the edge that the block before c on that axis owns; the
+// first active one of c, c - x, c - y, c - z writes the sum, taken in that order.
 __global__ void __launch_bounds__(kAdjWarps * 32) adjoint_gather_kernel(const __grid_constant__ AdjArgs a) {
     const Problem &p = a.p;
+    const GridDiv dv = grid_div(p);
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, W = blockDim.x >> 5;
-    const uint32_t B = p.B, B1 = B + 1;
-    const uint32_t rB1 = (uint32_t)((0x100000000ull + B) / B1);
+    const uint32_t B = p.B, B1 = B + 1, BB = B * B;
+    const uint32_t rB = (uint32_t)((0x100000000ull + B - 1) / B);
+    const uint32_t st[3] = {1u, B1, B1 * B1};  // tile steps
     for (uint32_t r = blockIdx.x * W + warp; r < a.n; r += gridDim.x * W) {
-        const uint32_t id = __ldg(a.ids + r);
-        const Geo g = block_geo(id, p, false, 4);
-        for (uint32_t i = lane; i < a.T3; i += 32) {
-            const uint32_t iq = fdiv(i, rB1);
-            const uint32_t lx = i - iq * B1, lz = fdiv(iq, rB1), ly = iq - lz * B1;
-            const uint32_t wx = g.ox + lx, wy = g.oy + ly, wz = g.oz + lz;
-            if (wx >= p.X || wy >= p.Y || wz >= p.Z) continue;
-            // containing block and the coordinates of w in it
-            const uint32_t cx = g.bx + (lx == B), cy = g.by + (ly == B), cz = g.bz + (lz == B);
-            const uint32_t ux = lx == B ? 0 : lx, uy = ly == B ? 0 : ly, uz = lz == B ? 0 : lz;
-            uint32_t first = kNoVertex;
-            float sum = 0.0f;
-            for (uint32_t d = 0; d < 8; ++d) {
-                const uint32_t dx = d & 1u, dy = (d >> 1) & 1u, dz = d >> 2;
-                if ((dx && (ux || !cx)) || (dy && (uy || !cy)) || (dz && (uz || !cz))) continue;
-                const uint32_t bx = cx - dx, by = cy - dy, bz = cz - dz;
-                if (bx >= p.GX || by >= p.GY || bz >= p.GZ) continue;
-                const uint32_t rk = __ldg(a.rank_map + ((uint64_t)bz * p.GY + by) * p.GX + bx);
-                if (rk == kNoVertex) continue;
-                if (first == kNoVertex) {
-                    first = rk;
-                    if (first != r) break;
-                }
-                const uint32_t j = ((uz + dz * B) * B1 + (uy + dy * B)) * B1 + (ux + dx * B);
-                sum = __fadd_rn(sum, __ldcg(a.partial + (uint64_t)rk * a.T3 + j));
+        const Geo g = block_geo(__ldg(a.ids + r), p, false, 4, dv);
+        // ranks, one a lane: lanes 0-2 the blocks before this one along x, y, z; 3-5 those after it; 6 + 2 k, 7 + 2 k
+        // the blocks before the one after it along axis k, on the other two axes in order
+        uint32_t rk = kNoVertex;
+        if (lane < 12) {
+            int b[3] = {(int)g.bx, (int)g.by, (int)g.bz};
+            if (lane < 3) {
+                --b[lane];
+            } else if (lane < 6) {
+                ++b[lane - 3];
+            } else {
+                const uint32_t k = (lane - 6) >> 1, o = (lane & 1u) ? (k == 2 ? 1u : 2u) : (k == 0 ? 1u : 0u);
+                ++b[k];
+                --b[o];
             }
-            if (first == r) a.dfield[((uint64_t)wz * p.Y + wy) * p.X + wx] = sum;
+            if (b[0] >= 0 && b[1] >= 0 && b[2] >= 0 && b[0] < (int)p.GX && b[1] < (int)p.GY && b[2] < (int)p.GZ)
+                rk = __ldg(a.rank_map + ((uint64_t)b[2] * p.GY + b[1]) * p.GX + b[0]);
+        }
+        uint32_t nb[12];
+#pragma unroll
+        for (int k = 0; k < 12; ++k) nb[k] = __shfl_sync(0xffffffffu, rk, k);
+        const float *own = a.partial + (uint64_t)r * a.T3;
+        auto put = [&](uint32_t lx, uint32_t ly, uint32_t lz, float t) {
+            const uint32_t wx = g.ox + lx, wy = g.oy + ly, wz = g.oz + lz;
+            if (t != 0.0f && wx < p.X && wy < p.Y && wz < p.Z)
+                a.dfield[((uint64_t)wz * p.Y + wy) * p.X + wx] = t;
+        };
+        auto from = [&](uint32_t rank, uint32_t i) { return __ldcg(a.partial + (uint64_t)rank * a.T3 + i); };
+        // this block's voxels on its low faces: z == 0 (B^2), then y == 0 (B (B-1)), then x == 0 ((B-1)^2)
+        const uint32_t nlow = BB + B * (B - 1) + (B - 1) * (B - 1);
+        for (uint32_t j = lane; j < nlow; j += 32) {
+            uint32_t lx, ly, lz;
+            if (j < BB) {
+                ly = fdiv(j, rB);
+                lx = j - ly * B;
+                lz = 0;
+            } else if (j < BB + B * (B - 1)) {
+                const uint32_t i = j - BB;
+                lz = 1 + fdiv(i, rB);
+                lx = i - (lz - 1) * B;
+                ly = 0;
+            } else {
+                const uint32_t i = j - BB - B * (B - 1);
+                lz = 1 + i / (B - 1);
+                ly = 1 + i % (B - 1);
+                lx = 0;
+            }
+            const uint32_t i = (lz * B1 + ly) * B1 + lx;
+            float t = __ldcg(own + i);
+            if (!lx && nb[0] != kNoVertex) t = __fadd_rn(t, from(nb[0], i + B * st[0]));
+            if (!ly && nb[1] != kNoVertex) t = __fadd_rn(t, from(nb[1], i + B * st[1]));
+            if (!lz && nb[2] != kNoVertex) t = __fadd_rn(t, from(nb[2], i + B * st[2]));
+            put(lx, ly, lz, t);
+        }
+        // voxels of the block after this one along axis k, where that one is not active
+#pragma unroll
+        for (uint32_t k = 0; k < 3; ++k) {
+            if (nb[3 + k] != kNoVertex) continue;
+            const uint32_t u = k == 0 ? 1u : 0u, v = k == 2 ? 1u : 2u;  // the other axes, in order
+            const uint32_t ru = nb[6 + 2 * k], rv = nb[7 + 2 * k];
+            for (uint32_t j = lane; j < BB; j += 32) {
+                const uint32_t lv = fdiv(j, rB), lu = j - lv * B;
+                const uint32_t i = B * st[k] + lu * st[u] + lv * st[v];
+                const bool tu = !lu && ru != kNoVertex, tv = !lv && rv != kNoVertex;
+                // a block before that one on an axis before k writes the voxel
+                if ((tu && u < k) || (tv && v < k)) continue;
+                float t = __ldcg(own + i);
+                const uint32_t c = lu * st[u] + lv * st[v];  // the voxel in its own block's tile
+                if (tu) t = __fadd_rn(t, from(ru, c + B * st[u]));
+                if (tv) t = __fadd_rn(t, from(rv, c + B * st[v]));
+                put(k == 0 ? B : lu, k == 1 ? B : (k == 0 ? lu : lv), k == 2 ? B : lv, t);
+            }
         }
     }
 }
@@ -180,6 +362,12 @@ __global__ void __launch_bounds__(kIsoThreads) adjoint_iso_kernel(const float *_
         __syncthreads();
     }
     if (threadIdx.x == 0) *out = (float)s[0];
+}
+
+template <typename T>
+static auto adjoint_fn(bool det, uint32_t B) {
+    return det ? (B == 8 ? adjoint_block_kernel<T, true, 8> : adjoint_block_kernel<T, true, 0>)
+               : (B == 8 ? adjoint_block_kernel<T, false, 8> : adjoint_block_kernel<T, false, 0>);
 }
 
 MTX_BC_READER(bc_take_adjoint)
@@ -208,8 +396,7 @@ extern "C" mtx_status mtx_extract_backward(mtx_context_t c, const mtx_volume *vo
     if (n && (!meshlets || !filt->compactedBlockIdBuffer.ptr || !filt->blockRankBuffer.ptr ||
               (vertexCount && !dl_dvertex)))
         return fail(c, MTX_ERR_INVALID_ARG, "forward outputs are missing");
-    if ((rs = load_case_tables(c)) != MTX_OK) return rs;
-    cudaStream_t s = c->stream;
+        cudaStream_t s = c->stream;
     mtx_profiler *prof = c->prof;
     prof_begin(prof, "Mesh_Extraction_Backward", s);
     MTX_CUDA(c, cudaMemsetAsync(dl_dfield, 0, nvox(vol->dims) * sizeof(float), s));
@@ -238,11 +425,11 @@ extern "C" mtx_status mtx_extract_backward(mtx_context_t c, const mtx_volume *vo
     a.iso_part = (float *)c->adj_iso.ptr;
     a.T3 = T3;
     a.st = &c->ctrl->status;
-    const WPlan pl = make_wplan(B);
-    a.off_acc = pl.bytes;
-    a.ws_bytes = pl.bytes + (det ? align_up(4 * T3, 128) : 0u);
-    const uint32_t smem = kAdjWarps * a.ws_bytes;
-    auto kern = det ? adjoint_block_kernel<true> : adjoint_block_kernel<false>;
+    const WPlan pl = make_adjoint_plan(B, det);
+    const uint32_t smem = kAdjWarps * pl.bytes;
+    auto kern = p.dtype == MTX_DTYPE_U8    ? adjoint_fn<uint8_t>(det, B)
+                : p.dtype == MTX_DTYPE_U16 ? adjoint_fn<uint16_t>(det, B)
+                                           : adjoint_fn<float>(det, B);
     int occ = 0;
     if ((rs = ctas_per_sm(c, reinterpret_cast<const void *>(kern), kAdjWarps * 32, smem, &occ)) != MTX_OK) return rs;
     if (occ < 1) return fail(c, MTX_ERR_UNSUPPORTED, "adjoint warp layout does not fit shared memory");

@@ -62,29 +62,6 @@ __host__ __device__ inline uint32_t tile_pitch(uint32_t B, uint32_t esz, bool tm
     return align_up(xoff_max + B + 1, A);
 }
 
-// A warp's shared memory for a float tile staged by plain loads, its inside
-// rows, crossing rows and row prefixes (the adjoint).
-__host__ __device__ inline WPlan make_wplan(uint32_t B) {
-    WPlan p{};
-    p.B = B;
-    p.B1 = B + 1;
-    p.BB = B * B;
-    p.nb3 = 3 * B * B + 3 * B + 1;  // voxels of the (B+1)^3 context outside the block
-    p.rB = (uint32_t)((0x100000000ull + B - 1) / B);
-    p.rB1 = (uint32_t)((0x100000000ull + B) / (B + 1));
-    p.PX = B + 1;
-    p.tile_bytes = 4 * p.PX * p.B1 * p.B1;
-    uint32_t o = align_up(p.tile_bytes, 16);
-    p.off_rows = o;
-    o = align_up(o + 4 * p.B1 * p.B1, 16);
-    p.off_cross = o;
-    o = align_up(o + 12 * p.BB, 16);
-    p.off_vp = o;
-    o = align_up(o + 4 * p.BB, 16);
-    p.bytes = align_up(o, 128);
-    return p;
-}
-
 // n / d and n % d for the block-local sizes (n < 70000, 2 <= d < 300), exact.
 __device__ __forceinline__ uint32_t fdiv(uint32_t n, uint32_t r) { return __umulhi(n, r); }
 __device__ __forceinline__ uint32_t fmod(uint32_t n, uint32_t r, uint32_t d) { return n - __umulhi(n, r) * d; }
@@ -170,41 +147,6 @@ __device__ __forceinline__ bool tile_wait(const WPlan &pl, unsigned char *ws, co
     }
     parity ^= 1u;
     return true;
-}
-
-// Plain loads of a block's (B+1)^3 tile from a volume of run-time dtype
-// p.dtype, stored as float (exact for uint8 and uint16), so that one set of
-// block bodies serves every dtype.
-template <typename S>
-__device__ __forceinline__ void tile_load_float_from(const Problem &p, const WPlan &pl, float *tile, const Geo &g) {
-    constexpr uint32_t kLdgBatch = 8;
-    const S *vol = reinterpret_cast<const S *>(p.vol);
-    const uint32_t n = pl.B1 * pl.B1 * pl.B1;
-    for (uint32_t i0 = 0; i0 < n; i0 += 32 * kLdgBatch) {
-        float v[kLdgBatch];
-        uint32_t dst[kLdgBatch];
-#pragma unroll
-        for (uint32_t k = 0; k < kLdgBatch; ++k) {
-            const uint32_t i = i0 + k * 32 + (threadIdx.x & 31);
-            const uint32_t iq = fdiv(i, pl.rB1);
-            const uint32_t x = i - iq * pl.B1, z = fdiv(iq, pl.rB1), y = iq - z * pl.B1;
-            const uint32_t gx = g.ox + x, gy = g.oy + y, gz = g.oz + z;
-            v[k] = 0.0f;
-            dst[k] = i < n ? (z * pl.B1 + y) * pl.PX + x : 0xffffffffu;
-            if (i < n && gx < p.X && gy < p.Y && gz < p.Z)
-                v[k] = Vox<S>::val(__ldg(vol + ((uint64_t)gz * p.Y + gy) * p.X + gx));
-        }
-#pragma unroll
-        for (uint32_t k = 0; k < kLdgBatch; ++k)
-            if (dst[k] != 0xffffffffu && MTX_BC(dst[k], pl.PX * pl.B1 * pl.B1, kBcTile)) tile[dst[k]] = v[k];
-    }
-    __syncwarp();
-}
-
-__device__ __forceinline__ void tile_load_float(const Problem &p, const WPlan &pl, float *tile, const Geo &g) {
-    if (p.dtype == MTX_DTYPE_U8) tile_load_float_from<uint8_t>(p, pl, tile, g);
-    else if (p.dtype == MTX_DTYPE_U16) tile_load_float_from<uint16_t>(p, pl, tile, g);
-    else tile_load_float_from<float>(p, pl, tile, g);
 }
 
 // Inside bitmask of every tile row: bit x <=> voxel at or below iso and inside
@@ -366,13 +308,6 @@ __device__ __forceinline__ void block_counts(const Problem &p, const WPlan &pl, 
     __syncwarp();
     nv = tv;
     nt = tt;
-}
-
-// Block-relative index of the first vertex owned by voxel (x, y, z).
-__device__ __forceinline__ uint32_t voxel_prefix(const uint32_t *cross, const uint32_t *vp, uint32_t BB, uint32_t q,
-                                                 uint32_t x) {
-    const uint32_t below = (1u << x) - 1u;
-    return vp[q] + __popc(cross[q] & below) + __popc(cross[BB + q] & below) + __popc(cross[2 * BB + q] & below);
 }
 
 // ------------------------------------------------------------- numerics

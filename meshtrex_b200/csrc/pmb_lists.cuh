@@ -26,7 +26,7 @@ constexpr uint32_t kTris = 820;
 static __device__ uint16_t g_mc_tri[kTris];
 static __device__ uint16_t g_mc_first[256];
 
-static mtx_status load_list_tables(mtx_context *c) {
+[[maybe_unused]] static mtx_status load_list_tables(mtx_context *c) {
     static bool loaded[128] = {false};
     mtx_status r = load_case_tables(c);
     if (r != MTX_OK || (c->device >= 0 && c->device < 128 && loaded[c->device])) return r;
