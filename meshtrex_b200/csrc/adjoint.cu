@@ -5,14 +5,15 @@
 //
 // One warp per active block builds the inside bits of the block's rows from the
 // volume, lists the voxels that own a cut edge in canonical order (so vertex
-// ids follow the forward's) and, axis by axis, one voxel a lane, recomputes t's
-// inputs:
+// ids follow the forward's) and, 32 voxels a step, one a lane, recomputes t's
+// inputs for their edges:
 //   dL/df(u)  = g (iso - f(v)) / d^2,  dL/df(v) = g (f(u) - iso) / d^2,
 //   dL/diso   = g / d,                 d = f(v) - f(u), v = u + e_axis.
 // ATOMIC mode adds the field terms into dL/dfield with FP32 atomics.
 // DETERMINISTIC mode accumulates them into a private (B+1)^3 tile in shared
-// memory in six sweeps (axis x, y, z; the edge's first, then second voxel),
-// in each of which every tile voxel has at most one writer.  The tile's inner
+// memory in four additions a step (the edges' first voxels, then their second
+// ones along x, y and z), in each of which every tile voxel has at most one
+// writer.  The tile's inner
 // voxels belong to this block alone and go straight to dL/dfield; the others
 // are kept as the block's partial, and a gather pass gives each of them one
 // designated block that sums the partials of the blocks that own an edge at it
@@ -119,7 +120,6 @@ __device__ __forceinline__ float iso_term(float gv, float scale, float den) {
 
 template <typename T, bool DET, int BC>
 __global__ void __launch_bounds__(kAdjWarps * 32) adjoint_block_kernel(const __grid_constant__ AdjArgs a) {
-    constexpr bool kBig = BC == 0;  // the run-time form's list rounds; BC = 8 has one
     extern __shared__ __align__(128) unsigned char smem[];
     Problem p = a.p;
     if (BC) p.B = BC;
@@ -150,8 +150,7 @@ __global__ void __launch_bounds__(kAdjWarps * 32) adjoint_block_kernel(const __g
         const bool keep = cr.nl <= nterm;  // else the terms are computed again below
         ListWalk l;
         uint32_t run = vbase, seen = 0;
-        while (const uint32_t n = !ok ? 0u : !kBig ? list_next<false>(l, pl, ws)
-                                           : B > 8 ? list_next<true>(l, pl, ws) : list_next<false>(l, pl, ws)) {
+        while (const uint32_t n = ok ? list_take<BC>(l, pl, ws) : 0u) {
             uint32_t m = 0, cell = 0;
             if (lane < n) {
                 cell = list[l.done + lane];

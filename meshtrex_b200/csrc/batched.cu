@@ -27,7 +27,7 @@
 #include <vector>
 
 #include "minmax_device.cuh"
-#include "pmb_balanced.cuh"
+#include "pmb_lists.cuh"
 
 namespace mtx {
 
@@ -35,15 +35,18 @@ constexpr uint32_t kBThreads = 256;
 constexpr uint32_t kBItems = 4;
 constexpr uint32_t kBTile = kBThreads * kBItems;
 constexpr uint32_t kBWarps = kBThreads / 32;
+// triangle table, the cases' first triangles and triangle counts
+constexpr uint32_t kBFixedBytes = (8 * kTris + 512 + 256 + 127) / 128 * 128;
 constexpr uint32_t kBChunk = 2;                 // active blocks per warp ticket
 constexpr uint32_t kPhaseSpinLimit = 1u << 26;  // about 17 s of polling at the longest back-off
 
 struct BVol {
     Problem p;      // isovalue unset
-    WPlan pl;       // region sizes of this volume, offsets of the batch's shared warp layout
+    WPlan pl;       // this volume's block edge, offsets of the batch's shared warp layout
     GridDiv dv;     // reciprocals of the grid's row and slice sizes (block_geo)
-    uint32_t nXS, nbs, zchunk, wide;  // min/max: strips, blocks a strip, words a lane (RowCut); slabs a warp
-    bool nan_zero;      // minmax_leaf_rows_warp
+    uint32_t nXS, nbs, zchunk;  // min/max: strips, blocks a strip (RowCut), slabs a warp
+    uint32_t wide, aligned;     // RowCut
+    bool nan_zero;              // minmax_leaf_rows_warp
     uint64_t leaf_off;  // first leaf entry of the volume in the pooled leaf array
     uint64_t mm_begin;  // first min/max warp of the volume
 };
@@ -70,13 +73,14 @@ struct BatchArgs {
     const uint32_t *tile_job;
     const uint2 *leaf;
     uint32_t njobs, n_ftiles;
-    uint32_t ws_bytes, face_stride;
-    uint32_t block_warps, pad0;  // warps of a CTA that take count/emit work (the layout fits that many)
+    uint32_t ws_bytes, face_stride, state_stride;
+    uint32_t block_warps;  // warps of a CTA that take count/emit work (the layout fits that many)
     uint32_t *rank_pool;
     uint32_t *ids, *job_of;
     uint64_t block_cap;
     mtx_meshlet_descriptor *desc;
-    uint32_t *faces;
+    uint16_t *faces;
+    uint32_t *state;  // inside rows of each active block (count -> emit)
     uint32_t *filter_status;
     uint64_t *scan_status;
     mtx_batch_job_result *res;
@@ -120,18 +124,26 @@ __global__ void __launch_bounds__(128) batch_minmax_kernel(const BVol *__restric
         }
         return;
     }
-#define MTX_MM(T, W, NR)                                                                                               \
-    minmax_leaf_rows_warp<T, W, NR, sizeof(T) == 4>((const T *)p.vol, p.X, p.Y, p.Z, p.B, p.GX, p.GY, p.GZ, v.nXS, v.nbs, \
-                                                    v.zchunk, lw, out, s_col[threadIdx.x >> 5], v.nan_zero)
-    switch (p.dtype * 4 + (p.B == 8) * 2 + v.wide) {
-    case MTX_DTYPE_U8 * 4: MTX_MM(uint8_t, 1, 0); break;
-    case MTX_DTYPE_U8 * 4 + 1: MTX_MM(uint8_t, 2, 0); break;
-    case MTX_DTYPE_U8 * 4 + 2: MTX_MM(uint8_t, 1, 9); break;
-    case MTX_DTYPE_U8 * 4 + 3: MTX_MM(uint8_t, 2, 9); break;
-    case MTX_DTYPE_U16 * 4 + 1: MTX_MM(uint16_t, 2, 0); break;
-    case MTX_DTYPE_U16 * 4 + 3: MTX_MM(uint16_t, 2, 9); break;
-    case MTX_DTYPE_F32 * 4 + 1: MTX_MM(float, 2, 0); break;
-    default: MTX_MM(float, 2, 9); break;
+#define MTX_MM(T, W, NR, AL)                                                                                          \
+    minmax_leaf_rows_warp<T, W, NR, AL>((const T *)p.vol, p.X, p.Y, p.Z, p.B, p.GX, p.GY, p.GZ, v.nXS, v.nbs, v.zchunk, \
+                                        lw, out, s_col[threadIdx.x >> 5], v.nan_zero)
+    // type, words of a row a lane, block edge 8 at compile time, aligned rows
+    switch (p.dtype * 8 + (p.B == 8) * 4 + v.wide * 2 + v.aligned) {
+    case MTX_DTYPE_U8 * 8 + 0: MTX_MM(uint8_t, 1, 0, false); break;
+    case MTX_DTYPE_U8 * 8 + 1: MTX_MM(uint8_t, 1, 0, true); break;
+    case MTX_DTYPE_U8 * 8 + 2: MTX_MM(uint8_t, 2, 0, false); break;
+    case MTX_DTYPE_U8 * 8 + 3: MTX_MM(uint8_t, 2, 0, true); break;
+    case MTX_DTYPE_U8 * 8 + 4: MTX_MM(uint8_t, 1, 9, false); break;
+    case MTX_DTYPE_U8 * 8 + 5: MTX_MM(uint8_t, 1, 9, true); break;
+    case MTX_DTYPE_U8 * 8 + 6: MTX_MM(uint8_t, 2, 9, false); break;
+    case MTX_DTYPE_U8 * 8 + 7: MTX_MM(uint8_t, 2, 9, true); break;
+    case MTX_DTYPE_U16 * 8 + 2: MTX_MM(uint16_t, 2, 0, false); break;
+    case MTX_DTYPE_U16 * 8 + 3: MTX_MM(uint16_t, 2, 0, true); break;
+    case MTX_DTYPE_U16 * 8 + 6: MTX_MM(uint16_t, 2, 9, false); break;
+    case MTX_DTYPE_U16 * 8 + 7: MTX_MM(uint16_t, 2, 9, true); break;
+    case MTX_DTYPE_F32 * 8 + 2:
+    case MTX_DTYPE_F32 * 8 + 3: MTX_MM(float, 2, 0, true); break;
+    default: MTX_MM(float, 2, 9, true); break;
     }
 #undef MTX_MM
 }
@@ -447,68 +459,150 @@ __device__ __forceinline__ void batch_bases(const BatchArgs &a, uint32_t n, uint
 }
 
 // ------------------------------------------------------------ per block
-// The tile of every block is staged as float whatever the volume's dtype
-// (exact for uint8 and uint16: the same compares and interpolation bits as
-// the single-volume kernels), so one copy of each block body serves all
-// dtypes and the kernel's instruction footprint stays small.  The bodies are
-// the balanced ones (pmb_balanced.cuh): batches of many volumes and
-// isovalues tend to have dense blocks.
+// The list bodies of the single-volume passes (pmb_lists.cuh).  A block hands
+// its inside rows over, not its list: batches of many volumes and isovalues tend
+// to have dense blocks, and the emit phase lists the cells again in less time
+// than the longer lists take through memory.  Only the inside rows are built
+// per voxel type; vertices switch on it at their two loads, so that the kernel's
+// code stays small.  Bound by instruction issue (2.2 a cycle and SM, 4600 a block
+// of 122 vertices and 238 triangles) and the latency of L2-only loads: 46 jobs on
+// 16 mixed volumes (39,800 blocks), 280 us of which 20 compaction, 100 counts,
+// 12 offsets; float tiles staged in both phases, with a vertex table of 5 bytes a
+// voxel, took 313.  Loading the next block's job and place under the current one
+// was slower (315: registers).
+template <int BC>
 __device__ __forceinline__ void batch_count_block(const BatchArgs &a, const Problem &p, const WPlan &pl,
                                                   const GridDiv &dv, unsigned char *ws, const uint8_t *ntab,
                                                   uint32_t id, uint32_t r) {
     const Geo g = block_geo(id, p, false, 4, dv);
-    tile_load_rows(p, pl, ws, g);
-    count_block_balanced(p, pl, ws, g, ntab, a.desc + r, a.faces + (uint64_t)r * a.face_stride);
+    if (p.dtype == MTX_DTYPE_U8) load_rows<uint8_t, BC>(p, pl, ws, g, nullptr);
+    else if (p.dtype == MTX_DTYPE_U16) load_rows<uint16_t, BC>(p, pl, ws, g, nullptr);
+    else load_rows<float, BC>(p, pl, ws, g, nullptr);
+    count_block_list<BC, true>(p, pl, ws, g, ntab, nullptr, a.desc + r, a.faces + (uint64_t)r * a.face_stride,
+                               a.state + (uint64_t)r * a.state_stride);
 }
 
-template <int CPL, bool GENERIC, bool EO>
+template <bool GENERIC, int BC>
 __device__ __forceinline__ void batch_emit_block(const BatchArgs &a, const Problem &p, const WPlan &pl,
-                                                 const GridDiv &dv, unsigned char *ws, const uint64_t *tab,
-                                                 const uint8_t *ntab, const uint8_t *owner, uint32_t id, uint32_t r,
+                                                 const GridDiv &dv, unsigned char *ws, const uint64_t *tri,
+                                                 const uint16_t *first, uint32_t edge8, uint32_t id, uint32_t r,
                                                  uint64_t rank_off, const mtx_batch_job_result &jr) {
+    const uint32_t lane = threadIdx.x & 31;
     const Geo g = block_geo(id, p, false, 4, dv);
-    const uint4 q = __ldcg(reinterpret_cast<const uint4 *>(a.desc + r));
-    const mtx_meshlet_descriptor d{q.x, q.y, q.z, q.w};
+    const uint4 d = __ldcg(reinterpret_cast<const uint4 *>(a.desc + r));
     const uint32_t nb_rk = neighbour_rank<false>(p, g, id, a.rank_pool + rank_off);
     const uint32_t nb_vb = nb_rk != kNoVertex ? __ldcg(&a.desc[nb_rk].vertexOffset) : kNoVertex;
-    tile_load_rows(p, pl, ws, g);
+    const uint32_t miss = __ballot_sync(0xffffffffu, nb_rk == kNoVertex) & 0xfeu;
+    const uint64_t face_words = a.block_cap * a.face_stride;
+    Ctx8 c8;
+    if (BC == 8) c8 = ctx8_load<false>(a.faces, nb_rk, edge8, face_words);
+    uint32_t *rows = reinterpret_cast<uint32_t *>(ws + pl.off_rows);
+    const uint32_t *own = a.state + (uint64_t)r * a.state_stride;
+    for (uint32_t i = lane; i < pl.B1 * pl.B1; i += 32) rows[i] = __ldcg(own + i);
+    __syncwarp();
+    const uint32_t tbase = d.y / 3u, nv = d.z, nt = d.w;
     void *verts = a.vertices ? (void *)((char *)a.vertices + jr.vertexOffset * a.vsz) : nullptr;
-    if (!emit_vertices_balanced<GENERIC>(p, pl, ws, g, d, ntab, jr.indexCount / 3u, verts, jr.vertexCount, a.vfmt,
-                                         a.frame, a.normals, &a.ctrl->status, r))
+    if ((uint64_t)tbase + nt > jr.indexCount / 3u || (verts && (uint64_t)d.x + nv > jr.vertexCount)) {
+        if (lane == 0) report(&a.ctrl->status, MTX_ERR_CAPACITY, kSiteEmitCapacity, r, 2);
         return;
-    // the tile is dead: the vertex table takes its place, its context layer
-    // gathered from the neighbours' face records
-    uint32_t rec[CPL];
-    gather_issue<CPL, false>(p, pl, g, nb_rk, a.faces, a.face_stride, rec);
-    fill_context_vertices<CPL>(pl, ws, nb_vb, rec);
-    emit_triangles_balanced<EO>(p, pl, ws, g, d, tab, ntab, owner, a.indices + jr.indexOffset, &a.ctrl->status, r);
+    }
+    if (!(nt || (verts && nv))) return;
+    const bool inner = g.ox + pl.B < p.X && g.oy + pl.B < p.Y && g.oz + pl.B < p.Z;
+    list_bits<BC>(p, pl, ws, g);
+    uint32_t *jobs = reinterpret_cast<uint32_t *>(ws + pl.off_jobs);
+    uint32_t *nbase = reinterpret_cast<uint32_t *>(ws + pl.off_nvid);
+    uint16_t *vtab = reinterpret_cast<uint16_t *>(ws + pl.off_vtab);
+    const uint16_t *list = reinterpret_cast<const uint16_t *>(ws + pl.off_list);
+    if (lane < 8) nbase[lane] = lane ? nb_vb : d.x;
+
+    // vertices, and this block's entries of the vertex table
+    ListWalk l;
+    uint32_t vrun = 0, out = 0;
+    while (vrun < nv) {
+        const uint32_t n = list_take<BC>(l, pl, ws);
+        if (!n) break;
+        const uint32_t e = lane < n ? listed_cell(p, pl, g, rows, list[l.done + lane], inner) : 0u;
+        l.done += n;
+        uint32_t vt;
+        const uint32_t rel = vrun + step_vertices(e >> 28, vt);
+        queue_vertices(pl, e, rel, vtab, jobs);
+        vrun += vt;
+        __syncwarp();
+        if (verts) {
+            const uint32_t avail = min(vrun, nv);
+            while (avail - out >= (vrun >= nv ? 1u : 32u)) {
+                const uint32_t k = min(32u, avail - out);
+                put_vertices<AnyVoxel, GENERIC>(p, pl, g, jobs, out, k, inner, verts, d.x, a.vfmt, a.frame, a.normals);
+                out += k;
+            }
+        }
+    }
+    // the context layer's entries
+    if (BC == 8) {
+        ctx8_store(c8, edge8, vtab);
+    } else {
+        for (uint32_t j0 = 0; j0 < pl.nb3; j0 += 32) {
+            const uint32_t j = j0 + lane, c = ctx_entry(pl, min(j, pl.nb3 - 1));
+            const uint32_t rk = __shfl_sync(0xffffffffu, nb_rk, c & 7u);
+            const uint64_t at = (uint64_t)rk * a.face_stride + ((c >> 3) & 1023u);
+            if (j < pl.nb3)
+                vtab[c >> 13] = rk != kNoVertex && MTX_BC(at, face_words, kBcFaces) ? __ldcg(a.faces + at) : (uint16_t)0;
+        }
+    }
+    __syncwarp();
+
+    // triangles
+    bool bad = vrun != nv;
+    uint32_t top = 0;
+    out = 0;
+    if (BC == 8) l.done = 0;  // the list is still there
+    else l = ListWalk{};
+    while (top < nt) {
+        const uint32_t n = list_take<BC>(l, pl, ws);
+        if (!n) break;
+        const uint32_t e = lane < n ? listed_cell(p, pl, g, rows, list[l.done + lane], inner) : 0u;
+        l.done += n;
+        const uint32_t f = first[(e >> 12) & 0xffu];
+        uint32_t total;
+        const uint32_t before = warp_excl_scan(f >> 12, total);
+        queue_triangles(pl, e, f, top + before, jobs);
+        top += total;
+        __syncwarp();
+        const uint32_t avail = min(top, nt);
+        const uint32_t least = top >= nt ? 1u : 32u;
+        while (avail - out >= least) {
+            const uint32_t k = min(32u, avail - out);
+            put_triangles(ws + pl.off_vtab, tri, jobs, nbase, out, k, a.indices + jr.indexOffset + 3ull * tbase, miss,
+                          bad);
+            out += k;
+        }
+    }
+    bad |= top != nt;
+    if (bad) report(&a.ctrl->status, MTX_ERR_INTERNAL, kSiteEmitNeighbour, r, 3);
+    __syncwarp();
 }
 
 // ------------------------------------------------------------ the kernel
 // BC: every volume's block edge at compile time (0: each volume's own, at run
 // time).  When all volumes of a batch have edge 8 the plan and every division
 // by the edge fold to constants, and the kernel's code gets smaller.  Its
-// register use is held to four CTAs per SM (62 registers, no spills), the
-// occupancy of the run-time-edge variants.
-template <int CPL, bool GENERIC, int BC>
-__global__ void __launch_bounds__(kBThreads, BC ? 4 : 1) batch_extract_kernel(const __grid_constant__ BatchArgs a) {
+// register use is held to four CTAs per SM.
+template <bool GENERIC, int BC>
+__global__ void __launch_bounds__(kBThreads, BC ? 4 : 2) batch_extract_kernel(const __grid_constant__ BatchArgs a) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ uint32_t s_u[4];
     __shared__ uint32_t s_tmp[kBWarps + 1];
     __shared__ uint64_t s_tmp64[kBWarps + 1];
     __shared__ uint32_t s_f[kBWarps];
     __shared__ uint64_t s_carry[1];
-    uint64_t *tab = reinterpret_cast<uint64_t *>(smem);
-    uint8_t *ntab = smem + 2048;
-    uint8_t *owner = smem + 2048 + 256;
+    uint64_t *tri = reinterpret_cast<uint64_t *>(smem);
+    uint16_t *first = reinterpret_cast<uint16_t *>(smem + 8 * kTris);
+    uint8_t *ntab = smem + 8 * kTris + 512;
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    unsigned char *ws = smem + kTableBytes + min(warp, a.block_warps - 1) * a.ws_bytes;
-    for (uint32_t i = tid; i < 256; i += kBThreads) {
-        tab[i] = c_mc_cases[i];
-        ntab[i] = (uint8_t)(c_mc_cases[i] & 0xFu);
-    }
-    if (tid < 12) owner[tid] = c_mc_owner[tid];
-    if (BC) edge_offsets(reinterpret_cast<uint16_t *>(owner + 16), BC + 1);  // the edge is known: table_vertex<true>
+    unsigned char *ws = smem + kBFixedBytes + min(warp, a.block_warps - 1) * a.ws_bytes;
+    for (uint32_t i = tid; i < 256; i += kBThreads) ntab[i] = (uint8_t)(c_mc_cases[i] & 0xFu);
+    build_tris(BC ? make_batch_plan(BC) : a.vols[0].pl, tri, first);  // one table row for all volumes (S1)
+    const uint32_t edge8 = BC == 8 ? ctx8_edge(lane) : 0u;
     __syncthreads();
     BCtrl *ctrl = a.ctrl;
     DevStatus *st = &ctrl->status;
@@ -541,8 +635,8 @@ __global__ void __launch_bounds__(kBThreads, BC ? 4 : 1) batch_extract_kernel(co
             Problem p = v.p;
             p.iso = job.iso;
             if (BC) p.B = BC;
-            const WPlan pl = BC ? make_wplan_balanced(BC) : v.pl;
-            batch_count_block(a, p, pl, v.dv, ws, ntab, id, r);
+            const WPlan pl = BC ? make_batch_plan(BC) : v.pl;
+            batch_count_block<BC>(a, p, pl, v.dv, ws, ntab, id, r);
             ++done;
         }
     }
@@ -585,13 +679,13 @@ __global__ void __launch_bounds__(kBThreads, BC ? 4 : 1) batch_extract_kernel(co
             Problem p = v.p;
             p.iso = job.iso;
             if (BC) p.B = BC;
-            const WPlan pl = BC ? make_wplan_balanced(BC) : v.pl;
+            const WPlan pl = BC ? make_batch_plan(BC) : v.pl;
             mtx_batch_job_result jr;
             jr.vertexOffset = __ldcg(&a.res[j].vertexOffset);
             jr.indexOffset = __ldcg(&a.res[j].indexOffset);
             jr.vertexCount = __ldcg(&a.res[j].vertexCount);
             jr.indexCount = __ldcg(&a.res[j].indexCount);
-            batch_emit_block<CPL, GENERIC, BC != 0>(a, p, pl, v.dv, ws, tab, ntab, owner, id, r, job.rank_off, jr);
+            batch_emit_block<GENERIC, BC>(a, p, pl, v.dv, ws, tri, first, edge8, id, r, job.rank_off, jr);
         }
     }
 }
@@ -609,7 +703,7 @@ struct mtx_batch {
     uint64_t mm_warps = 0;
     uint32_t grid = 0, smem = 0, vsz = 12;
     uint64_t block_cap = 0, vcap = 0, tcap = 0;
-    int variant = 0;  // CPL 8/32 x GENERIC (0-3), edge 8 at compile time x GENERIC (4-5)
+    int variant = 0;  // edge at run time (0-1), edge 8 at compile time (2-3); + 1: GENERIC
     std::vector<void *> allocs;
     BVol *vols = nullptr;
     uint2 *leaf = nullptr;
@@ -627,27 +721,18 @@ namespace {
 using KernelFn = void (*)(BatchArgs);
 KernelFn batch_kernel(int variant) {
     switch (variant) {
-    case 0: return batch_extract_kernel<8, false, 0>;
-    case 1: return batch_extract_kernel<8, true, 0>;
-    case 2: return batch_extract_kernel<32, false, 0>;
-    case 3: return batch_extract_kernel<32, true, 0>;
-    case 4: return batch_extract_kernel<8, false, 8>;
-    default: return batch_extract_kernel<8, true, 8>;
+    case 0: return batch_extract_kernel<false, 0>;
+    case 1: return batch_extract_kernel<true, 0>;
+    case 2: return batch_extract_kernel<false, 8>;
+    default: return batch_extract_kernel<true, 8>;
     }
 }
 
+// Block edge B in the warp layout of the batch's largest.
 WPlan plan_in_layout(uint32_t B, const WPlan &L) {
-    WPlan p = make_wplan_balanced(B);
-    p.off_tile = L.off_tile;
-    p.off_vtab = L.off_vtab;
-    p.off_bar = L.off_bar;
-    p.off_rows = L.off_rows;
-    p.off_cross = L.off_cross;
-    p.off_vp = L.off_vp;
-    p.off_list = L.off_list;
-    p.off_vmsk = L.off_vmsk;
-    p.off_jobs = L.off_jobs;
-    p.bytes = L.bytes;
+    WPlan p = L;
+    plan_block(p, B);
+    p.S1 = L.S1;
     return p;
 }
 
@@ -696,7 +781,7 @@ mtx_status mtx_batch_create(mtx_context_t c, const mtx_batch_desc *d, mtx_batch_
         return fail(c, MTX_ERR_INVALID_ARG, "batch: empty volume or job list");
     if (d->vertexFormat > MTX_VERTEX_DATA || d->frame > MTX_FRAME_NDC)
         return fail(c, MTX_ERR_INVALID_ARG, "batch: bad vertex format or frame");
-    mtx_status rs = load_case_tables(c);
+    mtx_status rs = load_list_tables(c);
     if (rs != MTX_OK) return rs;
 
     mtx_batch *b = new mtx_batch();
@@ -714,9 +799,12 @@ mtx_status mtx_batch_create(mtx_context_t c, const mtx_batch_desc *d, mtx_batch_
         if (B < 2 || B > 16) { batch_release(b); return fail(c, MTX_ERR_INVALID_ARG, "batch: block edge outside 2..16"); }
         Bmax = std::max(Bmax, B);
     }
-    const WPlan L = make_wplan_balanced(Bmax);  // float tile, vertex table in its place
+    const WPlan L = make_batch_plan(Bmax);
     std::vector<BVol> vols(b->nvol);
-    uint64_t leaf_total = 0, want = (uint64_t)c->sm_count * 48;
+    // min/max warps: four waves of them, shared out by the volumes' sizes
+    uint64_t leaf_total = 0, want = (uint64_t)c->sm_count * 48 * 4;
+    double voxels = 0;
+    for (uint32_t v = 0; v < b->nvol; ++v) voxels += (double)nvox(d->volumes[v].dims);
     for (uint32_t v = 0; v < b->nvol; ++v) {
         const mtx_volume &mv = d->volumes[v];
         const uint32_t B = d->blockEdges[v], esz = dtype_size(mv.dtype);
@@ -744,11 +832,12 @@ mtx_status mtx_batch_create(mtx_context_t c, const mtx_batch_desc *d, mtx_batch_
         }
         const RowCut cut = row_cut(p, esz);
         bv.wide = cut.wide;
+        bv.aligned = cut.aligned;
         bv.nan_zero = (uintptr_t)p.vol % 16 != 0 || ((uint64_t)p.X * esz) % 16 != 0 || (B != 4 && B != 8 && B != 16);
         bv.nXS = cut.nXS;
         bv.nbs = cut.nbs;
         const uint64_t cols = (uint64_t)bv.nXS * p.GY;
-        const uint64_t share = std::max<uint64_t>(1, want / b->nvol);
+        const uint64_t share = std::max<uint64_t>(1, (uint64_t)((double)want * (double)nvox(mv.dims) / voxels));
         const uint32_t nzc = (uint32_t)std::min<uint64_t>(p.GZ, std::max<uint64_t>(1, (share + cols - 1) / cols));
         bv.zchunk = ceil_div(p.GZ, nzc);
         b->mm_warps += cols * ceil_div(p.GZ, bv.zchunk);
@@ -776,11 +865,11 @@ mtx_status mtx_batch_create(mtx_context_t c, const mtx_batch_desc *d, mtx_batch_
     b->block_cap = d->maxActiveBlocks ? std::min<uint64_t>(d->maxActiveBlocks, blocks_total) : blocks_total;
     b->vcap = d->vertexCapacity ? d->vertexCapacity : b->block_cap * 4ull * Bmax * Bmax;
     b->tcap = d->triangleCapacity ? d->triangleCapacity : b->block_cap * 8ull * Bmax * Bmax;
-    const uint32_t face_stride = 3 * Bmax * Bmax;
+    const uint32_t face_stride = face_stride16(Bmax), state_stride = row_state_words(Bmax);
     const uint64_t n_stiles = (b->block_cap + kBTile - 1) / kBTile;
 
     // device memory
-    void *p_vols, *p_jobs, *p_tiles, *p_leaf, *p_rank, *p_ids, *p_jobof, *p_desc, *p_faces, *p_verts, *p_idx;
+    void *p_vols, *p_jobs, *p_tiles, *p_leaf, *p_rank, *p_ids, *p_jobof, *p_desc, *p_faces, *p_state, *p_verts, *p_idx;
     b->ctrl_bytes = align256(sizeof(BCtrl));
     const size_t off_fst = b->ctrl_bytes;
     const size_t off_sst = align256(off_fst + 4ull * b->n_ftiles);
@@ -795,7 +884,8 @@ mtx_status mtx_batch_create(mtx_context_t c, const mtx_batch_desc *d, mtx_batch_
         (rs = batch_alloc(b, &p_ids, 4ull * b->block_cap)) != MTX_OK ||
         (rs = batch_alloc(b, &p_jobof, 4ull * b->block_cap)) != MTX_OK ||
         (rs = batch_alloc(b, &p_desc, sizeof(mtx_meshlet_descriptor) * b->block_cap)) != MTX_OK ||
-        (rs = batch_alloc(b, &p_faces, 4ull * face_stride * b->block_cap)) != MTX_OK ||
+        (rs = batch_alloc(b, &p_faces, 2ull * face_stride * b->block_cap)) != MTX_OK ||
+        (rs = batch_alloc(b, &p_state, 4ull * state_stride * b->block_cap)) != MTX_OK ||
         (rs = batch_alloc(b, &p_verts, (size_t)b->vsz * b->vcap)) != MTX_OK ||
         (rs = batch_alloc(b, &p_idx, 12ull * b->tcap)) != MTX_OK ||
         (rs = batch_alloc(b, &b->ctrl_region, b->ctrl_bytes)) != MTX_OK) {
@@ -822,12 +912,14 @@ mtx_status mtx_batch_create(mtx_context_t c, const mtx_batch_desc *d, mtx_batch_
     a.n_ftiles = b->n_ftiles;
     a.ws_bytes = L.bytes;
     a.face_stride = face_stride;
+    a.state_stride = state_stride;
     a.rank_pool = (uint32_t *)p_rank;
     a.ids = (uint32_t *)p_ids;
     a.job_of = (uint32_t *)p_jobof;
     a.block_cap = b->block_cap;
     a.desc = (mtx_meshlet_descriptor *)p_desc;
-    a.faces = (uint32_t *)p_faces;
+    a.faces = (uint16_t *)p_faces;
+    a.state = (uint32_t *)p_state;
     a.filter_status = (uint32_t *)(cr + off_fst);
     a.scan_status = (uint64_t *)(cr + off_sst);
     a.res = (mtx_batch_job_result *)(cr + off_res);
@@ -846,11 +938,11 @@ mtx_status mtx_batch_create(mtx_context_t c, const mtx_batch_desc *d, mtx_batch_
     const bool generic = d->vertexFormat != MTX_VERTEX_XYZ || d->frame != MTX_FRAME_VOXEL;
     bool all8 = true;
     for (uint32_t v = 0; v < b->nvol; ++v) all8 = all8 && d->blockEdges[v] == 8;
-    b->variant = all8 ? 4 + (generic ? 1 : 0) : (Bmax > 8 ? 2 : 0) + (generic ? 1 : 0);
+    b->variant = (all8 ? 2 : 0) + (generic ? 1 : 0);
     // as many block warps per CTA as the shared memory holds (8 unless the
-    // largest plan is a 16^3 float32 tile)
+    // largest block edge is near 16)
     const int static_smem = 1024;
-    const int room = (c->max_smem_optin > 0 ? c->max_smem_optin : 227 * 1024) - (int)kTableBytes - static_smem;
+    const int room = (c->max_smem_optin > 0 ? c->max_smem_optin : 227 * 1024) - (int)kBFixedBytes - static_smem;
     a.block_warps = (uint32_t)std::min<int>(kBWarps, std::max(0, room / (int)L.bytes));
     if (d->blockWarps > kBWarps) {
         batch_release(b);
@@ -861,7 +953,7 @@ mtx_status mtx_batch_create(mtx_context_t c, const mtx_batch_desc *d, mtx_batch_
         batch_release(b);
         return fail(c, MTX_ERR_UNSUPPORTED, "batch: warp layout does not fit shared memory");
     }
-    b->smem = kTableBytes + a.block_warps * L.bytes;
+    b->smem = kBFixedBytes + a.block_warps * L.bytes;
     KernelFn fn = batch_kernel(b->variant);
     e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b->smem);
     // all of the unified L1 as shared memory: more resident warps hide the

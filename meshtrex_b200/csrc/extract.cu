@@ -110,10 +110,10 @@ __global__ void __launch_bounds__(kScanThreads)
 // the rest by ticket, drawn one block ahead.  Warps' blocks differ in work, and
 // with about ten blocks a warp (80,000 active blocks of a 1024^3 volume) fixed
 // shares alone leave most warps waiting for the unluckiest; tickets alone are
-// bound by the counter, which serves fewer than one draw a nanosecond
-// (emit of the 1024^3 uint16
-// ball at block 8: 183 us by stride, 161 by tickets, 158 so; the count pass, at
-// half the work a block, gets slower, 94 -> 134 us, and keeps the stride).
+// bound by the counter, which serves fewer than one draw a nanosecond (emit of
+// the 1024^3 uint16 ball at block 8: 183 us by stride, 161 by tickets, 158 so;
+// the count pass, at half the work a block, gets slower, 94 -> 134 us, and keeps
+// the stride).
 struct BlockShare {
     uint32_t fixed, stride;  // blocks given out by stride, warps of the grid
     uint32_t *ticket;
@@ -285,14 +285,7 @@ __global__ void __launch_bounds__(kMaxWarps * 32, GENERIC ? 1 : 4)
                     before = (e >> 20) & 0xffu;
                     total = __shfl_sync(0xffffffffu, before + n, 31);
                 }
-                const uint32_t cell = e & 0xfffu, q = fdiv(cell, pl.rB), x = cell - q * pl.B;
-                const uint32_t z = fdiv(q, pl.rB), y = q - z * pl.B;
-                const uint32_t end = (x + 1 == pl.B ? 1u << 26 : 0u) | (y + 1 == pl.B ? 1u << 27 : 0u) |
-                                     (z + 1 == pl.B ? 1u << 28 : 0u);
-                const uint32_t job = (((q + z) * pl.B1 + x) << 1) | ((f & 0xfffu) << 16) | end;
-#pragma unroll
-                for (uint32_t t = 0; t < 5; ++t)  // at most five triangles a case
-                    if (t < n) jobs[(top + before + t) & (kJobWin - 1)] = job + (t << 16);
+                queue_triangles(pl, e, f, top + before, jobs);
                 top += total;
                 __syncwarp();
                 const uint32_t avail = min(top, nt);  // never past the block's triangles

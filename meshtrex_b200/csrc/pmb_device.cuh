@@ -31,11 +31,6 @@ static mtx_status load_case_tables(mtx_context *c) {
 }
 
 constexpr uint32_t kNoVertex = 0xffffffffu;
-// packed cases (2048 B), triangle counts (256 B), owners (16 B), the emit
-// pass's edge offsets (24 B, edge_offsets), rounded up so that every warp's
-// region -- and the TMA tile at its start -- is 128-byte aligned
-constexpr uint32_t kTableBytes = 2432;
-static_assert(kTableBytes % 128 == 0 && kTableBytes >= 2048 + 256 + 16 + 24, "table region must keep warp regions aligned");
 constexpr uint32_t kJobWin = 256;                   // jobs (vertices or triangles) resolved per window
 constexpr int kMaxWarps = 8;                        // warps per CTA of the extraction kernels
 
@@ -44,10 +39,11 @@ __host__ __device__ inline uint32_t align_up(uint32_t v, uint32_t a) { return (v
 // ------------------------------------------------------- per-warp smem plan
 struct WPlan {
     uint32_t B, B1, BB, PX, nb3;
+    uint32_t S1;       // row of the vertex table: B + 1, or in a batch the largest block edge + 1
     uint32_t rB, rB1;  // ceil(2^32 / d) reciprocals: n / d == __umulhi(n, r) for the sizes used here
-    uint32_t off_tile, off_bar, off_rows, off_cross, off_vp, off_tp, off_nvid, off_jobs;
-    uint32_t off_case, off_mm;             // pmb_lists.cuh: face records and bitstream, list bits
-    uint32_t off_vtab, off_vmsk, off_list;
+    uint32_t off_tile, off_bar, off_rows, off_vp, off_nvid, off_jobs;
+    uint32_t off_case, off_mm;  // face records and bitstream, list bits
+    uint32_t off_vtab, off_list;
     uint32_t bytes;       // per warp
     uint32_t tile_bytes;  // one tile (the TMA transaction size)
 };
@@ -62,9 +58,8 @@ __host__ __device__ inline uint32_t tile_pitch(uint32_t B, uint32_t esz, bool tm
     return align_up(xoff_max + B + 1, A);
 }
 
-// n / d and n % d for the block-local sizes (n < 70000, 2 <= d < 300), exact.
+// n / d for the block-local sizes (n < 70000, 2 <= d < 300), exact.
 __device__ __forceinline__ uint32_t fdiv(uint32_t n, uint32_t r) { return __umulhi(n, r); }
-__device__ __forceinline__ uint32_t fmod(uint32_t n, uint32_t r, uint32_t d) { return n - __umulhi(n, r) * d; }
 
 struct Geo {
     uint32_t ox, oy, oz;  // block origin (voxels)
@@ -100,19 +95,6 @@ __device__ __forceinline__ Geo block_geo(uint32_t id, const Problem &p, bool tma
     const uint32_t rest = id - g.bz * dv.dxy;
     g.by = div_by(rest, dv.mx, dv.dx);
     g.bx = rest - g.by * dv.dx;
-    g.ox = g.bx * p.B;
-    g.oy = g.by * p.B;
-    g.oz = g.bz * p.B;
-    g.nx = min(p.B, p.X - g.ox);
-    g.xoff = tma ? (g.ox % (16 / esz)) : 0u;
-    return g;
-}
-
-__device__ __forceinline__ Geo block_geo(uint32_t id, const Problem &p, bool tma, uint32_t esz) {
-    Geo g;
-    g.bx = id % p.GX;
-    g.by = (id / p.GX) % p.GY;
-    g.bz = id / (p.GX * p.GY);
     g.ox = g.bx * p.B;
     g.oy = g.by * p.B;
     g.oz = g.bz * p.B;
@@ -239,77 +221,6 @@ __device__ __forceinline__ uint32_t warp_excl_scan(uint32_t v, uint32_t &total) 
     return x - v;
 }
 
-// Cells x of cell row (y, z) whose case is neither 0 nor 255 (bit x set), and
-// those that are entirely inside (all 8 corners at or below iso).
-__device__ __forceinline__ uint32_t mixed_cells(const Problem &p, const WPlan &pl, const Geo &g, const uint32_t *rows,
-                                                uint32_t y, uint32_t z, uint32_t &all_inside) {
-    all_inside = 0;
-    if (g.oy + y + 1 >= p.Y || g.oz + z + 1 >= p.Z || g.ox + 1 >= p.X) return 0;
-    const uint32_t ncell = min(pl.B, p.X - 1 - g.ox), B1 = pl.B1;
-    const uint32_t cells = (1u << ncell) - 1u;
-    const uint32_t r00 = rows[z * B1 + y], r01 = rows[z * B1 + y + 1];
-    const uint32_t r10 = rows[(z + 1) * B1 + y], r11 = rows[(z + 1) * B1 + y + 1];
-    const uint32_t all = r00 & r01 & r10 & r11, any = r00 | r01 | r10 | r11;
-    all_inside = all & (all >> 1) & cells;
-    return (any | (any >> 1)) & ~(all & (all >> 1)) & cells;
-}
-
-// Per-row crossing masks, vertex prefixes and (want_tris) triangle prefixes,
-// and the block's vertex/triangle counts.  Lane l owns rows [l*R, l*R + R) so
-// that the row prefixes follow from one warp scan. 
-__device__ __forceinline__ void block_counts(const Problem &p, const WPlan &pl, unsigned char *ws, const Geo &g,
-                                             const uint8_t *ntab, bool want_tris, uint32_t &nv,
-                                             uint32_t &nt) {
-    const uint32_t lane = threadIdx.x & 31;
-    const uint32_t *rows = reinterpret_cast<const uint32_t *>(ws + pl.off_rows);
-    uint32_t *cross = reinterpret_cast<uint32_t *>(ws + pl.off_cross);
-    uint32_t *vp = reinterpret_cast<uint32_t *>(ws + pl.off_vp);
-    uint32_t *tp = reinterpret_cast<uint32_t *>(ws + pl.off_tp);
-    const uint32_t B = pl.B, BB = pl.BB;
-    const uint32_t R = (BB + 31) / 32;
-    uint32_t sv = 0, stri = 0;
-    for (uint32_t k = 0; k < R; ++k) {
-        const uint32_t q = lane * R + k;
-        if (q >= BB) break;
-        const uint32_t z = fdiv(q, pl.rB), y = q - z * B;
-        uint32_t xc, yc, zc;
-        row_cross(p, pl, g, rows, y, z, xc, yc, zc);
-        cross[q] = xc;
-        cross[BB + q] = yc;
-        cross[2 * BB + q] = zc;
-        vp[q] = sv;  // lane-local prefixes, rebased below
-        sv += __popc(xc) + __popc(yc) + __popc(zc);
-        if (want_tris) {
-            tp[q] = stri;
-            uint32_t inside;
-            uint32_t mm = mixed_cells(p, pl, g, rows, y, z, inside);
-            // the four rows of the cell row, read once for all its mixed cells
-            const uint32_t r00 = mm ? rows[z * pl.B1 + y] : 0u, r01 = mm ? rows[z * pl.B1 + y + 1] : 0u;
-            const uint32_t r10 = mm ? rows[(z + 1) * pl.B1 + y] : 0u, r11 = mm ? rows[(z + 1) * pl.B1 + y + 1] : 0u;
-            while (mm) {
-                const uint32_t x = __ffs(mm) - 1;
-                mm &= mm - 1u;
-                const uint32_t a = r00 >> x, b = r01 >> x, c = r10 >> x, e = r11 >> x;
-                const uint32_t cfg = (a & 3u) | ((b & 2u) << 1) | ((b & 1u) << 3) | ((c & 3u) << 4) | ((e & 2u) << 5) |
-                                     ((e & 1u) << 7);
-                stri += ntab[cfg];
-            }
-        }
-    }
-    uint32_t tv, tt;
-    const uint32_t pv = warp_excl_scan(sv, tv);
-    const uint32_t pt = warp_excl_scan(stri, tt);
-    for (uint32_t k = 0; k < R; ++k) {
-        const uint32_t q = lane * R + k;
-        if (q >= BB) break;
-        vp[q] += pv;
-        if (want_tris) tp[q] += pt;
-    }
-    __syncwarp();
-    nv = tv;
-    nt = tt;
-}
-
 // ------------------------------------------------------------- numerics
 // Edge parameter (marching_cubes_pmb.mesh.glsl:129-134): t = (iso - a)/(b - a)
 // when |b - a| > 1e-5 else 0.5, clamped to [0, 1]; every operation rounds once.
@@ -378,29 +289,6 @@ static __device__ __noinline__ float3 vertex_normal_any(const Problem &p, uint32
     return vertex_normal<float>(p, gx, gy, gz, a, t);
 }
 
-// Position of the vertex on the +axis edge of block voxel (x,y,z); its edge
-// parameter goes to *tout.
-template <typename T>
-__device__ __forceinline__ float3 vertex_pos(const Problem &p, const WPlan &pl, const T *tile, const Geo &g, uint32_t x,
-                                             uint32_t y, uint32_t z, uint32_t a, bool ndc, float *tout) {
-    uint32_t i0 = (z * pl.B1 + y) * pl.PX + g.xoff + x;
-    uint32_t i1 = i0 + (a == 0 ? 1u : a == 1 ? pl.PX : pl.PX * pl.B1);
-    if (!MTX_BC(i1, pl.PX * pl.B1 * pl.B1, kBcTile)) i1 = i0 = 0;
-    const float t = edge_t(Vox<T>::val(tile[i0]), Vox<T>::val(tile[i1]), p.iso);
-    *tout = t;
-    float3 pos = make_float3((float)(g.ox + x), (float)(g.oy + y), (float)(g.oz + z));
-    if (a == 0) pos.x = __fadd_rn(pos.x, t);
-    else if (a == 1) pos.y = __fadd_rn(pos.y, t);
-    else pos.z = __fadd_rn(pos.z, t);
-    if (ndc) {
-        pos.x = __fsub_rn(__fmul_rn(__fdiv_rn(pos.x, (float)p.X), 2.0f), 1.0f);
-        pos.y = __fsub_rn(__fmul_rn(__fdiv_rn(pos.y, (float)p.Y), 2.0f), 1.0f);
-        pos.z = __fsub_rn(__fmul_rn(__fdiv_rn(pos.z, (float)p.Z), 2.0f), 1.0f);
-    }
-    return pos;
-}
-
-
 // -------------------------------------------------------------- emit pass
 // Context voxel of compact index j: the (B+1)^2 voxels with x == B first, then
 // those with y == B, then those with z == B.
@@ -420,16 +308,6 @@ __device__ __forceinline__ void ctx_voxel(const WPlan &pl, uint32_t j, uint32_t 
         z = B;
         y = fdiv(i, pl.rB);
         x = i - y * B;
-    }
-}
-
-// Edge offsets of the vertex table for one CTA (B <= 8): entry e holds the
-// table offset of cube edge e's owner voxel from the cell's low corner,
-// dx + dy (B+1) + dz (B+1)^2, and its axis << 8 (from the owner table).
-__device__ __forceinline__ void edge_offsets(uint16_t *eoff, uint32_t B1) {
-    if (threadIdx.x < 12) {
-        const uint32_t o = c_mc_owner[threadIdx.x];
-        eoff[threadIdx.x] = (uint16_t)((o & 1u) + ((o >> 1) & 1u) * B1 + ((o >> 2) & 1u) * B1 * B1 + ((o >> 3) << 8));
     }
 }
 
@@ -525,58 +403,6 @@ __device__ __forceinline__ uint32_t neighbour_rank(const Problem &p, const Geo &
             rk = ld_in<NC>(rank_map + id + dx + dy * p.GX + dz * p.GX * p.GY);
     }
     return rk;
-}
-
-// Issues the loads of the face records of the block's +x/+y/+z context layer
-// (all of them before any is used); bit 31 of rec marks a present record and
-// bits 27-29 hold the number c of the neighbour it came from (face records
-// use bits 0-26).
-template <int CPL, bool NC = true>
-__device__ __forceinline__ void gather_issue(const Problem &p, const WPlan &pl, const Geo &g, uint32_t nb_rk,
-                                             const uint32_t *faces, uint32_t face_stride, uint32_t rec[CPL]) {
-    const uint32_t lane = threadIdx.x & 31, B = pl.B, BB = pl.BB, nb3 = pl.nb3;
-#pragma unroll
-    for (uint32_t k = 0; k < CPL; ++k) {
-        rec[k] = 0;
-        if (k * 32 >= nb3) continue;  // warp-uniform
-        const uint32_t j = k * 32 + lane;
-        uint32_t x, y, z;
-        ctx_voxel(pl, j < nb3 ? j : 0, x, y, z);
-        const uint32_t dx = x == B, dy = y == B, dz = z == B;
-        const uint32_t c = j < nb3 ? (dx | (dy << 1) | (dz << 2)) : 1u;
-        const uint32_t rk = __shfl_sync(0xffffffffu, nb_rk, c);
-        if (j < nb3 && rk != kNoVertex && g.ox + x < p.X && g.oy + y < p.Y && g.oz + z < p.Z) {
-            const uint32_t lx = dx ? 0 : x, ly = dy ? 0 : y, lz = dz ? 0 : z;
-            const uint32_t e = dx ? lz * B + ly : (dy ? BB + lz * B + lx : 2 * BB + ly * B + lx);
-            rec[k] = ld_in<NC>(faces + (uint64_t)rk * face_stride + e) | 0x80000000u | (c << 27);
-        }
-    }
-}
-
-// The block's low-face records from its crossing rows and row prefixes:
-// block-relative first vertex | owned-edge mask << 24 of the voxels with
-// x == 0 (index z*B + y), y == 0 (BB + z*B + x) and z == 0 (2BB + y*B + x).
-// 2B lanes walk the y == 0 and z == 0 rows along x with a running first vertex.
-__device__ __forceinline__ void write_face_records(const WPlan &pl, const unsigned char *ws, uint32_t *fr) {
-    const uint32_t lane = threadIdx.x & 31, B = pl.B, BB = pl.BB;
-    const uint32_t *cross = reinterpret_cast<const uint32_t *>(ws + pl.off_cross);
-    const uint32_t *vp = reinterpret_cast<const uint32_t *>(ws + pl.off_vp);
-    if (lane < 2 * B) {
-        // lane l < 2B walks row (y = 0, z = l) or (y = l - B, z = 0) along x
-        const bool yface = lane < B;
-        const uint32_t q = yface ? lane * B : lane - B;
-        uint32_t *o = fr + (yface ? BB + lane * B : 2 * BB + (lane - B) * B);
-        const uint32_t xc = cross[q], yc = cross[BB + q], zc = cross[2 * BB + q];
-        uint32_t run = vp[q];
-        for (uint32_t x = 0; x < B; ++x) {
-            const uint32_t m = ((xc >> x) & 1u) | (((yc >> x) & 1u) << 1) | (((zc >> x) & 1u) << 2);
-            if (MTX_BC((uint32_t)(o - fr) + x, 3 * BB, kBcFaces)) o[x] = run | (m << 24);
-            run += __popc(m);
-        }
-    }
-    // x == 0 face: record z*B + y is voxel (0, y, z), the first of row q = z*B + y
-    for (uint32_t q = lane; q < BB; q += 32)
-        fr[q] = vp[q] | (((cross[q] & 1u) | ((cross[BB + q] & 1u) << 1) | ((cross[2 * BB + q] & 1u) << 2)) << 24);
 }
 
 // Exclusive scan of the per-block vertex and triangle counts in rank order,

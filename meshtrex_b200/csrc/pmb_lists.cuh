@@ -16,6 +16,8 @@
 // cells, as walks along the rows did.
 #pragma once
 
+#include <type_traits>
+
 #include "pmb_device.cuh"
 
 namespace mtx {
@@ -65,6 +67,7 @@ __host__ __device__ inline uint32_t list_words(uint32_t B) { return (B * B * B +
 __host__ __device__ inline void plan_block(WPlan &p, uint32_t B) {
     p.B = B;
     p.B1 = B + 1;
+    p.S1 = B + 1;
     p.BB = B * B;
     p.nb3 = 3 * B * B + 3 * B + 1;
     p.rB = (uint32_t)((0x100000000ull + B - 1) / B);
@@ -129,6 +132,32 @@ __host__ __device__ inline WPlan make_emit_plan(uint32_t B) {
     return p;
 }
 
+// In the batched kernel, whose emit phase always takes inside rows over: both
+// phases' regions, the count phase's face records and bitstream in the vertex
+// table's place.
+__host__ __device__ inline WPlan make_batch_plan(uint32_t B) {
+    WPlan p{};
+    plan_block(p, B);
+    uint32_t o = 0;
+    p.off_jobs = o;
+    o += 4 * kJobWin;
+    p.off_nvid = o;
+    o += 32;
+    p.off_vtab = p.off_case = o;
+    const uint32_t T3 = p.B1 * p.B1 * p.B1;
+    o = align_up(o + std::max(2 * T3, std::max(2 * face_stride16(B), 4 * ((T3 + 31) / 32 + 1))), 16);
+    p.off_rows = o;
+    o = align_up(o + 4 * p.B1 * p.B1, 16);
+    p.off_mm = o;
+    o = align_up(o + 4 * list_words(B), 16);
+    p.off_list = o;
+    o = align_up(o + 2 * list_cap(B), 16);
+    p.bytes = o;
+    return p;
+}
+// Words of inside rows a block hands over there.
+__host__ __device__ inline uint32_t row_state_words(uint32_t B) { return ((B + 1) * (B + 1) + 3) / 4 * 4; }
+
 // Shared memory of an emit CTA before its warps' regions: the triangles as
 // vertex-table offsets, the cases' first triangles, the context-layer map.
 __host__ __device__ inline uint32_t emit_fixed_bytes(uint32_t B) {
@@ -151,6 +180,7 @@ __device__ __forceinline__ void load_rows(const Problem &p, const WPlan &pl, uns
     const uint32_t lane = threadIdx.x & 31, B1 = pl.B1, n = B1 * B1 * B1, nw = (n + 31) / 32;
     const bool inner = g.ox + pl.B < p.X && g.oy + pl.B < p.Y && g.oz + pl.B < p.Z;
     const T *base = vol + ((uint64_t)g.oz * p.Y + g.oy) * p.X + g.ox;
+    const bool narrow = ((uint64_t)B1 * p.X * p.Y >> 32) == 0;  // the tile's offsets fit 32 bits
     for (uint32_t w0 = 0; w0 < nw; w0 += kBatch) {
         T v[kBatch];
         uint32_t in = 0;
@@ -161,6 +191,9 @@ __device__ __forceinline__ void load_rows(const Problem &p, const WPlan &pl, uns
             v[k] = T(0);
             if (inner && off) {
                 if (on) v[k] = __ldg(base + off[i]);
+            } else if (inner && narrow) {
+                const uint32_t iq = fdiv(i, pl.rB1), z = fdiv(iq, pl.rB1);
+                if (on) v[k] = __ldg(base + ((z * p.Y + iq - z * B1) * p.X + i - iq * B1));
             } else {
                 const uint32_t iq = fdiv(i, pl.rB1);
                 const uint32_t x = i - iq * B1, z = fdiv(iq, pl.rB1), y = iq - z * B1;
@@ -334,6 +367,13 @@ __device__ __forceinline__ uint32_t list_next(ListWalk &l, const WPlan &pl, unsi
     return min(32u, l.top - l.done);
 }
 
+// list_next for the block edge BC, or at run time (0).
+template <int BC>
+__device__ __forceinline__ uint32_t list_take(ListWalk &l, const WPlan &pl, unsigned char *ws) {
+    if constexpr (BC != 0) return list_next<(BC > 8)>(l, pl, ws);
+    else return pl.B > 8 ? list_next<true>(l, pl, ws) : list_next<false>(l, pl, ws);
+}
+
 // A list word: cell (bits 0-11), case (12-19; 0 for a voxel that starts no
 // cell), triangles before it in its step of 32 (20-27), cut owned edges (28-30).
 __device__ __forceinline__ uint32_t listed_cell(const Problem &p, const WPlan &pl, const Geo &g, const uint32_t *rows,
@@ -364,8 +404,9 @@ __device__ __forceinline__ uint32_t step_vertices(uint32_t m, uint32_t &total) {
 // Block whose inside rows are built: list and counts, the face records -- for
 // each voxel with x == 0 (index z B + y), y == 0 (BB + z B + x) or z == 0 (2BB +
 // y B + x) that owns a vertex, its first vertex in the block (14 bits) and
-// whether its x and y edges are cut (bits 14, 15) -- and the state.
-template <int BC>
+// whether its x and y edges are cut (bits 14, 15) -- and the state: the list for
+// B <= 8, else, or with ROWS, the inside rows.
+template <int BC, bool ROWS = false>
 __device__ __forceinline__ void count_block_list(const Problem &p, const WPlan &pl, unsigned char *ws, const Geo &g,
                                                  const uint8_t *ntab, uint8_t *cases_out, mtx_meshlet_descriptor *dr,
                                                  uint16_t *faces, uint32_t *state) {
@@ -381,19 +422,18 @@ __device__ __forceinline__ void count_block_list(const Problem &p, const WPlan &
             const uint32_t q = fdiv(c, pl.rB), x = c - q * B, z = fdiv(q, pl.rB), y = q - z * B;
             cases_out[c] = cell_valid(p, g, x, y, z) ? (uint8_t)cell_case(rows, pl.B1, x, y, z) : (uint8_t)0;
         }
-    if (B > 8)
+    if (ROWS || B > 8)
         for (uint32_t i = lane; i < pl.B1 * pl.B1; i += 32) state[i] = rows[i];
-    constexpr bool kBig = BC > 8;  // the run-time form takes the rounds of B > 8
     ListWalk l;
     uint32_t nv = 0, nt = 0, steps = 0;
-    while (const uint32_t n = BC ? list_next<kBig>(l, pl, ws) : B > 8 ? list_next<true>(l, pl, ws) : list_next<false>(l, pl, ws)) {
+    while (const uint32_t n = list_take<BC>(l, pl, ws)) {
         uint32_t e = 0;
         if (lane < n) e = listed_cell(p, pl, g, rows, list[l.done + lane], inner);
         const uint32_t m = e >> 28, tris = lane < n ? ntab[(e >> 12) & 0xffu] : 0u;
         uint32_t vt, tt;
         const uint32_t rel = nv + step_vertices(m, vt);
         const uint32_t before = warp_excl_scan(tris, tt);
-        if (B <= 8 && MTX_BC(steps + lane, list_state_words(B), kBcState)) state[steps + lane] = e | (before << 20);
+        if (!ROWS && B <= 8 && MTX_BC(steps + lane, list_state_words(B), kBcState)) state[steps + lane] = e | (before << 20);
         steps += 32;
         if (m) {
             const uint32_t cell = e & 0xfffu, q = fdiv(cell, pl.rB), x = cell - q * B, z = fdiv(q, pl.rB), y = q - z * B;
@@ -432,7 +472,7 @@ __device__ __forceinline__ void build_tris(const WPlan &pl, uint64_t *tri, uint1
         uint64_t w = 0;
         for (uint32_t k = 0; k < 3; ++k) {
             const uint32_t o = c_mc_owner[(e3 >> (4 * k)) & 0xfu], ax = o >> 3;
-            const uint32_t off = (o & 1u) + ((o >> 1) & 1u) * pl.B1 + ((o >> 2) & 1u) * pl.B1 * pl.B1;
+                const uint32_t off = (o & 1u) + ((o >> 1) & 1u) * pl.S1 + ((o >> 2) & 1u) * pl.S1 * pl.S1;
             w |= (uint64_t)((off << 1) | ((o & 7u) << 10) | (((1u << ax) - 1u) << 14)) << (16 * k);
         }
         tri[i] = w;
@@ -449,7 +489,7 @@ __device__ __forceinline__ uint32_t ctx_entry(const WPlan &pl, uint32_t j) {
     const uint32_t dx = x == B, dy = y == B, dz = z == B;
     const uint32_t lx = dx ? 0 : x, ly = dy ? 0 : y, lz = dz ? 0 : z;
     const uint32_t e = dx ? lz * B + ly : (dy ? BB + lz * B + lx : 2 * BB + ly * B + lx);
-    return (dx | (dy << 1) | (dz << 2)) | (e << 3) | (((z * pl.B1 + y) * pl.B1 + x) << 13);
+    return (dx | (dy << 1) | (dz << 2)) | (e << 3) | (((z * pl.S1 + y) * pl.S1 + x) << 13);
 }
 
 // The context layer: face records of the neighbours (nb_rk: lane c holds
@@ -466,6 +506,8 @@ __device__ __forceinline__ uint32_t ctx8_edge(uint32_t lane) {  // map entry (ct
     if (lane < 24) return 6u | ((64 + k) << 3) | (((8 * 9 + 8) * 9 + k) << 13);
     return lane == 24 ? 7u | (728u << 13) : 0u;
 }
+// NC: the records come from an earlier launch (ld_in).
+template <bool NC = true>
 __device__ __forceinline__ Ctx8 ctx8_load(const uint16_t *faces, uint32_t nb_rk, uint32_t edge, uint64_t face_words) {
     const uint32_t lane = threadIdx.x & 31;
     Ctx8 c;
@@ -475,12 +517,12 @@ __device__ __forceinline__ Ctx8 ctx8_load(const uint16_t *faces, uint32_t nb_rk,
         const uint64_t at = (uint64_t)rk * 192 + 64 * f + 2 * lane;
         c.face[f] = 0;
         if (rk != kNoVertex && MTX_BC(at + 1, face_words, kBcFaces))
-            c.face[f] = __ldg(reinterpret_cast<const uint32_t *>(faces + at));
+            c.face[f] = ld_in<NC>(reinterpret_cast<const uint32_t *>(faces + at));
     }
     const uint32_t rk = __shfl_sync(0xffffffffu, nb_rk, edge & 7u);
     const uint64_t at = (uint64_t)rk * 192 + ((edge >> 3) & 1023u);
     c.edge = 0;
-    if (edge && rk != kNoVertex && MTX_BC(at, face_words, kBcFaces)) c.edge = __ldg(faces + at);
+    if (edge && rk != kNoVertex && MTX_BC(at, face_words, kBcFaces)) c.edge = ld_in<NC>(faces + at);
     return c;
 }
 __device__ __forceinline__ void ctx8_store(const Ctx8 &c, uint32_t edge, uint16_t *vtab) {
@@ -529,12 +571,25 @@ __device__ __forceinline__ void queue_vertices(const WPlan &pl, uint32_t e, uint
                                                uint32_t *jobs) {
     const uint32_t m = e >> 28, cell = e & 0xfffu;
     if (!m) return;
-    const uint32_t q = fdiv(cell, pl.rB), x = cell - q * pl.B;
-    const uint32_t ti = (q + fdiv(q, pl.rB)) * pl.B1 + x;  // row q = z B + y
-    if (MTX_BC(ti, pl.B1 * pl.B1 * pl.B1, kBcVoxTab)) vtab[ti] = (uint16_t)(rel | (m << 14));
+    const uint32_t q = fdiv(cell, pl.rB), x = cell - q * pl.B, z = fdiv(q, pl.rB), y = q - z * pl.B;
+    const uint32_t ti = (z * pl.S1 + y) * pl.S1 + x;
+    if (MTX_BC(ti, pl.S1 * pl.S1 * pl.S1, kBcVoxTab)) vtab[ti] = (uint16_t)(rel | (m << 14));
     if (m & 1u) jobs[rel++ & (kJobWin - 1)] = cell;
     if (m & 2u) jobs[rel++ & (kJobWin - 1)] = cell | (1u << 12);
     if (m & 4u) jobs[rel & (kJobWin - 1)] = cell | (2u << 12);
+}
+
+// A voxel's value; AnyVoxel: of the volume's run-time type.
+struct AnyVoxel {};
+template <typename T>
+__device__ __forceinline__ float voxel_value(const Problem &p, uint64_t i) {
+    if constexpr (std::is_same<T, AnyVoxel>::value) {
+        if (p.dtype == MTX_DTYPE_U8) return Vox<uint8_t>::val(__ldg(reinterpret_cast<const uint8_t *>(p.vol) + i));
+        if (p.dtype == MTX_DTYPE_U16) return Vox<uint16_t>::val(__ldg(reinterpret_cast<const uint16_t *>(p.vol) + i));
+        return __ldg(reinterpret_cast<const float *>(p.vol) + i);
+    } else {
+        return Vox<T>::val(__ldg(reinterpret_cast<const T *>(p.vol) + i));
+    }
 }
 
 // Writes vertices [done, done + n) of the block, n <= 32, one a lane; the first
@@ -550,9 +605,9 @@ __device__ __forceinline__ void put_vertices(const Problem &p, const WPlan &pl, 
     const uint32_t gx = g.ox + x, gy = g.oy + y, gz = g.oz + z;
     // (a list the count pass did not finish must not lead past the volume)
     if (lane < n && (inner || (gx + (a == 0) < p.X && gy + (a == 1) < p.Y && gz + (a == 2) < p.Z))) {
-        const T *v = reinterpret_cast<const T *>(p.vol) + ((uint64_t)gz * p.Y + gy) * p.X + gx;
+        const uint64_t v = ((uint64_t)gz * p.Y + gy) * p.X + gx;
         const uint64_t step = a == 0 ? 1ull : a == 1 ? (uint64_t)p.X : (uint64_t)p.X * p.Y;
-        const float t = edge_t(Vox<T>::val(__ldg(v)), Vox<T>::val(__ldg(v + step)), p.iso);
+        const float t = edge_t(voxel_value<T>(p, v), voxel_value<T>(p, v + step), p.iso);
         float3 pos = make_float3((float)gx, (float)gy, (float)gz);
         if (a == 0) pos.x = __fadd_rn(pos.x, t);
         if (a == 1) pos.y = __fadd_rn(pos.y, t);
@@ -570,13 +625,29 @@ __device__ __forceinline__ void put_vertices(const Problem &p, const WPlan &pl, 
             o[2] = pos.z;
         } else {
             float3 nn = make_float3(0.0f, 0.0f, 0.0f);
-            if (normals) nn = vertex_normal<T>(p, gx, gy, gz, a, t);
+            if (normals) {
+                if constexpr (std::is_same<T, AnyVoxel>::value) nn = vertex_normal_any(p, gx, gy, gz, a, t);
+                else nn = vertex_normal<T>(p, gx, gy, gz, a, t);
+            }
             float4 *o = reinterpret_cast<float4 *>(vertices) + 2 * at;
             o[0] = make_float4(pos.x, pos.y, pos.z, 1.0f);
             o[1] = make_float4(nn.x, nn.y, nn.z, 0.0f);
         }
     }
     __syncwarp();
+}
+
+// Queues the triangles of this lane's list word e, numbers [at, at + n) of the
+// block; f: the entry of its case in `first`.
+__device__ __forceinline__ void queue_triangles(const WPlan &pl, uint32_t e, uint32_t f, uint32_t at, uint32_t *jobs) {
+    const uint32_t cell = e & 0xfffu, n = f >> 12, q = fdiv(cell, pl.rB), x = cell - q * pl.B;
+    const uint32_t z = fdiv(q, pl.rB), y = q - z * pl.B;
+    const uint32_t end =
+        (x + 1 == pl.B ? 1u << 26 : 0u) | (y + 1 == pl.B ? 1u << 27 : 0u) | (z + 1 == pl.B ? 1u << 28 : 0u);
+    const uint32_t job = (((z * pl.S1 + y) * pl.S1 + x) << 1) | ((f & 0xfffu) << 16) | end;
+#pragma unroll
+    for (uint32_t t = 0; t < 5; ++t)  // at most five triangles a case
+        if (t < n) jobs[(at + t) & (kJobWin - 1)] = job + (t << 16);
 }
 
 // Writes triangles [done, done + n) of the block, n <= 32, one a lane, each lane
