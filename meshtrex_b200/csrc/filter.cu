@@ -200,13 +200,13 @@ __global__ void __launch_bounds__(kFilterThreads, 4)
                          uint64_t *tile_status, uint64_t *ticket, DevStatus *st, uint32_t spin_limit, uint32_t skip,
                          const __grid_constant__ PyrAll L) {
     static_assert(kPyrThreads == kFilterThreads, "one CTA size for both");
-    __shared__ uint2 s_part[8][8];
+    __shared__ uint2 s_part[2][8][8];
     __shared__ uint32_t s_last;
     if (blockIdx.x < ntiles)
         filter_tile<kFilterItems, true>(leaf, nblocks, ntiles, dtype, iso, ids, rank_map, count_out, tile_status,
                                         ticket, st, spin_limit, skip);
     else
-        pyramid_tile(L, blockIdx.x - ntiles, s_part, &s_last);
+        pyramid_part(L, blockIdx.x - ntiles, s_part, &s_last);
 }
 
 MTX_BC_READER(bc_take_filter)
@@ -223,7 +223,7 @@ mtx_status launch_filter(mtx_context *c, const Problem &p, const uint2 *leaf, ui
     uint64_t *words = (uint64_t *)c->filter_status.ptr;
     const uint32_t polls = c->wait_polls ? c->wait_polls : kSpinLimit, skip = c->withhold & 1u;
     if (octree && octree->ntiles)
-        filter_octree_kernel<<<ntiles + octree->ntiles, kFilterThreads, 0, s>>>(
+        filter_octree_kernel<<<ntiles + octree->ctas, kFilterThreads, 0, s>>>(
             leaf, p.nblocks, ntiles, p.dtype, p.iso, ids, rank_map, count, words, &c->ctrl->filter_ticket,
             &c->ctrl->status, polls, skip, *octree);
     else

@@ -360,9 +360,9 @@ __global__ void __launch_bounds__(128) minmax_leaf_one_kernel(const T *__restric
 }
 
 __global__ void __launch_bounds__(kPyrThreads) pyramid_all_kernel(const __grid_constant__ PyrAll L) {
-    __shared__ uint2 s_part[8][8];
+    __shared__ uint2 s_part[2][8][8];
     __shared__ uint32_t s_last;
-    pyramid_tile(L, blockIdx.x, s_part, &s_last);
+    pyramid_part(L, blockIdx.x, s_part, &s_last);
 }
 
 // ------------------------------------------------------------------ host
@@ -557,8 +557,18 @@ mtx_status pyramid_levels(mtx_context *c, uint2 *all, int levels, const uint32_t
         for (int a = 0; a < 3; ++a) P->ext[k][a] = ext[start + k][a];
     }
     P->tiles_x = ceil_div(P->ext[0][0], kPyrTileX);
-    P->tiles_y = ceil_div(P->ext[0][1], kPyrTileYZ);
-    P->ntiles = P->tiles_x * P->tiles_y * ceil_div(P->ext[0][2], kPyrTileYZ);
+    // Four CTAs an SM, each with several tiles where there are more; tiles of 2 x 2
+    // steps where there are enough of them for that (below, a CTA would take its
+    // four steps in turn while others have none: octrees of 10^6 texels and less
+    // take 4 to 8 us either way).
+    const uint32_t slots = 4u * (uint32_t)c->sm_count;
+    for (P->quad = 1;; P->quad = 0) {
+        const uint32_t yz = kPyrTileYZ << P->quad;
+        P->tiles_y = ceil_div(P->ext[0][1], yz);
+        P->ntiles = P->tiles_x * P->tiles_y * ceil_div(P->ext[0][2], yz);
+        if (!P->quad || P->ntiles >= slots) break;
+    }
+    P->ctas = std::min(P->ntiles, slots);
     P->done = &c->ctrl->pyr_done;
     return MTX_OK;
 }
@@ -568,7 +578,7 @@ mtx_status launch_pyramid(mtx_context *c, uint2 *all, int levels, const uint32_t
     PyrAll P;
     const mtx_status r = pyramid_levels(c, all, levels, ext, offset, start, &P);
     if (r != MTX_OK || !P.ntiles) return r;
-    pyramid_all_kernel<<<P.ntiles, kPyrThreads, 0, s>>>(P);
+    pyramid_all_kernel<<<P.ctas, kPyrThreads, 0, s>>>(P);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(c, e, "pyramid launch");
     return MTX_OK;

@@ -540,25 +540,31 @@ __device__ __forceinline__ void minmax_leaf_one(const T *__restrict__ vol, uint3
 
 // ------------------------------------------------------------ octree
 // Every octree level in one launch (minMaxOctreeReduce.comp.glsl:23-59 runs
-// one dispatch per level).  A CTA takes 32 x 8 x 8 texels of the launch's first
-// level (the leaf level, or level 1 when the leaf pass wrote it): each thread
-// reads the 2 x 2 x 2 texels of one texel of the next level, all eight loads in
-// flight, and the two levels after that follow by shuffles and one exchange
-// through shared memory.  The CTA that finishes last builds the rest from the
-// third level and zeroes the counter (zero since the context's creation) for
-// the next launch.  Each texel is the min/max of its up-to-8 children; children
-// past their level's extent are skipped (minMaxOctreeReduce.comp.glsl:37-47),
-// which the identity {~0, 0} in their place does.
-// Latency-bound: a tile costs one round of loads, one barrier and one counter.
-// An 8^3 tile a CTA of 512 threads, a barrier pair a level, took 203 us for the
-// 342 x 342 x 105 grid of a 1024 x 1024 x 314 volume at B = 3; this takes 56.
+// one dispatch per level).  A step of a CTA takes 32 x 8 x 8 texels of the
+// launch's first level (the leaf level, or level 1 when the leaf pass wrote it):
+// each thread reads the 2 x 2 x 2 texels of one texel of the next level, all
+// eight loads in flight and those of its next step behind them, and the two
+// levels after that follow by shuffles and one exchange through shared memory.
+// A tile is one step, or 2 x 2 of them in y and z (`quad`), whose level-3
+// texels make one level more.  The CTA that finishes last builds the rest and
+// zeroes the counter (zero since the context's creation) for the next launch.
+// Each texel is the min/max of its up-to-8 children; children past their
+// level's extent are skipped (minMaxOctreeReduce.comp.glsl:37-47), which the
+// identity {~0, 0} in their place does.
+// Latency-bound: a step costs a round of loads and a barrier, so the CTAs of the
+// launch stay and load ahead instead of one CTA a step with a counter each, and
+// the serial levels of the last CTA begin one level higher.  For the 342 x 342 x
+// 105 grid of a 1024 x 1024 x 314 volume at B = 3: 55 us with a CTA a step, 30 so
+// (a CTA of 512 threads per 8^3 texels with a barrier pair a level: 203).
 constexpr int kPyrMaxLevels = 32;
 constexpr uint32_t kPyrThreads = 256, kPyrTileX = 32, kPyrTileYZ = 8;
 struct PyrAll {
     uint2 *base[kPyrMaxLevels];
     uint32_t ext[kPyrMaxLevels][3];
     int levels;
+    uint32_t quad;  // 1: tiles of 2 x 2 steps
     uint32_t tiles_x, tiles_y, ntiles;
+    uint32_t ctas;  // CTAs of the launch that work on the octree, at most ntiles
     uint32_t *done;
 };
 
@@ -571,60 +577,94 @@ __device__ __forceinline__ void texel_store(const PyrAll &L, int k, uint32_t x, 
         L.base[k][((uint64_t)z * L.ext[k][1] + y) * L.ext[k][0] + x] = v;
 }
 
-// One tile of the launch by a CTA of kPyrThreads threads (all of them).
-__device__ __forceinline__ void pyramid_tile(const PyrAll &L, uint32_t tile, uint2 (*s_part)[8], uint32_t *s_last) {
+// The part of CTA `cta` of L.ctas, by all kPyrThreads threads of it.
+__device__ __forceinline__ void pyramid_part(const PyrAll &L, uint32_t cta, uint2 (*s_part)[8][8], uint32_t *s_last) {
     const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    const uint32_t tx = tile % L.tiles_x, ty = (tile / L.tiles_x) % L.tiles_y, tz = tile / (L.tiles_x * L.tiles_y);
-    {
-        // next level: 16 x 4 x 4 texels a tile, a warp 16 x 2 of them
-        const uint32_t x = tx * 16 + (t & 15), y = ty * 4 + ((t >> 4) & 3), z = tz * 4 + (t >> 6);
-        uint2 v[8];
+    const uint32_t ox = t & 15, oy = (t >> 4) & 3, oz = t >> 6;  // 16 x 4 x 4 level-1 texels a step, a warp 16 x 2
+    const uint32_t steps = L.quad ? 4u : 1u;
+    uint32_t tx = 0, ty = 0, tz = 0;  // the step to load next, in steps
+    auto place = [&](uint32_t tile, uint32_t s) {
+        const uint32_t rest = tile / L.tiles_x;
+        tx = tile - rest * L.tiles_x;
+        tz = rest / L.tiles_y;
+        ty = rest - tz * L.tiles_y;
+        if (L.quad) {
+            ty = 2 * ty + (s & 1);
+            tz = 2 * tz + (s >> 1);
+        }
+    };
+    uint2 v[8];
+    auto load = [&]() {
+        const uint32_t x = 2 * (tx * 16 + ox), y = 2 * (ty * 4 + oy), z = 2 * (tz * 4 + oz);
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
-            const uint32_t ux = 2 * x + (c & 1), uy = 2 * y + ((c >> 1) & 1), uz = 2 * z + (c >> 2);
+            const uint32_t ux = x + (c & 1), uy = y + ((c >> 1) & 1), uz = z + (c >> 2);
             v[c] = make_uint2(~0u, 0u);
             if (ux < L.ext[0][0] && uy < L.ext[0][1] && uz < L.ext[0][2])
                 v[c] = L.base[0][((uint64_t)uz * L.ext[0][1] + uy) * L.ext[0][0] + ux];
         }
-        uint2 r = v[0];
+    };
+    place(cta, 0);
+    load();
+    uint32_t buf = 0;
+    for (uint32_t tile = cta; tile < L.ntiles; tile += L.ctas) {
+        uint2 quad = make_uint2(~0u, 0u);  // warp 0: the tile's level-3 texels so far
+        for (uint32_t s = 0; s < steps; ++s) {
+            const uint32_t sx = tx, sy = ty, sz = tz;
+            uint2 r = v[0];
 #pragma unroll
-        for (int c = 1; c < 8; ++c) r = texel_join(r, v[c]);
-        texel_store(L, 1, x, y, z, r);
-        if (L.levels <= 2) return;
-        r = texel_xor(texel_xor(r, 1), 16);  // pairs in x and y
-        if (lane < 16 && !(lane & 1)) s_part[warp][lane >> 1] = r;
-    }
-    __syncthreads();
-    if (warp == 0) {
-        // level 2: 8 x 2 x 2 texels, lane = x | y << 3 | z << 4; warp 2 z + (y of level 1) / 2 holds a pair in y
-        const uint32_t x = lane & 7, y = (lane >> 3) & 1, z = lane >> 4;
-        uint2 r = texel_join(s_part[4 * z + y][x], s_part[4 * z + 2 + y][x]);
-        texel_store(L, 2, tx * 8 + x, ty * 2 + y, tz * 2 + z, r);
-        r = texel_xor(texel_xor(texel_xor(r, 1), 8), 16);
-        if (!(lane & 25)) texel_store(L, 3, tx * 4 + (x >> 1), ty, tz, r);
-        if (L.levels > 4) {  // level 3 of every tile is written: the last CTA to get here builds the rest
-            __threadfence();
-            __syncwarp();
-            if (lane == 0) *s_last = atomicAdd(L.done, 1u) == L.ntiles - 1;
+            for (int c = 1; c < 8; ++c) r = texel_join(r, v[c]);
+            if (s + 1 < steps) {
+                place(tile, s + 1);
+                load();
+            } else if (tile + L.ctas < L.ntiles) {
+                place(tile + L.ctas, 0);
+                load();
+            }
+            texel_store(L, 1, sx * 16 + ox, sy * 4 + oy, sz * 4 + oz, r);
+            if (L.levels <= 2) continue;
+            r = texel_xor(texel_xor(r, 1), 16);  // pairs in x and y
+            if (lane < 16 && !(lane & 1)) s_part[buf][warp][lane >> 1] = r;
+            __syncthreads();  // and warp 0 is done with the other buffer, two steps old
+            if (warp == 0) {
+                // level 2: 8 x 2 x 2 texels, lane = x | y << 3 | z << 4; warp 2 z + (y of level 1) / 2 holds a pair in y
+                const uint32_t x = lane & 7, y = (lane >> 3) & 1, z = lane >> 4;
+                r = texel_join(s_part[buf][4 * z + y][x], s_part[buf][4 * z + 2 + y][x]);
+                texel_store(L, 2, sx * 8 + x, sy * 2 + y, sz * 2 + z, r);
+                r = texel_xor(texel_xor(texel_xor(r, 1), 8), 16);
+                if (!(lane & 25)) texel_store(L, 3, sx * 4 + (x >> 1), sy, sz, r);
+                quad = texel_join(quad, r);
+                if (L.quad && s == 3) {
+                    quad = texel_xor(quad, 2);
+                    if (!(lane & 27)) texel_store(L, 4, sx * 2 + (x >> 2), sy >> 1, sz >> 1, quad);
+                }
+            }
+            buf ^= 1;
         }
     }
-    if (L.levels <= 4) return;
+    const int top = L.quad ? 5 : 4;  // the levels below are written by the tiles
+    if (L.levels <= top) return;
+    if (warp == 0) {
+        __threadfence();
+        __syncwarp();
+        if (lane == 0) *s_last = atomicAdd(L.done, 1u) == L.ctas - 1;
+    }
     __syncthreads();
     if (!*s_last) return;
     __threadfence();
-    for (int k = 4; k < L.levels; ++k) {
-        const uint32_t ex = L.ext[k][0], ey = L.ext[k][1], ez = L.ext[k][2];
+    for (int k = top; k < L.levels; ++k) {
+        const uint32_t ex = L.ext[k][0], ey = L.ext[k][1];
         const uint32_t px = L.ext[k - 1][0], py = L.ext[k - 1][1], pz = L.ext[k - 1][2];
-        const uint64_t cnt = (uint64_t)ex * ey * ez;
+        const uint32_t cnt = ex * ey * L.ext[k][2];  // below 2^30 / 8^3
 #pragma unroll 2
-        for (uint64_t i = t; i < cnt; i += kPyrThreads) {
-            const uint32_t x = (uint32_t)(i % ex), y = (uint32_t)((i / ex) % ey), z = (uint32_t)(i / ((uint64_t)ex * ey));
+        for (uint32_t i = t; i < cnt; i += kPyrThreads) {
+            const uint32_t q = i / ex, x = i - q * ex, z = q / ey, y = q - z * ey;
             uint2 r = make_uint2(~0u, 0u);
 #pragma unroll
             for (int c = 0; c < 8; ++c) {
                 const uint32_t ux = 2 * x + (c & 1), uy = 2 * y + ((c >> 1) & 1), uz = 2 * z + (c >> 2);
                 if (ux < px && uy < py && uz < pz)
-                    r = texel_join(r, __ldcg(&L.base[k - 1][((uint64_t)uz * py + uy) * px + ux]));
+                    r = texel_join(r, __ldcg(&L.base[k - 1][(uz * py + uy) * px + ux]));
             }
             L.base[k][i] = r;
         }

@@ -22,7 +22,7 @@ struct Ctrl {
     uint32_t active_count;   // compaction result
     uint32_t totals[4];      // vertexCount, indexCount, meshletCount, activeBlockCount
     uint32_t batch_ticket[4];
-    uint32_t pyr_done;       // octree tiles finished (the last one builds the top levels)
+    uint32_t pyr_done;       // octree CTAs finished (the last one builds the top levels)
     uint32_t emit_done;      // CTAs of the emit pass finished (the last one writes status_out)
     uint32_t emit_ticket;    // emit pass: blocks handed out by ticket (zeroed by the scan pass)
     uint32_t pad1;
