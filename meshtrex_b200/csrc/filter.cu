@@ -4,12 +4,12 @@
 //
 // meshtrex scans within a workgroup and then takes one atomicAdd per
 // workgroup, so the compacted list is ordered only inside a workgroup.  Here
-// each CTA takes a tile of consecutive block ids by ticket (4096 a tile, 16
-// per thread, so that a 1024^3 volume at block 8 is one wave of CTAs; 1024 in
-// the no-allocation entry point, whose scratch is sized for them), counts its
-// active blocks (two ballots a round of 64 blocks), and resolves its global offset with a
-// single-pass decoupled look-back over the tiles before it: the list comes out
-// in ascending block order, which is the order the CPU rule produces.  It
+// the CTAs take tiles of consecutive block ids by ticket (4096 a tile, 16
+// per thread, so that a 1024^3 volume at block 8 is one tile a CTA; 1024 in
+// the no-allocation entry point, whose scratch is sized for them), count their
+// active blocks (two ballots a round of 64 blocks), and resolve their global offsets with a
+// single-pass decoupled look-back over the tiles before them: the list comes out
+// in ascending block order, which is the order the CPU rule produces.  The pass
 // also writes the rank of every block (0xffffffff for inactive ones), which
 // the extraction uses to find a neighbouring block's vertices.
 #include <mutex>
@@ -20,6 +20,7 @@ namespace mtx {
 
 constexpr int kFilterThreads = 256;
 constexpr int kFilterItems = 16;       // blocks a thread: tiles of 4096
+constexpr uint32_t kFilterCtas = 4;    // CTAs an SM
 constexpr int kNoallocItems = 4;       // tiles of 1024 in mtx_filter_active_blocks_noalloc
 constexpr int kFilterTile = kFilterThreads * kFilterItems;
 constexpr int kNoallocTile = kFilterThreads * kNoallocItems;
@@ -54,129 +55,181 @@ template <> struct TileWord<true> {
         return ((uint32_t)(w >> 32) & 0x3fffffffu) == epoch ? (uint32_t)(w >> 62) : 0u;
     }
     __device__ __forceinline__ static uint32_t count(U w) { return (uint32_t)w; }
-    __device__ __forceinline__ static uint32_t draw(U *ticket, uint32_t ntiles, uint32_t &epoch) {
+    __device__ __forceinline__ static uint32_t draw(U *ticket, uint32_t draws, uint32_t &epoch) {
         const U t = atomicAdd(reinterpret_cast<unsigned long long *>(ticket), 1ull);
         epoch = (uint32_t)(t >> 32);
-        if ((uint32_t)t == ntiles - 1) st_volatile(ticket, (U)((epoch + 1) & 0x3fffffffu) << 32);
+        if ((uint32_t)t == draws - 1) st_volatile(ticket, (U)((epoch + 1) & 0x3fffffffu) << 32);
         return (uint32_t)t;
     }
 };
 
-// A CTA's tile is ITEMS / 2 rounds of 64 consecutive blocks a warp, lane l
-// taking blocks 2 l and 2 l + 1 of each round: the loads and the rank stores
-// are coalesced and the ranks follow from two ballots a round.  skip: failure
-// injection, the tickets start at tile `skip`.
+// A tile is ITEMS / 2 rounds of 64 consecutive blocks a warp, lane l taking
+// blocks 2 l and 2 l + 1 of each round: the loads and the rank stores are
+// coalesced and the ranks follow from two ballots a round.  A CTA takes tiles
+// until its ticket is past the last one: each of the `ctas` CTAs draws one
+// ticket too many, so a launch draws ntiles - skip + ctas.  Before a tile is
+// resolved, the next one's blocks are counted and published and the loads of
+// the one after are on their way: a look-back finds the tiles before it
+// published, instead of waiting for loads that are behind other tiles' waits.
+// Nothing waits for a tile that no running CTA holds: a CTA publishes and
+// resolves its tiles in the order of their tickets, and what a look-back needs
+// of an earlier tile, its count, is published before that tile's CTA waits for
+// anything later.
+// skip: failure injection, the tickets start at tile `skip`.
+// Bound by that chain of tiles: keys and ranks of 12.3 million blocks (1024 x
+// 1024 x 314 at B = 3) take 25 us without it.  One tile a CTA, its look-back
+// behind its own loads, 62 us; with the next tile's loads ahead, 54; with the
+// next tile's count published ahead as well, 32 (windows of 128 tiles a round of
+// reads: 37).  512^2 x 1024 blocks and fewer, a tile or less a CTA: 1 to 2 us less.
 template <int ITEMS, bool EPOCH>
-__device__ __forceinline__ void filter_tile(const uint2 *__restrict__ leaf, uint64_t nblocks, uint32_t ntiles,
-                                            uint32_t dtype, float iso, uint32_t *__restrict__ ids,
-                                            uint32_t *__restrict__ rank_map, uint32_t *__restrict__ count_out,
-                                            typename TileWord<EPOCH>::U *tile_status,
-                                            typename TileWord<EPOCH>::U *ticket, DevStatus *st, uint32_t spin_limit,
-                                            uint32_t skip) {
+__device__ __forceinline__ void filter_tiles(const uint2 *__restrict__ leaf, uint64_t nblocks, uint32_t ntiles,
+                                             uint32_t ctas, uint32_t dtype, float iso, uint32_t *__restrict__ ids,
+                                             uint32_t *__restrict__ rank_map, uint32_t *__restrict__ count_out,
+                                             typename TileWord<EPOCH>::U *tile_status,
+                                             typename TileWord<EPOCH>::U *ticket, DevStatus *st, uint32_t spin_limit,
+                                             uint32_t skip) {
     using TW = TileWord<EPOCH>;
-    constexpr int R = ITEMS / 2;
-    __shared__ uint32_t s_tile, s_epoch, s_prefix, s_abort;
-    __shared__ uint32_t s_tmp[kFilterThreads / 32];
-    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    constexpr int R = ITEMS / 2, W = kFilterThreads / 32;
+    static_assert(ITEMS <= 32, "a tile's ballots, one a lane");
+    __shared__ uint32_t s_draw[2], s_epoch, s_prefix, s_abort;
+    __shared__ uint32_t s_sum[2][W];  // active blocks of each warp, of the present tile and the next
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, lt = (1u << lane) - 1u;
+    const uint32_t draws = ntiles - skip + ctas;
     if (threadIdx.x == 0) {
         uint32_t epoch;
-        s_tile = TW::draw(ticket, ntiles, epoch) + skip;
+        s_draw[0] = TW::draw(ticket, draws, epoch) + skip;
         s_epoch = epoch;
     }
     __syncthreads();
-    const uint32_t t = s_tile, epoch = s_epoch;
+    uint32_t t = s_draw[0], e;
+    const uint32_t epoch = s_epoch;
     if (t >= ntiles) return;
 
-    const uint64_t base = (uint64_t)t * (kFilterThreads * ITEMS) + (uint64_t)warp * (32 * ITEMS) + 2 * lane;
-    uint4 v[R];
+    auto base_of = [&](uint32_t tile) {
+        return (uint64_t)tile * (kFilterThreads * ITEMS) + (uint64_t)warp * (32 * ITEMS) + 2 * lane;
+    };
+    uint4 v[R];  // the blocks of the tile to count next
+    auto load = [&](uint32_t tile) {
+        const uint64_t base = base_of(tile);
 #pragma unroll
-    for (int k = 0; k < R; ++k) {  // all loads before any use; {0, 0} is an inactive block
-        const uint64_t i = base + 64 * k;
-        v[k] = make_uint4(0, 0, 0, 0);
-        if (i + 1 < nblocks) {
-            v[k] = __ldg(reinterpret_cast<const uint4 *>(leaf + i));
-        } else if (i < nblocks) {
-            const uint2 one = __ldg(leaf + i);
-            v[k].x = one.x;
-            v[k].y = one.y;
-        }
-    }
-    uint32_t b0[R], b1[R], total_w = 0;  // active first and second blocks of each round's lanes
-#pragma unroll
-    for (int k = 0; k < R; ++k) {
-        b0[k] = __ballot_sync(0xffffffffu, block_active(dtype, v[k].x, v[k].y, iso));
-        b1[k] = __ballot_sync(0xffffffffu, block_active(dtype, v[k].z, v[k].w, iso));
-        total_w += __popc(b0[k]) + __popc(b1[k]);
-    }
-    if (lane == 0) s_tmp[warp] = total_w;
-    __syncthreads();
-    uint32_t total = 0, excl = 0;
-#pragma unroll
-    for (uint32_t w = 0; w < kFilterThreads / 32; ++w) {
-        if (w == warp) excl = total;
-        total += s_tmp[w];
-    }
-
-    if (warp == 0) {
-        uint32_t prefix = 0;
-        bool abort = false;
-        if (t == 0) {
-            if (lane == 0) st_volatile(&tile_status[0], TW::make(kFlagInc, epoch, total));
-        } else {
-            if (lane == 0) st_volatile(&tile_status[t], TW::make(kFlagAgg, epoch, total));
-            int64_t j = (int64_t)t - 1;
-            uint32_t spins = 0;
-            while (true) {
-                const int64_t k = j - (int64_t)lane;
-                const typename TW::U w = k >= 0 ? ld_volatile(&tile_status[k]) : TW::make(kFlagInc, epoch, 0);
-                const uint32_t flag = TW::flag(w, epoch);
-                if (__any_sync(0xffffffffu, flag == kFlagAbort)) { abort = true; break; }
-                const uint32_t inc = __ballot_sync(0xffffffffu, flag == kFlagInc);
-                const uint32_t emp = __ballot_sync(0xffffffffu, flag == 0u);
-                const uint32_t first = inc ? (uint32_t)(__ffs(inc) - 1) : 32u;
-                const uint32_t window = first >= 31 ? 0xffffffffu : ((2u << first) - 1u);
-                if (emp & window) {
-                    if (++spins >= spin_limit) {
-                        if (lane == 0) report(st, MTX_ERR_TIMEOUT, kSiteFilterLookback, t, (uint32_t)j);
-                        abort = true;
-                        break;
-                    }
-                    backoff(spins);
-                    continue;
-                }
-                uint32_t c = lane <= first ? TW::count(w) : 0u;
-#pragma unroll
-                for (int o = 16; o; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
-                prefix += c;
-                if (first < 32) break;
-                j -= 32;
+        for (int k = 0; k < R; ++k) {  // {0, 0} is an inactive block
+            const uint64_t i = base + 64 * k;
+            v[k] = make_uint4(0, 0, 0, 0);
+            if (i + 1 < nblocks) {
+                v[k] = __ldg(reinterpret_cast<const uint4 *>(leaf + i));
+            } else if (i < nblocks) {
+                const uint2 one = __ldg(leaf + i);
+                v[k].x = one.x;
+                v[k].y = one.y;
             }
-            if (lane == 0)
-                st_volatile(&tile_status[t],
-                            abort ? TW::make(kFlagAbort, epoch, 0) : TW::make(kFlagInc, epoch, prefix + total));
         }
-        if (lane == 0) {
-            s_prefix = prefix;
-            s_abort = abort ? 1u : 0u;
-            if (t == ntiles - 1) *count_out = abort ? 0u : prefix + total;
-        }
-    }
-    __syncthreads();
-    if (s_abort) return;
-    uint32_t r = s_prefix + excl;
-    const uint32_t lt = (1u << lane) - 1u;
+    };
+    // The ballots of v, lane 2 k the first and 2 k + 1 the second blocks' of round k; the warp's sum.
+    auto count = [&](uint32_t *sum) {
+        uint32_t bits = 0;
 #pragma unroll
-    for (int k = 0; k < R; ++k) {
-        const uint64_t i = base + 64 * k;
-        const bool f0 = (b0[k] >> lane) & 1u, f1 = (b1[k] >> lane) & 1u;
-        const uint32_t r0 = r + __popc(b0[k] & lt) + __popc(b1[k] & lt), r1 = r0 + f0;
-        if (f0 && MTX_BC(r0, nblocks, kBcRank)) ids[r0] = (uint32_t)i;
-        if (f1 && MTX_BC(r1, nblocks, kBcRank)) ids[r1] = (uint32_t)i + 1;
-        // rank of every block of the tile: its rank if active, else kNoRank
-        const uint2 rk = make_uint2(f0 ? r0 : 0xffffffffu, f1 ? r1 : 0xffffffffu);
-        if (i + 1 < nblocks) *reinterpret_cast<uint2 *>(rank_map + i) = rk;
-        else if (i < nblocks) rank_map[i] = rk.x;
-        r += __popc(b0[k]) + __popc(b1[k]);
+        for (int k = 0; k < R; ++k) {
+            const uint32_t b0 = __ballot_sync(0xffffffffu, block_active(dtype, v[k].x, v[k].y, iso));
+            const uint32_t b1 = __ballot_sync(0xffffffffu, block_active(dtype, v[k].z, v[k].w, iso));
+            if (lane == 2 * k) bits = b0;
+            if (lane == 2 * k + 1) bits = b1;
+        }
+        const uint32_t n = __reduce_add_sync(0xffffffffu, (uint32_t)__popc(bits));
+        if (lane == 0) sum[warp] = n;
+        return bits;
+    };
+    auto publish = [&](uint32_t tile, const uint32_t *sum) {  // warp 0
+        const uint32_t n = __reduce_add_sync(0xffffffffu, lane < W ? sum[lane] : 0u);
+        if (lane == 0) st_volatile(&tile_status[tile], TW::make(tile ? kFlagAgg : kFlagInc, epoch, n));
+    };
+
+    load(t);
+    if (threadIdx.x == 0) s_draw[1] = TW::draw(ticket, draws, e) + skip;
+    uint32_t bits = count(s_sum[0]);
+    __syncthreads();
+    if (warp == 0) publish(t, s_sum[0]);
+    uint32_t next = s_draw[1];
+    if (next < ntiles) load(next);
+    for (uint32_t buf = 0; t < ntiles; buf ^= 1) {
+        uint32_t after = next, bits_next = 0;
+        if (next < ntiles) {
+            if (threadIdx.x == 0) s_draw[0] = TW::draw(ticket, draws, e) + skip;
+            bits_next = count(s_sum[buf ^ 1]);
+        }
+        __syncthreads();
+        if (next < ntiles) {
+            after = s_draw[0];
+            if (warp == 0) publish(next, s_sum[buf ^ 1]);
+            if (after < ntiles) load(after);
+        }
+        uint32_t total = 0, excl = 0;
+#pragma unroll
+        for (uint32_t w = 0; w < W; ++w) {
+            if (w == warp) excl = total;
+            total += s_sum[buf][w];
+        }
+        if (warp == 0) {
+            uint32_t prefix = 0;
+            bool abort = false;
+            if (t > 0) {
+                int64_t j = (int64_t)t - 1;
+                uint32_t spins = 0;
+                while (true) {
+                    const int64_t k = j - (int64_t)lane;
+                    const typename TW::U w = k >= 0 ? ld_volatile(&tile_status[k]) : TW::make(kFlagInc, epoch, 0);
+                    const uint32_t flag = TW::flag(w, epoch);
+                    abort = __any_sync(0xffffffffu, flag == kFlagAbort);
+                    if (abort) break;
+                    const uint32_t inc = __ballot_sync(0xffffffffu, flag == kFlagInc);
+                    const uint32_t emp = __ballot_sync(0xffffffffu, flag == 0u);
+                    const uint32_t first = inc ? (uint32_t)(__ffs(inc) - 1) : 32u;
+                    const uint32_t window = first >= 31 ? 0xffffffffu : ((2u << first) - 1u);
+                    if (emp & window) {
+                        if (++spins >= spin_limit) {
+                            if (lane == 0) report(st, MTX_ERR_TIMEOUT, kSiteFilterLookback, t, (uint32_t)j);
+                            abort = true;
+                            break;
+                        }
+                        backoff(spins);
+                        continue;
+                    }
+                    prefix += lane <= first ? TW::count(w) : 0u;
+                    if (first < 32) break;
+                    j -= 32;
+                }
+                prefix = __reduce_add_sync(0xffffffffu, prefix);
+                if (lane == 0)
+                    st_volatile(&tile_status[t],
+                                abort ? TW::make(kFlagAbort, epoch, 0) : TW::make(kFlagInc, epoch, prefix + total));
+            }
+            if (lane == 0) {
+                s_prefix = prefix;
+                s_abort = abort ? 1u : 0u;
+                if (t == ntiles - 1) *count_out = abort ? 0u : prefix + total;
+            }
+        }
+        __syncthreads();
+        if (!s_abort) {
+            uint32_t r = s_prefix + excl;
+            const uint64_t base = base_of(t);
+#pragma unroll
+            for (int k = 0; k < R; ++k) {
+                const uint64_t i = base + 64 * k;
+                const uint32_t b0 = __shfl_sync(0xffffffffu, bits, 2 * k), b1 = __shfl_sync(0xffffffffu, bits, 2 * k + 1);
+                const bool f0 = (b0 >> lane) & 1u, f1 = (b1 >> lane) & 1u;
+                const uint32_t r0 = r + __popc(b0 & lt) + __popc(b1 & lt), r1 = r0 + f0;
+                if (f0 && MTX_BC(r0, nblocks, kBcRank)) ids[r0] = (uint32_t)i;
+                if (f1 && MTX_BC(r1, nblocks, kBcRank)) ids[r1] = (uint32_t)i + 1;
+                // rank of every block of the tile: its rank if active, else kNoRank
+                const uint2 rk = make_uint2(f0 ? r0 : 0xffffffffu, f1 ? r1 : 0xffffffffu);
+                if (i + 1 < nblocks) *reinterpret_cast<uint2 *>(rank_map + i) = rk;
+                else if (i < nblocks) rank_map[i] = rk.x;
+                r += __popc(b0) + __popc(b1);
+            }
+        }
+        t = next;
+        next = after;
+        bits = bits_next;
     }
 }
 
@@ -186,8 +239,8 @@ __global__ void __launch_bounds__(kFilterThreads, 4)
                           float iso, uint32_t *__restrict__ ids, uint32_t *__restrict__ rank_map,
                           uint32_t *__restrict__ count_out, typename TileWord<EPOCH>::U *tile_status,
                           typename TileWord<EPOCH>::U *ticket, DevStatus *st, uint32_t spin_limit, uint32_t skip) {
-    filter_tile<ITEMS, EPOCH>(leaf, nblocks, ntiles, dtype, iso, ids, rank_map, count_out, tile_status, ticket, st,
-                              spin_limit, skip);
+    filter_tiles<ITEMS, EPOCH>(leaf, nblocks, ntiles, gridDim.x, dtype, iso, ids, rank_map, count_out, tile_status,
+                               ticket, st, spin_limit, skip);
 }
 
 // The compaction and the octree in one launch (the asynchronous whole-path
@@ -198,15 +251,15 @@ __global__ void __launch_bounds__(kFilterThreads, 4)
     filter_octree_kernel(const uint2 *__restrict__ leaf, uint64_t nblocks, uint32_t ntiles, uint32_t dtype, float iso,
                          uint32_t *__restrict__ ids, uint32_t *__restrict__ rank_map, uint32_t *__restrict__ count_out,
                          uint64_t *tile_status, uint64_t *ticket, DevStatus *st, uint32_t spin_limit, uint32_t skip,
-                         const __grid_constant__ PyrAll L) {
+                         uint32_t ctas, const __grid_constant__ PyrAll L) {
     static_assert(kPyrThreads == kFilterThreads, "one CTA size for both");
     __shared__ uint2 s_part[2][8][8];
     __shared__ uint32_t s_last;
-    if (blockIdx.x < ntiles)
-        filter_tile<kFilterItems, true>(leaf, nblocks, ntiles, dtype, iso, ids, rank_map, count_out, tile_status,
-                                        ticket, st, spin_limit, skip);
+    if (blockIdx.x < ctas)
+        filter_tiles<kFilterItems, true>(leaf, nblocks, ntiles, ctas, dtype, iso, ids, rank_map, count_out,
+                                         tile_status, ticket, st, spin_limit, skip);
     else
-        pyramid_part(L, blockIdx.x - ntiles, s_part, &s_last);
+        pyramid_part(L, blockIdx.x - ctas, s_part, &s_last);
 }
 
 MTX_BC_READER(bc_take_filter)
@@ -221,13 +274,14 @@ mtx_status launch_filter(mtx_context *c, const Problem &p, const uint2 *leaf, ui
     if (c->filter_status.size != before)  // new words: no epoch's
         MTX_CUDA(c, cudaMemsetAsync(c->filter_status.ptr, 0, c->filter_status.size, s));
     uint64_t *words = (uint64_t *)c->filter_status.ptr;
+    const uint32_t ctas = std::min(ntiles, kFilterCtas * (uint32_t)c->sm_count);
     const uint32_t polls = c->wait_polls ? c->wait_polls : kSpinLimit, skip = c->withhold & 1u;
     if (octree && octree->ntiles)
-        filter_octree_kernel<<<ntiles + octree->ctas, kFilterThreads, 0, s>>>(
+        filter_octree_kernel<<<ctas + octree->ctas, kFilterThreads, 0, s>>>(
             leaf, p.nblocks, ntiles, p.dtype, p.iso, ids, rank_map, count, words, &c->ctrl->filter_ticket,
-            &c->ctrl->status, polls, skip, *octree);
+            &c->ctrl->status, polls, skip, ctas, *octree);
     else
-        filter_compact_kernel<kFilterItems, true><<<ntiles, kFilterThreads, 0, s>>>(
+        filter_compact_kernel<kFilterItems, true><<<ctas, kFilterThreads, 0, s>>>(
             leaf, p.nblocks, ntiles, p.dtype, p.iso, ids, rank_map, count, words, &c->ctrl->filter_ticket,
             &c->ctrl->status, polls, skip);
     cudaError_t e = cudaGetLastError();
@@ -331,8 +385,9 @@ extern "C" mtx_status mtx_filter_active_blocks_noalloc(const uint32_t *leaf_minm
         return MTX_ERR_INVALID_ARG;
     if (total_blocks > (uint64_t)kNoallocMaxTiles * kNoallocTile) return MTX_ERR_CAPACITY;
     const uint32_t ntiles = (uint32_t)((total_blocks + kNoallocTile - 1) / kNoallocTile);
-    int device = 0;
-    if (cudaGetDevice(&device) != cudaSuccess) {
+    int device = 0, sms = 0;
+    if (cudaGetDevice(&device) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) {
         cudaGetLastError();
         return MTX_ERR_NO_DEVICE;
     }
@@ -351,7 +406,7 @@ extern "C" mtx_status mtx_filter_active_blocks_noalloc(const uint32_t *leaf_minm
         cudaGetLastError();
         return MTX_ERR_CUDA;
     }
-    filter_compact_kernel<kNoallocItems, false><<<ntiles, kFilterThreads, 0, s>>>(
+    filter_compact_kernel<kNoallocItems, false><<<std::min(ntiles, kFilterCtas * (uint32_t)sms), kFilterThreads, 0, s>>>(
         reinterpret_cast<const uint2 *>(leaf_minmax), total_blocks, ntiles, dtype, isovalue, compacted_ids, block_rank,
         active_count, sc, sc + kNoallocTicket, st, kSpinLimit, 0u);
     if (cudaGetLastError() != cudaSuccess) return MTX_ERR_CUDA;
