@@ -19,15 +19,29 @@
 namespace mtx {
 
 // ------------------------------------------------------------- count pass
+// Warps a CTA at most: for B > 8 the shared memory of a warp (15 KB in the emit
+// pass, 13 to 30 in the count pass) and not the registers bounds the warps of an
+// SM, and one CTA with all of them wastes least of it.  640 x 512 x 448 uint16 at
+// B = 16 (2869 active blocks), CTAs of 4 and 8 warps: count 37 us, emit 112; one
+// CTA of 11 and 14: 30.5 and 85.
+constexpr int kBigWarps = 16;
+constexpr int cta_warps_max(int BC) { return BC == 0 || BC > 8 ? kBigWarps : kMaxWarps; }
+
+// A warp's first block.  For B > 8 a volume has few blocks, each long: they go
+// round the CTAs; else neighbours in a CTA share voxels and records in L1.
+__device__ __forceinline__ uint32_t first_block(uint32_t B, uint32_t warp, uint32_t W) {
+    return B > 8 ? warp * gridDim.x + blockIdx.x : blockIdx.x * W + warp;
+}
+
 // BC: the block edge at compile time (0: p.B at run time): the warp's
 // shared-memory plan and every division by the edge fold to constants.
 // Bound by instruction issue (2.6 a cycle and SM, 880 a block at B = 8).  Row
 // walks over the crossing rows with case bytes and prefixes kept for every cell
 // took 108 us for the 80,600 active blocks of the 1024^3 uint16 ball at B = 8;
 // the list takes 94; 1024 x 1024 x 314 uint8 at B = 3 179 -> 127; 384 x 320 x
-// 256 float32 at B = 4 58 -> 42; 640 x 512 x 448 uint16 at B = 16 53 -> 36.
+// 256 float32 at B = 4 58 -> 42; 640 x 512 x 448 uint16 at B = 16 53 -> 30.5.
 template <typename T, bool TMA, int BC>
-__global__ void __launch_bounds__(kMaxWarps * 32, 4)
+__global__ void __launch_bounds__(cta_warps_max(BC) * 32, BC == 0 ? 2 : BC > 8 ? 1 : 4)
     pmb_count_kernel(Problem p_, const __grid_constant__ CUtensorMap map, const uint32_t *__restrict__ ids,
                      const uint32_t *__restrict__ count_ptr, mtx_meshlet_descriptor *__restrict__ desc,
                      uint64_t desc_cap, uint16_t *__restrict__ faces, uint32_t *__restrict__ state,
@@ -61,7 +75,7 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 4)
     const uint32_t B3 = pl.BB * pl.B, slot = list_state_words(p.B), fslot = face_stride16(p.B);
     uint32_t parity = 0;
 
-    uint32_t r = blockIdx.x * W + warp;
+    uint32_t r = first_block(p.B, warp, W);
     const uint32_t nw = gridDim.x * W;
     Geo g{};
     if (r < count) {
@@ -119,7 +133,7 @@ struct BlockShare {
     uint32_t *ticket;
     __device__ __forceinline__ BlockShare(uint32_t count, uint32_t warps, uint32_t *t) : stride(warps), ticket(t) {
         const uint32_t rounds = count / warps;
-        fixed = rounds ? rounds * 3 / 4 * warps : ~0u;
+        fixed = rounds ? max(rounds * 3 / 4, 1u) * warps : ~0u;  // the first round is by stride, always
     }
     // The block after block r of this warp (lane 0's value is the block for tickets: take it by shuffle).
     __device__ __forceinline__ uint32_t after(uint32_t r) const {
@@ -138,9 +152,9 @@ struct BlockShare {
 // slower.  Against the tile, the rows and the row walks of the former pass:
 // 1024^3 uint16 ball at B = 8, 231 -> 157 us; 512^3 float32 gyroid at B = 8,
 // 225 -> 135; 640 x 512 x 448 uint16 at B = 16, one CTA of four warps an SM
-// before, 411 -> 110; 1024 x 1024 x 314 uint8 at B = 3, 251 -> 152.
+// before, 411 -> 85; 1024 x 1024 x 314 uint8 at B = 3, 251 -> 152.
 template <typename T, bool GENERIC, int BC, bool BIG>
-__global__ void __launch_bounds__(kMaxWarps * 32, GENERIC ? 1 : 4)
+__global__ void __launch_bounds__((BIG ? kBigWarps : kMaxWarps) * 32, GENERIC || BIG ? 1 : 4)
     pmb_emit_kernel(Problem p_, const uint32_t *__restrict__ ids, const uint32_t *__restrict__ rank_map,
                     const uint32_t *__restrict__ count_ptr, const mtx_meshlet_descriptor *__restrict__ desc,
                     const uint16_t *__restrict__ faces, const uint32_t *__restrict__ state,
@@ -173,7 +187,7 @@ __global__ void __launch_bounds__(kMaxWarps * 32, GENERIC ? 1 : 4)
     const uint32_t edge8 = BC == 8 ? ctx8_edge(lane) : 0u;
 
     const BlockShare share(count, gridDim.x * W, ticket);
-    uint32_t r = blockIdx.x * W + warp, drawn = share.after(r), nb_rk = kNoVertex;
+    uint32_t r = first_block(p.B, warp, W), drawn = share.after(r), nb_rk = kNoVertex;
     Geo g{};
     mtx_meshlet_descriptor d{};
     if (r < count) {
@@ -346,12 +360,12 @@ static mtx_status grid_for(mtx_context *c, K kernel, int threads, uint32_t smem,
     return MTX_OK;
 }
 
-// Warps a CTA: threads/32 of the options, else the context's tuning, else the
-// pass's own choice, and no more than the shared memory holds.
+// Warps a CTA: threads/32 of the options, else the context's tuning (up to
+// kMaxWarps), else the pass's own choice, and no more than the shared memory holds.
 static uint32_t cta_warps(const mtx_context *c, const ExtractArgs &a, uint32_t fixed, uint32_t per_warp,
                           uint32_t own) {
-    uint32_t W = a.threads ? a.threads / 32 : (c->tuning.extractWarps ? c->tuning.extractWarps : own);
-    W = std::min<uint32_t>(std::max<uint32_t>(W, 1), kMaxWarps);
+    const uint32_t asked = a.threads ? std::max(a.threads / 32, 1u) : c->tuning.extractWarps;
+    const uint32_t W = asked ? std::min<uint32_t>(asked, kMaxWarps) : own;
     const uint32_t room = c->max_smem_optin > (int)fixed ? (uint32_t)c->max_smem_optin - fixed : 0u;
     return std::min<uint32_t>(W, std::max<uint32_t>(1, room / per_warp));
 }
@@ -380,11 +394,11 @@ static mtx_status run_count(mtx_context *c, const Problem &p, const ExtractArgs 
     // the tile's element offsets in shared memory, where they fit 32 bits and B <= 8 keeps them small
     const bool use_off = !tma && p.B <= 8 && (uint64_t)(p.B + 1) * p.X * p.Y < (1ull << 32);
     const WPlan pl = make_count_plan(p.B, sizeof(T), tma);
-    const uint32_t fixed = count_fixed_bytes(p.B, use_off), W = cta_warps(c, a, fixed, pl.bytes, 4);
+    const uint32_t fixed = count_fixed_bytes(p.B, use_off), W = cta_warps(c, a, fixed, pl.bytes, p.B > 8 ? kBigWarps : 4);
     const uint32_t smem = fixed + W * pl.bytes;
     auto k = tma ? count_fn<T, true>(p.B) : count_fn<T, false>(p.B);
     unsigned grid;
-    mtx_status r = grid_for(c, k, W * 32, smem, a.host_count, W, grid);
+    mtx_status r = grid_for(c, k, W * 32, smem, a.host_count, p.B > 8 ? 1 : W, grid);
     if (r != MTX_OK) return r;
     k<<<grid, W * 32, smem, s>>>(p, map, a.ids, a.count, a.desc, a.desc_capacity, a.faces, a.state, a.totals,
                                  a.cell_cases, a.block_capacity, &c->ctrl->status, (uint64_t *)c->count_status.ptr,
@@ -409,12 +423,12 @@ static auto emit_fn(uint32_t B) {
 template <typename T>
 static mtx_status run_emit(mtx_context *c, const Problem &p, const ExtractArgs &a, cudaStream_t s) {
     const WPlan pl = make_emit_plan(p.B);
-    const uint32_t fixed = emit_fixed_bytes(p.B), W = cta_warps(c, a, fixed, pl.bytes, 8);
+    const uint32_t fixed = emit_fixed_bytes(p.B), W = cta_warps(c, a, fixed, pl.bytes, p.B > 8 ? kBigWarps : 8);
     const uint32_t smem = fixed + W * pl.bytes;
     const bool generic = a.vertices && (a.vertex_format != MTX_VERTEX_XYZ || a.frame != MTX_FRAME_VOXEL);
     auto k = generic ? emit_fn<T, true>(p.B) : emit_fn<T, false>(p.B);
     unsigned grid;
-    mtx_status r = grid_for(c, k, W * 32, smem, a.host_count, W, grid);
+    mtx_status r = grid_for(c, k, W * 32, smem, a.host_count, p.B > 8 ? 1 : W, grid);
     if (r != MTX_OK) return r;
     k<<<grid, W * 32, smem, s>>>(p, a.ids, a.rank_map, a.count, a.desc, a.faces, a.state, a.indices, a.tri_capacity,
                                  a.block_capacity, a.vertices, a.vertex_capacity, a.vertex_format, a.frame, a.normals,
