@@ -38,8 +38,8 @@ __device__ __forceinline__ uint32_t first_block(uint32_t B, uint32_t warp, uint3
 // Bound by instruction issue (2.6 a cycle and SM, 880 a block at B = 8).  Row
 // walks over the crossing rows with case bytes and prefixes kept for every cell
 // took 108 us for the 80,600 active blocks of the 1024^3 uint16 ball at B = 8;
-// the list takes 94; 1024 x 1024 x 314 uint8 at B = 3 179 -> 127; 384 x 320 x
-// 256 float32 at B = 4 58 -> 42; 640 x 512 x 448 uint16 at B = 16 53 -> 30.5.
+// the list takes 93; 1024 x 1024 x 314 uint8 at B = 3 179 -> 123; 384 x 320 x
+// 256 float32 at B = 4 58 -> 41; 640 x 512 x 448 uint16 at B = 16 53 -> 30.5.
 template <typename T, bool TMA, int BC>
 __global__ void __launch_bounds__(cta_warps_max(BC) * 32, BC == 0 ? 2 : BC > 8 ? 1 : 4)
     pmb_count_kernel(Problem p_, const __grid_constant__ CUtensorMap map, const uint32_t *__restrict__ ids,
@@ -394,7 +394,10 @@ static mtx_status run_count(mtx_context *c, const Problem &p, const ExtractArgs 
     // the tile's element offsets in shared memory, where they fit 32 bits and B <= 8 keeps them small
     const bool use_off = !tma && p.B <= 8 && (uint64_t)(p.B + 1) * p.X * p.Y < (1ull << 32);
     const WPlan pl = make_count_plan(p.B, sizeof(T), tma);
-    const uint32_t fixed = count_fixed_bytes(p.B, use_off), W = cta_warps(c, a, fixed, pl.bytes, p.B > 8 ? kBigWarps : 4);
+    // eight warps a CTA: the case counts are loaded half as often as with four and blocks
+    // next to each other share voxels in L1 (256^3 uint8 at B = 8 10.8 -> 9.7 us, 1024 x 1024 x 314
+    // at B = 3 127 -> 123, 1024^3 uint16 at B = 8 94.6 -> 93.1)
+    const uint32_t fixed = count_fixed_bytes(p.B, use_off), W = cta_warps(c, a, fixed, pl.bytes, p.B > 8 ? kBigWarps : 8);
     const uint32_t smem = fixed + W * pl.bytes;
     auto k = tma ? count_fn<T, true>(p.B) : count_fn<T, false>(p.B);
     unsigned grid;
