@@ -308,9 +308,13 @@ inline RowCut row_cut(const Problem &p, uint32_t esz) {
     return c;
 }
 
-// Whether the byte offsets of a block's rows fit 32 bits; wider rows take
-// minmax_leaf_one.
-inline bool rows_ok(const Problem &p, uint32_t esz) { return (uint64_t)p.X * esz * p.B < (1ull << 32); }
+// Whether the byte offsets of a block's rows fit 32 bits and every row is a
+// word or longer: then only the volume's first and last row have a word that
+// reaches past the volume (is_edge below).  Other rows take minmax_leaf_one.
+inline bool rows_ok(const Problem &p, uint32_t esz) {
+    const uint64_t row = (uint64_t)p.X * esz;
+    return row >= 4 && row * p.B < (1ull << 32);
+}
 
 // One warp's share of the leaf pass for any block edge and any row alignment:
 // a strip of nbs whole blocks of one block row over a run of zchunk slabs.
@@ -324,8 +328,8 @@ inline bool rows_ok(const Problem &p, uint32_t esz) { return (uint64_t)p.X * esz
 // four rows in flight.  s: 64 * W words of the warp's own shared memory.
 // nan_zero (float32): a NaN of positive sign takes the key of -0.0 instead of one
 // above +inf, which would leave its block without an isovalue -- what volumes
-// off the 16-byte passes have always had, while those passes keep the NaN's key.  The
-// B + 1 rows of a strip span less than 4 GiB (rows_ok).
+// off the 16-byte passes have always had, while those passes keep the NaN's key.  Rows
+// are 4 bytes or longer and the B + 1 rows of a strip span less than 4 GiB (rows_ok).
 // Bound by instruction issue (about 2.5 a cycle and SM): every word costs an
 // address, a load, for unaligned rows a shuffle and a shift, and half a
 // min/max pair.  Against one thread a block, whose byte loads read every voxel
@@ -393,7 +397,10 @@ __device__ __forceinline__ void minmax_leaf_rows_warp(const T *__restrict__ vol,
         const uintptr_t a = at + row_off(r);
         const uint32_t *src = reinterpret_cast<const uint32_t *>(ALIGNED ? a : a & ~(uintptr_t)3);
 #pragma unroll
-        for (int j = 0; j < W; ++j) raw[j] = on[j] ? __ldg(src + 32 * j) : 0u;
+        for (int j = 0; j < W; ++j) {
+            [[maybe_unused]] const uintptr_t last = reinterpret_cast<uintptr_t>(src + 32 * j) + 3;
+            raw[j] = on[j] && MTX_BC(last - vbeg, vend - vbeg, kBcVolume) ? __ldg(src + 32 * j) : 0u;
+        }
     };
     // the same for a row with a word that may reach past the volume: its bytes one by one
     auto load_edge = [&](uintptr_t at, uint32_t r, uint32_t raw[W]) {
@@ -517,7 +524,7 @@ __device__ __forceinline__ void minmax_leaf_rows_warp(const T *__restrict__ vol,
     if (bz < bz1) close(bz);
 }
 
-// One block by one thread: rows too long for the 32-bit offsets above.
+// One block by one thread: rows that rows_ok refuses.
 template <typename T>
 __device__ __forceinline__ void minmax_leaf_one(const T *__restrict__ vol, uint32_t X, uint32_t Y, uint32_t Z,
                                                 uint32_t B, uint32_t GX, uint32_t GY, uint64_t b,

@@ -61,6 +61,7 @@ enum : uint32_t {
     kBcRank = 110,      // rank map and compacted ids
     kBcLeaf = 111,      // min/max leaf level
     kBcDesc = 112,      // meshlet descriptors
+    kBcVolume = 113,    // voxel words of the rows leaf pass, in bytes of the volume
 };
 #ifdef MTX_BOUNDS_CHECK
 static __device__ DevStatus g_bc_record;
