@@ -104,10 +104,13 @@ __global__ void __launch_bounds__(cta_warps_max(BC) * 32, BC == 0 ? 2 : BC > 8 ?
 }
 
 // -------------------------------------------------------------- scan pass
+// capacity: descriptors that desc and the tile words hold.  With more active
+// blocks than that the count pass has reported the error and set the totals,
+// and there is nothing to scan.
 __global__ void __launch_bounds__(kScanThreads)
     pmb_scan_kernel(mtx_meshlet_descriptor *__restrict__ desc, const uint32_t *__restrict__ count_ptr,
-                    uint64_t *tile_status, uint32_t *ticket, uint32_t *totals, DevStatus *st, uint32_t spin_limit,
-                    uint32_t skip, uint32_t *emit_ticket) {
+                    uint64_t capacity, uint64_t *tile_status, uint32_t *ticket, uint32_t *totals, DevStatus *st,
+                    uint32_t spin_limit, uint32_t skip, uint32_t *emit_ticket) {
     if (blockIdx.x == 0 && threadIdx.x == 0) *emit_ticket = 0;  // for the emit pass that follows
     __shared__ uint32_t s_tile, s_ok;
     __shared__ uint64_t s_tmp[kScanThreads / 32 + 1];
@@ -116,7 +119,7 @@ __global__ void __launch_bounds__(kScanThreads)
     __syncthreads();
     const uint32_t t = s_tile;
     const uint32_t count = *count_ptr;
-    if (t >= (count + kScanTile - 1) / kScanTile) return;
+    if (count > capacity || t >= (count + kScanTile - 1) / kScanTile) return;
     scan_tile(desc, count, t, tile_status, totals, st, s_tmp, &s_ok, s_pre, spin_limit);
 }
 
@@ -459,10 +462,9 @@ size_t face_record_bytes(uint32_t B) { return 2 * (size_t)face_stride16(B); }
 // The scan over up to `capacity` descriptors, behind a kernel that ran scan_reset for it.
 static mtx_status run_scan(mtx_context *c, mtx_meshlet_descriptor *desc, const uint32_t *count, uint64_t capacity,
                            uint32_t *totals, uint32_t skip, cudaStream_t s) {
-    pmb_scan_kernel<<<scan_tiles(capacity), kScanThreads, 0, s>>>(desc, count, (uint64_t *)c->count_status.ptr,
-                                                                  &c->ctrl->count_ticket, totals, &c->ctrl->status,
-                                                                  c->wait_polls ? c->wait_polls : kSpinLimit, skip,
-                                                                  &c->ctrl->emit_ticket);
+    pmb_scan_kernel<<<scan_tiles(capacity), kScanThreads, 0, s>>>(
+        desc, count, capacity, (uint64_t *)c->count_status.ptr, &c->ctrl->count_ticket, totals, &c->ctrl->status,
+        c->wait_polls ? c->wait_polls : kSpinLimit, skip, &c->ctrl->emit_ticket);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(c, e, "scan launch");
     return MTX_OK;
