@@ -158,7 +158,7 @@ void dev_cache_release(int device) {
         }
     }
     for (const IdleBuf &b : drop) {
-        if (b.freed) cudaEventSynchronize(b.freed->ev);
+        if (b.freed && cudaEventSynchronize(b.freed->ev) != cudaSuccess) cudaGetLastError();
         cudaFree(b.ptr);
     }
     for (cudaEvent_t e : events) cudaEventDestroy(e);
@@ -179,7 +179,8 @@ mtx_status dev_alloc(mtx_context *c, void **p, size_t bytes) {
             if (e == cudaErrorNotReady) e = cudaStreamWaitEvent(c->stream, idle.freed->ev, 0);
             if (e != cudaSuccess) {
                 cudaGetLastError();
-                cudaEventSynchronize(idle.freed->ev);
+                // (an event last recorded in a capture has nothing to wait for)
+                if (cudaEventSynchronize(idle.freed->ev) != cudaSuccess) cudaGetLastError();
             }
         }
         *p = idle.ptr;
@@ -254,7 +255,7 @@ void dev_free(mtx_context *c, std::initializer_list<void *> ptrs) {
             }
         }
         if (!keep) {
-            if (mark) cudaEventSynchronize(mark->ev);
+            if (mark && cudaEventSynchronize(mark->ev) != cudaSuccess) cudaGetLastError();
             cudaFree(p);
         }
     }
@@ -277,6 +278,16 @@ mtx_status scratch_reserve(mtx_context *c, Scratch &s, size_t bytes) {
     mtx_status r = dev_alloc(c, &s.ptr, want);
     if (r != MTX_OK) return r;
     s.size = want;
+    return MTX_OK;
+}
+
+mtx_status rezero(mtx_context *c, cudaStream_t s) {
+    if (!c->rezero) return MTX_OK;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    MTX_CUDA(c, cudaStreamIsCapturing(s, &capture));
+    MTX_CUDA(c, cudaMemsetAsync(&c->ctrl->filter_ticket, 0, 8, s));
+    if (c->filter_status.ptr) MTX_CUDA(c, cudaMemsetAsync(c->filter_status.ptr, 0, c->filter_status.size, s));
+    if (capture == cudaStreamCaptureStatusNone) c->rezero = false;  // a captured memset has not run
     return MTX_OK;
 }
 

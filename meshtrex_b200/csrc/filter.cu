@@ -268,11 +268,11 @@ mtx_status launch_filter(mtx_context *c, const Problem &p, const uint2 *leaf, ui
                          uint32_t *count, cudaStream_t s, const PyrAll *octree) {
     if (p.nblocks >= (1ull << 30)) return fail(c, MTX_ERR_UNSUPPORTED, "more than 2^30 blocks");
     const uint32_t ntiles = (uint32_t)((p.nblocks + kFilterTile - 1) / kFilterTile);
-    const size_t before = c->filter_status.size;
+    const void *before = c->filter_status.ptr;
+    const size_t size = c->filter_status.size;
     mtx_status rs = scratch_reserve(c, c->filter_status, sizeof(uint64_t) * (size_t)ntiles);
-    if (rs != MTX_OK) return rs;
-    if (c->filter_status.size != before)  // new words: no epoch's
-        MTX_CUDA(c, cudaMemsetAsync(c->filter_status.ptr, 0, c->filter_status.size, s));
+    if (c->filter_status.ptr != before || c->filter_status.size != size) c->rezero = true;  // new words: no epoch's
+    if (rs != MTX_OK || (rs = rezero(c, s)) != MTX_OK) return rs;
     uint64_t *words = (uint64_t *)c->filter_status.ptr;
     const uint32_t ctas = std::min(ntiles, kFilterCtas * (uint32_t)c->sm_count);
     const uint32_t polls = c->wait_polls ? c->wait_polls : kSpinLimit, skip = c->withhold & 1u;

@@ -68,6 +68,9 @@ struct mtx_context {
         int ctas;
     };
     std::vector<Occupancy> occupancy;  // ctas_per_sm
+    // Whether the compaction's look-back words and ticket are zeroed ahead of its
+    // next launch: they are new, and no launch outside a capture has zeroed them yet.
+    bool rezero = false;
 };
 
 namespace mtx {
@@ -98,6 +101,7 @@ void dev_free(mtx_context *c, std::initializer_list<void *> ptrs);
 void dev_free(mtx_context *c, void *p);  // ordered on c's stream (c may be null: a device-wide wait)
 mtx_status ctas_per_sm(mtx_context *c, const void *kernel, int threads, uint32_t smem, int *out);
 mtx_status scratch_reserve(mtx_context *c, Scratch &s, size_t bytes);
+mtx_status rezero(mtx_context *c, cudaStream_t s);  // where mtx_context::rezero asks for it
 // Makes the context's stream wait for an extraction still running on its
 // extraction stream (mtx_context_set_extract_stream); every entry point that
 // queues work on the context or touches its scratch calls it first.
