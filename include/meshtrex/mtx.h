@@ -196,6 +196,10 @@ uint32_t mtx_abi_version(void);
  * scratch arena. */
 mtx_status mtx_context_create(int device, void *stream, mtx_context_t *out);
 mtx_status mtx_context_destroy(mtx_context_t ctx);
+/* Later calls go to `stream`.  A context's calls share its scratch and its
+ * counters, so the caller orders them: work still queued on the former stream,
+ * and replays of a captured call on another one, must come before later calls
+ * on the new stream (an event, or a wait) and not overlap them. */
 mtx_status mtx_context_set_stream(mtx_context_t ctx, void *stream);
 /* A second stream for the count, scan and emit passes of
  * mtx_extract_plain_async (NULL: none, everything on the context's stream).

@@ -110,8 +110,8 @@ __global__ void __launch_bounds__(cta_warps_max(BC) * 32, BC == 0 ? 2 : BC > 8 ?
 __global__ void __launch_bounds__(kScanThreads)
     pmb_scan_kernel(mtx_meshlet_descriptor *__restrict__ desc, const uint32_t *__restrict__ count_ptr,
                     uint64_t capacity, uint64_t *tile_status, uint32_t *ticket, uint32_t *totals, DevStatus *st,
-                    uint32_t spin_limit, uint32_t skip, uint32_t *emit_ticket) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) *emit_ticket = 0;  // for the emit pass that follows
+                    uint32_t spin_limit, uint32_t skip, uint32_t *emit_ticket, uint32_t *emit_done) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) *emit_ticket = *emit_done = 0;  // for the emit pass that follows
     __shared__ uint32_t s_tile, s_ok;
     __shared__ uint64_t s_tmp[kScanThreads / 32 + 1];
     __shared__ uint64_t s_pre[2];
@@ -330,7 +330,6 @@ __global__ void __launch_bounds__((BIG ? kBigWarps : kMaxWarps) * 32, GENERIC ||
             __threadfence();
             if (atomicAdd(done, 1u) == gridDim.x - 1) {
                 __threadfence();
-                *done = 0;
                 *status_out = ld_volatile(&st->code);
             }
         }
@@ -464,7 +463,7 @@ static mtx_status run_scan(mtx_context *c, mtx_meshlet_descriptor *desc, const u
                            uint32_t *totals, uint32_t skip, cudaStream_t s) {
     pmb_scan_kernel<<<scan_tiles(capacity), kScanThreads, 0, s>>>(
         desc, count, capacity, (uint64_t *)c->count_status.ptr, &c->ctrl->count_ticket, totals, &c->ctrl->status,
-        c->wait_polls ? c->wait_polls : kSpinLimit, skip, &c->ctrl->emit_ticket);
+        c->wait_polls ? c->wait_polls : kSpinLimit, skip, &c->ctrl->emit_ticket, &c->ctrl->emit_done);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(c, e, "scan launch");
     return MTX_OK;

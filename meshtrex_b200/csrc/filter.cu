@@ -30,9 +30,13 @@ constexpr int kNoallocTile = kFilterThreads * kNoallocItems;
 // word epoch << 32 | ticket; the CTA that draws a launch's last ticket starts
 // the next epoch, so that the words of earlier launches read as empty and
 // nothing has to be zeroed between launches (three memsets of about 4 us
-// each on the timeline before; the words are zeroed once, when the scratch
-// grows).  Otherwise (the no-allocation entry point, whose array holds 32-bit
-// words): flag << 30 | count, zeroed before the launch.
+// each on the timeline before).  The words and the ticket are zeroed when the
+// scratch grows, after an error and when the context's stream changes
+// (rezero): launches of one context that overlapped would leave the ticket
+// short of an epoch's end or past it, and every later one waiting for tiles
+// that are never handed out; a ticket past the last is reported.  Otherwise (the
+// no-allocation entry point, whose array holds 32-bit words): flag << 30 |
+// count, zeroed before the launch.
 // flag: 0 empty, 1 aggregate, 2 inclusive, 3 aborted.
 constexpr uint32_t kFlagAgg = 1u, kFlagInc = 2u, kFlagAbort = 3u;
 template <bool EPOCH> struct TileWord;
@@ -45,6 +49,7 @@ template <> struct TileWord<false> {
         epoch = 0;
         return atomicAdd(ticket, 1u);
     }
+    __device__ __forceinline__ static bool torn(uint32_t, uint32_t) { return false; }
 };
 template <> struct TileWord<true> {
     using U = uint64_t;
@@ -61,6 +66,8 @@ template <> struct TileWord<true> {
         if ((uint32_t)t == draws - 1) st_volatile(ticket, (U)((epoch + 1) & 0x3fffffffu) << 32);
         return (uint32_t)t;
     }
+    // A ticket past a launch's last: the word was not left at an epoch's start.
+    __device__ __forceinline__ static bool torn(uint32_t t, uint32_t draws) { return t >= draws; }
 };
 
 // A tile is ITEMS / 2 rounds of 64 consecutive blocks a warp, lane l taking
@@ -97,8 +104,12 @@ __device__ __forceinline__ void filter_tiles(const uint2 *__restrict__ leaf, uin
     const uint32_t draws = ntiles - skip + ctas;
     if (threadIdx.x == 0) {
         uint32_t epoch;
-        s_draw[0] = TW::draw(ticket, draws, epoch) + skip;
+        const uint32_t first = TW::draw(ticket, draws, epoch);
+        s_draw[0] = first + skip;
         s_epoch = epoch;
+        const bool torn = TW::torn(first, draws);
+        if (torn) report(st, MTX_ERR_INTERNAL, kSiteFilterTicket, first, draws);
+        if (torn || skip >= ntiles) *count_out = 0;  // no CTA may take the last tile
     }
     __syncthreads();
     uint32_t t = s_draw[0], e;
@@ -271,7 +282,8 @@ mtx_status launch_filter(mtx_context *c, const Problem &p, const uint2 *leaf, ui
     const void *before = c->filter_status.ptr;
     const size_t size = c->filter_status.size;
     mtx_status rs = scratch_reserve(c, c->filter_status, sizeof(uint64_t) * (size_t)ntiles);
-    if (c->filter_status.ptr != before || c->filter_status.size != size) c->rezero = true;  // new words: no epoch's
+    if (c->filter_status.ptr != before || c->filter_status.size != size)
+        c->rezero = mtx_context::kRezeroNeeded;  // new words: no epoch's
     if (rs != MTX_OK || (rs = rezero(c, s)) != MTX_OK) return rs;
     uint64_t *words = (uint64_t *)c->filter_status.ptr;
     const uint32_t ctas = std::min(ntiles, kFilterCtas * (uint32_t)c->sm_count);

@@ -576,8 +576,8 @@ mtx_status pyramid_levels(mtx_context *c, uint2 *all, int levels, const uint32_t
 mtx_status launch_pyramid(mtx_context *c, uint2 *all, int levels, const uint32_t ext[][3],
                           const uint64_t *offset, cudaStream_t s, int start) {
     PyrAll P;
-    const mtx_status r = pyramid_levels(c, all, levels, ext, offset, start, &P);
-    if (r != MTX_OK || !P.ntiles) return r;
+    mtx_status r = pyramid_levels(c, all, levels, ext, offset, start, &P);
+    if (r != MTX_OK || !P.ntiles || (r = rezero(c, s)) != MTX_OK) return r;
     pyramid_all_kernel<<<P.ctas, kPyrThreads, 0, s>>>(P);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(c, e, "pyramid launch");

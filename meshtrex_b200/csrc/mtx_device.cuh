@@ -30,6 +30,7 @@ enum : uint32_t {
     kSiteBatched = 7,
     kSiteAdjoint = 8,
     kSiteMinMaxTma = 9,
+    kSiteFilterTicket = 10,
 };
 
 __device__ __forceinline__ void report(DevStatus *st, uint32_t code, uint32_t where, uint32_t i0 = 0,

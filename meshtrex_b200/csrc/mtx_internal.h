@@ -17,14 +17,16 @@ namespace mtx {
 // Per-pipeline control words in device memory.
 struct Ctrl {
     DevStatus status;        // first error recorded by any kernel
+    // These two every launch leaves as the next one needs them (rezero).
     uint64_t filter_ticket;  // compaction: epoch << 32 | tile ticket
+    uint32_t pyr_done;       // octree CTAs finished (the last one builds the top levels)
+    uint32_t pad0;
     uint32_t count_ticket;   // tile tickets of the count scan
     uint32_t active_count;   // compaction result
     uint32_t totals[4];      // vertexCount, indexCount, meshletCount, activeBlockCount
     uint32_t batch_ticket[4];
-    uint32_t pyr_done;       // octree CTAs finished (the last one builds the top levels)
     uint32_t emit_done;      // CTAs of the emit pass finished (the last one writes status_out)
-    uint32_t emit_ticket;    // emit pass: blocks handed out by ticket (zeroed by the scan pass)
+    uint32_t emit_ticket;    // emit pass: blocks handed out by ticket (both zeroed by the scan pass)
     uint32_t pad1;
 };
 
@@ -68,9 +70,13 @@ struct mtx_context {
         int ctas;
     };
     std::vector<Occupancy> occupancy;  // ctas_per_sm
-    // Whether the compaction's look-back words and ticket are zeroed ahead of its
-    // next launch: they are new, and no launch outside a capture has zeroed them yet.
-    bool rezero = false;
+    // When the compaction's look-back words and ticket and the octree's counter
+    // are zeroed ahead of a launch: kRezeroEager before the next launch that is
+    // not captured (the stream changed, and launches on two streams that
+    // overlapped would have left them torn), kRezeroNeeded before any (new words,
+    // or an error).
+    enum Rezero { kRezeroNo, kRezeroEager, kRezeroNeeded };
+    Rezero rezero = kRezeroNo;
 };
 
 namespace mtx {
@@ -101,7 +107,7 @@ void dev_free(mtx_context *c, std::initializer_list<void *> ptrs);
 void dev_free(mtx_context *c, void *p);  // ordered on c's stream (c may be null: a device-wide wait)
 mtx_status ctas_per_sm(mtx_context *c, const void *kernel, int threads, uint32_t smem, int *out);
 mtx_status scratch_reserve(mtx_context *c, Scratch &s, size_t bytes);
-mtx_status rezero(mtx_context *c, cudaStream_t s);  // where mtx_context::rezero asks for it
+mtx_status rezero(mtx_context *c, cudaStream_t s);  // as mtx_context::rezero asks for
 // Makes the context's stream wait for an extraction still running on its
 // extraction stream (mtx_context_set_extract_stream); every entry point that
 // queues work on the context or touches its scratch calls it first.
