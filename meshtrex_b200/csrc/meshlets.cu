@@ -142,6 +142,94 @@ __global__ void __launch_bounds__(kMeshletWarps * 32)
     }
 }
 
+// The same rule for meshlets of few triangles.  A warp has the corners of
+// kFewTriangles triangles one a lane, and a step takes as many of them as join
+// the current meshlet: equal vertices are found by a match across the lanes, so
+// there is no table to fill and clear.  A meshlet that has room for more keeps its
+// vertices one a lane, and the next step's corners are compared with each.
+// The words ahead are in registers, as where a meshlet ends is known only at
+// its end.
+// Taken (few_triangles) for up to kFewTriangles triangles a meshlet or
+// kFewVertices vertices; above, meshlets outgrow a step.  Count and emit of a
+// 201 x 243 x 257 volume at B = 8, us, one triangle at a time / 32 a step / so:
+// (maxVertices, maxPrimitives) = (3, 1) and (3, 126) 1314 / 1737 / 976, (4, 126)
+// 1225 / 1129 / 671, (8, 126) 1152 / 446 / 302, (64, 10) 1124 / 196 / 169; 32 a
+// step take 182 at (64, 11) and 272 at (12, 126).
+constexpr uint32_t kFewTriangles = 10, kFewVertices = 8;
+static bool few_triangles(uint32_t maxV, uint32_t maxP) { return maxP <= kFewTriangles || maxV <= kFewVertices; }
+
+template <bool EMIT>
+__global__ void __launch_bounds__(kMeshletWarps * 32)
+    meshlet_few_kernel(const mtx_meshlet_descriptor *__restrict__ blocks, const uint32_t *__restrict__ count_ptr,
+                       const uint32_t *__restrict__ indices, uint32_t maxV, uint32_t maxP,
+                       mtx_meshlet_descriptor *__restrict__ per_block, mtx_meshlet_descriptor *__restrict__ meshlets,
+                       uint32_t *__restrict__ mverts, uint32_t *__restrict__ midx, uint64_t *scan_words,
+                       uint32_t scan_ntiles, uint32_t *scan_ticket, uint32_t *totals) {
+    if (!EMIT) scan_reset(scan_words, scan_ntiles, scan_ticket, totals);
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, tri = lane / 3u;
+    const uint32_t upto = lane < 3 * kFewTriangles ? (8u << (3 * tri)) - 1u : 0u;  // corners up to this one's triangle's last
+    const uint32_t n = *count_ptr;
+    for (uint32_t r = blockIdx.x * kMeshletWarps + warp; r < n; r += gridDim.x * kMeshletWarps) {
+        const mtx_meshlet_descriptor b = blocks[r];
+        const uint32_t t0 = b.indexOffset / 3u, nt = b.primitiveCount, words = 3 * nt;
+        uint32_t mbase = 0, vbase = 0;  // EMIT: the block's first meshlet and first meshlet vertex
+        if (EMIT) {
+            mbase = per_block[r].indexOffset / 3u;
+            vbase = per_block[r].vertexOffset;
+        }
+        const uint32_t *src = indices + 3ull * t0;
+        auto load = [&](uint32_t w) { return w < words ? __ldg(src + w) : 0u; };
+        uint32_t mcount = 0, vused = 0;                 // meshlets closed, their vertices
+        uint32_t cur_v = 0, cur_p = 0, mine = 0;        // the current one's; lane v: its vertex v
+        uint32_t base = 0, w0 = load(lane), w1 = load(32 + lane);  // the block's words from base on
+        for (uint32_t t = 0; t < nt;) {
+            if (3 * t - base >= 32) {  // a step moves by 30 words at most
+                w0 = w1;
+                base += 32;
+                w1 = load(base + 32 + lane);
+            }
+            const uint32_t at = 3 * t - base + lane;
+            const uint32_t a0 = __shfl_sync(0xffffffffu, w0, at & 31), a1 = __shfl_sync(0xffffffffu, w1, at & 31);
+            const uint32_t id = at < 32 ? a0 : a1;
+            const bool on = upto && cur_p + tri < maxP && t + tri < nt;
+            uint32_t num = kNoId;  // the corner's vertex in the meshlet, where it has it already
+            for (uint32_t v = 0; v < cur_v; ++v)
+                if (__shfl_sync(0xffffffffu, mine, v) == id) num = v;
+            const uint32_t live = __ballot_sync(0xffffffffu, on);
+            const uint32_t first = __ffs(__match_any_sync(0xffffffffu, id) & live) - 1;  // the vertex's first corner
+            const bool own = on && first == lane && num == kNoId;
+            const uint32_t fresh = __ballot_sync(0xffffffffu, own);
+            const uint32_t fit = __ballot_sync(0xffffffffu, on && cur_v + __popc(fresh & upto) <= maxV);
+            const uint32_t corners = __ffs(~fit) - 1, take = corners / 3u;  // triangles that join the meshlet
+            const uint32_t used = __popc(fresh & ((1u << corners) - 1u));
+            if (EMIT && lane < corners) {
+                if (num == kNoId) num = cur_v + __popc(fresh & ((1u << first) - 1u));
+                midx[3ull * (t0 + t) + lane] = vbase + vused + num;
+                if (own) mverts[vbase + vused + num] = id;
+            }
+            t += take;
+            if (take == kFewTriangles && cur_p + take < maxP && t < nt) {  // room for more
+                const uint32_t k = lane - cur_v;
+                const uint32_t from = k < used ? __fns(fresh, 0, (int)k + 1) : 0u;
+                const uint32_t got = __shfl_sync(0xffffffffu, id, from);
+                if (k < used) mine = got;
+                cur_v += used;
+                cur_p += take;
+                continue;
+            }
+            cur_v += used;
+            cur_p += take;
+            if (EMIT && lane == 0)
+                meshlets[mbase + mcount] =
+                    mtx_meshlet_descriptor{vbase + vused, 3u * (t0 + t - cur_p), cur_v, cur_p};
+            vused += cur_v;
+            ++mcount;
+            cur_v = cur_p = 0;
+        }
+        if (!EMIT && lane == 0) per_block[r] = mtx_meshlet_descriptor{0u, 0u, vused, mcount};
+    }
+}
+
 // vertexData[j] = vertices[mverts[j]], stride words of type V per record (16-byte
 // words for the 32-byte records, else floats); 64-bit indices and divisions by a
 // run-time stride, a float a thread, took 12.5 us where this takes 6.4 (the same volume).
@@ -195,9 +283,10 @@ extern "C" mtx_status mtx_build_meshlets(mtx_context_t c, const mtx_extraction_o
     uint32_t ntiles, *ticket;
     if ((r = desc_scan_words(c, nb, &words, &ntiles, &ticket)) != MTX_OK) return bail(r);
     const uint32_t grid = std::min<uint32_t>((nb + kMeshletWarps - 1) / kMeshletWarps, 16u * c->sm_count);
-    meshlet_kernel<false><<<grid, kMeshletWarps * 32, 0, s>>>(blocks, count, indices, maxVertices, maxPrimitives,
-                                                              (mtx_meshlet_descriptor *)per_block, nullptr, nullptr,
-                                                              nullptr, words, ntiles, ticket, (uint32_t *)counters);
+    const bool few = few_triangles(maxVertices, maxPrimitives);
+    (few ? meshlet_few_kernel<false> : meshlet_kernel<false>)<<<grid, kMeshletWarps * 32, 0, s>>>(
+        blocks, count, indices, maxVertices, maxPrimitives, (mtx_meshlet_descriptor *)per_block, nullptr, nullptr,
+        nullptr, words, ntiles, ticket, (uint32_t *)counters);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return bail(cuda_fail(c, e, "meshlet count launch"));
     if ((r = launch_desc_scan(c, (mtx_meshlet_descriptor *)per_block, count, nb, (uint32_t *)counters, s)) != MTX_OK)
@@ -216,10 +305,9 @@ extern "C" mtx_status mtx_build_meshlets(mtx_context_t c, const mtx_extraction_o
     out->indexBuffer = {p_idx, 12ull * T};
     if ((r = dev_alloc(c, &p_vd, 4ull * stride * MV)) != MTX_OK) return bail(r);
     out->vertexBuffer = {p_vd, 4ull * stride * MV};
-    meshlet_kernel<true><<<grid, kMeshletWarps * 32, 0, s>>>(blocks, count, indices, maxVertices, maxPrimitives,
-                                                             (mtx_meshlet_descriptor *)per_block,
-                                                             (mtx_meshlet_descriptor *)p_desc, (uint32_t *)p_mv,
-                                                             (uint32_t *)p_idx, nullptr, 0, nullptr, nullptr);
+    (few ? meshlet_few_kernel<true> : meshlet_kernel<true>)<<<grid, kMeshletWarps * 32, 0, s>>>(
+        blocks, count, indices, maxVertices, maxPrimitives, (mtx_meshlet_descriptor *)per_block,
+        (mtx_meshlet_descriptor *)p_desc, (uint32_t *)p_mv, (uint32_t *)p_idx, nullptr, 0, nullptr, nullptr);
     if ((e = cudaGetLastError()) != cudaSuccess) return bail(cuda_fail(c, e, "meshlet emit launch"));
     const bool wide = stride == 8 && ((uintptr_t)ext->vertexBuffer.ptr | (uintptr_t)p_vd) % 16 == 0;
     const uint64_t work = (uint64_t)MV * (wide ? 2 : stride);
