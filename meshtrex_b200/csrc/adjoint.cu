@@ -24,7 +24,11 @@
 // Staging each tile as float and walking its rows took 49 us (ATOMIC) for the
 // 7,700 active blocks of a 512^3 volume, after 88 us of zeroing, and 34 us, with
 // 36 us for a gather over whole tiles, for the 1,250 of 250 x 198 x 171
-// (DETERMINISTIC); this takes 31, and 14 with 9.
+// (DETERMINISTIC); this takes 31, and 14 with 9.  Blocks with more terms than the
+// shared memory holds list their voxels again for each axis: a noisy 300 x 400 x
+// 512 float32 ball at B = 8, 232 vertices a block, takes 81 us, 132 with its gather
+// (126 and 271 by tiles and rows; 142 and 223 with terms kept for at most 256 voxels
+// a block and rows walked again by lane).
 #include "pmb_lists.cuh"
 
 namespace mtx {
@@ -49,8 +53,10 @@ struct AdjArgs {
     DevStatus *st;
 };
 
-// Listed voxels of a block whose dL/diso terms are kept in shared memory.
-__host__ __device__ inline uint32_t iso_terms(uint32_t B) { return B <= 8 ? 256u : 768u; }
+// dL/diso terms, one a vertex, that a warp's shared memory holds: all that a block
+// of edge 6 or less can have, half of the most one of edge 8 can, and more than a
+// surface through it has.
+__host__ __device__ inline uint32_t iso_terms(uint32_t B) { return std::min(3 * B * B * B, B <= 8 ? 768u : 2304u); }
 
 // A warp's shared memory: inside rows, list bits, list, the plain loads'
 // bitstream, dL/diso terms, and for DETERMINISTIC the accumulation tile
@@ -69,7 +75,7 @@ __host__ __device__ inline WPlan make_adjoint_plan(uint32_t B, bool det) {
     p.off_case = o;
     o = align_up(o + 4 * ((T3 + 31) / 32 + 1), 16);
     p.off_vp = o;  // dL/diso terms, axis by axis
-    o += 12 * iso_terms(B);
+    o = align_up(o + 4 * iso_terms(B), 16);
     p.off_tile = o;
     if (det) o = align_up(o + 4 * T3, 16);
     p.bytes = o;
@@ -77,10 +83,11 @@ __host__ __device__ inline WPlan make_adjoint_plan(uint32_t B, bool det) {
 }
 
 // List bits of the voxels that own a cut edge.  Lane l takes rows [l R, l R + R),
-// R = ceil(B^2 / 32): its listed voxels are list[at, at + n), its vertices the
-// block's from vat on; nl and nv are the block's.
+// R = ceil(B^2 / 32): of the block's cut edges along an axis its own are
+// [at, at + own).
 struct CutRows {
-    uint32_t at, n, vat, nl, nv;
+    uint32_t at[2], own[2];  // of x | y << 16, z
+    uint32_t nx, ny, nz;     // the block's
 };
 template <int BC>
 __device__ __forceinline__ CutRows cut_bits(const Problem &p, const WPlan &pl, unsigned char *ws, const Geo &g) {
@@ -90,14 +97,13 @@ __device__ __forceinline__ CutRows cut_bits(const Problem &p, const WPlan &pl, u
     for (uint32_t i = lane; i < list_words(B); i += 32) bits[i] = 0;
     __syncwarp();
     CutRows c{};
-    uint32_t nv = 0;
     for (uint32_t q = lane * R; q < min(pl.BB, lane * R + R); ++q) {
         const uint32_t z = fdiv(q, pl.rB), y = q - z * B;
         uint32_t xc, yc, zc;
         row_cross(p, pl, g, rows, y, z, xc, yc, zc);
-        nv += __popc(xc) + __popc(yc) + __popc(zc);
+        c.own[0] += __popc(xc) | (__popc(yc) << 16);
+        c.own[1] += __popc(zc);
         const uint32_t m = xc | yc | zc;
-        c.n += __popc(m);
         if constexpr (BC == 8) {
             reinterpret_cast<uint8_t *>(bits)[q] = (uint8_t)m;
         } else if (m) {
@@ -107,9 +113,24 @@ __device__ __forceinline__ CutRows cut_bits(const Problem &p, const WPlan &pl, u
         }
     }
     __syncwarp();
-    c.at = warp_excl_scan(c.n, c.nl);
-    c.vat = warp_excl_scan(nv, c.nv);
+    uint32_t xy;  // at most 4096 an axis
+    c.at[0] = warp_excl_scan(c.own[0], xy);
+    c.nx = xy & 0xffffu;
+    c.ny = xy >> 16;
+    c.at[1] = warp_excl_scan(c.own[1], c.nz);
     return c;
+}
+
+// Of the step's cut edges along each axis, those of the voxels before this lane's
+// and all of them (m: this lane's cut owned edges).
+__device__ __forceinline__ void step_edges(uint32_t m, uint32_t before[3], uint32_t all[3]) {
+    const uint32_t lt = (1u << (threadIdx.x & 31)) - 1u;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const uint32_t b = __ballot_sync(0xffffffffu, (m >> k) & 1u);
+        before[k] = __popc(b & lt);
+        all[k] = __popc(b);
+    }
 }
 
 // One vertex's dL/diso term (the gradient along its edge over the edge's value
@@ -118,8 +139,18 @@ __device__ __forceinline__ float iso_term(float gv, float scale, float den) {
     return fabsf(den) > 1e-5f ? __fdiv_rn(__fmul_rn(gv, scale), den) : 0.0f;
 }
 
+// CTAs an SM that the register count has to allow, where the compiler's own choice
+// takes more registers than pay (0: its choice).  Block edge 5, ATOMIC: 122
+// registers 337 us, 64 registers 263 (300 x 400 x 512 uint16, 35 vertices a
+// block); run-time edges, DETERMINISTIC: 96 registers 585, 80 registers 538 (B = 6);
+// at B = 2, 4 and 8 a bound of the same register count is 2 to 5% slower than none.
+constexpr int adjoint_min_ctas(bool det, int BC) {
+    return BC == 0 ? (det ? 6 : 8) : BC == 5 ? (det ? 7 : 8) : BC == 3 && !det ? 8 : 0;
+}
+
 template <typename T, bool DET, int BC>
-__global__ void __launch_bounds__(kAdjWarps * 32) adjoint_block_kernel(const __grid_constant__ AdjArgs a) {
+__global__ void __launch_bounds__(kAdjWarps * 32, adjoint_min_ctas(DET, BC))
+    adjoint_block_kernel(const __grid_constant__ AdjArgs a) {
     extern __shared__ __align__(128) unsigned char smem[];
     Problem p = a.p;
     if (BC) p.B = BC;
@@ -140,24 +171,25 @@ __global__ void __launch_bounds__(kAdjWarps * 32) adjoint_block_kernel(const __g
         const bool inner = g.ox + B < p.X && g.oy + B < p.Y && g.oz + B < p.Z;
         load_rows<T, BC>(p, pl, ws, g, nullptr);
         const CutRows cr = cut_bits<BC>(p, pl, ws, g);
-        const bool ok = cr.nv == nv && (uint64_t)vbase + nv <= a.vcount;
-        if (!ok && lane == 0) report(a.st, MTX_ERR_INTERNAL, kSiteAdjoint, r, cr.nv);
+        const bool ok = cr.nx + cr.ny + cr.nz == nv && (uint64_t)vbase + nv <= a.vcount;
+        if (!ok && lane == 0) report(a.st, MTX_ERR_INTERNAL, kSiteAdjoint, r, cr.nx + cr.ny + cr.nz);
         if (DET) {
             for (uint32_t i = lane; i < T3; i += 32) acc[i] = 0.0f;
             __syncwarp();
         }
-        const uint32_t nterm = iso_terms(B);
-        const bool keep = cr.nl <= nterm;  // else the terms are computed again below
+        const bool keep = nv <= iso_terms(B);  // else the terms are computed again below
         ListWalk l;
-        uint32_t run = vbase, seen = 0;
+        // the next vertex, and each axis's next term (x | y << 16, z)
+        uint32_t run = vbase, to[2] = {cr.nx << 16, cr.nx + cr.ny};
         while (const uint32_t n = ok ? list_take<BC>(l, pl, ws) : 0u) {
             uint32_t m = 0, cell = 0;
             if (lane < n) {
                 cell = list[l.done + lane];
                 m = listed_cell(p, pl, g, rows, cell, inner) >> 28;
             }
-            uint32_t vt;
-            const uint32_t first = run + step_vertices(m, vt);
+            uint32_t before[3], all[3];
+            step_edges(m, before, all);
+            const uint32_t first = run + before[0] + before[1] + before[2];
             const uint32_t q = fdiv(cell, pl.rB), x = cell - q * B, z = fdiv(q, pl.rB), y = q - z * B;
             const uint64_t v0 = ((uint64_t)(g.oz + z) * p.Y + (g.oy + y)) * p.X + (g.ox + x);
             const uint64_t gstep[3] = {1ull, (uint64_t)p.X, (uint64_t)p.X * p.Y};
@@ -181,7 +213,8 @@ __global__ void __launch_bounds__(kAdjWarps * 32) adjoint_block_kernel(const __g
                 on[k] = ((m >> k) & 1u) && fabsf(den) > 1e-5f;  // else t = 0.5: no gradient
                 far[k] = 0.0f;
                 const float s = (m >> k) & 1u ? iso_term(gv[k], a.gscale[k], den) : 0.0f;
-                if (keep && lane < n) term[k * nterm + seen + lane] = s;
+                if (keep && ((m >> k) & 1u))
+                    term[(k == 0 ? to[0] & 0xffffu : k == 1 ? to[0] >> 16 : to[1]) + before[k]] = s;
                 if (on[k]) {
                     const float ta = __fdiv_rn(__fmul_rn(s, __fsub_rn(iso, fb)), den);
                     far[k] = __fdiv_rn(__fmul_rn(s, __fsub_rn(fa, iso)), den);
@@ -205,38 +238,60 @@ __global__ void __launch_bounds__(kAdjWarps * 32) adjoint_block_kernel(const __g
                     __syncwarp();
                 }
             }
-            run += vt;
-            seen += n;
+            run += all[0] + all[1] + all[2];
+            to[0] += all[0] | (all[1] << 16);
+            to[1] += all[2];
             l.done += n;
         }
         // dL/diso: each lane its rows' terms, axis by axis in canonical order, then the lanes' sums
         float diso = 0.0f;
         __syncwarp();
         if (ok && keep) {
-            for (uint32_t k = 0; k < 3; ++k)
-                for (uint32_t i = cr.at; i < cr.at + cr.n; ++i) diso = __fadd_rn(diso, term[k * nterm + i]);
+            // (y's terms begin where x's end, z's where y's do)
+            const float *tx = term + (cr.at[0] & 0xffffu), *ty = term + (to[0] & 0xffffu) + (cr.at[0] >> 16),
+                        *tz = term + (to[0] >> 16) + cr.at[1];
+            for (uint32_t i = 0; i < (cr.own[0] & 0xffffu); ++i) diso = __fadd_rn(diso, tx[i]);
+            for (uint32_t i = 0; i < (cr.own[0] >> 16); ++i) diso = __fadd_rn(diso, ty[i]);
+            for (uint32_t i = 0; i < cr.own[1]; ++i) diso = __fadd_rn(diso, tz[i]);
         } else if (ok) {
-            const uint32_t R = (pl.BB + 31) / 32;
+            // the list once more for each axis, its terms summed whenever they fill the room for them
             for (uint32_t k = 0; k < 3; ++k) {
-                uint64_t vid = vbase + cr.vat;
-                for (uint32_t q = lane * R; q < min(pl.BB, lane * R + R); ++q) {
-                    const uint32_t z = fdiv(q, pl.rB), y = q - z * B;
-                    uint32_t xc, yc, zc;
-                    row_cross(p, pl, g, rows, y, z, xc, yc, zc);
-                    for (uint32_t any = xc | yc | zc; any; any &= any - 1u) {
-                        const uint32_t x = __ffs(any) - 1;
-                        const uint32_t m = ((xc >> x) & 1u) | (((yc >> x) & 1u) << 1) | (((zc >> x) & 1u) << 2);
-                        if ((m >> k) & 1u) {
-                            const T *v = reinterpret_cast<const T *>(p.vol) +
-                                         ((uint64_t)(g.oz + z) * p.Y + (g.oy + y)) * p.X + (g.ox + x);
-                            const uint64_t step = k == 0 ? 1ull : k == 1 ? (uint64_t)p.X : (uint64_t)p.X * p.Y;
-                            const float den = __fsub_rn(Vox<T>::val(__ldg(v + step)), Vox<T>::val(__ldg(v)));
-                            const float gk = __ldg(a.g + (vid + __popc(m & ((1u << k) - 1u))) * a.gstride + k);
-                            diso = __fadd_rn(diso, iso_term(gk, a.gscale[k], den));
-                        }
-                        vid += __popc(m);
+                l = ListWalk{};
+                run = vbase;
+                uint32_t t0 = 0, held = 0;  // of the axis's terms, [t0, t0 + held) are held
+                const uint64_t step = k == 0 ? 1ull : k == 1 ? (uint64_t)p.X : (uint64_t)p.X * p.Y;
+                const uint32_t at = k == 0 ? cr.at[0] & 0xffffu : k == 1 ? cr.at[0] >> 16 : cr.at[1];
+                const uint32_t own = k == 0 ? cr.own[0] & 0xffffu : k == 1 ? cr.own[0] >> 16 : cr.own[1];
+                uint32_t n;
+                do {
+                    n = list_take<BC>(l, pl, ws);
+                    if (!n || held + 32 > iso_terms(B)) {
+                        __syncwarp();
+                        const uint32_t i1 = min(at + own, t0 + held);
+                        for (uint32_t i = max(at, t0); i < i1; ++i) diso = __fadd_rn(diso, term[i - t0]);
+                        __syncwarp();
+                        t0 += held;
+                        held = 0;
                     }
-                }
+                    uint32_t m = 0, cell = 0;
+                    if (lane < n) {
+                        cell = list[l.done + lane];
+                        m = listed_cell(p, pl, g, rows, cell, inner) >> 28;
+                    }
+                    uint32_t before[3], all[3];
+                    step_edges(m, before, all);
+                    if ((m >> k) & 1u) {
+                        const uint32_t q = fdiv(cell, pl.rB), x = cell - q * B, z = fdiv(q, pl.rB), y = q - z * B;
+                        const T *v = reinterpret_cast<const T *>(p.vol) +
+                                     ((uint64_t)(g.oz + z) * p.Y + (g.oy + y)) * p.X + (g.ox + x);
+                        const float den = __fsub_rn(Vox<T>::val(__ldg(v + step)), Vox<T>::val(__ldg(v)));
+                        const uint32_t vid = run + before[0] + before[1] + before[2] + __popc(m & ((1u << k) - 1u));
+                        term[held + before[k]] = iso_term(__ldg(a.g + (uint64_t)vid * a.gstride + k), a.gscale[k], den);
+                    }
+                    run += all[0] + all[1] + all[2];
+                    held += all[k];
+                    l.done += n;
+                } while (n);
             }
         }
 #pragma unroll
@@ -363,10 +418,20 @@ __global__ void __launch_bounds__(kIsoThreads) adjoint_iso_kernel(const float *_
     if (threadIdx.x == 0) *out = (float)s[0];
 }
 
+template <typename T, bool DET>
+static auto adjoint_fn(uint32_t B) {
+    switch (B) {
+    case 2: return adjoint_block_kernel<T, DET, 2>;
+    case 3: return adjoint_block_kernel<T, DET, 3>;
+    case 4: return adjoint_block_kernel<T, DET, 4>;
+    case 5: return adjoint_block_kernel<T, DET, 5>;
+    case 8: return adjoint_block_kernel<T, DET, 8>;
+    default: return adjoint_block_kernel<T, DET, 0>;
+    }
+}
 template <typename T>
 static auto adjoint_fn(bool det, uint32_t B) {
-    return det ? (B == 8 ? adjoint_block_kernel<T, true, 8> : adjoint_block_kernel<T, true, 0>)
-               : (B == 8 ? adjoint_block_kernel<T, false, 8> : adjoint_block_kernel<T, false, 0>);
+    return det ? adjoint_fn<T, true>(B) : adjoint_fn<T, false>(B);
 }
 
 MTX_BC_READER(bc_take_adjoint)
