@@ -55,9 +55,13 @@ def _current_stream_ptr() -> int:
         return _stream_ptr()
 
 
-def device_copy(ptr: int, shape, dtype: torch.dtype) -> torch.Tensor:
-    """A library buffer's contents as a new tensor: one copy on torch's current
-    stream (a third of the host time of cloning a view of it)."""
+def device_copy(ptr: int, shape, dtype: torch.dtype, device: int | None = None) -> torch.Tensor:
+    """The contents of a library buffer on `device` (None: the current one) as a
+    new tensor on the current device: one copy on torch's current stream (a third
+    of the host time of cloning a view of it).  From another device torch makes
+    the copy, which it orders behind the current streams of both."""
+    if device is not None and device != torch.cuda.current_device():
+        return device_view(ptr, shape, dtype).clone()
     out = torch.empty(shape, dtype=dtype, device="cuda")
     n = out.numel()
     if n and ptr:
@@ -72,6 +76,7 @@ class Context:
 
     def __init__(self, device: int = 0, stream=None):
         self.handle = C.c_void_p()
+        self.device = device
         self.stream_ptr = _stream_ptr(stream)
         L.check(L.lib().mtx_context_create(device, C.c_void_p(self.stream_ptr),
                                            C.byref(self.handle)), "mtx_context_create")
@@ -188,11 +193,11 @@ class MinMax:
         """uint32 [gz, gy, gx, 2] {min,max} keys of mip level l (a copy)."""
         e = self.out.levelExtent[l]
         base = self.out.minMaxImage.ptr + 8 * int(self.out.levelOffset[l])
-        return device_copy(base, (e[2], e[1], e[0], 2), torch.int32)
+        return device_copy(base, (e[2], e[1], e[0], 2), torch.int32, self.ctx.device)
 
     def all_levels(self) -> torch.Tensor:
         n = self.out.minMaxImage.size // 8
-        return device_copy(self.out.minMaxImage.ptr, (n, 2), torch.int32)
+        return device_copy(self.out.minMaxImage.ptr, (n, 2), torch.int32, self.ctx.device)
 
     def free(self):
         if self.out.minMaxImage.ptr:
@@ -211,7 +216,7 @@ class Filtering:
 
     def ids(self) -> torch.Tensor:
         n = self.out.activeBlockCount
-        return device_copy(self.out.compactedBlockIdBuffer.ptr, (n,), torch.int32)
+        return device_copy(self.out.compactedBlockIdBuffer.ptr, (n,), torch.int32, self.ctx.device)
 
     def device_count(self) -> int:
         return int(device_view(self.out.activeBlockCountBuffer.ptr, (1,), torch.int32).item())
@@ -242,17 +247,17 @@ class Extraction:
     def vertices(self) -> torch.Tensor:
         """float32 [V, 3] (xyz format) or [V, 8] (VertexData)."""
         w = self.out.vertexStride // 4
-        return device_copy(self.out.vertexBuffer.ptr, (self.out.vertexCount, w), torch.float32)
+        return device_copy(self.out.vertexBuffer.ptr, (self.out.vertexCount, w), torch.float32, self.ctx.device)
 
     def indices(self) -> torch.Tensor:
-        return device_copy(self.out.indexBuffer.ptr, (self.out.indexCount // 3, 3), torch.int32)
+        return device_copy(self.out.indexBuffer.ptr, (self.out.indexCount // 3, 3), torch.int32, self.ctx.device)
 
     def meshlets(self) -> torch.Tensor:
         return device_copy(self.out.meshletDescriptorBuffer.ptr, (self.out.meshletCount, 4),
-                           torch.int32)
+                           torch.int32, self.ctx.device)
 
     def counters(self) -> torch.Tensor:
-        return device_copy(self.out.vertexCountBuffer.ptr, (3,), torch.int32)
+        return device_copy(self.out.vertexCountBuffer.ptr, (3,), torch.int32, self.ctx.device)
 
     def free(self):
         if self.out.vertexCountBuffer.ptr or self.out.meshletDescriptorBuffer.ptr:
@@ -392,10 +397,10 @@ def build_meshlets(ctx: Context, x: Extraction, max_vertices: int = 64, max_prim
     L.check(L.lib().mtx_build_meshlets(ctx.handle, C.byref(x.out), max_vertices, max_primitives, C.byref(o)),
             "mtx_build_meshlets", ctx.handle)
     w = max(o.vertexStride // 4, 1)
-    m = Meshlets(device_copy(o.meshletDescriptorBuffer.ptr, (o.meshletCount, 4), torch.int32),
-                 device_copy(o.meshletVertexBuffer.ptr, (o.vertexCount,), torch.int32),
-                 device_copy(o.vertexBuffer.ptr, (o.vertexCount, w), torch.float32),
-                 device_copy(o.indexBuffer.ptr, (o.indexCount // 3, 3), torch.int32))
+    m = Meshlets(device_copy(o.meshletDescriptorBuffer.ptr, (o.meshletCount, 4), torch.int32, ctx.device),
+                 device_copy(o.meshletVertexBuffer.ptr, (o.vertexCount,), torch.int32, ctx.device),
+                 device_copy(o.vertexBuffer.ptr, (o.vertexCount, w), torch.float32, ctx.device),
+                 device_copy(o.indexBuffer.ptr, (o.indexCount // 3, 3), torch.int32, ctx.device))
     ctx.fence()
     L.lib().mtx_meshlet_output_free(ctx.handle, C.byref(o))
     return m
