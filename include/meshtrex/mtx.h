@@ -532,7 +532,8 @@ typedef struct mtx_tuning {
     uint32_t minmaxZChunk;  /* block slabs per warp in the min/max pass */
     uint32_t minmaxSlices;  /* 0 (default): a TMA ring of z slices for 2- and 4-byte voxels, row words for uint8;
                                1, 2 or 4: the load-based pass with that many z slices in flight */
-    uint32_t extractWarps;  /* warps per CTA of the extraction passes: 1, 2, 4 or 8; 0: 8, or as many as fit for B > 8 */
+    uint32_t extractWarps;  /* warps per CTA of the extraction passes: 1, 2, 4 or 8 (0 = 8; for B > 8, 8 is as many as
+                               fit, up to 16) */
     uint32_t staging;       /* mtx_staging used when the extract options say AUTO */
     uint32_t extractCtasPerSm; /* at most this many CTAs an SM in the count and emit passes (0 = as many as
                                   fit): leaves room on each SM for another stream's min/max pass */

@@ -362,11 +362,15 @@ static mtx_status grid_for(mtx_context *c, K kernel, int threads, uint32_t smem,
     return MTX_OK;
 }
 
-// Warps a CTA: threads/32 of the options, else the context's tuning (up to
-// kMaxWarps), else the pass's own choice, and no more than the shared memory holds.
-static uint32_t cta_warps(const mtx_context *c, const ExtractArgs &a, uint32_t fixed, uint32_t per_warp,
-                          uint32_t own) {
-    const uint32_t asked = a.threads ? std::max(a.threads / 32, 1u) : c->tuning.extractWarps;
+// Warps a CTA: threads/32 of the options (up to kMaxWarps), else the context's
+// tuning, else the pass's own choice -- eight, for B > 8 as many as fit -- and no
+// more than the shared memory holds.  The tuning's largest count is for B > 8 the
+// own choice too, so that mtx_autotune, which tries 2, 4 and 8, reaches it (CTAs of
+// 8 and of 11 to 14 warps at B = 16: count 37 and 30.5 us, emit 112 and 85, the
+// volume of kBigWarps).
+static uint32_t cta_warps(const mtx_context *c, const ExtractArgs &a, uint32_t B, uint32_t fixed, uint32_t per_warp) {
+    const uint32_t own = B > 8 ? kBigWarps : kMaxWarps, tuned = c->tuning.extractWarps;
+    const uint32_t asked = a.threads ? std::max(a.threads / 32, 1u) : B > 8 && tuned == kMaxWarps ? 0u : tuned;
     const uint32_t W = asked ? std::min<uint32_t>(asked, kMaxWarps) : own;
     const uint32_t room = c->max_smem_optin > (int)fixed ? (uint32_t)c->max_smem_optin - fixed : 0u;
     return std::min<uint32_t>(W, std::max<uint32_t>(1, room / per_warp));
@@ -399,7 +403,7 @@ static mtx_status run_count(mtx_context *c, const Problem &p, const ExtractArgs 
     // eight warps a CTA: the case counts are loaded half as often as with four and blocks
     // next to each other share voxels in L1 (256^3 uint8 at B = 8 10.8 -> 9.7 us, 1024 x 1024 x 314
     // at B = 3 127 -> 123, 1024^3 uint16 at B = 8 94.6 -> 93.1)
-    const uint32_t fixed = count_fixed_bytes(p.B, use_off), W = cta_warps(c, a, fixed, pl.bytes, p.B > 8 ? kBigWarps : 8);
+    const uint32_t fixed = count_fixed_bytes(p.B, use_off), W = cta_warps(c, a, p.B, fixed, pl.bytes);
     const uint32_t smem = fixed + W * pl.bytes;
     auto k = tma ? count_fn<T, true>(p.B) : count_fn<T, false>(p.B);
     unsigned grid;
@@ -428,7 +432,7 @@ static auto emit_fn(uint32_t B) {
 template <typename T>
 static mtx_status run_emit(mtx_context *c, const Problem &p, const ExtractArgs &a, cudaStream_t s) {
     const WPlan pl = make_emit_plan(p.B);
-    const uint32_t fixed = emit_fixed_bytes(p.B), W = cta_warps(c, a, fixed, pl.bytes, p.B > 8 ? kBigWarps : 8);
+    const uint32_t fixed = emit_fixed_bytes(p.B), W = cta_warps(c, a, p.B, fixed, pl.bytes);
     const uint32_t smem = fixed + W * pl.bytes;
     const bool generic = a.vertices && (a.vertex_format != MTX_VERTEX_XYZ || a.frame != MTX_FRAME_VOXEL);
     auto k = generic ? emit_fn<T, true>(p.B) : emit_fn<T, false>(p.B);
