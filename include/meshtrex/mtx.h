@@ -536,7 +536,8 @@ typedef struct mtx_tuning {
                                fit, up to 16) */
     uint32_t staging;       /* mtx_staging used when the extract options say AUTO */
     uint32_t extractCtasPerSm; /* at most this many CTAs an SM in the count and emit passes (0 = as many as
-                                  fit): leaves room on each SM for another stream's min/max pass */
+                                  fit), of 4 warps where extractWarps is 0: leaves room on each SM for another
+                                  stream's min/max pass */
 } mtx_tuning;
 mtx_status mtx_context_set_tuning(mtx_context_t ctx, const mtx_tuning *t);
 mtx_status mtx_context_get_tuning(mtx_context_t ctx, mtx_tuning *t);

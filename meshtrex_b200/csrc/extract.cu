@@ -367,10 +367,12 @@ static mtx_status grid_for(mtx_context *c, K kernel, int threads, uint32_t smem,
 // more than the shared memory holds.  The tuning's largest count is for B > 8 the
 // own choice too, so that mtx_autotune, which tries 2, 4 and 8, reaches it (CTAs of
 // 8 and of 11 to 14 warps at B = 16: count 37 and 30.5 us, emit 112 and 85, the
-// volume of kBigWarps).
+// volume of kBigWarps).  A cap on the CTAs of an SM counts CTAs of four warps:
+// it is set for the room that they leave to another stream's kernels.
 static uint32_t cta_warps(const mtx_context *c, const ExtractArgs &a, uint32_t B, uint32_t fixed, uint32_t per_warp) {
-    const uint32_t own = B > 8 ? kBigWarps : kMaxWarps, tuned = c->tuning.extractWarps;
-    const uint32_t asked = a.threads ? std::max(a.threads / 32, 1u) : B > 8 && tuned == kMaxWarps ? 0u : tuned;
+    const bool capped = c->tuning.extractCtasPerSm != 0;
+    const uint32_t own = capped ? 4 : B > 8 ? kBigWarps : kMaxWarps, tuned = c->tuning.extractWarps;
+    const uint32_t asked = a.threads ? std::max(a.threads / 32, 1u) : B > 8 && tuned == kMaxWarps && !capped ? 0u : tuned;
     const uint32_t W = asked ? std::min<uint32_t>(asked, kMaxWarps) : own;
     const uint32_t room = c->max_smem_optin > (int)fixed ? (uint32_t)c->max_smem_optin - fixed : 0u;
     return std::min<uint32_t>(W, std::max<uint32_t>(1, room / per_warp));

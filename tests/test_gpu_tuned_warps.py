@@ -64,3 +64,12 @@ def test_tuned_warps(oracle, block):
     assert _sizes(a, block, ref, extract_warps=8) == own
     assert _sizes(a, block, ref, extract_warps=4) == (4, 4)
     assert _sizes(a, block, ref, extract_warps=8, options=api.extract_options(threads=64)) == (2, 2)
+
+
+@pytest.mark.parametrize("block", [4, 8, 16])
+def test_capped_ctas_keep_their_size(oracle, block):
+    """extractCtasPerSm leaves room on each SM: the CTAs it counts stay at four warps."""
+    a = blob_volume((40, 36, 48), np.uint16, seed=2)
+    ref = oracle.extract(a, block, mid_iso(a))
+    assert _sizes(a, block, ref, extract_ctas_per_sm=2) == (4, 4)
+    assert _sizes(a, block, ref, extract_ctas_per_sm=2, extract_warps=2) == (2, 2)
