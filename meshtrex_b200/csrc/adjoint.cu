@@ -213,9 +213,9 @@ __global__ void __launch_bounds__(kAdjWarps * 32, adjoint_min_ctas(DET, BC))
                 on[k] = ((m >> k) & 1u) && fabsf(den) > 1e-5f;  // else t = 0.5: no gradient
                 far[k] = 0.0f;
                 const float s = (m >> k) & 1u ? iso_term(gv[k], a.gscale[k], den) : 0.0f;
-                if (keep && ((m >> k) & 1u))
-                    term[(k == 0 ? to[0] & 0xffffu : k == 1 ? to[0] >> 16 : to[1]) + before[k]] = s;
-                if (on[k]) {
+                const uint32_t at = (k == 0 ? to[0] & 0xffffu : k == 1 ? to[0] >> 16 : to[1]) + before[k];
+                if (keep && ((m >> k) & 1u) && MTX_BC(at, iso_terms(B), kBcTerms)) term[at] = s;
+                if (on[k] && MTX_BC(v0 + gstep[k], (uint64_t)p.X * p.Y * p.Z, kBcField)) {
                     const float ta = __fdiv_rn(__fmul_rn(s, __fsub_rn(iso, fb)), den);
                     far[k] = __fdiv_rn(__fmul_rn(s, __fsub_rn(fa, iso)), den);
                     if (DET) {
@@ -229,12 +229,12 @@ __global__ void __launch_bounds__(kAdjWarps * 32, adjoint_min_ctas(DET, BC))
             if (DET) {
                 // one writer a tile voxel in each of the four additions
                 const uint32_t i = (z * B1 + y) * B1 + x;
-                if (m) acc[i] = __fadd_rn(acc[i], own);
+                if (m && MTX_BC(i, T3, kBcTile)) acc[i] = __fadd_rn(acc[i], own);
                 __syncwarp();
 #pragma unroll
                 for (uint32_t k = 0; k < 3; ++k) {
                     const uint32_t j = i + (k == 0 ? 1u : k == 1 ? B1 : B1 * B1);
-                    if (on[k]) acc[j] = __fadd_rn(acc[j], far[k]);
+                    if (on[k] && MTX_BC(j, T3, kBcTile)) acc[j] = __fadd_rn(acc[j], far[k]);
                     __syncwarp();
                 }
             }
@@ -280,7 +280,7 @@ __global__ void __launch_bounds__(kAdjWarps * 32, adjoint_min_ctas(DET, BC))
                     }
                     uint32_t before[3], all[3];
                     step_edges(m, before, all);
-                    if ((m >> k) & 1u) {
+                    if (((m >> k) & 1u) && MTX_BC(held + before[k], iso_terms(B), kBcTerms)) {
                         const uint32_t q = fdiv(cell, pl.rB), x = cell - q * B, z = fdiv(q, pl.rB), y = q - z * B;
                         const T *v = reinterpret_cast<const T *>(p.vol) +
                                      ((uint64_t)(g.oz + z) * p.Y + (g.oy + y)) * p.X + (g.ox + x);
@@ -305,7 +305,9 @@ __global__ void __launch_bounds__(kAdjWarps * 32, adjoint_min_ctas(DET, BC))
                 const float t = acc[i];
                 if (lx % B == 0 || ly % B == 0 || lz % B == 0)  // shared with a neighbour: the gather pass's
                     dst[i] = t;
-                else if (t != 0.0f)  // (voxels outside the volume have none)
+                else if (t != 0.0f &&  // (voxels outside the volume have none)
+                         MTX_BC(g.ox + lx, p.X, kBcField) && MTX_BC(g.oy + ly, p.Y, kBcField) &&
+                         MTX_BC(g.oz + lz, p.Z, kBcField))
                     a.dfield[((uint64_t)(g.oz + lz) * p.Y + (g.oy + ly)) * p.X + (g.ox + lx)] = t;
             }
         }
@@ -346,13 +348,16 @@ __global__ void __launch_bounds__(kAdjWarps * 32) adjoint_gather_kernel(const __
         uint32_t nb[12];
 #pragma unroll
         for (int k = 0; k < 12; ++k) nb[k] = __shfl_sync(0xffffffffu, rk, k);
-        const float *own = a.partial + (uint64_t)r * a.T3;
         auto put = [&](uint32_t lx, uint32_t ly, uint32_t lz, float t) {
             const uint32_t wx = g.ox + lx, wy = g.oy + ly, wz = g.oz + lz;
             if (t != 0.0f && wx < p.X && wy < p.Y && wz < p.Z)
                 a.dfield[((uint64_t)wz * p.Y + wy) * p.X + wx] = t;
         };
-        auto from = [&](uint32_t rank, uint32_t i) { return __ldcg(a.partial + (uint64_t)rank * a.T3 + i); };
+        auto from = [&](uint32_t rank, uint32_t i) {
+            return MTX_BC(rank, a.n, kBcPartial) && MTX_BC(i, a.T3, kBcPartial)
+                       ? __ldcg(a.partial + (uint64_t)rank * a.T3 + i)
+                       : 0.0f;
+        };
         // this block's voxels on its low faces: z == 0 (B^2), then y == 0 (B (B-1)), then x == 0 ((B-1)^2)
         const uint32_t nlow = BB + B * (B - 1) + (B - 1) * (B - 1);
         for (uint32_t j = lane; j < nlow; j += 32) {
@@ -373,7 +378,7 @@ __global__ void __launch_bounds__(kAdjWarps * 32) adjoint_gather_kernel(const __
                 lx = 0;
             }
             const uint32_t i = (lz * B1 + ly) * B1 + lx;
-            float t = __ldcg(own + i);
+            float t = from(r, i);
             if (!lx && nb[0] != kNoVertex) t = __fadd_rn(t, from(nb[0], i + B * st[0]));
             if (!ly && nb[1] != kNoVertex) t = __fadd_rn(t, from(nb[1], i + B * st[1]));
             if (!lz && nb[2] != kNoVertex) t = __fadd_rn(t, from(nb[2], i + B * st[2]));
@@ -391,7 +396,7 @@ __global__ void __launch_bounds__(kAdjWarps * 32) adjoint_gather_kernel(const __
                 const bool tu = !lu && ru != kNoVertex, tv = !lv && rv != kNoVertex;
                 // a block before that one on an axis before k writes the voxel
                 if ((tu && u < k) || (tv && v < k)) continue;
-                float t = __ldcg(own + i);
+                float t = from(r, i);
                 const uint32_t c = lu * st[u] + lv * st[v];  // the voxel in its own block's tile
                 if (tu) t = __fadd_rn(t, from(ru, c + B * st[u]));
                 if (tv) t = __fadd_rn(t, from(rv, c + B * st[v]));

@@ -525,14 +525,15 @@ __device__ __forceinline__ void batch_emit_block(const BatchArgs &a, const Probl
         l.done += n;
         uint32_t vt;
         const uint32_t rel = vrun + step_vertices(e >> 28, vt);
-        queue_vertices(pl, e, rel, vtab, jobs);
+        queue_vertices(pl, e, rel, vtab, jobs, verts ? out : vrun);
         vrun += vt;
         __syncwarp();
         if (verts) {
             const uint32_t avail = min(vrun, nv);
             while (avail - out >= (vrun >= nv ? 1u : 32u)) {
                 const uint32_t k = min(32u, avail - out);
-                put_vertices<AnyVoxel, GENERIC>(p, pl, g, jobs, out, k, inner, verts, d.x, a.vfmt, a.frame, a.normals);
+                put_vertices<AnyVoxel, GENERIC>(p, pl, g, jobs, out, k, nv, inner, verts, d.x, a.vfmt, a.frame,
+                                                a.normals);
                 out += k;
             }
         }
@@ -545,7 +546,7 @@ __device__ __forceinline__ void batch_emit_block(const BatchArgs &a, const Probl
             const uint32_t j = j0 + lane, c = ctx_entry(pl, min(j, pl.nb3 - 1));
             const uint32_t rk = __shfl_sync(0xffffffffu, nb_rk, c & 7u);
             const uint64_t at = (uint64_t)rk * a.face_stride + ((c >> 3) & 1023u);
-            if (j < pl.nb3)
+            if (j < pl.nb3 && MTX_BC(c >> 13, pl.S1 * pl.S1 * pl.S1, kBcVoxTab))
                 vtab[c >> 13] = rk != kNoVertex && MTX_BC(at, face_words, kBcFaces) ? __ldcg(a.faces + at) : (uint16_t)0;
         }
     }
@@ -565,15 +566,15 @@ __device__ __forceinline__ void batch_emit_block(const BatchArgs &a, const Probl
         const uint32_t f = first[(e >> 12) & 0xffu];
         uint32_t total;
         const uint32_t before = warp_excl_scan(f >> 12, total);
-        queue_triangles(pl, e, f, top + before, jobs);
+        queue_triangles(pl, e, f, top + before, jobs, out);
         top += total;
         __syncwarp();
         const uint32_t avail = min(top, nt);
         const uint32_t least = top >= nt ? 1u : 32u;
         while (avail - out >= least) {
             const uint32_t k = min(32u, avail - out);
-            put_triangles(ws + pl.off_vtab, tri, jobs, nbase, out, k, a.indices + jr.indexOffset + 3ull * tbase, miss,
-                          bad);
+            put_triangles(pl, ws + pl.off_vtab, tri, jobs, nbase, out, k, nt, a.indices + jr.indexOffset + 3ull * tbase,
+                          miss, bad);
             out += k;
         }
     }

@@ -251,14 +251,14 @@ __global__ void __launch_bounds__((BIG ? kBigWarps : kMaxWarps) * 32, GENERIC ||
                 if (!BIG && (e & 0xfffu) >= B3) e = 0;  // a list the count pass did not finish (reported there)
                 uint32_t vt;
                 const uint32_t rel = vrun + step_vertices(e >> 28, vt);
-                queue_vertices(pl, e, rel, vtab, jobs);
+                queue_vertices(pl, e, rel, vtab, jobs, vertices ? out : vrun);
                 vrun += vt;
                 __syncwarp();
                 if (vertices) {
                     const uint32_t avail = min(vrun, nv);  // never past the block's vertices
                     while (avail - out >= (vrun >= nv ? 1u : 32u)) {
                         const uint32_t k = min(32u, avail - out);
-                        put_vertices<T, GENERIC>(p, pl, g, jobs, out, k, inner, vertices, d.vertexOffset, vfmt,
+                        put_vertices<T, GENERIC>(p, pl, g, jobs, out, k, nv, inner, vertices, d.vertexOffset, vfmt,
                                                  frame, normals);
                         out += k;
                     }
@@ -302,14 +302,14 @@ __global__ void __launch_bounds__((BIG ? kBigWarps : kMaxWarps) * 32, GENERIC ||
                     before = (e >> 20) & 0xffu;
                     total = __shfl_sync(0xffffffffu, before + n, 31);
                 }
-                queue_triangles(pl, e, f, top + before, jobs);
+                queue_triangles(pl, e, f, top + before, jobs, out);
                 top += total;
                 __syncwarp();
                 const uint32_t avail = min(top, nt);  // never past the block's triangles
                 const bool last = top >= nt;
                 while (avail - out >= (last ? 1u : 32u)) {
                     const uint32_t k = min(32u, avail - out);
-                    put_triangles(vtab_b, tri, jobs, nbase, out, k, indices + 3ull * tbase, miss, bad);
+                    put_triangles(pl, vtab_b, tri, jobs, nbase, out, k, nt, indices + 3ull * tbase, miss, bad);
                     out += k;
                 }
             }

@@ -580,7 +580,9 @@ __device__ __forceinline__ uint2 texel_xor(uint2 a, int o) {
     return texel_join(a, make_uint2(__shfl_xor_sync(0xffffffffu, a.x, o), __shfl_xor_sync(0xffffffffu, a.y, o)));
 }
 __device__ __forceinline__ void texel_store(const PyrAll &L, int k, uint32_t x, uint32_t y, uint32_t z, uint2 v) {
-    if (k < L.levels && x < L.ext[k][0] && y < L.ext[k][1] && z < L.ext[k][2])
+    if (k < L.levels && x < L.ext[k][0] && y < L.ext[k][1] && z < L.ext[k][2] &&
+        MTX_BC(((uint64_t)z * L.ext[k][1] + y) * L.ext[k][0] + x, (uint64_t)L.ext[k][0] * L.ext[k][1] * L.ext[k][2],
+               kBcOctree))
         L.base[k][((uint64_t)z * L.ext[k][1] + y) * L.ext[k][0] + x] = v;
 }
 
@@ -670,7 +672,8 @@ __device__ __forceinline__ void pyramid_part(const PyrAll &L, uint32_t cta, uint
 #pragma unroll
             for (int c = 0; c < 8; ++c) {
                 const uint32_t ux = 2 * x + (c & 1), uy = 2 * y + ((c >> 1) & 1), uz = 2 * z + (c >> 2);
-                if (ux < px && uy < py && uz < pz)
+                if (ux < px && uy < py && uz < pz &&
+                    MTX_BC((uz * py + uy) * px + ux, (uint64_t)px * py * pz, kBcOctree))
                     r = texel_join(r, __ldcg(&L.base[k - 1][(uz * py + uy) * px + ux]));
             }
             L.base[k][i] = r;

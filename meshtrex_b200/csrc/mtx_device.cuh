@@ -50,19 +50,24 @@ __device__ __forceinline__ void report(DevStatus *st, uint32_t code, uint32_t wh
 // the record as MTX_ERR_INTERNAL.  There is no trap.  In the normal build
 // MTX_BC is the constant true and the checks compile away.
 enum : uint32_t {
-    kBcTile = 101,      // voxel tile in shared memory
-    kBcRows = 102,      // inside masks, crossing rows, prefixes, case bytes, mixed masks
-    kBcJobs = 103,      // job window
-    kBcVertex = 104,    // vertex buffer
-    kBcIndex = 105,     // index buffer
+    kBcTile = 101,      // voxel tile in shared memory; the adjoint's accumulation tile
+    kBcRows = 102,      // inside rows
+    kBcJobs = 103,      // job window: jobs not yet resolved, and a job's triangle
+    kBcVertex = 104,    // vertex buffer: a vertex's number in its block
+    kBcIndex = 105,     // index buffer: a triangle's number in its block
     kBcFaces = 106,     // face records (read and write)
-    kBcContext = 107,   // context layer (neighbour ids and masks)
-    kBcVoxTab = 108,    // voxel table
+    kBcContext = 107,   // context layer: a face record's number in its block
+    kBcVoxTab = 108,    // vertex table
     kBcState = 109,     // block state
     kBcRank = 110,      // rank map and compacted ids
     kBcLeaf = 111,      // min/max leaf level
     kBcDesc = 112,      // meshlet descriptors
     kBcVolume = 113,    // voxel words of the rows leaf pass, in bytes of the volume
+    kBcList = 114,      // a warp's list of cells
+    kBcOctree = 115,    // octree levels
+    kBcTerms = 116,     // the adjoint's dL/diso terms
+    kBcPartial = 117,   // the adjoint's partial tiles
+    kBcField = 118,     // dL/dfield
 };
 #ifdef MTX_BOUNDS_CHECK
 static __device__ DevStatus g_bc_record;

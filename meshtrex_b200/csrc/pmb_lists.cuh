@@ -359,7 +359,8 @@ __device__ __forceinline__ uint32_t list_next(ListWalk &l, const WPlan &pl, unsi
         }
         uint32_t total;
         uint32_t at = l.top + warp_excl_scan(__popc(b), total);
-        for (uint32_t c = u * unit; b; b &= b - 1u) list[at++] = (uint16_t)(c + __ffs(b) - 1);
+        for (uint32_t c = u * unit; b; b &= b - 1u, ++at)
+            if (MTX_BC(at, list_cap(pl.B), kBcList)) list[at] = (uint16_t)(c + __ffs(b) - 1);
         l.top += total;
         l.next += 32;
         __syncwarp();
@@ -438,9 +439,9 @@ __device__ __forceinline__ void count_block_list(const Problem &p, const WPlan &
         if (m) {
             const uint32_t cell = e & 0xfffu, q = fdiv(cell, pl.rB), x = cell - q * B, z = fdiv(q, pl.rB), y = q - z * B;
             const uint16_t rec = (uint16_t)(rel | ((m & 3u) << 14));
-            if (x == 0) fr[z * B + y] = rec;
-            if (y == 0) fr[BB + z * B + x] = rec;
-            if (z == 0) fr[2 * BB + y * B + x] = rec;
+            if (x == 0 && MTX_BC(z * B + y, BB, kBcFaces)) fr[z * B + y] = rec;
+            if (y == 0 && MTX_BC(z * B + x, BB, kBcFaces)) fr[BB + z * B + x] = rec;
+            if (z == 0 && MTX_BC(y * B + x, BB, kBcFaces)) fr[2 * BB + y * B + x] = rec;
         }
         nv += vt;
         nt += tt;
@@ -534,7 +535,7 @@ __device__ __forceinline__ void ctx8_store(const Ctx8 &c, uint32_t edge, uint16_
     y[1] = (uint16_t)(c.face[1] >> 16);
     z[0] = (uint16_t)c.face[2];
     z[1] = (uint16_t)(c.face[2] >> 16);
-    if (edge) vtab[edge >> 13] = (uint16_t)c.edge;
+    if (edge && MTX_BC(edge >> 13, 9 * 9 * 9, kBcVoxTab)) vtab[edge >> 13] = (uint16_t)c.edge;
 }
 
 // Any B, through the map: up to 32 N context voxels from j0 on.
@@ -550,7 +551,9 @@ __device__ __forceinline__ void ctx_load(const WPlan &pl, const uint16_t *faces,
         const uint32_t c = cmap[min(j, pl.nb3 - 1)];
         const uint32_t rk = __shfl_sync(0xffffffffu, nb_rk, c & 7u);
         const uint64_t at = (uint64_t)rk * face_stride16(pl.B) + ((c >> 3) & 1023u);
-        if (j < pl.nb3 && rk != kNoVertex && MTX_BC(at, face_words, kBcFaces)) rec[k] = __ldg(faces + at);
+        if (j < pl.nb3 && rk != kNoVertex && MTX_BC((c >> 3) & 1023u, 3 * pl.BB, kBcContext) &&
+            MTX_BC(at, face_words, kBcFaces))
+            rec[k] = __ldg(faces + at);
     }
 }
 template <int N>
@@ -566,14 +569,16 @@ __device__ __forceinline__ void ctx_store(const WPlan &pl, uint16_t *vtab, const
 
 // One step of the vertex phase: this lane's list word e (0: none) and its first
 // vertex rel -> the voxel's table entry, and a job (cell | axis << 12) for each
-// of its vertices, queued at the vertex's own number.
+// of its vertices, queued at the vertex's own number.  done: vertices written,
+// or all before this step where none are (the jobs are not read then).
 __device__ __forceinline__ void queue_vertices(const WPlan &pl, uint32_t e, uint32_t rel, uint16_t *vtab,
-                                               uint32_t *jobs) {
+                                               uint32_t *jobs, [[maybe_unused]] uint32_t done) {
     const uint32_t m = e >> 28, cell = e & 0xfffu;
     if (!m) return;
     const uint32_t q = fdiv(cell, pl.rB), x = cell - q * pl.B, z = fdiv(q, pl.rB), y = q - z * pl.B;
     const uint32_t ti = (z * pl.S1 + y) * pl.S1 + x;
     if (MTX_BC(ti, pl.S1 * pl.S1 * pl.S1, kBcVoxTab)) vtab[ti] = (uint16_t)(rel | (m << 14));
+    if (!MTX_BC(rel + __popc(m) - 1 - done, kJobWin, kBcJobs)) return;
     if (m & 1u) jobs[rel++ & (kJobWin - 1)] = cell;
     if (m & 2u) jobs[rel++ & (kJobWin - 1)] = cell | (1u << 12);
     if (m & 4u) jobs[rel & (kJobWin - 1)] = cell | (2u << 12);
@@ -592,19 +597,21 @@ __device__ __forceinline__ float voxel_value(const Problem &p, uint64_t i) {
     }
 }
 
-// Writes vertices [done, done + n) of the block, n <= 32, one a lane; the first
-// is vertex vbase of the mesh.
+// Writes vertices [done, done + n) of the block's nv, n <= 32, one a lane; the
+// first is vertex vbase of the mesh.
 template <typename T, bool GENERIC>
 __device__ __forceinline__ void put_vertices(const Problem &p, const WPlan &pl, const Geo &g, const uint32_t *jobs,
-                                             uint32_t done, uint32_t n, bool inner, void *vertices, uint64_t vbase,
-                                             uint32_t vfmt, uint32_t frame, uint32_t normals) {
+                                             uint32_t done, uint32_t n, [[maybe_unused]] uint32_t nv, bool inner,
+                                             void *vertices, uint64_t vbase, uint32_t vfmt, uint32_t frame,
+                                             uint32_t normals) {
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t job = jobs[(done + lane) & (kJobWin - 1)];
     const uint32_t cell = job & 0xfffu, a = job >> 12;
     const uint32_t q = fdiv(cell, pl.rB), x = cell - q * pl.B, z = fdiv(q, pl.rB), y = q - z * pl.B;
     const uint32_t gx = g.ox + x, gy = g.oy + y, gz = g.oz + z;
     // (a list the count pass did not finish must not lead past the volume)
-    if (lane < n && (inner || (gx + (a == 0) < p.X && gy + (a == 1) < p.Y && gz + (a == 2) < p.Z))) {
+    if (lane < n && MTX_BC(done + lane, nv, kBcVertex) &&
+        (inner || (gx + (a == 0) < p.X && gy + (a == 1) < p.Y && gz + (a == 2) < p.Z))) {
         const uint64_t v = ((uint64_t)gz * p.Y + gy) * p.X + gx;
         const uint64_t step = a == 0 ? 1ull : a == 1 ? (uint64_t)p.X : (uint64_t)p.X * p.Y;
         const float t = edge_t(voxel_value<T>(p, v), voxel_value<T>(p, v + step), p.iso);
@@ -638,8 +645,9 @@ __device__ __forceinline__ void put_vertices(const Problem &p, const WPlan &pl, 
 }
 
 // Queues the triangles of this lane's list word e, numbers [at, at + n) of the
-// block; f: the entry of its case in `first`.
-__device__ __forceinline__ void queue_triangles(const WPlan &pl, uint32_t e, uint32_t f, uint32_t at, uint32_t *jobs) {
+// block, of which `done` are written; f: the entry of its case in `first`.
+__device__ __forceinline__ void queue_triangles(const WPlan &pl, uint32_t e, uint32_t f, uint32_t at, uint32_t *jobs,
+                                                [[maybe_unused]] uint32_t done) {
     const uint32_t cell = e & 0xfffu, n = f >> 12, q = fdiv(cell, pl.rB), x = cell - q * pl.B;
     const uint32_t z = fdiv(q, pl.rB), y = q - z * pl.B;
     const uint32_t end =
@@ -647,25 +655,27 @@ __device__ __forceinline__ void queue_triangles(const WPlan &pl, uint32_t e, uin
     const uint32_t job = (((z * pl.S1 + y) * pl.S1 + x) << 1) | ((f & 0xfffu) << 16) | end;
 #pragma unroll
     for (uint32_t t = 0; t < 5; ++t)  // at most five triangles a case
-        if (t < n) jobs[(at + t) & (kJobWin - 1)] = job + (t << 16);
+        if (t < n && MTX_BC(at + t - done, kJobWin, kBcJobs)) jobs[(at + t) & (kJobWin - 1)] = job + (t << 16);
 }
 
-// Writes triangles [done, done + n) of the block, n <= 32, one a lane, each lane
-// its own 12 bytes from dst on.  Job: the cell's byte offset in the vertex table
+// Writes triangles [done, done + n) of the block's nt, n <= 32, one a lane, each
+// lane its own 12 bytes from dst on.  Job: the cell's byte offset in the vertex table
 // (bits 0-15), the triangle (16-25), whether the cell is the block's last along
 // x, y and z (26-28).  miss: bit c, neighbour c is not active.
-__device__ __forceinline__ void put_triangles(const unsigned char *vtab, const uint64_t *tri, const uint32_t *jobs,
-                                              const uint32_t *nbase, uint32_t done, uint32_t n, uint32_t *dst,
-                                              uint32_t miss, bool &bad) {
+__device__ __forceinline__ void put_triangles(const WPlan &pl, const unsigned char *vtab, const uint64_t *tri,
+                                              const uint32_t *jobs, const uint32_t *nbase, uint32_t done, uint32_t n,
+                                              [[maybe_unused]] uint32_t nt, uint32_t *dst, uint32_t miss, bool &bad) {
     const uint32_t lane = threadIdx.x & 31;
-    if (lane < n) {
+    if (lane < n && MTX_BC(done + lane, nt, kBcIndex)) {
         const uint32_t job = jobs[(done + lane) & (kJobWin - 1)];
-        const uint64_t w = tri[(job >> 16) & 0x3ffu];
+        const uint64_t w = MTX_BC((job >> 16) & 0x3ffu, kTris, kBcJobs) ? tri[(job >> 16) & 0x3ffu] : 0ull;
         const uint32_t ti = job & 0xffffu, c[3] = {(uint32_t)w, (uint32_t)w >> 16, (uint32_t)(w >> 32)};
         uint32_t id[3], from = 0;
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
-            const uint32_t e = *reinterpret_cast<const uint16_t *>(vtab + ti + (c[k] & 0x3ffu));
+            const uint32_t e = MTX_BC(ti + (c[k] & 0x3ffu), 2 * pl.S1 * pl.S1 * pl.S1, kBcVoxTab)
+                                   ? *reinterpret_cast<const uint16_t *>(vtab + ti + (c[k] & 0x3ffu))
+                                   : 0u;
             const uint32_t b = (c[k] >> 10) & (job >> 26) & 7u;
             id[k] = nbase[b] + (e & kRelMask) + __popc(e & c[k] & kCutMask);
             from |= miss >> b;
