@@ -283,15 +283,16 @@ mtx_status scratch_reserve(mtx_context *c, Scratch &s, size_t bytes) {
 }
 
 mtx_status rezero(mtx_context *c, cudaStream_t s) {
-    if (c->rezero == mtx_context::kRezeroNo) return MTX_OK;
+    if (!c->rezero) return MTX_OK;
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     MTX_CUDA(c, cudaStreamIsCapturing(s, &capture));
     const bool eager = capture == cudaStreamCaptureStatusNone;
-    if (!eager && c->rezero != mtx_context::kRezeroNeeded) return MTX_OK;
+    const uint32_t why = eager ? c->rezero : c->rezero & ~(uint32_t)mtx_context::kStreamChanged;
+    if (!why) return MTX_OK;
     static_assert(offsetof(Ctrl, pyr_done) == offsetof(Ctrl, filter_ticket) + 8, "Ctrl layout");
-    MTX_CUDA(c, cudaMemsetAsync(&c->ctrl->filter_ticket, 0, 12, s));
+    if (why != mtx_context::kNewWords) MTX_CUDA(c, cudaMemsetAsync(&c->ctrl->filter_ticket, 0, 12, s));
     if (c->filter_status.ptr) MTX_CUDA(c, cudaMemsetAsync(c->filter_status.ptr, 0, c->filter_status.size, s));
-    if (eager) c->rezero = mtx_context::kRezeroNo;  // a captured memset has not run
+    if (eager) c->rezero = 0;  // a captured memset has not run
     return MTX_OK;
 }
 
@@ -476,7 +477,7 @@ static mtx_status sync_and_check(mtx_context *c, const void *src = nullptr, uint
         }
 #endif
     if (h->code == 0) return MTX_OK;
-    c->rezero = mtx_context::kRezeroNeeded;
+    c->rezero |= mtx_context::kAfterError;
     const DevStatus e = *h;
     MTX_CUDA(c, cudaMemset(&c->ctrl->status, 0, sizeof(e)));
     char buf[160];
@@ -554,7 +555,7 @@ mtx_status mtx_context_destroy(mtx_context_t c) {
 mtx_status mtx_context_set_stream(mtx_context_t c, void *stream) {
     if (!c) return MTX_ERR_INVALID_ARG;
     DeviceGuard g(c->device);
-    if (c->stream != (cudaStream_t)stream) c->rezero = std::max(c->rezero, mtx_context::kRezeroEager);
+    if (c->stream != (cudaStream_t)stream) c->rezero |= mtx_context::kStreamChanged;
     c->stream = (cudaStream_t)stream;
     return join_extract(c);  // the new stream waits for an extraction still in flight
 }

@@ -283,7 +283,7 @@ mtx_status launch_filter(mtx_context *c, const Problem &p, const uint2 *leaf, ui
     const size_t size = c->filter_status.size;
     mtx_status rs = scratch_reserve(c, c->filter_status, sizeof(uint64_t) * (size_t)ntiles);
     if (c->filter_status.ptr != before || c->filter_status.size != size)
-        c->rezero = mtx_context::kRezeroNeeded;  // new words: no epoch's
+        c->rezero |= mtx_context::kNewWords;  // no epoch's
     if (rs != MTX_OK || (rs = rezero(c, s)) != MTX_OK) return rs;
     uint64_t *words = (uint64_t *)c->filter_status.ptr;
     const uint32_t ctas = std::min(ntiles, kFilterCtas * (uint32_t)c->sm_count);

@@ -70,13 +70,12 @@ struct mtx_context {
         int ctas;
     };
     std::vector<Occupancy> occupancy;  // ctas_per_sm
-    // When the compaction's look-back words and ticket and the octree's counter
-    // are zeroed ahead of a launch: kRezeroEager before the next launch that is
-    // not captured (the stream changed, and launches on two streams that
-    // overlapped would have left them torn), kRezeroNeeded before any (new words,
-    // or an error).
-    enum Rezero { kRezeroNo, kRezeroEager, kRezeroNeeded };
-    Rezero rezero = kRezeroNo;
+    // Why the compaction's look-back words are zeroed ahead of its next launch,
+    // and but for kNewWords its ticket and the octree's counter too: an error, or
+    // the stream changed (launches on two streams that overlapped would have left
+    // them torn), which can wait for a launch that is not captured.
+    enum : uint32_t { kNewWords = 1, kAfterError = 2, kStreamChanged = 4 };
+    uint32_t rezero = 0;
 };
 
 namespace mtx {
