@@ -169,7 +169,7 @@ __global__ void __launch_bounds__(kAdjWarps * 32, adjoint_min_ctas(DET, BC))
         const uint4 dq = __ldg(reinterpret_cast<const uint4 *>(a.desc + r));
         const uint32_t vbase = dq.x, nv = dq.z;
         const bool inner = g.ox + B < p.X && g.oy + B < p.Y && g.oz + B < p.Z;
-        load_rows<T, BC>(p, pl, ws, g, nullptr);
+        load_rows<T>(p, pl, ws, g, nullptr);
         const CutRows cr = cut_bits<BC>(p, pl, ws, g);
         const bool ok = cr.nx + cr.ny + cr.nz == nv && (uint64_t)vbase + nv <= a.vcount;
         if (!ok && lane == 0) report(a.st, MTX_ERR_INTERNAL, kSiteAdjoint, r, cr.nx + cr.ny + cr.nz);
@@ -465,7 +465,7 @@ extern "C" mtx_status mtx_extract_backward(mtx_context_t c, const mtx_volume *vo
     if (n && (!meshlets || !filt->compactedBlockIdBuffer.ptr || !filt->blockRankBuffer.ptr ||
               (vertexCount && !dl_dvertex)))
         return fail(c, MTX_ERR_INVALID_ARG, "forward outputs are missing");
-        cudaStream_t s = c->stream;
+    cudaStream_t s = c->stream;
     mtx_profiler *prof = c->prof;
     prof_begin(prof, "Mesh_Extraction_Backward", s);
     MTX_CUDA(c, cudaMemsetAsync(dl_dfield, 0, nvox(vol->dims) * sizeof(float), s));

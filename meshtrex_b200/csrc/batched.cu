@@ -475,9 +475,9 @@ __device__ __forceinline__ void batch_count_block(const BatchArgs &a, const Prob
                                                   const GridDiv &dv, unsigned char *ws, const uint8_t *ntab,
                                                   uint32_t id, uint32_t r) {
     const Geo g = block_geo(id, p, false, 4, dv);
-    if (p.dtype == MTX_DTYPE_U8) load_rows<uint8_t, BC>(p, pl, ws, g, nullptr);
-    else if (p.dtype == MTX_DTYPE_U16) load_rows<uint16_t, BC>(p, pl, ws, g, nullptr);
-    else load_rows<float, BC>(p, pl, ws, g, nullptr);
+    if (p.dtype == MTX_DTYPE_U8) load_rows<uint8_t>(p, pl, ws, g, nullptr);
+    else if (p.dtype == MTX_DTYPE_U16) load_rows<uint16_t>(p, pl, ws, g, nullptr);
+    else load_rows<float>(p, pl, ws, g, nullptr);
     count_block_list<BC, true>(p, pl, ws, g, ntab, nullptr, a.desc + r, a.faces + (uint64_t)r * a.face_stride,
                                a.state + (uint64_t)r * a.state_stride);
 }

@@ -93,7 +93,7 @@ __global__ void __launch_bounds__(cta_warps_max(BC) * 32, BC == 0 ? 2 : BC > 8 ?
             else build_rows<T>(p, pl, ws, g);
             if (have_next) tile_issue<T>(pl, ws, gn, &map);  // the tile is dead once the rows are built
         } else {
-            load_rows<T, BC>(p, pl, ws, g, use_off ? off : nullptr);
+            load_rows<T>(p, pl, ws, g, use_off ? off : nullptr);
         }
         count_block_list<BC>(p, pl, ws, g, ntab, cell_cases ? cell_cases + (uint64_t)r * B3 : nullptr, desc + r,
                              faces + (uint64_t)r * fslot, state + (uint64_t)r * slot);
@@ -130,7 +130,10 @@ __global__ void __launch_bounds__(kScanThreads)
 // bound by the counter, which serves fewer than one draw a nanosecond (emit of
 // the 1024^3 uint16 ball at block 8: 183 us by stride, 161 by tickets, 158 so;
 // the count pass, at half the work a block, gets slower, 94 -> 134 us, and keeps
-// the stride).
+// the stride).  A half, 5/8, 3/4, 7/8 and all by stride, us: 512^3 float32 gyroid at B
+// = 8 293, 293, 293, 317, 342; 1024 x 1024 x 314 uint8 at B = 3 741, 733, 726, 729, 788;
+// a noisy 1024^3 uint16 ball of 209,000 dense blocks 974, 1043, 1099, 1187, 1246; with two
+// or three blocks a warp (201 x 243 x 257 gyroid at B = 8) 50.8, 51.1, 50.8, 51.9, 45.3.
 struct BlockShare {
     uint32_t fixed, stride;  // blocks given out by stride, warps of the grid
     uint32_t *ticket;

@@ -87,7 +87,8 @@ template <> struct TileWord<true> {
 // 1024 x 314 at B = 3) take 25 us without it.  One tile a CTA, its look-back
 // behind its own loads, 62 us; with the next tile's loads ahead, 54; with the
 // next tile's count published ahead as well, 32 (windows of 128 tiles a round of
-// reads: 37).  512^2 x 1024 blocks and fewer, a tile or less a CTA: 1 to 2 us less.
+// reads: 37).  2.4 million blocks and fewer (4096 a CTA, four CTAs an SM), a tile or
+// less a CTA: 1 to 2 us less.
 template <int ITEMS, bool EPOCH>
 __device__ __forceinline__ void filter_tiles(const uint2 *__restrict__ leaf, uint64_t nblocks, uint32_t ntiles,
                                              uint32_t ctas, uint32_t dtype, float iso, uint32_t *__restrict__ ids,

@@ -502,8 +502,11 @@ static cudaError_t dispatch_leaf(const Problem &p, uint2 *leaf, cudaStream_t s, 
     const bool vec_ok = ((uintptr_t)p.vol % 16 == 0) && (((uint64_t)p.X * sizeof(T)) % 16 == 0) &&
                         (p.B == 4 || p.B == 8 || p.B == 16);
     // uint8 takes the rows pass for 16-byte rows too: a 512-byte strip of 16
-    // voxels a lane leaves a 256^3 volume half of its lanes and few warps (19.8
-    // against 7.7 us at B = 8)
+    // voxels a lane leaves narrow volumes half of their lanes and few warps, and its
+    // byte min/max are wider in instructions.  16-byte pass and rows pass, us, at B =
+    // 4 / 8 / 16: 64^3 6.5, 3.0 / 15.7, 4.1 / 51.7, 7.3; 256^3 18.8, 8.2 / 19.9, 7.7 /
+    // 52.5, 8.9; 512^3 63, 51 / 58, 41 / 71, 45; 1024^3 419, 262 / 357, 207 / 453, 196;
+    // and no shape from 64 x 64 x 64 to 1024^3, rows of 64 to 2048, the other way round
     if (!vec_ok || (sizeof(T) == 1 && !slices)) return launch_rows<T>(p, leaf, s, sm, zover);
     switch (slices) {
     case 1: return dispatch_b<T, 1>(p, leaf, s, sm, zover);

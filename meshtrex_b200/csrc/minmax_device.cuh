@@ -291,7 +291,10 @@ struct RowCut {
 };
 inline RowCut row_cut(const Problem &p, uint32_t esz) {
     RowCut c{};
-    // uint8 rows of up to 160 voxels leave most of a 256-column strip's lanes idle
+    // uint8 rows of up to 160 voxels leave most of a 256-column strip's lanes idle.  256 x
+    // 256 slices of such rows, us with one word a lane and two, at B = 3 / B = 8: X = 61
+    // 7.1, 9.3 / 6.6, 8.1; 96 5.3, 6.6 / 4.3, 5.2; 128 8.4, 7.2 / 5.0, 5.3; 192 8.4, 7.2 /
+    // 5.0, 5.4; 250 14.5, 15.9 / 11.4, 12.5; 1024 (and 1024 x 314) 152, 112 at B = 3
     c.wide = esz > 1 || p.X > 160;
     const uint32_t W = c.wide ? 2u : 1u, vpw = 4u / esz;
     // blocks are word-aligned columns apart when `step` of them are

@@ -170,7 +170,7 @@ __host__ __device__ inline uint32_t emit_fixed_bytes(uint32_t B) {
 // a time, their inside bits are one ballot, and row q is the B+1 bits from bit
 // q (B+1) of that stream on.  off: element offsets of the tile's voxels
 // (row_offsets), null where they do not fit 32 bits.
-template <typename T, int BC>
+template <typename T>
 __device__ __forceinline__ void load_rows(const Problem &p, const WPlan &pl, unsigned char *ws, const Geo &g,
                                           const uint32_t *off) {
     constexpr uint32_t kBatch = 8;
@@ -473,7 +473,7 @@ __device__ __forceinline__ void build_tris(const WPlan &pl, uint64_t *tri, uint1
         uint64_t w = 0;
         for (uint32_t k = 0; k < 3; ++k) {
             const uint32_t o = c_mc_owner[(e3 >> (4 * k)) & 0xfu], ax = o >> 3;
-                const uint32_t off = (o & 1u) + ((o >> 1) & 1u) * pl.S1 + ((o >> 2) & 1u) * pl.S1 * pl.S1;
+            const uint32_t off = (o & 1u) + ((o >> 1) & 1u) * pl.S1 + ((o >> 2) & 1u) * pl.S1 * pl.S1;
             w |= (uint64_t)((off << 1) | ((o & 7u) << 10) | (((1u << ax) - 1u) << 14)) << (16 * k);
         }
         tri[i] = w;
