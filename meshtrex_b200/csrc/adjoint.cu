@@ -142,18 +142,16 @@ __device__ __forceinline__ float iso_term(float gv, float scale, float den) {
 // CTAs an SM that the register count has to allow, where the compiler's own choice
 // takes more registers than pay (0: its choice).  Block edge 5, ATOMIC: 122
 // registers 337 us, 64 registers 263 (300 x 400 x 512 uint16, 35 vertices a
-// block); run-time edges, DETERMINISTIC: 96 registers 585, 80 registers 538 (B = 6);
-// at B = 2, 4 and 8 a bound of the same register count is 2 to 5% slower than none.
-constexpr int adjoint_min_ctas(bool det, int BC) {
-    return BC == 0 ? (det ? 6 : 8) : BC == 5 ? (det ? 7 : 8) : BC == 3 && !det ? 8 : 0;
-}
+// block); at B = 2, 4 and 8 a bound of the same register count is 2 to 5% slower than
+// none.
+constexpr int adjoint_min_ctas(bool det, int BC) { return BC == 5 ? (det ? 7 : 8) : BC == 3 && !det ? 8 : 0; }
 
 template <typename T, bool DET, int BC>
 __global__ void __launch_bounds__(kAdjWarps * 32, adjoint_min_ctas(DET, BC))
     adjoint_block_kernel(const __grid_constant__ AdjArgs a) {
     extern __shared__ __align__(128) unsigned char smem[];
     Problem p = a.p;
-    if (BC) p.B = BC;
+    p.B = BC;  // known at compile time: the plan and every division by the edge fold to constants
     const WPlan pl = make_adjoint_plan(p.B, DET);
     const GridDiv dv = grid_div(p);
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, W = blockDim.x >> 5;
@@ -423,6 +421,10 @@ __global__ void __launch_bounds__(kIsoThreads) adjoint_iso_kernel(const float *_
     if (threadIdx.x == 0) *out = (float)s[0];
 }
 
+// Every block edge at compile time: against one kernel for run-time edges the block
+// pass of a 300 x 400 x 512 float32 gyroid takes, us, ATOMIC / DETERMINISTIC, at B = 3
+// 455, 517 where that takes 589, 898; at B = 6 211, 271 (238, 440); at B = 16 288, 1087
+// (310, 1708).
 template <typename T, bool DET>
 static auto adjoint_fn(uint32_t B) {
     switch (B) {
@@ -430,8 +432,17 @@ static auto adjoint_fn(uint32_t B) {
     case 3: return adjoint_block_kernel<T, DET, 3>;
     case 4: return adjoint_block_kernel<T, DET, 4>;
     case 5: return adjoint_block_kernel<T, DET, 5>;
+    case 6: return adjoint_block_kernel<T, DET, 6>;
+    case 7: return adjoint_block_kernel<T, DET, 7>;
     case 8: return adjoint_block_kernel<T, DET, 8>;
-    default: return adjoint_block_kernel<T, DET, 0>;
+    case 9: return adjoint_block_kernel<T, DET, 9>;
+    case 10: return adjoint_block_kernel<T, DET, 10>;
+    case 11: return adjoint_block_kernel<T, DET, 11>;
+    case 12: return adjoint_block_kernel<T, DET, 12>;
+    case 13: return adjoint_block_kernel<T, DET, 13>;
+    case 14: return adjoint_block_kernel<T, DET, 14>;
+    case 15: return adjoint_block_kernel<T, DET, 15>;
+    default: return adjoint_block_kernel<T, DET, 16>;  // MTX_MAX_BLOCK_EDGE (check_pc)
     }
 }
 template <typename T>

@@ -1,6 +1,6 @@
 """The adjoint on blocks with more cut edges than its shared memory holds
-dL/diso terms for (a checkerboard cuts every edge) and on noise, at compile-time
-and run-time block edges: dL/dfield against the oracle's FP64 adjoint, and
+dL/diso terms for (a checkerboard cuts every edge) and on noise, at every kind
+of block edge: dL/dfield against the oracle's FP64 adjoint, and
 dL/diso bit for bit in the order the kernels state -- each lane over its rows,
 axis by axis, the lanes by a butterfly, the blocks in rank order in double."""
 import numpy as np
