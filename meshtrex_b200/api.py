@@ -47,10 +47,11 @@ def _stream_ptr(stream=None) -> int:
     return int(s.cuda_stream)
 
 
-def _current_stream_ptr() -> int:
-    """torch's current stream as a raw handle, without a Stream object."""
+def _current_stream_ptr(device: int | None = None) -> int:
+    """torch's current stream as a raw handle, without a Stream object (device: the
+    current one, where the caller has asked for it already)."""
     try:
-        return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+        return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if device is None else device)
     except AttributeError:
         return _stream_ptr()
 
@@ -60,12 +61,13 @@ def device_copy(ptr: int, shape, dtype: torch.dtype, device: int | None = None) 
     new tensor on the current device: one copy on torch's current stream (a third
     of the host time of cloning a view of it).  From another device torch makes
     the copy, which it orders behind the current streams of both."""
-    if device is not None and device != torch.cuda.current_device():
+    current = torch.cuda.current_device()
+    if device is not None and device != current:
         return device_view(ptr, shape, dtype).clone()
     out = torch.empty(shape, dtype=dtype, device="cuda")
     n = out.numel()
     if n and ptr:
-        e = L.lib().mtxpy_copy(out.data_ptr(), int(ptr), n * out.element_size(), _current_stream_ptr())
+        e = L.lib().mtxpy_copy(out.data_ptr(), int(ptr), n * out.element_size(), _current_stream_ptr(current))
         if e:
             raise RuntimeError(f"copy of a device buffer failed (CUDA error {e})")
     return out

@@ -23,7 +23,7 @@ def test_accessors_copy_by_the_contexts_device(monkeypatch, device, way):
     calls = []
     empty = torch.empty
     monkeypatch.setattr(api.torch.cuda, "current_device", lambda: 0)
-    monkeypatch.setattr(api, "_current_stream_ptr", lambda: 0)
+    monkeypatch.setattr(api, "_current_stream_ptr", lambda *a: 0)
     monkeypatch.setattr(api.L, "lib", lambda: _Lib(calls))
     monkeypatch.setattr(api.torch, "empty", lambda shape, dtype=None, device=None: empty(shape, dtype=dtype))
 
